@@ -395,16 +395,15 @@ def work(case):
     return {"bytes": 2 * mats + 4 * T * z["hidden"] + 4 * len(lens) * (mem + conv), "flops": 2 * T * mats + per * T * mem}
 
 
-# Relative errors (2-norms) between this engine's fast and plain kernels and float64, times four; a whole step's grows with
-# its layers because a rounding in one travels through all that follow.
-_TOLERANCE = {"decode": 3e-2, "prompt": 3e-2, "attention": 1.5e-2, "latent": 1.5e-2, "experts": 1.5e-2, "mamba2": 1.5e-2, "mlstm": 1.5e-2,
-              "gla": 1.5e-2, "delta": 1.5e-2}
-
-
+# Measured 2-norm errors against float64, about four times each: 0.0038 to 0.0050 for the single layers, 0.0066 to 0.011 for the steps
+# through 4 and 8 layers, 0.020 for the 28 layers of decode_0.6b_b1 (a rounding in one layer travels through all that follow, so two
+# correct forms are up to 1.4 times that apart), 3.1e-6 for the float32 prompt.
 def tolerance(case):
     if case["dtype"] == "float32":
-        return {"rel": 1e-5}
-    return {"rel": _TOLERANCE[case["kind"]]}
+        return {"rel": 1.2e-5}
+    if case["kind"] in ("decode", "prompt"):
+        return {"rel": 6e-2 if case["layers"] > 8 else 4e-2}
+    return {"rel": 1.6e-2}
 
 
 # ---------------------------------------------------------------------------- the same in 64 bits
