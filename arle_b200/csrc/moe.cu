@@ -381,26 +381,7 @@ __device__ __forceinline__ void mma_tile_64x128(const __nv_bfloat16* __restrict_
       }
 }
 
-__global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int lda, const int* __restrict__ rows,
-                                                           const __nv_bfloat16* __restrict__ W, int ldw, long w_expert,
-                                                           __nv_bfloat16* __restrict__ C, int ldc, const int* __restrict__ plan, int E,
-                                                           int N, int K, const float* __restrict__ place_scale, int act) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int tile = blockIdx.y;
-  if (tile >= plan[E + 1]) return;
-  const int* tt = plan + E + 2 + 3 * tile;
-  const int expert = tt[0], p0 = tt[1], M = tt[2];
-  __shared__ __align__(16) __nv_bfloat16 As[kStages][TM * TPITCH];
-  __shared__ __align__(16) __nv_bfloat16 Ws[kStages][TN * TPITCH];
-  __shared__ int arow[TM];
-  if (threadIdx.x < TM) arow[threadIdx.x] = (int)threadIdx.x < M ? (rows ? rows[p0 + threadIdx.x] : p0 + (int)threadIdx.x) : -1;
-  __syncthreads();
-  mma_tile_64x128(A, lda, arow, W + (size_t)expert * w_expert, ldw, C, ldc, (size_t)p0, M, blockIdx.x * TN, N, K, As, Ws,
-                  [&](float v, size_t row, int) { return finish_sum(v, place_scale ? place_scale[row] : 1.f, act); });
-}
-
-// The same tile for one matrix per head, heads side by side in the rows of A and C (see arle_gemm_heads): grid (column
+// The tile for one matrix per head, heads side by side in the rows of A and C (see arle_gemm_heads): grid (column
 // tiles, row tiles, heads).  With a gate [M][heads * N] a sum is multiplied by sigmoid(gate) before it is stored.
 template <typename TC>
 __global__ void __launch_bounds__(256) gemm_heads_mma_kernel(const __nv_bfloat16* __restrict__ A, int lda, int a_head,
@@ -473,7 +454,7 @@ __global__ void __launch_bounds__(256) moe_gemv_kernel(const __nv_bfloat16* __re
 
 // dtype: type of A and C; w_dtype: type of W [E][N][K] (an expert every w_expert elements).  pairs: places in all.
 // place_scale float32 [pairs] or null, act 0 none / 1 square of relu: see finish_sum.
-// fast: bfloat16 operands with aligned rows may take the tensor-core tiles or, for few pairs, the dot products.
+// fast: few pairs of bfloat16 operands with aligned rows take the dot products (many take moe_tcgen05.cu).
 ARLE_API int arle_moe_gemm(const void* A, int lda, const int* rows, const void* W, int ldw, long w_expert, void* C, int ldc,
                            int dtype, int w_dtype, const int* plan, int E, int pairs, int N, int K, int fast,
                            const float* place_scale, int act, cudaStream_t s) {
@@ -481,15 +462,10 @@ ARLE_API int arle_moe_gemm(const void* A, int lda, const int* rows, const void* 
   if (K <= 0 || E <= 0 || (act != 0 && act != 1)) return ARLE_E_BADARG;
   const int max_tiles = pairs / kMoeTile + E + 1;
   if (max_tiles > 65535) return ARLE_E_UNSUPPORTED;
-  if (fast && dtype == 1 && w_dtype == 1 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && w_expert % 8 == 0 &&
+  if (fast && pairs <= 128 && dtype == 1 && w_dtype == 1 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && w_expert % 8 == 0 &&
       ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0) {
-    if (pairs <= 128) {
-      launch_kernel(moe_gemv_kernel, dim3((N + 7) / 8, pairs), dim3(256), 0, s, 1, (const __nv_bfloat16*)A, lda, rows,
-                    (const __nv_bfloat16*)W, ldw, w_expert, (__nv_bfloat16*)C, ldc, plan, E, N, K, place_scale, act);
-    } else {
-      launch_kernel(moe_gemm_mma_kernel, dim3((N + TN - 1) / TN, max_tiles), dim3(256), 0, s, 1, (const __nv_bfloat16*)A, lda, rows,
-                    (const __nv_bfloat16*)W, ldw, w_expert, (__nv_bfloat16*)C, ldc, plan, E, N, K, place_scale, act);
-    }
+    launch_kernel(moe_gemv_kernel, dim3((N + 7) / 8, pairs), dim3(256), 0, s, 1, (const __nv_bfloat16*)A, lda, rows,
+                  (const __nv_bfloat16*)W, ldw, w_expert, (__nv_bfloat16*)C, ldc, plan, E, N, K, place_scale, act);
     return launch_status();
   }
   dim3 grid((N + GN - 1) / GN, max_tiles);

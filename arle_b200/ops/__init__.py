@@ -104,6 +104,8 @@ _SIGNATURES = {
     "arle_moe_select": [_P, _I, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P, _I, _P],
     "arle_moe_plan": [_P, _I, _I, _I, _P, _P, _P, _P, _P, _P],
     "arle_moe_gemm": [_P, _I, _P, _P, _I, ctypes.c_long, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _P, _I, _P],
+    "arle_moe_rows": [_P, _I, _P, _P, _I, _I, _P],
+    "arle_moe_gemm_tcgen05": [_P, _I, _I, _P, _P, _P, _I, _P, _I, _I, _I, _I, _P, _I, _F, _F, _P, _P],
     "arle_layernorm": [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P],
     "arle_branch_layernorm_add": [_P, _P, _I, _P, _P, _I, _I, _I, _F, _P, _I, _P, ctypes.c_long, _P, _P, _P],
     "arle_input_conv": [_P, _P, _P, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
@@ -1551,8 +1553,8 @@ def moe_gemm(x, rows, w, out, plan, experts: int, place_scale=None, act: str = "
     """out[place] = act(place_scale[place] * x[rows[place]] . w[expert of place]^T) for every place of the plan (rows None: x is
     in place order; place_scale float32 [pairs] or None: ones; ``act`` "none" or "square_relu", on the float32 sums).
     x [*, K], w [experts, N, K] contiguous, out [pairs, N] in x's type; float32 sums, k ascending.  With the fast kernel
-    set, bfloat16 operands with rows on 16-byte boundaries run on the tensor cores (many pairs) or as one dot product a
-    warp (up to 128 pairs: a decode step)."""
+    set, bfloat16 operands with rows on 16-byte boundaries run on the tensor cores (from MOE_TCGEN05_MIN_PAIRS pairs on) or as one
+    dot product a warp."""
     pairs, N = out.shape
     K = x.shape[1]
     if (w.dim() != 3 or w.shape[0] != experts or w.shape[1] != N or w.shape[2] != K or not w.is_contiguous() or x.stride(1) != 1
@@ -1561,9 +1563,62 @@ def moe_gemm(x, rows, w, out, plan, experts: int, place_scale=None, act: str = "
     if act not in MOE_ACTS or (place_scale is not None and (place_scale.dtype != torch.float32 or place_scale.numel() < pairs)):
         raise KernelError(f"moe_gemm: act {act!r} (known: {', '.join(MOE_ACTS)}); place_scale must be float32 [pairs]")
     _i32(rows, "rows"), _i32(plan, "plan")
+    if _moe_tcgen05_takes(x, w, pairs, experts):
+        _moe_gemm_tcgen05(x, rows, w, out, plan, experts, place_scale, MOE_ACTS[act], 0.0, 0.0)
+        return
     _check(library().arle_moe_gemm(_ptr(x), x.stride(0), _ptr(rows), _ptr(w), K, N * K, _ptr(out), out.stride(0), _dt(x), _dt(w),
                                    _ptr(plan), experts, pairs, N, K, int(_KERNEL_SET == "fast"), _ptr(place_scale), MOE_ACTS[act], _stream()),
            "moe_gemm")
+
+
+# Pairs from which the experts' products run on the two-SM tcgen05 tiles; below, a warp forms each dot product.  A whole routed
+# feed-forward took, dot products and tiles (us): 32 experts of 3 x 3,072 x 4,096: 16 pairs 199 and 209, 24 pairs 273 and 250, 64 pairs
+# 602 and 343; 16 experts of 3 x 768 x 1,024: 16 pairs 50 and 50, 24 pairs 54 and 49.
+MOE_TCGEN05_MIN_PAIRS = 24
+
+
+def _moe_tcgen05_takes(x, w, pairs: int, experts: int) -> bool:
+    return (_KERNEL_SET == "fast" and pairs >= MOE_TCGEN05_MIN_PAIRS and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+            and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and experts <= 1024
+            and experts * w.shape[1] < 1 << 31)
+
+
+def _moe_gemm_tcgen05(x, rows, w, out, plan, experts, place_scale, finish: int, limit: float, alpha: float) -> None:
+    _check(library().arle_moe_gemm_tcgen05(_ptr(x), x.stride(0), x.shape[0], _ptr(rows), _ptr(w), _ptr(out), out.stride(0), _ptr(plan), experts,
+                                           out.shape[0], w.shape[1], x.shape[1], _ptr(place_scale), finish, limit, alpha,
+                                           _ptr(error_flag(x.device)), _stream()), "moe_gemm_tcgen05")
+
+
+def moe_tcgen05_takes(x, w, pairs: int) -> bool:
+    """Whether the products of ``pairs`` rows of x with the experts' matrices w run on the tcgen05 tiles (``moe_rows`` in front of the
+    first then pays)."""
+    return x.is_cuda and x.stride(1) == 1 and w.is_contiguous() and _moe_tcgen05_takes(x, w, pairs, w.shape[0])
+
+
+def moe_rows(x, rows, out) -> None:
+    """out[place] = x[rows[place]]: the places' token rows side by side (bfloat16, rows of a multiple of 8 numbers on 16-byte boundaries)."""
+    if (x.dtype != torch.bfloat16 or out.dtype != x.dtype or out.shape[1] != x.shape[1] or not out.is_contiguous() or x.stride(1) != 1
+            or rows.numel() != out.shape[0]):
+        raise KernelError(f"moe_rows: shapes x {tuple(x.shape)} out {tuple(out.shape)}")
+    _i32(rows, "rows")
+    _check(library().arle_moe_rows(_ptr(x), x.stride(0), _ptr(rows), _ptr(out), out.shape[0], x.shape[1], _stream()), "moe_rows")
+
+
+MOE_GATES = {"silu": 2, "gelu_tanh": 3, "clamped_glu": 4}
+
+
+def moe_gemm_gated(x, rows, w, out, plan, experts: int, activation: str, place_scale=None, limit: float = 0.0, alpha: float = 0.0) -> None:
+    """out[place, i] = act(g, u) with g and u the products of ``moe_gemm`` with the expert's rows 2i and 2i + 1 (times place_scale):
+    ``activation`` "silu" or "gelu_tanh": act(g) * u; "clamped_glu": what ``clamped_glu`` does with ``limit`` and ``alpha``.  The gate is
+    applied to the float32 sums and rounded once.  x [*, K], w [experts, 2I, K] contiguous, out [pairs, I], all bfloat16."""
+    pairs, I = out.shape
+    if (w.dim() != 3 or w.shape[0] != experts or w.shape[1] != 2 * I or w.shape[2] != x.shape[1] or out.stride(1) != 1 or out.dtype != torch.bfloat16
+            or not moe_tcgen05_takes(x, w, pairs)):
+        raise KernelError(f"moe_gemm_gated: shapes x {tuple(x.shape)} w {tuple(w.shape)} out {tuple(out.shape)}")
+    if activation not in MOE_GATES or (place_scale is not None and (place_scale.dtype != torch.float32 or place_scale.numel() < pairs)):
+        raise KernelError(f"moe_gemm_gated: activation {activation!r} (known: {', '.join(MOE_GATES)}); place_scale must be float32 [pairs]")
+    _i32(rows, "rows"), _i32(plan, "plan")
+    _moe_gemm_tcgen05(x, rows, w, out, plan, experts, place_scale, MOE_GATES[activation], float(limit), float(alpha))
 
 
 def moe_combine(y, place_of_pair, weights, shared, gate, out, top: int = None) -> None:

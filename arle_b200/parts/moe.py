@@ -153,17 +153,26 @@ class RoutedExperts(FeedForward):
         on_input = s.weight_on == "input"
         of_place = ctx.ws.get("moe_weight_of_place", (pairs,), torch.float32) if on_input else None
         ops.moe_plan(ids, E, plan, place_of_pair, row_of_place, weights if on_input else None, of_place)
-        gu = ctx.ws.get("moe_gate_up", (pairs, self.first_rows), x.dtype)
-        ops.moe_gemm(x, row_of_place, self.w_gate_up, gu, plan, E, place_scale=of_place, act="none" if s.gated else s.activation)
-        if not s.gated:
-            act = gu                                    # the activation is the product's last act
-        else:
-            act = ctx.ws.get("moe_act", (pairs, ff), x.dtype)
-            if s.activation == "clamped_glu":
-                ops.clamped_glu(gu, act, s.act_limit, s.act_alpha)
-            else:
-                ops.act_mul(gu, act, s.activation)
         y = ctx.ws.get("moe_y", (pairs, s.hidden_size), x.dtype)
+        src, src_rows = x, row_of_place
+        tiles = ops.moe_tcgen05_takes(x, self.w_gate_up, pairs)
+        if tiles:                                           # the first product reads its rows side by side; y is written after it
+            ops.moe_rows(x, row_of_place, y)
+            src, src_rows = y, None
+        if s.gated and tiles:                               # the gate is applied in the product's epilogue
+            act = ctx.ws.get("moe_act", (pairs, ff), x.dtype)
+            ops.moe_gemm_gated(src, src_rows, self.w_gate_up, act, plan, E, s.activation, of_place, s.act_limit or 0.0, s.act_alpha)
+        else:
+            gu = ctx.ws.get("moe_gate_up", (pairs, self.first_rows), x.dtype)
+            ops.moe_gemm(src, src_rows, self.w_gate_up, gu, plan, E, place_scale=of_place, act="none" if s.gated else s.activation)
+            if not s.gated:
+                act = gu                                    # the activation is the product's last act
+            else:
+                act = ctx.ws.get("moe_act", (pairs, ff), x.dtype)
+                if s.activation == "clamped_glu":
+                    ops.clamped_glu(gu, act, s.act_limit, s.act_alpha)
+                else:
+                    ops.act_mul(gu, act, s.activation)
         ops.moe_gemm(act, None, self.w_down, y, plan, E)
         shared = self.shared.forward(x, ctx) if self.shared is not None else None
         out = ctx.ws.get("moe_out", (T, s.hidden_size), x.dtype)
