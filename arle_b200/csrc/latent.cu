@@ -28,10 +28,11 @@
 using namespace arle;
 
 template <typename T>
-__global__ void latent_prep_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ dkv, int dkv_stride,
+__global__ void latent_prep_kernel(const T* q, int q_stride, const T* __restrict__ dkv, int dkv_stride,
                                    const int* __restrict__ positions, const int* __restrict__ slot_mapping,
                                    const float* __restrict__ c_weight, float eps, const float* __restrict__ inv_freq,
-                                   int rot_dims, int pairing, float amplitude, T* __restrict__ cache, T* __restrict__ q_abs, int H, int dn, int dr, int rank) {
+                                   int rot_dims, int pairing, float amplitude, T* __restrict__ cache, T* q_out, long out_stride, int out_head,
+                                   int out_at, int H, int dn, int dr, int rank) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float2 turn[];                 // (cos, sin) of the token's angles, evaluated once for the key and all heads
@@ -75,13 +76,16 @@ __global__ void latent_prep_kernel(const T* __restrict__ q, int q_stride, const 
 #pragma unroll 4
   for (int idx = threadIdx.x; idx < H * units; idx += blockDim.x) {
     const int h = idx / units, i = idx - h * units;
-    turned(q + (size_t)t * q_stride + (size_t)h * (dn + dr) + dn, q_abs + ((size_t)t * H + h) * kd + rank, i);
+    turned(q + (size_t)t * q_stride + (size_t)h * (dn + dr) + dn, q_out + (size_t)t * out_stride + (size_t)h * out_head + out_at, i);
   }
 }
 
+// A head's rotated numbers go to q_out[t * out_stride + h * out_head + out_at ..]; that may be the place in q that they come from (a
+// thread reads and writes a pair).
 ARLE_API int arle_latent_prep(const void* q, int q_stride, const void* dkv, int dkv_stride, int dtype, const int* positions,
                               const int* slot_mapping, const float* c_weight, float eps, const float* inv_freq, int rot_dims, int pairing, float amplitude,
-                              void* cache, void* q_abs, int H, int dn, int dr, int rank, int num_tokens, cudaStream_t s) {
+                              void* cache, void* q_out, long out_stride, int out_head, int out_at, int H, int dn, int dr, int rank, int num_tokens,
+                              cudaStream_t s) {
   if (num_tokens <= 0) return 0;
   if (H <= 0 || dn < 0 || dr < 0 || rank <= 0 || rot_dims < 0 || rot_dims > dr || (rot_dims & 1) || (pairing != 0 && pairing != 1)) return ARLE_E_BADARG;
   const int threads = H * dr >= 1024 ? 256 : 128;
@@ -89,11 +93,12 @@ ARLE_API int arle_latent_prep(const void* q, int q_stride, const void* dkv, int 
   if (smem > 40 * 1024) return ARLE_E_UNSUPPORTED;
   if (dtype == 0)
     launch_kernel(latent_prep_kernel<float>, dim3(num_tokens), dim3(threads), smem, s, 1, (const float*)q, q_stride, (const float*)dkv,
-                  dkv_stride, positions, slot_mapping, c_weight, eps, inv_freq, rot_dims, pairing, amplitude, (float*)cache, (float*)q_abs, H, dn, dr, rank);
+                  dkv_stride, positions, slot_mapping, c_weight, eps, inv_freq, rot_dims, pairing, amplitude, (float*)cache, (float*)q_out,
+                  out_stride, out_head, out_at, H, dn, dr, rank);
   else if (dtype == 1)
     launch_kernel(latent_prep_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), smem, s, 1, (const __nv_bfloat16*)q, q_stride,
                   (const __nv_bfloat16*)dkv, dkv_stride, positions, slot_mapping, c_weight, eps, inv_freq, rot_dims, pairing, amplitude,
-                  (__nv_bfloat16*)cache, (__nv_bfloat16*)q_abs, H, dn, dr, rank);
+                  (__nv_bfloat16*)cache, (__nv_bfloat16*)q_out, out_stride, out_head, out_at, H, dn, dr, rank);
   else
     return ARLE_E_BADARG;
   return launch_status();
@@ -208,7 +213,8 @@ template <int R64>
 __global__ void __launch_bounds__(128) latent_attention_mma_kernel(
     const __nv_bfloat16* __restrict__ q_abs, __nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
     const __nv_bfloat16* __restrict__ cache, const int* __restrict__ positions, const int* __restrict__ row_of_token,
-    const int* __restrict__ block_table, int bt_stride, int H, int kd, int page_size, float scale, int window, int splits) {
+    const int* __restrict__ block_table, int bt_stride, int H, int kd, int page_size, float scale, int window, int splits,
+    const int* __restrict__ q_indptr, int shorter_than) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr int rank = 64 * R64;
@@ -222,7 +228,9 @@ __global__ void __launch_bounds__(128) latent_attention_mma_kernel(
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
   const int pos = positions[t];
-  const int* bt = block_table + (size_t)row_of_token[t] * bt_stride;
+  const int row = row_of_token[t];
+  if (shorter_than > 0 && q_indptr[row + 1] - q_indptr[row] >= shorter_than) return;      // latent_prefill_tc.cu runs the long rows
+  const int* bt = block_table + (size_t)row * bt_stride;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
   const int ntiles = (pos - lo) / kMmaTile + 1;
   const int tps = (ntiles + splits - 1) / splits;
@@ -406,7 +414,7 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_o, const floa
 template <int R64>
 static int launch_latent_mma(const void* q_abs, void* out, float* part_o, float* part_ml, const void* cache, const int* positions,
                              const int* row_of_token, const int* block_table, int bt_stride, int H, int kd, int page_size, float scale,
-                             int window, int num_tokens, int splits, cudaStream_t s) {
+                             int window, int num_tokens, int splits, const int* q_indptr, int shorter_than, cudaStream_t s) {
   const size_t smem = (size_t)(16 + kMmaTile) * (kd + 8) * 2 + 16 * kPPitch * 2 + 64 * sizeof(float);
   if (smem > 220 * 1024) return ARLE_E_UNSUPPORTED;
   cudaError_t e = cudaFuncSetAttribute(latent_attention_mma_kernel<R64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -414,7 +422,7 @@ static int launch_latent_mma(const void* q_abs, void* out, float* part_o, float*
   dim3 grid(num_tokens, (H + 15) / 16, splits);
   launch_kernel(latent_attention_mma_kernel<R64>, dim3(grid), dim3(128), smem, s, 1, (const __nv_bfloat16*)q_abs, (__nv_bfloat16*)out,
                 part_o, part_ml, (const __nv_bfloat16*)cache, positions, row_of_token, block_table, bt_stride, H, kd, page_size, scale,
-                window, splits);
+                window, splits, q_indptr, shorter_than);
   if (splits > 1)
     launch_kernel(latent_merge_kernel, dim3(num_tokens * H), dim3(64 * R64 >= 256 ? 256 : 64), 0, s, 1, (const float*)part_o,
                   (const float*)part_ml, (__nv_bfloat16*)out, 64 * R64, splits);
@@ -422,18 +430,19 @@ static int launch_latent_mma(const void* q_abs, void* out, float* part_o, float*
 }
 
 // The tensor-core form: bfloat16, rank 64 / 128 / 256 / 512, kd - rank a multiple of 16.  splits > 1 needs part_o float32
-// [T * H * splits * rank] and part_ml float32 [T * H * splits * 2].
+// [T * H * splits * rank] and part_ml float32 [T * H * splits * 2].  shorter_than > 0: tokens of rows (q_indptr) with that many tokens or
+// more are left alone.
 ARLE_API int arle_latent_attention_mma(const void* q_abs, void* out, float* part_o, float* part_ml, const void* cache,
                                        const int* positions, const int* row_of_token, const int* block_table, int bt_stride, int H,
                                        int rank, int kd, int page_size, float scale, int window, int num_tokens, int splits,
-                                       cudaStream_t s) {
+                                       const int* q_indptr, int shorter_than, cudaStream_t s) {
   if (num_tokens <= 0) return 0;
   if (H <= 0 || kd < rank || (kd - rank) % 16 || page_size <= 0 || splits < 1 || splits > 65535 || splits > 64 || (H + 15) / 16 > 65535 ||
       (splits > 1 && (!part_o || !part_ml)))
     return ARLE_E_BADARG;
 #define ARLE_LAT(R) \
   return launch_latent_mma<R>(q_abs, out, part_o, part_ml, cache, positions, row_of_token, block_table, bt_stride, H, kd, page_size, \
-                              scale, window, num_tokens, splits, s)
+                              scale, window, num_tokens, splits, q_indptr, shorter_than, s)
   if (rank == 64) ARLE_LAT(1);
   if (rank == 128) ARLE_LAT(2);
   if (rank == 256) ARLE_LAT(4);

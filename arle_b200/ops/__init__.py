@@ -88,8 +88,11 @@ _SIGNATURES = {
     "arle_dyt_norm": [_P, _P, _P, _P, _P, _F, _P, _I, _I, _I, _I, _P],
     "arle_gemm_heads_mma": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, ctypes.c_long, _I, _P, _I, _P],
     "arle_gemm_heads": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, ctypes.c_long, _I, _P],
-    "arle_latent_prep": [_P, _I, _P, _I, _I, _P, _P, _P, _F, _P, _I, _I, _F, _P, _P, _I, _I, _I, _I, _I, _P],
-    "arle_latent_attention_mma": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P],
+    "arle_latent_prep": [_P, _I, _P, _I, _I, _P, _P, _P, _F, _P, _I, _I, _F, _P, _P, ctypes.c_long, _I, _I, _I, _I, _I, _I, _I, _P],
+    "arle_latent_attention_mma": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _I, _P],
+    "arle_latent_plan": [_P, _P, _I, _I, _I, _P, _P],
+    "arle_latent_gather": [_P, _P, _I, _P, _P, _I, _I, _I, _P, _I, _P],
+    "arle_latent_prefill_tc": [_P, _I, _I, _P, _P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _I, _I, _I, _I, _P, _P],
     "arle_latent_attention": [_P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
     "arle_decay_scan": [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _I, _P],
     "arle_decay_chunk_plan_ints": [_I, _I],
@@ -1212,7 +1215,7 @@ def latent_prep(q, dkv, positions, slot_mapping, c_weight, eps: float, inv_freq,
     2i + 1, by position * inv_freq[i], cosine and sine times ``amplitude``);
     both go to cache[slot_mapping[t]] (cache [pages, 1, page_size, rank + dr]; None: nothing is stored).  q [T, >= heads
     * (dn + dr)]: every head's last ``dr`` numbers are rotated the same way into q_abs[t, h, rank:] (q_abs [T, heads,
-    rank + dr], contiguous)."""
+    rank + dr], contiguous); ``q_abs`` None: in place, in q."""
     T = q.shape[0]
     kd = rank + dr
     if pairing not in ROTARY_PAIRINGS:
@@ -1222,7 +1225,8 @@ def latent_prep(q, dkv, positions, slot_mapping, c_weight, eps: float, inv_freq,
     elif dkv is None or c_weight is None:
         raise KernelError("latent_prep: a cache to store into needs dkv and the latent's norm weight")
     if (q.stride(1) != 1 or dkv.stride(1) != 1 or q.shape[1] < heads * (dn + dr) or (cache is not None and dkv.shape[1] < kd)
-            or q.dtype != dkv.dtype or tuple(q_abs.shape) != (T, heads, kd) or not q_abs.is_contiguous() or q_abs.dtype != q.dtype):
+            or q.dtype != dkv.dtype
+            or (q_abs is not None and (tuple(q_abs.shape) != (T, heads, kd) or not q_abs.is_contiguous() or q_abs.dtype != q.dtype))):
         raise KernelError("latent_prep: q, dkv or q_abs do not fit the sizes given")
     if c_weight is not None and (c_weight.dtype != torch.float32 or c_weight.numel() != rank):
         raise KernelError("latent_prep: the latent's norm weight must be float32 [rank]")
@@ -1236,7 +1240,8 @@ def latent_prep(q, dkv, positions, slot_mapping, c_weight, eps: float, inv_freq,
     _check(library().arle_latent_prep(_ptr(q), q.stride(0), _ptr(dkv), dkv.stride(0), _dt(q), _ptr(positions),
                                       _ptr(slot_mapping) if cache is not None else None, _ptr(c_weight), float(eps),
                                       _ptr(inv_freq) if rot_dims else None, int(rot_dims), ROTARY_PAIRINGS[pairing], float(amplitude),
-                                      _ptr(cache), _ptr(q_abs), heads, dn, dr, rank, T, _stream()), "latent_prep")
+                                      _ptr(cache), *((_ptr(q), q.stride(0), dn + dr, dn) if q_abs is None else (_ptr(q_abs), heads * kd, kd, rank)),
+                                      heads, dn, dr, rank, T, _stream()), "latent_prep")
 
 
 def latent_mma_supported(q_abs, rank: int) -> bool:
@@ -1248,12 +1253,13 @@ def latent_mma_supported(q_abs, rank: int) -> bool:
 
 
 def latent_attention(q_abs, out, cache, positions, row_of_token, block_table, rank: int, page_size: int, scale: float, window,
-                     batch=None) -> None:
+                     batch=None, shorter_than: int = 0) -> None:
     """Causal attention of folded queries q_abs [T, heads, kd] over records cache [pages, 1, page_size, kd]: head h's score
     against record j is (q_abs[t, h] . record_j) * scale, its output sum_j softmax_j * record_j[:rank] (out [T, heads,
     rank]).  ``window`` None or <= 0: all keys; W: keys p - W + 1 .. p.  Scores, softmax and sums are float32.  ``batch`` (a
     StepContext, for its scratch buffers) lets the tensor-core kernel run where the shapes allow it; with few tokens in
-    the step a token's keys are shared out among several blocks."""
+    the step a token's keys are shared out among several blocks.  ``shorter_than`` > 0 (with ``batch``): the outputs of tokens in rows of
+    that many tokens or more need not be written."""
     T, heads, kd = q_abs.shape
     if (not q_abs.is_contiguous() or tuple(out.shape) != (T, heads, rank) or not out.is_contiguous() or out.dtype != q_abs.dtype
             or cache.dtype != q_abs.dtype or tuple(cache.shape[1:]) != (1, page_size, kd) or not cache.is_contiguous()):
@@ -1273,7 +1279,8 @@ def latent_attention(q_abs, out, cache, positions, row_of_token, block_table, ra
             part_ml = batch.ws.get("latent_part_ml", (T * heads * splits * 2,), torch.float32)
         _check(library().arle_latent_attention_mma(_ptr(q_abs), _ptr(out), _ptr(part_o), _ptr(part_ml), _ptr(cache), _ptr(positions),
                                                    _ptr(row_of_token), _ptr(block_table), block_table.stride(0), heads, rank, kd,
-                                                   page_size, float(scale), int(window) if window else 0, T, splits, _stream()),
+                                                   page_size, float(scale), int(window) if window else 0, T, splits,
+                                                   _ptr(batch.q_indptr) if shorter_than else None, int(shorter_than), _stream()),
                "latent_attention_mma")
         if splits > 1:
             add_launches(1)
@@ -1281,6 +1288,76 @@ def latent_attention(q_abs, out, cache, positions, row_of_token, block_table, ra
     _check(library().arle_latent_attention(_ptr(q_abs), _ptr(out), _ptr(cache), _dt(q_abs), _ptr(positions), _ptr(row_of_token),
                                            _ptr(block_table), block_table.stride(0), heads, rank, kd, page_size, float(scale),
                                            int(window) if window else 0, T, _stream()), "latent_attention")
+
+
+# Rows of the step for which keys and values are built from the latent records.  A latent attention layer on one row, folded and built (us):
+# 32 heads of 128 + 64 at rank 512, width 4,096: 64 queries 57 and 48 (behind 2,048 tokens 239 and 114, behind 6,144 599 and 213), 512
+# queries 275 and 90 (4,054 and 281); 16 heads of 64 + 32 at rank 256, width 1,024: 64 queries 35 and 32 (68 and 65; 143 and 131), 512
+# queries 92 and 45 (801 and 145).  With 16 queries the two are equal without a context and the folded form wins behind one.
+LATENT_BUILT_LEAST = 64             # queries of a row from which its keys and values are built
+LATENT_BUILT_MOST = 8               # records that are laid side by side, a token of the step ...
+LATENT_BUILT_PLACES = 1 << 16       # ... or this many, whichever is more: what the step's buffers leave room for
+LATENT_BUILT_NUMBERS = 1 << 25      # keys' numbers that are built at a time, where the step's tokens do not give room for more
+
+
+def latent_built_places(batch, q, dn: int, dr: int, vdim: int, rank: int, page_size: int, window) -> int:
+    """Records (each row's padded to a multiple of 16) that ``latent_prefill`` would build keys and values from for this step's rows of
+    LATENT_BUILT_LEAST tokens and more; 0: none, the folded attention runs every row."""
+    if not (batch.max_q_len >= LATENT_BUILT_LEAST and _KERNEL_SET == "fast" and q.is_cuda and q.dtype == torch.bfloat16 and dn in (64, 128)
+            and vdim == dn and dr <= 64 and dr % 8 == 0 and rank % 8 == 0 and page_size % 16 == 0 and q.stride(0) % 8 == 0
+            and q.data_ptr() % 16 == 0):
+        return 0
+    places = 0
+    for n, kv in zip(batch.q_lens, batch.kv_lens_host):
+        if n >= LATENT_BUILT_LEAST:
+            first = max(0, kv - n - int(window) + 1) if window else 0
+            places += (kv - first // 16 * 16 + 15) // 16 * 16
+    return places if places <= max(LATENT_BUILT_MOST * batch.num_tokens, LATENT_BUILT_PLACES) else 0
+
+
+def latent_prefill(q, out, records, batch, block_table, w_ukv, heads: int, places: int, dr: int, rank: int, page_size: int, scale: float, window,
+                   gate=None) -> None:
+    """What folding the key map into the queries, ``latent_attention`` and the heads' value map do together, for the step's rows of
+    LATENT_BUILT_LEAST tokens and more: their keys and values are built from the records [pages, 1, page_size, rank + dr] once and attended
+    to on the tensor cores.  q [T, heads * (dn + dr)], the last dr numbers of a head rotated; w_ukv [2 * heads * dn, rank]: the heads' key
+    maps, then their value maps; out [T, heads * dn]: other rows are left alone.  ``gate`` [T, heads * dn]: the sums times sigmoid(gate).
+    ``places``: ``latent_built_places``.  Where the records are many more than the tokens, keys and values are built for some heads at a
+    time."""
+    T = q.shape[0]
+    dn = w_ukv.shape[0] // (2 * heads)
+    kd = rank + dr
+    if (q.shape[1] != heads * (dn + dr) or q.stride(1) != 1 or tuple(out.shape) != (T, heads * dn) or not out.is_contiguous()
+            or tuple(w_ukv.shape) != (2 * heads * dn, rank) or tuple(records.shape[1:]) != (1, page_size, kd) or not records.is_contiguous()
+            or q.dtype != out.dtype or places <= 0 or (gate is not None and (gate.shape != out.shape or gate.stride(1) != 1 or gate.dtype != out.dtype))):
+        raise KernelError("latent_prefill: q, out, records or the heads' maps do not fit")
+    _i32(block_table, "block_table")
+    lib, s = library(), _stream()
+    R, window = batch.num_rows, int(window) if window else 0
+    key = ("latent_plan", window)
+    plan = batch.memo.get(key)
+    if plan is None:
+        plan = batch.ws.get(f"latent_plan_{window}", (R + 1, 2), torch.int32)
+        _check(lib.arle_latent_plan(_ptr(batch.q_indptr), _ptr(batch.kv_lens), R, LATENT_BUILT_LEAST, window, _ptr(plan), s), "latent_plan")
+        batch.memo[key] = plan
+    lat = batch.ws.get("latent_gathered", (places, kd), q.dtype)
+    _check(lib.arle_latent_gather(_ptr(records), _ptr(block_table), block_table.stride(0), _ptr(batch.kv_lens), _ptr(plan), R, page_size, kd,
+                                  _ptr(lat), places, s), "latent_gather")
+    width = heads * dn
+    group = min(heads, max(T * heads // places, LATENT_BUILT_NUMBERS // (places * dn), 1))
+    for h0 in range(0, heads, group):
+        hg = min(group, heads - h0)
+        built = batch.ws.get("latent_built", (places, 2 * hg * dn), q.dtype)
+        if hg == heads:
+            gemm(lat[:, :rank], w_ukv, built)
+        else:
+            gemm(lat[:, :rank], w_ukv[h0 * dn: (h0 + hg) * dn], built[:, : hg * dn])
+            gemm(lat[:, :rank], w_ukv[width + h0 * dn: width + (h0 + hg) * dn], built[:, hg * dn:])
+        at = h0 * dn * 2
+        _check(lib.arle_latent_prefill_tc(_ptr(q) + h0 * (dn + dr) * 2, q.stride(0), T, _ptr(built), _ptr(built) + 2 * hg * dn, 2 * hg * dn,
+                                          _ptr(lat), places, _ptr(out) + at, out.stride(0), _ptr(batch.q_indptr), _ptr(batch.kv_lens), _ptr(plan),
+                                          hg, dn, dr, rank, float(scale), _ptr(gate) + at if gate is not None else None,
+                                          gate.stride(0) if gate is not None else 0, window, R, batch.max_q_len, _ptr(error_flag(q.device)), s),
+               "latent_prefill_tc")
 
 
 # ------------------------------------------------------------------ matrix memories with a scalar decay

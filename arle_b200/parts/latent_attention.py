@@ -11,6 +11,8 @@ maps are folded into the queries (one small product per head), every head then a
 keys [c | k_rot] and values c, and W_uv[h] is applied to the head's weighted sum of latents afterwards.  The
 position encoding is the rotary part's (either pairing, with its amplitude); it turns the first ``rotary_dim`` of the dr
 numbers.
+For rows of many queries (bfloat16, ``ops.latent_built_places``) the keys and values are built instead, once for all of the
+row's queries: a score then costs dn + dr products instead of rank + dr, a sum dv instead of rank.
 A ``window`` keeps the last ``window`` positions visible (itself included) and lets older pages go back.
 
 ``q_rank``: the queries go through a latent of their own, c_q = rmsnorm(W_dq x) * weight, q = W_uq c_q (tensors ``dq``,
@@ -78,7 +80,7 @@ class LatentAttention(Mixer):
         self.gate_at = self.rows                        # the gate's columns, on a 16-byte boundary
         if spec.out_gate:
             self.rows += -(-spec.num_heads * spec.value_dim // 8) * 8
-        self.w_in = self.w_uk_t = self.w_uv = self.w_o = self.latent_norm = self.w_uq = self.q_latent_norm = None
+        self.w_in = self.w_ukv = self.w_uk_t = self.w_uv = self.w_o = self.latent_norm = self.w_uq = self.q_latent_norm = None
 
     def _name(self, role: str) -> str:
         return self.spec.prefix + self.names[role]
@@ -116,6 +118,10 @@ class LatentAttention(Mixer):
         uk, uv, o = (tensors[self._name(n)] for n in ("uk", "uv", "o"))
         # head h's key map transposed: [rank, nope_dim], the matrix that folds it into the head's query
         self.w_uk_t = uk.to(device=device, dtype=kept([uk])).view(s.num_heads, s.nope_dim, s.kv_rank).transpose(1, 2).contiguous()
+        if dtype == torch.bfloat16 and s.nope_dim in (64, 128) and s.value_dim == s.nope_dim:
+            # as stored, one below the other: the product that builds the heads' keys and values; w_uv is its second half
+            self.w_ukv = torch.cat([uk.to(device=device, dtype=dtype), uv.to(device=device, dtype=dtype)], dim=0).contiguous()
+            uv = self.w_ukv[s.num_heads * s.nope_dim:]
         self.w_uv = uv.to(device=device, dtype=kept([uv])).view(s.num_heads, s.value_dim, s.kv_rank).contiguous()
         self.w_o = o.to(device=device, dtype=kept([o])).contiguous()
         if s.own_latent:
@@ -132,7 +138,8 @@ class LatentAttention(Mixer):
 
     def scratch_elements_per_token(self):
         s = self.spec
-        return self.rows + s.num_heads * (self.record + s.kv_rank + s.value_dim) + s.hidden_size + (self.first + self.q_width if s.q_rank else 0)
+        return self.rows + s.num_heads * (self.record + s.kv_rank + s.value_dim) + s.hidden_size + (self.first + self.q_width if s.q_rank else 0) + (
+            ops.LATENT_BUILT_MOST * self.record + s.num_heads * (s.nope_dim + s.value_dim) if self.w_ukv is not None else 0)
 
     # ------------------------------------------------------------------ cache
     def cache_need(self):
@@ -159,22 +166,36 @@ class LatentAttention(Mixer):
             ops.gemm(cq, self.w_uq, q)
         else:
             q = proj[:, : self.q_width]
-        q_abs = ctx.ws.get("latent_q", (T, H, self.record), x.dtype)
         records = cache.streams[0]
         stores = cache.writable and s.own_latent
-        if stores or dr:
-            ops.latent_prep(q, proj[:, self.first: self.first + self.record] if s.own_latent else None, ctx.positions, cache.slot_mapping,
-                            self.latent_norm, s.norm_eps, inv_freq, rdim, records if stores else None, q_abs, H, dn, dr, rank,
+        places = ops.latent_built_places(ctx, q, dn, dr, s.value_dim, rank, cache.page_size, s.window) if self.w_ukv is not None else 0
+        all_built = places > 0 and min(ctx.q_lens) >= ops.LATENT_BUILT_LEAST
+        q_abs = None if all_built else ctx.ws.get("latent_q", (T, H, self.record), x.dtype)
+
+        def prepare(into, record, store):
+            ops.latent_prep(q, record, ctx.positions, cache.slot_mapping, self.latent_norm if record is not None else None, s.norm_eps, inv_freq,
+                            rdim, records if store else None, into, H, dn, dr, rank,
                             pairing=getattr(self.position, "pairing", "half"), amplitude=getattr(self.position, "amplitude", 1.0))
-        if dn:
-            ops.gemm_heads(q.unflatten(1, (H, dn + dr))[:, :, :dn], self.w_uk_t, q_abs[:, :, :rank])
-        else:
-            q_abs[:, :, :rank].zero_()
-        o_lat = ctx.ws.get("latent_o", (T, H, rank), x.dtype)
-        ops.latent_attention(q_abs, o_lat, records, ctx.positions, ctx.row_of_token, cache.block_table, rank, cache.page_size,
-                             s.scale, s.window, batch=ctx)
+
+        if stores or dr:
+            prepare(q_abs, proj[:, self.first: self.first + self.record] if s.own_latent else None, stores)
         heads_out = ctx.ws.get("attn_out", (T, H, s.value_dim), x.dtype)
-        ops.gemm_heads(o_lat, self.w_uv, heads_out, gate=proj[:, self.gate_at: self.gate_at + H * s.value_dim] if s.out_gate else None)
+        gate = proj[:, self.gate_at: self.gate_at + H * s.value_dim] if s.out_gate else None
+        if not all_built:
+            if dn:
+                ops.gemm_heads(q.unflatten(1, (H, dn + dr))[:, :, :dn], self.w_uk_t, q_abs[:, :, :rank])
+            else:
+                q_abs[:, :, :rank].zero_()
+            o_lat = ctx.ws.get("latent_o", (T, H, rank), x.dtype)
+            short = {"shorter_than": ops.LATENT_BUILT_LEAST} if places else {}
+            ops.latent_attention(q_abs, o_lat, records, ctx.positions, ctx.row_of_token, cache.block_table, rank, cache.page_size,
+                                 s.scale, s.window, batch=ctx, **short)
+            ops.gemm_heads(o_lat, self.w_uv, heads_out, gate=gate)
+        if places:
+            if dr and not all_built:
+                prepare(None, None, False)              # the rotated numbers in q itself
+            ops.latent_prefill(q, heads_out.view(T, H * s.value_dim), records, ctx, cache.block_table, self.w_ukv, H, places, dr, rank,
+                               cache.page_size, s.scale, s.window, gate=gate)
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)
         return None if ops.gemm(heads_out.view(T, H * s.value_dim), self.w_o, out, sink=sink) else out
 
