@@ -8,7 +8,20 @@
 // float32 sum) is the plain twin of the tensor-core products: the engine's "plain"
 // kernel set runs it for every projection, so that a bfloat16 discrepancy can be put
 // down to the fast kernels or to the arithmetic.
+//
+// float32 A runs on one of three kernels, all with that order of sums, so all with the same bits:
+//  * gemm_f32_rows (up to 16 rows): a thread per column of C, W staged by cp.async.  Bound by W's bytes for one row, by the loads from
+//    shared memory for more.
+//  * gemm_f32_tiles: tiles of 64 x 128 to 32 x 32, 8 x 4 or 4 x 4 sums a thread, the next 16 numbers of k on their way while the present
+//    ones are multiplied; two neighbouring sums are one packed instruction (fma.rn.f32x2: each half the same rounded fused product).
+//    Bound by the loads from shared memory and, since no sum may be split along k, by how few tiles there are: the launcher takes the
+//    tile that leaves the busiest SM the least.
+//  * gemm_f32 (rows that are not on 16-byte boundaries, and bfloat16 A): the general one, tiles of 64 x 64.
+// Measured, the general kernel and these (us): 301 rows, 4,096 x 1,024 168 and 98, 1,024 x 2,048 150 and 89, 6,144 x 1,024 222 and 117,
+// 1,024 x 3,072 224 and 130; 1,024 rows of 24,576 x 4,096 8,726 and 4,420 (47 TFLOP/s); one row, 151,936 x 1,024 880 and 58 (5.3 TB/s),
+// 4,096 x 1,024 76 and 12; 8 rows 883 and 117.
 #include "common.cuh"
+#include "mma_utils.cuh"
 using namespace arle;
 
 constexpr int BM = 64, BN = 64, BK = 16;
@@ -76,12 +89,226 @@ static int launch_plain(const void* A, const void* W, void* C, int M, int N, int
   return launch_status();
 }
 
+// TM, TN: rows and columns of C a thread holds, in groups of four that are BM / (TM / 4) and BN / (TN / 4) apart; two neighbouring
+// columns' sums stand in one 64-bit register.
+template <typename TW, int BM_, int BN_, int TM, int TN>
+__global__ void __launch_bounds__((BM_ / TM) * (BN_ / TN)) gemm_f32_tiles_kernel(const float* __restrict__ A, const TW* __restrict__ W,
+                                                                                 float* __restrict__ C, int M, int N, int K, int lda,
+                                                                                 int ldw, int ldc) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int THREADS = (BM_ / TM) * (BN_ / TN);
+  constexpr int AI = BM_ * 4 / THREADS, WI = BN_ * 4 / THREADS;      // groups of four numbers of k a thread stages
+  static_assert(BM_ * 4 % THREADS == 0 && BN_ * 4 % THREADS == 0, "staging");
+  __shared__ __align__(16) float As[2][BK][BM_ + 4];
+  __shared__ __align__(16) float Ws[2][BK][BN_ + 4];
+  const int tid = threadIdx.x;
+  const int tx = tid % (BN_ / TN), ty = tid / (BN_ / TN);
+  const int m0 = blockIdx.y * BM_, n0 = blockIdx.x * BN_;
+  unsigned long long acc[TM][TN / 2];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0;
+  Pack<float, 4> ar[AI];
+  Pack<TW, 4> wr[WI];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < AI; ++i) {
+      const int idx = tid + i * THREADS, r = m0 + (idx >> 2), k = k0 + (idx & 3) * 4;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) ar[i].e[g] = 0.f;
+      if (r < M && k < K) ar[i] = *reinterpret_cast<const Pack<float, 4>*>(A + (size_t)r * lda + k);
+    }
+#pragma unroll
+    for (int i = 0; i < WI; ++i) {
+      const int idx = tid + i * THREADS, r = n0 + (idx >> 2), k = k0 + (idx & 3) * 4;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) wr[i].e[g] = from_f32<TW>(0.f);
+      if (r < N && k < K) wr[i] = *reinterpret_cast<const Pack<TW, 4>*>(W + (size_t)r * ldw + k);
+    }
+  };
+  auto put = [&](int b) {
+#pragma unroll
+    for (int i = 0; i < AI; ++i) {
+      const int idx = tid + i * THREADS;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) As[b][(idx & 3) * 4 + g][idx >> 2] = ar[i].e[g];
+    }
+#pragma unroll
+    for (int i = 0; i < WI; ++i) {
+      const int idx = tid + i * THREADS;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) Ws[b][(idx & 3) * 4 + g][idx >> 2] = to_f32(wr[i].e[g]);
+    }
+  };
+  const int nk = (K + BK - 1) / BK;
+  fetch(0);
+  put(0);
+  __syncthreads();
+  for (int kt = 0; kt < nk; ++kt) {
+    const int b = kt & 1;
+    if (kt + 1 < nk) fetch((kt + 1) * BK);
+    auto frag = [&](int kk, float (&a)[TM], unsigned long long (&w)[TN / 2]) {
+#pragma unroll
+      for (int g = 0; g < TM / 4; ++g) load_vec<float, 4>(&As[b][kk][g * (BM_ / (TM / 4)) + ty * 4], reinterpret_cast<float(&)[4]>(a[4 * g]));
+#pragma unroll
+      for (int g = 0; g < TN / 4; ++g) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&Ws[b][kk][g * (BN_ / (TN / 4)) + tx * 4]);
+        w[2 * g] = x.x;
+        w[2 * g + 1] = x.y;
+      }
+    };
+    float a[2][TM];
+    unsigned long long w[2][TN / 2];
+    frag(0, a[0], w[0]);
+#pragma unroll
+    for (int kk = 0; kk < BK; ++kk) {
+      if (kk + 1 < BK) frag(kk + 1, a[(kk + 1) & 1], w[(kk + 1) & 1]);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        unsigned long long aa;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a[kk & 1][i]));
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(aa), "l"(w[kk & 1][j]));
+      }
+    }
+    if (kt + 1 < nk) put(b ^ 1);                       // the other buffer was last read before the barrier that ended the tile before
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int gm = m0 + (i >> 2) * (BM_ / (TM / 4)) + ty * 4 + (i & 3);
+    if (gm >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int gn = n0 + (j >> 2) * (BN_ / (TN / 4)) + tx * 4 + (j & 3);
+      if (gn < N) C[(size_t)gm * ldc + gn] = __uint_as_float((unsigned)(j & 1 ? acc[i][j / 2] >> 32 : acc[i][j / 2]));
+    }
+  }
+}
+
+// Up to 16 rows of A: a thread holds one column of C for all rows.  A block stages 128 rows of W, 64 numbers of k at a time, three
+// stages; a staged row is 16 bytes longer than its numbers, so that eight lanes' 16-byte reads fall on different banks.
+constexpr int kRowsN = 128, kRowsK = 64, kRowsStages = 3;
+
+template <typename TW, int MR>
+__global__ void __launch_bounds__(kRowsN) gemm_f32_rows_kernel(const float* __restrict__ A, const TW* __restrict__ W, float* __restrict__ C,
+                                                               int M, int N, int K, int lda, int ldw, int ldc) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int PER = 16 / sizeof(TW);                       // numbers in 16 bytes
+  constexpr int CH = kRowsK / PER, PITCH = kRowsK + PER;     // 16-byte pieces of a row, numbers to the next row
+  extern __shared__ __align__(16) unsigned char rows_sm[];
+  TW* ws = reinterpret_cast<TW*>(rows_sm);                                              // [stages][128][PITCH]
+  float* as = reinterpret_cast<float*>(rows_sm + sizeof(TW) * kRowsStages * kRowsN * PITCH);      // [stages][MR][64]
+  const int n0 = blockIdx.x * kRowsN, tid = threadIdx.x;
+  const int nk = (K + kRowsK - 1) / kRowsK;
+  auto load = [&](int kt) {
+    const int st = kt % kRowsStages, k0 = kt * kRowsK;
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const int idx = tid + i * kRowsN, r = idx / CH, c = idx % CH * PER;
+      const bool ok = n0 + r < N && k0 + c < K;
+      cp_async16(smem_u32(ws + ((size_t)st * kRowsN + r) * PITCH + c), ok ? W + (size_t)(n0 + r) * ldw + k0 + c : W, ok ? 16 : 0);
+    }
+    for (int idx = tid; idx < MR * (kRowsK / 4); idx += kRowsN) {
+      const int r = idx / (kRowsK / 4), c = idx % (kRowsK / 4) * 4;
+      const bool ok = r < M && k0 + c < K;
+      cp_async16(smem_u32(as + ((size_t)st * MR + r) * kRowsK + c), ok ? A + (size_t)r * lda + k0 + c : A, ok ? 16 : 0);
+    }
+  };
+  float acc[MR];
+#pragma unroll
+  for (int r = 0; r < MR; ++r) acc[r] = 0.f;
+  load(0);
+  cp_commit();
+  if (nk > 1) load(1);
+  cp_commit();
+  for (int kt = 0; kt < nk; ++kt) {
+    cp_wait<1>();
+    __syncthreads();
+    if (kt + 2 < nk) load(kt + 2);
+    cp_commit();
+    const int st = kt % kRowsStages;
+    const TW* w = ws + ((size_t)st * kRowsN + tid) * PITCH;
+    const float* a = as + (size_t)st * MR * kRowsK;
+#pragma unroll
+    for (int c = 0; c < kRowsK; c += PER) {
+      float wv[PER];
+      load_vec<TW, PER>(w + c, wv);
+#pragma unroll
+      for (int g = 0; g < PER; g += 4)
+#pragma unroll
+        for (int r = 0; r < MR; ++r) {
+          const float4 x = *reinterpret_cast<const float4*>(a + r * kRowsK + c + g);
+          acc[r] = fmaf(x.x, wv[g], acc[r]);
+          acc[r] = fmaf(x.y, wv[g + 1], acc[r]);
+          acc[r] = fmaf(x.z, wv[g + 2], acc[r]);
+          acc[r] = fmaf(x.w, wv[g + 3], acc[r]);
+        }
+    }
+  }
+  cp_wait<0>();
+  if (n0 + tid < N)
+#pragma unroll
+    for (int r = 0; r < MR; ++r)
+      if (r < M) C[(size_t)r * ldc + n0 + tid] = acc[r];
+}
+
+template <typename TW, int MR>
+static int launch_rows(const float* A, const TW* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+  constexpr size_t smem = sizeof(TW) * kRowsStages * kRowsN * (kRowsK + 16 / sizeof(TW)) + sizeof(float) * kRowsStages * MR * kRowsK;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<TW, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  launch_kernel(gemm_f32_rows_kernel<TW, MR>, dim3((N + kRowsN - 1) / kRowsN), dim3(kRowsN), smem, s, 1, A, W, C, M, N, K, lda, ldw, ldc);
+  return launch_status();
+}
+
+template <typename TW, int BM_, int BN_, int TM, int TN>
+static int launch_tiles(const float* A, const TW* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+  dim3 grid((N + BN_ - 1) / BN_, (M + BM_ - 1) / BM_);
+  if (grid.y > 65535) return ARLE_E_UNSUPPORTED;
+  launch_kernel(gemm_f32_tiles_kernel<TW, BM_, BN_, TM, TN>, grid, dim3((BM_ / TM) * (BN_ / TN)), 0, s, 1, A, W, C, M, N, K, lda, ldw, ldc);
+  return launch_status();
+}
+
+template <typename TW>
+static int launch_f32(const float* A, const void* Wv, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+  const TW* W = (const TW*)Wv;
+  constexpr int PER = 16 / sizeof(TW);
+  if (K % PER || lda % 4 || ldw % PER || ((uintptr_t)A & 15) || ((uintptr_t)Wv & 15))
+    return launch_plain<float, TW, float>(A, Wv, C, M, N, K, lda, ldw, ldc, s);
+  if (M <= 16) {
+    if (M == 1) return launch_rows<TW, 1>(A, W, C, M, N, K, lda, ldw, ldc, s);
+    if (M <= 4) return launch_rows<TW, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+    if (M <= 8) return launch_rows<TW, 8>(A, W, C, M, N, K, lda, ldw, ldc, s);
+    return launch_rows<TW, 16>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  }
+  // Microseconds per 1,024 of k: what a tile takes by itself on an SM, and what it adds to an SM that is full of them; in between the
+  // cube root of the sum of cubes is within a tenth of what was measured at 1,024 to 24,576 columns and 12 to 1,024 rows.
+  auto cost = [&](int bm, int bn, float alone, float added) {
+    const float b = (float)(((long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn) + 147) / 148) * added;
+    return alone * alone * alone + b * b * b;
+  };
+  const float c0 = cost(64, 128, 70.f, 53.f), c1 = cost(64, 64, 60.f, 29.f), c2 = cost(32, 64, 39.4f, 20.2f), c3 = cost(32, 32, 37.4f, 11.f);
+  const float best = fminf(fminf(c0, c1), fminf(c2, c3));
+  if (best == c0) return launch_tiles<TW, 64, 128, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  if (best == c1) return launch_tiles<TW, 64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  if (best == c2) return launch_tiles<TW, 32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  return launch_tiles<TW, 32, 32, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+}
+
 ARLE_API int arle_gemm_f32(const float* A, const void* W, int w_dtype, float* C, int M, int N, int K, int lda,
                            int ldw, int ldc, cudaStream_t s) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return ARLE_E_BADARG;
-  if (w_dtype == 0) return launch_plain<float, float, float>(A, W, C, M, N, K, lda, ldw, ldc, s);
-  if (w_dtype == 1) return launch_plain<float, __nv_bfloat16, float>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  if (w_dtype == 0) return launch_f32<float>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  if (w_dtype == 1) return launch_f32<__nv_bfloat16>(A, W, C, M, N, K, lda, ldw, ldc, s);
   return ARLE_E_BADARG;
 }
 

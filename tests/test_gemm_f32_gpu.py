@@ -1,0 +1,25 @@
+"""The float32 products: every kernel sums k in ascending order, so the tiles and the row kernel give the bits of the general kernel (which
+runs when rows are not on 16-byte boundaries), at the edges of their tiles; and float64 stays within a K-term sum's error."""
+import pytest
+import torch
+
+from arle_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("wdtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 130, 301, 700])
+@pytest.mark.parametrize("N,K", [(31, 8), (32, 64), (129, 72), (1000, 136), (2049, 16), (20000, 24)])
+def test_same_bits_as_the_general_kernel(wdtype, M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g, device=DEV)
+    w = torch.randn(N, K, generator=g, device=DEV).to(wdtype)
+    odd = torch.empty(M, K + 1, device=DEV)[:, :K].copy_(x)            # rows off the boundaries: the general kernel
+    got, want = torch.full((M + 1, N), 7.0, device=DEV), torch.empty(M, N, device=DEV)
+    ops.gemm(x, w, got[:M])
+    ops.gemm(odd, w, want)
+    assert torch.equal(got[:M], want) and (got[M] == 7.0).all()
+    exact = x.double() @ w.double().t()
+    assert ((got[:M].double() - exact).abs() <= K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())).all()
