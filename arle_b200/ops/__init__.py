@@ -53,6 +53,7 @@ _SIGNATURES = {
     "arle_gla_out": [_P, _P, _I, _I, _P, _F, _F, _P, _I, _I, _I, _I, _I, _I, _P],
     "arle_attention_prep": [_P, _I, _I, _P, _P, _P, _P, _F, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     "arle_rotary_angles": [_P, _P, _P, _I, _I, _P],
+    "arle_attention_f32": [_P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P, _I, _I, _I, _I, _P],
     "arle_paged_attention_plain": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P, _I, _I, _F, _I, _P, _I, _P],
     "arle_attention_prep_post": [_P, _I, _I, _P, _P, _P, _P, _F, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "arle_branch_norm_add": [_P, _P, _I, _P, _P, _I, _I, _I, _F, _P],
@@ -635,12 +636,25 @@ def paged_attention(q, out, k_cache, v_cache, positions, row_of_token, block_tab
                                    page_size, scale, window, splits, part_o, part_ml, counters, sink=sink, keep_first=keep_first,
                                    softcap=softcap, chunk=chunk, score_bias=score_bias, gate=gate)
         return
+    least = 0
+    if (q.dtype == torch.float32 and batch is not None and _KERNEL_SET == "fast" and vd == hd and hd in (64, 128) and batch.max_q_len >= ATTENTION_F32_LEAST
+            and not (keep_first or softcap or chunk) and score_bias is None and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0):
+        least = ATTENTION_F32_LEAST
+        _check(library().arle_attention_f32(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(batch.q_indptr), _ptr(batch.kv_lens),
+                                            _ptr(block_table), block_table.stride(0), nq, nkv, hd, page_size, float(scale),
+                                            int(window) if window else 0, _ptr(sink), gate_p, gate_stride, batch.num_rows, batch.max_q_len, least,
+                                            _stream()), "attention_f32")
+        if min(batch.q_lens) >= least:
+            return
     _check(library().arle_paged_attention_plain(
         _ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _dt(q), _ptr(positions), _ptr(row_of_token),
         _ptr(block_table), block_table.stride(0), nq, nkv, hd, vd, page_size, float(scale),
         int(window) if window else 0, _ptr(sink), gate_p, gate_stride, keep_first, float(softcap or 0.0), chunk,
-        _ptr(score_bias), T, _stream()),
+        _ptr(score_bias), T, _ptr(batch.q_indptr) if least else None, least, _stream()),
         "paged_attention")
+
+
+ATTENTION_F32_LEAST = 16            # queries of a float32 row from which it runs on the tiles
 
 
 _SINKS: dict = {}
