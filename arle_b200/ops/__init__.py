@@ -654,7 +654,9 @@ def paged_attention(q, out, k_cache, v_cache, positions, row_of_token, block_tab
         "paged_attention")
 
 
-ATTENTION_F32_LEAST = 16            # queries of a float32 row from which it runs on the tiles
+# Queries of a float32 row from which it runs on the tiles (attention_f32.cu has the figures): a tile has room for 32, so rows of fewer
+# than 8 win there only while they are few, and many of them fill the machine better as a block a token.
+ATTENTION_F32_LEAST = 8
 
 
 _SINKS: dict = {}
