@@ -14,6 +14,7 @@
 //    memory, and the tokens are run again from the true incoming state; 32 channels x up to 32 segments a block, or 16
 //    channels x up to 64 segments for long rows of a narrow model.
 #include "common.cuh"
+#include "conv_window.cuh"
 using namespace arle;
 
 template <typename TI, typename TO>
@@ -67,7 +68,10 @@ static int launch_conv(const void* x, int x_stride, const float* in_bias, const 
   const int threads = 128;
   const int cb = (C + threads - 1) / threads;
   if (cb > 65535) return ARLE_E_UNSUPPORTED;
-  launch_kernel(causal_conv_kernel<TI, TO>, dim3(num_tokens, cb), dim3(threads), 0, s, 1, (const TI*)x, x_stride, in_bias, w, out_bias, act,
+  if (conv_window_takes<TI, TO>(x, x_stride, w, out, out_stride, num_tokens, R, C, taps))
+    launch_conv_window<TI, TO>(x, x_stride, in_bias, w, out_bias, act, state, slot_stride, conv_off, q_indptr, row_of_token, state_slots, out,
+                               out_stride, num_tokens, C, s);
+  else launch_kernel(causal_conv_kernel<TI, TO>, dim3(num_tokens, cb), dim3(threads), 0, s, 1, (const TI*)x, x_stride, in_bias, w, out_bias, act,
                 (const float*)state, slot_stride, conv_off, q_indptr, row_of_token, state_slots, (TO*)out, out_stride, C, taps);
   if (taps > 1)
     launch_kernel(causal_conv_state_kernel<TI>, dim3(R, cb), dim3(threads), 0, s, 1, (const TI*)x, x_stride, in_bias, state, slot_stride,
