@@ -96,6 +96,7 @@ _SIGNATURES = {
     "arle_latent_prefill_tc": [_P, _I, _I, _P, _P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _I, _I, _I, _I, _P, _P],
     "arle_latent_attention": [_P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
     "arle_decay_scan": [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _I, _P],
+    "arle_decay_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P],
     "arle_decay_chunk_plan_ints": [_I, _I],
     "arle_decay_chunk_tokens": [],
     "arle_decay_chunk_plan": [_P, _I, _I, _P, _P],
@@ -1426,6 +1427,47 @@ def decay_scan(q, k, v, a, b, state, q_indptr, state_slots, out, heads: int, kq_
                                      dim, vdim, vcols - vdim, float(q_scale), 0 if per_head else heads, int(act == "silu"), int(T > 16 * R),
                                      *_rotation_args(rotation, T, dim, act), int(longest), _stream()),
            "decay_scan")
+
+
+# Rows of up to this many tokens stay with the scan.  A Mamba-2 layer of 128 heads and a matrix LSTM of 8, width 4,096, on the scan and in
+# chunks (us): 40 tokens 106 and 91, 100 and 63; 128 tokens 161 and 109, 195 and 77; at a width of 1,024 55 and 44, 35 and 26 (40 tokens).
+DECAY_TC_LONGEST = 32
+
+
+def decay_tc_takes(q, k, v, dim: int, vdim: int, ones_column: bool, max_q_len: int) -> bool:
+    """Whether ``decay_memories`` would run this step's long rows on the tensor cores."""
+    return (_KERNEL_SET == "fast" and q.is_cuda and max_q_len > DECAY_TC_LONGEST and q.dtype == torch.bfloat16 and dim in (64, 128, 256)
+            and vdim % (64 if ones_column else 8) == 0 and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v)))
+
+
+def decay_memories(q, k, v, a, b, state, batch, out, heads: int, kq_heads: int, dim: int, vdim: int, ones_column: bool, q_scale: float) -> None:
+    """``decay_scan`` for decays a in [0, 1] (float32 [T, heads], as the mixers' gates make them): rows of more than DECAY_TC_LONGEST tokens run
+    in chunks of 64 tokens on the tensor cores where ``decay_tc_takes`` allows it, the others on the scan."""
+    chunks = decay_tc_takes(q, k, v, dim, vdim, ones_column, batch.max_q_len)
+    longest = DECAY_TC_LONGEST
+    if chunks:
+        short = sum(n <= longest for n in batch.q_lens)
+        if short * heads * -(-vdim // 64) <= 148:       # none, or so few that they run beside the long ones without a launch of their own
+            longest = 0
+    if not chunks or longest:
+        decay_scan(q, k, v, a, b, state, batch.q_indptr, batch.state_slots, out, heads, kq_heads, dim, vdim, ones_column, q_scale,
+                   **({"longest": longest} if chunks else {}))
+    if not chunks:
+        return
+    T, vcols = v.shape[0], vdim + int(bool(ones_column))
+    if (q.shape != (T, kq_heads * dim) or k.shape != q.shape or v.shape != (T, heads * vdim) or k.dtype != q.dtype or v.dtype != q.dtype
+            or q.stride(1) != 1 or k.stride(1) != 1 or v.stride(1) != 1):
+        raise KernelError("decay_memories: q, k [T, kq_heads*dim] and v [T, heads*vdim] of one type with unit inner stride")
+    for t_, n_ in ((a, "a"), (b, "b")):
+        if t_.dtype != torch.float32 or tuple(t_.shape) != (T, heads) or not t_.is_contiguous():
+            raise KernelError(f"decay_memories: {n_} must be contiguous float32 [T, heads]")
+    if state.dtype != torch.float32 or state.dim() != 2 or state.shape[1] < heads * vcols * dim or state.stride(1) != 1:
+        raise KernelError(f"decay_memories: state {tuple(state.shape)} must be float32 [slots, >= {heads * vcols * dim}]")
+    if out.dtype != torch.float32 or tuple(out.shape) != (T, heads, vcols) or not out.is_contiguous():
+        raise KernelError("decay_memories: out must be contiguous float32 [T, heads, vcols]")
+    _check(library().arle_decay_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(a), _ptr(b), _ptr(state), state.stride(0),
+                                   _ptr(batch.q_indptr), _ptr(batch.state_slots), _ptr(out), batch.num_rows, heads, kq_heads, dim, vdim, vcols,
+                                   float(q_scale), longest, _stream()), "decay_tc")
 
 
 DECAY_CHUNK = 64                    # tokens of a chunk

@@ -113,8 +113,7 @@ class Mamba2(Mixer):
         a, b = (ctx.ws.get(n, (T, H), torch.float32) for n in ("scan_a", "scan_b"))
         ops.ssm_gates(dt_raw, self.dt_bias, self.a_log, a, b)
         y = ctx.ws.get("scan_out", (T, H, P), torch.float32)
-        ops.decay_scan(xbc[:, inner + bc:], xbc[:, inner: inner + bc], xbc[:, :inner], a, b, state, ctx.q_indptr, ctx.state_slots, y,
-                       H, s.groups, N, P, False, 1.0)
+        ops.decay_memories(xbc[:, inner + bc:], xbc[:, inner: inner + bc], xbc[:, :inner], a, b, state, ctx, y, H, s.groups, N, P, False, 1.0)
         gated = ctx.ws.get("ssm_gated", (T, inner), x.dtype)
         ops.gated_group_norm(y.view(T, inner), xbc[:, :inner], self.skip, P, zxbc[:, :inner], self.norm, s.norm_eps, gated, s.norm_groups)
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)

@@ -114,8 +114,8 @@ class MatrixLstm(Mixer):
         ops.mlstm_gates(pre, self.bias_i, self.bias_f, s.gate_cap, ctx.q_indptr, ctx.state_slots, state, self.m_offset, a, b, floor)
         at = self.at
         num = ctx.ws.get("scan_out", (T, H, dv + 1), torch.float32)
-        ops.decay_scan(proj[:, at["q"]: at["q"] + H * dk], proj[:, at["k"]: at["k"] + H * dk], proj[:, at["v"]: at["v"] + H * dv],
-                       a, b, state, ctx.q_indptr, ctx.state_slots, num, H, H, dk, dv, True, dk ** -0.5)
+        ops.decay_memories(proj[:, at["q"]: at["q"] + H * dk], proj[:, at["k"]: at["k"] + H * dk], proj[:, at["v"]: at["v"] + H * dv],
+                           a, b, state, ctx, num, H, H, dk, dv, True, dk ** -0.5)
         gated = ctx.ws.get("mlstm_gated", (T, H * dv), x.dtype)
         ops.mlstm_out(num, floor, proj[:, at["gate"]: at["gate"] + H * dv], self.norm, s.norm_eps, gated, H, dv)
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)
