@@ -16,7 +16,10 @@
 //    consecutive key channels of each of four columns of S in registers (up to 32 consecutive lanes share a
 //    column; the state is stored [vdim][dim], so a column's lanes read one contiguous run), the step's
 //    q, k, alpha and v are staged in shared memory a chunk of tokens at a time, and o_t[j] is the sum
-//    over the column's lanes.  The order of every sum depends on (dim, vdim) only: a token's result
+//    over the column's lanes.  What bounds it is a warp's instructions: a scheduler of the SM has one warp of a single prompt.  So
+//    two channels are one packed instruction (fma.rn.f32x2), and the sums of eight tokens and four columns are added over the 32 lanes
+//    together, 31 exchanges instead of 48.  16 heads of 128 x 128, 2,048 tokens: 269 us (444 with single numbers and a token's sums by
+//    themselves).  The order of every sum depends on (dim, vdim) only: a token's result
 //    does not depend on how the prompt was cut or on what else is in the batch.
 //    With a bonus u (one number per head and key channel) the read-out comes before the update and sees the current
 //    token through u instead: o_t = (S_(t-1) + diag(u) k_t v_t^T)^T q_t.
@@ -90,6 +93,26 @@ __device__ __forceinline__ float4 widen4(uint2 u) {
 template <typename T, bool VEC> struct Raw4 { using type = float4; };
 template <> struct Raw4<__nv_bfloat16, true> { using type = uint2; };
 
+// Two float32 numbers in a 64-bit register, each with the rounding of the single instruction.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 pair2(float lo, float hi) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float low2(f32x2 x) { return __uint_as_float((unsigned)x); }
+__device__ __forceinline__ float high2(f32x2 x) { return __uint_as_float((unsigned)(x >> 32)); }
+
 // DPT: consecutive key channels that a thread keeps of each of its kScanCpt columns of the state (4 up to 128
 // channels, then 8, 16).  LPC: lanes that share a column (a power of two; LPC * DPT >= dim).  VEC: four channels
 // at a time can be fetched with one aligned load.  A chunk of CHUNK tokens is staged in shared memory; while it is
@@ -114,7 +137,8 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
   constexpr int QPT = (QUADS + kScanThreads - 1) / kScanThreads;
   constexpr int VPT = (CHUNK * COLS + kScanThreads - 1) / kScanThreads;
   __shared__ __align__(16) float qs[CHUNK * DPAD], ks[CHUNK * DPAD], as[CHUNK * DPAD];
-  __shared__ __align__(16) float vs[CHUNK * COLS];
+  constexpr int VD = LPC >= 4 ? 2 : 1;           // v's numbers stand twice side by side (a factor of both halves of a pair), where there is room
+  __shared__ __align__(16) float vs[CHUNK * COLS * VD];
   const int r = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * COLS;
   const int l = threadIdx.x & (LPC - 1), jl = threadIdx.x / LPC;
   const int jb = j0 + jl * CPT;                  // this thread's first column
@@ -122,12 +146,15 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
   // the state of a head is kept as [vdim][dim]: a thread's channels of a column are contiguous
   float* S_g = state + (size_t)state_slots[r] * slot_stride + ((size_t)h * vdim) * dim + l * DPT;
   const bool vec_state = (dim & 3) == 0 && (slot_stride & 3) == 0 && ((uintptr_t)state & 15) == 0;
-  float u[BONUS ? DPT : 1];
+  f32x2 u2[BONUS ? DPT / 2 : 1];
   if constexpr (BONUS) {
 #pragma unroll
-    for (int i = 0; i < DPT; ++i) u[i] = l * DPT + i < dim ? bonus[(size_t)h * dim + l * DPT + i] : 0.f;
+    for (int i = 0; i < DPT / 2; ++i) {
+      const int c = l * DPT + 2 * i;
+      u2[i] = pair2(c < dim ? bonus[(size_t)h * dim + c] : 0.f, c + 1 < dim ? bonus[(size_t)h * dim + c + 1] : 0.f);
+    }
   }
-  float S[CPT][DPT];
+  f32x2 S[CPT][DPT / 2];                         // channels 2i and 2i + 1 of a column
 #pragma unroll
   for (int cc = 0; cc < CPT; ++cc) {
     const bool col_ok = jb + cc < vdim;
@@ -138,10 +165,11 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
       if (vec_state) {
         float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
         if (col_ok && c < dim) u = *reinterpret_cast<const float4*>(sp + i);
-        S[cc][i] = u.x, S[cc][i + 1] = u.y, S[cc][i + 2] = u.z, S[cc][i + 3] = u.w;
+        S[cc][i / 2] = pair2(u.x, u.y), S[cc][i / 2 + 1] = pair2(u.z, u.w);
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[cc][i + e] = (col_ok && c + e < dim) ? sp[i + e] : 0.f;
+        for (int e = 0; e < 4; e += 2)
+          S[cc][(i + e) / 2] = pair2((col_ok && c + e < dim) ? sp[i + e] : 0.f, (col_ok && c + e + 1 < dim) ? sp[i + e + 1] : 0.f);
       }
     }
   }
@@ -207,7 +235,11 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
     for (int u = 0; u < VPT; ++u) {
       const int idx = threadIdx.x + u * kScanThreads;
       const int tt = idx / COLS, c = idx - tt * COLS;
-      if (idx < CHUNK * COLS) vs[idx] = (tt < n && j0 + c < vdim) ? to_f32(rv[u]) : 0.f;
+      if (idx < CHUNK * COLS) {
+        const float x = (tt < n && j0 + c < vdim) ? to_f32(rv[u]) : 0.f;
+        if (VD == 2) *reinterpret_cast<float2*>(vs + VD * idx) = make_float2(x, x);
+        else vs[idx] = x;
+      }
     }
   };
 
@@ -218,41 +250,72 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
     stage(n);
     __syncthreads();
     if (t0 + CHUNK < t_end) fetch(t0 + CHUNK, min(CHUNK, t_end - t0 - CHUNK));
-#pragma unroll 4
-    for (int tt = 0; tt < n; ++tt) {
-      const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT);
-      const float vj[CPT] = {v4.x, v4.y, v4.z, v4.w};
-      const float4* qt = reinterpret_cast<const float4*>(qs + tt * DPAD + l * PAD);
-      const float4* kt = reinterpret_cast<const float4*>(ks + tt * DPAD + l * PAD);
-      const float4* at = reinterpret_cast<const float4*>(as + tt * DPAD + l * PAD);
-      float o[CPT];
+    // one token: the memory's step and the thread's part of its columns' sums
+    auto token = [&](int tt, float (&o)[CPT]) {
+      f32x2 vj[CPT];
+      if constexpr (VD == 2) {
+        const ulonglong2 va = *reinterpret_cast<const ulonglong2*>(vs + (tt * COLS + jl * CPT) * 2);
+        const ulonglong2 vb = *reinterpret_cast<const ulonglong2*>(vs + (tt * COLS + jl * CPT) * 2 + 4);
+        vj[0] = va.x, vj[1] = va.y, vj[2] = vb.x, vj[3] = vb.y;
+      } else {
+        const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT);
+        vj[0] = pair2(v4.x, v4.x), vj[1] = pair2(v4.y, v4.y), vj[2] = pair2(v4.z, v4.z), vj[3] = pair2(v4.w, v4.w);
+      }
+      const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(qs + tt * DPAD + l * PAD);
+      const ulonglong2* kt = reinterpret_cast<const ulonglong2*>(ks + tt * DPAD + l * PAD);
+      const ulonglong2* at = reinterpret_cast<const ulonglong2*>(as + tt * DPAD + l * PAD);
+      f32x2 o2[CPT];
 #pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) o[cc] = 0.f;
+      for (int cc = 0; cc < CPT; ++cc) o2[cc] = 0;
 #pragma unroll
       for (int i = 0; i < DPT / 4; ++i) {
-        const float4 a4 = at[i], k4 = kt[i], q4 = qt[i];
+        const ulonglong2 a4 = at[i], k4 = kt[i], q4 = qt[i];
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
+          const f32x2 kv0 = mul2(k4.x, vj[cc]), kv1 = mul2(k4.y, vj[cc]);
           if constexpr (BONUS) {
-            const float kv0 = k4.x * vj[cc], kv1 = k4.y * vj[cc], kv2 = k4.z * vj[cc], kv3 = k4.w * vj[cc];
-            const float lo = fmaf(fmaf(u[4 * i], kv0, S[cc][4 * i]), q4.x, fmaf(u[4 * i + 1], kv1, S[cc][4 * i + 1]) * q4.y);
-            const float hi = fmaf(fmaf(u[4 * i + 2], kv2, S[cc][4 * i + 2]), q4.z, fmaf(u[4 * i + 3], kv3, S[cc][4 * i + 3]) * q4.w);
-            o[cc] += lo + hi;
-            S[cc][4 * i] = fmaf(a4.x, S[cc][4 * i], kv0);
-            S[cc][4 * i + 1] = fmaf(a4.y, S[cc][4 * i + 1], kv1);
-            S[cc][4 * i + 2] = fmaf(a4.z, S[cc][4 * i + 2], kv2);
-            S[cc][4 * i + 3] = fmaf(a4.w, S[cc][4 * i + 3], kv3);
-            continue;
+            o2[cc] = fma2(fma2(u2[2 * i], kv0, S[cc][2 * i]), q4.x, o2[cc]);
+            o2[cc] = fma2(fma2(u2[2 * i + 1], kv1, S[cc][2 * i + 1]), q4.y, o2[cc]);
           }
-          S[cc][4 * i] = fmaf(a4.x, S[cc][4 * i], k4.x * vj[cc]);
-          S[cc][4 * i + 1] = fmaf(a4.y, S[cc][4 * i + 1], k4.y * vj[cc]);
-          S[cc][4 * i + 2] = fmaf(a4.z, S[cc][4 * i + 2], k4.z * vj[cc]);
-          S[cc][4 * i + 3] = fmaf(a4.w, S[cc][4 * i + 3], k4.w * vj[cc]);
-          const float lo = fmaf(S[cc][4 * i], q4.x, S[cc][4 * i + 1] * q4.y);
-          const float hi = fmaf(S[cc][4 * i + 2], q4.z, S[cc][4 * i + 3] * q4.w);
-          o[cc] += lo + hi;
+          S[cc][2 * i] = fma2(a4.x, S[cc][2 * i], kv0);
+          S[cc][2 * i + 1] = fma2(a4.y, S[cc][2 * i + 1], kv1);
+          if constexpr (!BONUS) {
+            o2[cc] = fma2(S[cc][2 * i], q4.x, o2[cc]);
+            o2[cc] = fma2(S[cc][2 * i + 1], q4.y, o2[cc]);
+          }
         }
       }
+#pragma unroll
+      for (int cc = 0; cc < CPT; ++cc) o[cc] = low2(o2[cc]) + high2(o2[cc]);
+    };
+    int first = 0;
+    if constexpr (LPC == 32 && CHUNK % 8 == 0) {
+      // Eight tokens at a time: their 32 sums over 32 lanes in 31 exchanges, after which lane l holds token l / 4's sum of column
+      // l % 4.  A sum's additions are those of a token by itself (lanes 16 apart, then 8, 4, 2, 1).
+      for (; first + 8 <= n; first += 8) {
+        float x[32];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          float o[CPT];
+          token(first + g, o);
+#pragma unroll
+          for (int cc = 0; cc < CPT; ++cc) x[g * CPT + cc] = o[cc];
+        }
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) {
+          const bool up = (l & w) != 0;
+#pragma unroll
+          for (int i = 0; i < w; ++i) {
+            const float got = __shfl_xor_sync(0xffffffffu, up ? x[i] : x[i + w], w);
+            x[i] = (up ? x[i + w] : x[i]) + got;
+          }
+        }
+        if (jb + (l & 3) < vdim) out[(size_t)(t0 + first + (l >> 2)) * heads * vdim + hv + jb + (l & 3)] = x[0];
+      }
+    }
+    for (int tt = first; tt < n; ++tt) {
+      float o[CPT];
+      token(tt, o);
       // the four columns' sums over the LPC lanes: two exchanges halve what a lane holds, then a butterfly
       int mine = 0;                              // the column whose sum this lane ends up with
       float b;
@@ -286,11 +349,12 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
     for (int i = 0; i < DPT; i += 4) {
       const int c = l * DPT + i;
       if (vec_state) {
-        if (col_ok && c < dim) *reinterpret_cast<float4*>(sp + i) = make_float4(S[cc][i], S[cc][i + 1], S[cc][i + 2], S[cc][i + 3]);
+        if (col_ok && c < dim)
+          *reinterpret_cast<float4*>(sp + i) = make_float4(low2(S[cc][i / 2]), high2(S[cc][i / 2]), low2(S[cc][i / 2 + 1]), high2(S[cc][i / 2 + 1]));
       } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          if (col_ok && c + e < dim) sp[i + e] = S[cc][i + e];
+          if (col_ok && c + e < dim) sp[i + e] = e & 1 ? high2(S[cc][(i + e) / 2]) : low2(S[cc][(i + e) / 2]);
       }
     }
   }
