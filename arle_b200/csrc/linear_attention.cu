@@ -18,8 +18,9 @@
 //    q, k, alpha and v are staged in shared memory a chunk of tokens at a time, and o_t[j] is the sum
 //    over the column's lanes.  What bounds it is a warp's instructions: a scheduler of the SM has one warp of a single prompt.  So
 //    two channels are one packed instruction (fma.rn.f32x2), and the sums of eight tokens and four columns are added over the 32 lanes
-//    together, 31 exchanges instead of 48.  16 heads of 128 x 128, 2,048 tokens: 269 us (444 with single numbers and a token's sums by
-//    themselves).  The order of every sum depends on (dim, vdim) only: a token's result
+//    together, 31 exchanges instead of 48.  The next chunk's loads are pinned in front
+//    of the work that hides them (plain ones were moved behind it).  16 heads of 128 x 128, 2,048 tokens: 213 us (444 with single
+//    numbers and a token's sums by themselves, 269 before the loads were pinned).  The order of every sum depends on (dim, vdim) only: a token's result
 //    does not depend on how the prompt was cut or on what else is in the batch.
 //    With a bonus u (one number per head and key channel) the read-out comes before the update and sees the current
 //    token through u instead: o_t = (S_(t-1) + diag(u) k_t v_t^T)^T q_t.
@@ -28,6 +29,7 @@
 #include <initializer_list>
 
 #include "common.cuh"
+#include "scan_utils.cuh"
 using namespace arle;
 
 constexpr int kScanThreads = 128;
@@ -92,26 +94,6 @@ __device__ __forceinline__ float4 widen4(uint2 u) {
 }
 template <typename T, bool VEC> struct Raw4 { using type = float4; };
 template <> struct Raw4<__nv_bfloat16, true> { using type = uint2; };
-
-// Two float32 numbers in a 64-bit register, each with the rounding of the single instruction.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 pair2(float lo, float hi) {
-  f32x2 d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ float low2(f32x2 x) { return __uint_as_float((unsigned)x); }
-__device__ __forceinline__ float high2(f32x2 x) { return __uint_as_float((unsigned)(x >> 32)); }
 
 // DPT: consecutive key channels that a thread keeps of each of its kScanCpt columns of the state (4 up to 128
 // channels, then 8, 16).  LPC: lanes that share a column (a power of two; LPC * DPT >= dim).  VEC: four channels
@@ -191,9 +173,9 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
       const size_t row = ok ? (size_t)(t0 + tt) : (size_t)t_begin;
       const int cs = ok ? c : 0;
       if constexpr (VEC) {
-        rq[u] = load_raw4(q + row * in_stride + hq + cs);
-        rk[u] = load_raw4(k + row * in_stride + hq + cs);
-        ra[u] = *reinterpret_cast<const float4*>(alpha + row * a_stride + hq + cs);
+        rq[u] = load_now(q + row * in_stride + hq + cs, RawT());
+        rk[u] = load_now(k + row * in_stride + hq + cs, RawT());
+        ra[u] = load_now(alpha + row * a_stride + hq + cs, float4());
       } else {
         float4 fq = make_float4(0.f, 0.f, 0.f, 0.f), fk = fq, fa = fq;
         float* pq = &fq.x; float* pk = &fk.x; float* pa = &fa.x;
@@ -214,7 +196,7 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
       const int idx = threadIdx.x + u * kScanThreads;
       const int tt = idx / COLS, c = idx - tt * COLS;
       const bool ok = idx < CHUNK * COLS && tt < n && j0 + c < vdim;
-      rv[u] = v[(ok ? (size_t)(t0 + tt) : (size_t)t_begin) * in_stride + hv + (ok ? j0 + c : 0)];
+      rv[u] = load_now(v + (ok ? (size_t)(t0 + tt) : (size_t)t_begin) * in_stride + hv + (ok ? j0 + c : 0), T());
     }
   };
   auto stage = [&](int n) {                      // registers to shared memory, widened, q scaled on the way
