@@ -16,9 +16,13 @@
 //    round, and since S^T q = g S_old^T q + u (k . q) the read-out needs no second round.  16 tokens are staged in shared
 //    memory at a time as they are; their unit lengths are three sums a token (q . q, k . k, q . k) and enter as factors
 //    of the two products and of u.  Eight lanes a column (sixteen numbers a lane at dim 128) cost a third of the
-//    instructions of thirty-two lanes with four numbers.  The split of a column depends on dim alone, so a token's sums
+//    instructions of thirty-two lanes with four numbers.  Two numbers are one packed instruction (the same roundings), and the next
+//    chunk's q, k and v are on their way into registers while a chunk's tokens run.  What bounds a long row is the chain of a token: loads
+//    from shared memory, four dependent FMAs, three exchanges, the correction and the update, some 550 cycles.  Rows of 479, 701 and 819
+//    tokens, 32 heads of 128 x 128: 570 us (single numbers, loads waited for at each chunk: 633 to 680); one row of 2,048, 8 heads: 581 (710).  The split of a column depends on dim alone, so a token's sums
 //    have one order whatever the cutting or the batch.
 #include "common.cuh"
+#include "scan_utils.cuh"
 using namespace arle;
 
 __global__ void delta_gates_kernel(const float* __restrict__ pre, int pre_stride, const float* __restrict__ a_log,
@@ -57,7 +61,7 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int q_stride, int k_stride, int v_stride,
     const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ state, long slot_stride,
     const int* __restrict__ q_indptr, const int* __restrict__ state_slots, float* __restrict__ out, int H, int kq_heads, int dim,
-    int vdim, float q_scale, float unit_eps) {
+    int vdim, float q_scale, float unit_eps, int ahead) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
@@ -82,24 +86,82 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
   const bool col_live = c0 + cl < vdim;
   float* sp = state + (size_t)state_slots[r] * slot_stride + (size_t)h * vdim * dim + (size_t)(c0 + cl) * dim;
   const bool vec_state = dim % 4 == 0 && ((uintptr_t)sp & 15) == 0;
-  float S[EPL];
+  f32x2 S[EPL / 2];                                      // two neighbouring numbers each
 #pragma unroll
   for (int i = 0; i < NG; ++i) {
     const int e = 4 * (i * LPC + part);
     if (col_live && vec_state && e < dim) {
       const float4 x = *reinterpret_cast<const float4*>(sp + e);
-      S[4 * i] = x.x; S[4 * i + 1] = x.y; S[4 * i + 2] = x.z; S[4 * i + 3] = x.w;
+      S[2 * i] = pair2(x.x, x.y), S[2 * i + 1] = pair2(x.z, x.w);
     } else {
+      float x[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) S[4 * i + j] = (col_live && e + j < dim) ? sp[e + j] : 0.f;
+      for (int j = 0; j < 4; ++j) x[j] = (col_live && e + j < dim) ? sp[e + j] : 0.f;
+      S[2 * i] = pair2(x[0], x[1]), S[2 * i + 1] = pair2(x[2], x[3]);
     }
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = nthreads >> 5;
   const int stt = threadIdx.x & (kDeltaChunk - 1), sseg = threadIdx.x >> 4, nseg = nthreads >> 4;   // the sums: a token, a share of dim
 
+  // `ahead` (rows of q and k in whole 16-byte pieces): the next chunk's numbers are on their way into registers while this one's
+  // tokens run.  Places past the row's end read its first token and are zeroed when staged.
+  constexpr int PER = 16 / sizeof(T), PIECES = kDeltaChunk * DPAD / PER, MAXP = LONG ? (PIECES + 127) / 128 : 1;
+  constexpr int VPT = LONG ? (kDeltaChunk + LPC - 1) / LPC : 1;
+  uint4 rq[MAXP], rk[MAXP];
+  T rv[VPT];
+  float rg = 0.f, rb = 0.f;
+  auto fetch = [&](int t0) {
+    const int n = min(kDeltaChunk, end - t0);
+#pragma unroll
+    for (int u = 0; u < MAXP; ++u) {
+      const int idx = threadIdx.x + u * nthreads, tt = idx / (DPAD / PER), e = idx % (DPAD / PER) * PER;
+      const bool on = idx < PIECES && tt < n && e < dim;
+      const size_t t = on ? t0 + tt : beg;
+      rq[u] = load_now16(q + t * q_stride + (size_t)g * dim + (on ? e : 0));
+      rk[u] = load_now16(k + t * k_stride + (size_t)g * dim + (on ? e : 0));
+    }
+#pragma unroll
+    for (int u = 0; u < VPT; ++u) {
+      const int idx = threadIdx.x + u * nthreads, tt = idx / cpb, cc = idx - tt * cpb;
+      const bool on = tt < n && c0 + cc < vdim;
+      rv[u] = load_now(v + (size_t)(on ? t0 + tt : beg) * v_stride + (size_t)h * vdim + (on ? c0 + cc : 0), T());
+    }
+    if (threadIdx.x < kDeltaChunk) {
+      const size_t t = (int)threadIdx.x < n ? t0 + threadIdx.x : beg;
+      rg = load_now(decay + t * H + h, 0.f);
+      rb = load_now(beta + t * H + h, 0.f);
+    }
+  };
+  if (LONG && ahead && beg < end) fetch(beg);
   for (int t0 = beg; t0 < end; t0 += kDeltaChunk) {
     const int n = min(kDeltaChunk, end - t0);
     __syncthreads();
+    if (LONG && ahead) {
+#pragma unroll
+      for (int u = 0; u < MAXP; ++u) {
+        const int idx = threadIdx.x + u * nthreads, tt = idx / (DPAD / PER), e = idx % (DPAD / PER) * PER;
+        if (idx >= PIECES) continue;
+        const bool on = tt < n && e < dim;
+        const T* a = reinterpret_cast<const T*>(&rq[u]);
+        const T* b = reinterpret_cast<const T*>(&rk[u]);
+#pragma unroll
+        for (int i = 0; i < PER; i += 4) {
+          *reinterpret_cast<float4*>(qs + tt * ROW + e + i) =
+              on ? make_float4(to_f32(a[i]), to_f32(a[i + 1]), to_f32(a[i + 2]), to_f32(a[i + 3])) : make_float4(0.f, 0.f, 0.f, 0.f);
+          *reinterpret_cast<float4*>(ksm + tt * ROW + e + i) =
+              on ? make_float4(to_f32(b[i]), to_f32(b[i + 1]), to_f32(b[i + 2]), to_f32(b[i + 3])) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < VPT; ++u) {
+        const int idx = threadIdx.x + u * nthreads;
+        if (idx < kDeltaChunk * cpb) vs[idx] = c0 + idx % cpb < vdim ? to_f32(rv[u]) : 0.f;
+      }
+      if (threadIdx.x < n) {
+        gs[threadIdx.x] = rg;
+        bs[threadIdx.x] = rb;
+      }
+    } else {
     for (int e = threadIdx.x; e < DPAD; e += nthreads) {
       const bool in = e < dim;
       const T* qp = q + (size_t)t0 * q_stride + (size_t)g * dim + e;
@@ -132,7 +194,9 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
       gs[threadIdx.x] = decay[(size_t)(t0 + threadIdx.x) * H + h];
       bs[threadIdx.x] = beta[(size_t)(t0 + threadIdx.x) * H + h];
     }
+    }
     __syncthreads();
+    if (LONG && ahead && t0 + kDeltaChunk < end) fetch(t0 + kDeltaChunk);
     {
       float sq = 0.f, sk = 0.f, qk = 0.f;
       if (stt < n)
@@ -167,18 +231,18 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
     __syncthreads();
     auto step = [&](int tt) {
       const float gt = gs[tt], ik = iks[tt];
-      const float4* kt = reinterpret_cast<const float4*>(ksm + tt * ROW) + part;
-      const float4* qt = reinterpret_cast<const float4*>(qs + tt * ROW) + part;
-      float kk[EPL];
-      float pk0 = 0.f, pk1 = 0.f, pk2 = 0.f, pk3 = 0.f, pq0 = 0.f, pq1 = 0.f, pq2 = 0.f, pq3 = 0.f;
+      const ulonglong2* kt = reinterpret_cast<const ulonglong2*>(ksm + tt * ROW) + part;
+      const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(qs + tt * ROW) + part;
+      f32x2 kk[EPL / 2];
+      f32x2 pka = 0, pkb = 0, pqa = 0, pqb = 0;
 #pragma unroll
       for (int i = 0; i < NG; ++i) {
-        const float4 kv = kt[i * LPC], qv = qt[i * LPC];
-        kk[4 * i] = kv.x; kk[4 * i + 1] = kv.y; kk[4 * i + 2] = kv.z; kk[4 * i + 3] = kv.w;
-        pk0 = fmaf(S[4 * i], kv.x, pk0); pk1 = fmaf(S[4 * i + 1], kv.y, pk1); pk2 = fmaf(S[4 * i + 2], kv.z, pk2); pk3 = fmaf(S[4 * i + 3], kv.w, pk3);
-        pq0 = fmaf(S[4 * i], qv.x, pq0); pq1 = fmaf(S[4 * i + 1], qv.y, pq1); pq2 = fmaf(S[4 * i + 2], qv.z, pq2); pq3 = fmaf(S[4 * i + 3], qv.w, pq3);
+        const ulonglong2 kv = kt[i * LPC], qv = qt[i * LPC];
+        kk[2 * i] = kv.x, kk[2 * i + 1] = kv.y;
+        pka = fma2(S[2 * i], kv.x, pka), pkb = fma2(S[2 * i + 1], kv.y, pkb);
+        pqa = fma2(S[2 * i], qv.x, pqa), pqb = fma2(S[2 * i + 1], qv.y, pqb);
       }
-      float pk = (pk0 + pk1) + (pk2 + pk3), pq = (pq0 + pq1) + (pq2 + pq3);
+      float pk = (low2(pka) + high2(pka)) + (low2(pkb) + high2(pkb)), pq = (low2(pqa) + high2(pqa)) + (low2(pqb) + high2(pqb));
 #pragma unroll
       for (int o = LPC >> 1; o > 0; o >>= 1) {
         pk += __shfl_xor_sync(0xffffffffu, pk, o);
@@ -186,8 +250,9 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
       }
       const float u = bs[tt] * (vs[tt * cpb + cl] - gt * (ik * pk));
       const float uk = u * ik;
+      const f32x2 uk2 = pair2(uk, uk), gt2 = pair2(gt, gt);
 #pragma unroll
-      for (int i = 0; i < EPL; ++i) S[i] = fmaf(gt, S[i], kk[i] * uk);
+      for (int i = 0; i < EPL / 2; ++i) S[i] = fma2(gt2, S[i], mul2(kk[i], uk2));
       if (part == 0 && col_live) out[((size_t)(t0 + tt) * H + h) * vdim + c0 + cl] = fmaf(gt * iqs[tt], pq, u * kq[tt]);
     };
     if (LONG && n == kDeltaChunk) {                      // a full chunk unrolled: a token's loads from shared memory run ahead of
@@ -202,11 +267,11 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
     for (int i = 0; i < NG; ++i) {
       const int e = 4 * (i * LPC + part);
       if (vec_state && e < dim) {
-        *reinterpret_cast<float4*>(sp + e) = make_float4(S[4 * i], S[4 * i + 1], S[4 * i + 2], S[4 * i + 3]);
+        *reinterpret_cast<float4*>(sp + e) = make_float4(low2(S[2 * i]), high2(S[2 * i]), low2(S[2 * i + 1]), high2(S[2 * i + 1]));
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (e + j < dim) sp[e + j] = S[4 * i + j];
+          if (e + j < dim) sp[e + j] = j & 1 ? high2(S[2 * i + (j >> 1)]) : low2(S[2 * i + (j >> 1)]);
       }
     }
   }
@@ -227,9 +292,11 @@ static int launch_delta(const void* q, const void* k, const void* v, int q_strid
     cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<T, EPL, LPC, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
+  const int per = 16 / (int)sizeof(T);
+  const int ahead = dim % per == 0 && q_stride % per == 0 && k_stride % per == 0 && (((uintptr_t)q | (uintptr_t)k) & 15) == 0;
   dim3 grid((vdim + cpb - 1) / cpb, H, R);
   launch_kernel(delta_scan_kernel<T, EPL, LPC, LONG>, dim3(grid), dim3(threads), smem, s, 1, (const T*)q, (const T*)k, (const T*)v, q_stride,
-                k_stride, v_stride, beta, decay, state, slot_stride, q_indptr, state_slots, out, H, kq_heads, dim, vdim, q_scale, unit_eps);
+                k_stride, v_stride, beta, decay, state, slot_stride, q_indptr, state_slots, out, H, kq_heads, dim, vdim, q_scale, unit_eps, ahead);
   return launch_status();
 }
 
