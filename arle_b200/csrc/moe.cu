@@ -14,10 +14,8 @@
 //  * moe_gemm: C[place, :] = A[row(place), :] . W[expert(place)]^T in tiles of 64 x 64, float32 sums with k ascending
 //    (the per-expert twin of the plain product).  `rows` maps a place to its row of A (the token of the pair) or is
 //    absent (A is already in place order).
-//    In bfloat16 with aligned rows the same product runs on the tensor cores (moe_gemm_mma: tiles of 64 places x 128
-//    columns, mma.sync with float32 sums, operands brought in by cp.async in three stages), and a step of few pairs
-//    (decoding) runs it as one dot product a warp (moe_gemv: every chosen expert's rows are streamed once, 16 bytes
-//    a lane and load), since a tile of 64 places would be all but empty.
+//    In bfloat16 with aligned rows the same product runs on the tensor cores (moe_tcgen05.cu), and a step of very few pairs
+//    runs it as one dot product a warp (moe_gemv: every chosen expert's rows are streamed once, 16 bytes a lane and load).
 //    The sums may be finished before they are stored: times a number per place (the choice's weight, when it multiplies the
 //    expert's input: W (w x) = w (W x)), then through an activation (the square of relu).
 //  * moe_combine: out[t] = sum_k weight[t, k] * Y[place(t, k)] (k ascending; no weights: ones) + sigmoid(gate[t]) * shared[t].
