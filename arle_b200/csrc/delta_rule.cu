@@ -91,8 +91,8 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
   for (int i = 0; i < NG; ++i) {
     const int e = 4 * (i * LPC + part);
     if (col_live && vec_state && e < dim) {
-      const float4 x = *reinterpret_cast<const float4*>(sp + e);
-      S[2 * i] = pair2(x.x, x.y), S[2 * i + 1] = pair2(x.z, x.w);
+      const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(sp + e);      // as pairs: packing them here would wait for every load
+      S[2 * i] = x.x, S[2 * i + 1] = x.y;
     } else {
       float x[4];
 #pragma unroll
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
     for (int i = 0; i < NG; ++i) {
       const int e = 4 * (i * LPC + part);
       if (vec_state && e < dim) {
-        *reinterpret_cast<float4*>(sp + e) = make_float4(low2(S[2 * i]), high2(S[2 * i]), low2(S[2 * i + 1]), high2(S[2 * i + 1]));
+        *reinterpret_cast<ulonglong2*>(sp + e) = make_ulonglong2(S[2 * i], S[2 * i + 1]);
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j)

@@ -102,7 +102,8 @@ template <> struct Raw4<__nv_bfloat16, true> { using type = uint2; };
 // alpha that a thread reads from shared memory serves four columns: with one column a thread the kernel was bound by
 // shared-memory bandwidth.
 // BONUS: the read-out before the update, with the current token weighted by u.
-template <typename T, int DPT, int LPC, bool VEC, bool BONUS>
+// GROUPS: some row has eight tokens or more; the form without them, for decoded tokens, holds fewer registers.
+template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool GROUPS>
 __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int in_stride,
     const float* __restrict__ alpha, const float* __restrict__ bonus, float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
@@ -145,9 +146,9 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
     for (int i = 0; i < DPT; i += 4) {
       const int c = l * DPT + i;
       if (vec_state) {
-        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (col_ok && c < dim) u = *reinterpret_cast<const float4*>(sp + i);
-        S[cc][i / 2] = pair2(u.x, u.y), S[cc][i / 2 + 1] = pair2(u.z, u.w);
+        ulonglong2 x = make_ulonglong2(0, 0);    // as pairs: packing them here would wait for every load
+        if (col_ok && c < dim) x = *reinterpret_cast<const ulonglong2*>(sp + i);
+        S[cc][i / 2] = x.x, S[cc][i / 2 + 1] = x.y;
       } else {
 #pragma unroll
         for (int e = 0; e < 4; e += 2)
@@ -271,7 +272,7 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
       for (int cc = 0; cc < CPT; ++cc) o[cc] = low2(o2[cc]) + high2(o2[cc]);
     };
     int first = 0;
-    if constexpr (LPC == 32 && CHUNK % 8 == 0) {
+    if constexpr (GROUPS && LPC == 32 && CHUNK % 8 == 0) {
       // Eight tokens at a time: their 32 sums over 32 lanes in 31 exchanges, after which lane l holds token l / 4's sum of column
       // l % 4.  A sum's additions are those of a token by itself (lanes 16 apart, then 8, 4, 2, 1).
       for (; first + 8 <= n; first += 8) {
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
       const int c = l * DPT + i;
       if (vec_state) {
         if (col_ok && c < dim)
-          *reinterpret_cast<float4*>(sp + i) = make_float4(low2(S[cc][i / 2]), high2(S[cc][i / 2]), low2(S[cc][i / 2 + 1]), high2(S[cc][i / 2 + 1]));
+          *reinterpret_cast<ulonglong2*>(sp + i) = make_ulonglong2(S[cc][i / 2], S[cc][i / 2 + 1]);
       } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
@@ -438,14 +439,18 @@ namespace {
 
 template <typename T, int DPT, int LPC>
 int scan_launch(const void* q, const void* k, const void* v, int in_stride, const float* alpha, const float* bonus, float* state, long slot_stride, const int* q_indptr,
-                const int* state_slots, float* out, int rows, int heads, int dim, int vdim, float q_scale, cudaStream_t s) {
+                const int* state_slots, float* out, int rows, int heads, int dim, int vdim, float q_scale, int max_q_len, cudaStream_t s) {
   constexpr int COLS = kScanThreads / LPC * kScanCpt;
   dim3 grid((vdim + COLS - 1) / COLS, heads, rows);
   const size_t eb = sizeof(T) * 4;               // bytes of four elements of q or k
   const bool vec = dim % 4 == 0 && in_stride % 4 == 0 && ((uintptr_t)q % eb) == 0 && ((uintptr_t)k % eb) == 0 &&
                    ((uintptr_t)alpha % 16) == 0;
-  auto kernel = bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true> : gla_scan_kernel<T, DPT, LPC, false, true>)
-                      : (vec ? gla_scan_kernel<T, DPT, LPC, true, false> : gla_scan_kernel<T, DPT, LPC, false, false>);
+  constexpr bool G = LPC == 32;
+  const bool groups = G && max_q_len >= 8;
+  auto kernel = groups ? (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, G> : gla_scan_kernel<T, DPT, LPC, false, true, G>)
+                                : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, G> : gla_scan_kernel<T, DPT, LPC, false, false, G>))
+                       : (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, false> : gla_scan_kernel<T, DPT, LPC, false, true, false>)
+                                : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, false> : gla_scan_kernel<T, DPT, LPC, false, false, false>));
   launch_kernel(kernel, grid, dim3(kScanThreads), 0, s, 1, (const T*)q, (const T*)k, (const T*)v, in_stride, alpha, bonus, state, slot_stride,
                 q_indptr, state_slots, out, heads, dim, vdim, q_scale);
   return launch_status();
@@ -456,9 +461,9 @@ int scan_launch(const void* q, const void* k, const void* v, int in_stride, cons
 template <typename T>
 int scan_dispatch(const void* q, const void* k, const void* v, int in_stride, const float* alpha, const float* bonus, float* state,
                   long slot_stride, const int* q_indptr, const int* state_slots, float* out, int rows, int heads, int dim, int vdim, float q_scale,
-                  cudaStream_t s) {
+                  int max_q_len, cudaStream_t s) {
 #define ARLE_SCAN(D, L) \
-  return scan_launch<T, D, L>(q, k, v, in_stride, alpha, bonus, state, slot_stride, q_indptr, state_slots, out, rows, heads, dim, vdim, q_scale, s)
+  return scan_launch<T, D, L>(q, k, v, in_stride, alpha, bonus, state, slot_stride, q_indptr, state_slots, out, rows, heads, dim, vdim, q_scale, max_q_len, s)
   if (dim <= 4) ARLE_SCAN(4, 1);
   if (dim <= 8) ARLE_SCAN(4, 2);
   if (dim <= 16) ARLE_SCAN(4, 4);
@@ -480,9 +485,9 @@ ARLE_API int arle_gla_scan(const void* q, const void* k, const void* v, int dtyp
   if (heads <= 0 || dim <= 0 || vdim <= 0 || max_q_len <= 0 || slot_stride < (long)heads * vdim * dim) return ARLE_E_BADARG;
   if (dim > 512 || heads > 65535 || rows > 65535) return ARLE_E_UNSUPPORTED;
   if (dtype == 0)
-    return scan_dispatch<float>(q, k, v, in_stride, alpha, bonus, state, slot_stride, q_indptr, state_slots, out, rows, heads, dim, vdim, q_scale, s);
+    return scan_dispatch<float>(q, k, v, in_stride, alpha, bonus, state, slot_stride, q_indptr, state_slots, out, rows, heads, dim, vdim, q_scale, max_q_len, s);
   if (dtype == 1)
-    return scan_dispatch<__nv_bfloat16>(q, k, v, in_stride, alpha, bonus, state, slot_stride, q_indptr, state_slots, out, rows, heads, dim, vdim, q_scale, s);
+    return scan_dispatch<__nv_bfloat16>(q, k, v, in_stride, alpha, bonus, state, slot_stride, q_indptr, state_slots, out, rows, heads, dim, vdim, q_scale, max_q_len, s);
   return ARLE_E_BADARG;
 }
 
