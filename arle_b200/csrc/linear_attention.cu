@@ -102,9 +102,10 @@ template <> struct Raw4<__nv_bfloat16, true> { using type = uint2; };
 // alpha that a thread reads from shared memory serves four columns: with one column a thread the kernel was bound by
 // shared-memory bandwidth.
 // BONUS: the read-out before the update, with the current token weighted by u.
-// GROUPS: some row has eight tokens or more; the form without them, for decoded tokens, holds fewer registers.
+// GROUPS: some row has eight tokens or more; the form without them, for decoded tokens, is bound by memory and holds few enough registers
+// for five blocks an SM.
 template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool GROUPS>
-__global__ void __launch_bounds__(kScanThreads) gla_scan_kernel(
+__global__ void __launch_bounds__(kScanThreads, DPT == 4 && !GROUPS && !BONUS ? 5 : 1) gla_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int in_stride,
     const float* __restrict__ alpha, const float* __restrict__ bonus, float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
     const int* __restrict__ state_slots, float* __restrict__ out, int heads, int dim, int vdim, float q_scale) {
