@@ -30,6 +30,9 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
   return __float2bfloat16_rn(v);
 }
 
+// Whether one of two bfloat16 numbers is an infinity or a NaN.
+__device__ __forceinline__ bool bf16x2_odd(uint32_t w) { return (w & 0x7f80u) == 0x7f80u || (w & 0x7f800000u) == 0x7f800000u; }
+
 // VEC consecutive numbers of type T as one aligned access (p on a VEC * sizeof(T) boundary; 16 bytes an instruction).
 template <typename T, int VEC> struct alignas(sizeof(T) * VEC) Pack { T e[VEC]; };
 

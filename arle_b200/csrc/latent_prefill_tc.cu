@@ -10,6 +10,9 @@
 //    its keys start in the built arrays; -1 for the others (the folded kernel runs them).
 //  * latent_gather: the records of those rows from the pages, side by side, each row's padded to a multiple of 16 with zeros.
 //    The product that builds keys and values is the caller's (a plain matrix product over the gathered latents).
+//    A latent with an infinity or a NaN is gathered as zeros with NaN in the rotated numbers beside it (a record without rotated numbers
+//    gets eight, zero otherwise): its scores are NaN, so every query that sees it gets NaN as from the folded form, and no other query
+//    does, since a masked score is replaced and the built values, which meet a weight of zero, are finite.
 //  * latent_prefill_tc: the attention.  The scheme, the roles of the warps and the barriers are those of attention_prefill_tc.cu (two
 //    query tiles of 128 a CTA that share every key tile; scores and outputs in tensor memory, P over the scores; blocks drawn from a
 //    counter, heaviest first).  What differs: a key tile has NS slices of 64 numbers from the built keys and one of up to 64 from the
@@ -123,12 +126,20 @@ __global__ void __launch_bounds__(32) latent_plan_kernel(const int* __restrict__
   if (lane == 0) plan[R] = make_int2(carry, carry);
 }
 
-// A block copies 16 neighbouring records (pages hold a multiple of 16), 16 bytes a thread and step.
-__global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table, int bt_stride,
-                                                            const int* __restrict__ kv_lens, const int2* __restrict__ plan, int R, int page_size,
-                                                            int kd, __nv_bfloat16* __restrict__ out) {
+// Numbers of a gathered record behind its latent.
+__host__ __device__ constexpr int gathered_tail(int dr) { return dr ? dr : 8; }
+
+constexpr int kGatherThreads = 256, kGatherSteps = 16 * (512 + 64) / 8 / kGatherThreads + 1;     // 16-byte pieces a thread copies at most
+
+// A block copies 16 neighbouring records (pages hold a multiple of 16), 16 bytes a thread and step.  kd: numbers of a stored record, ko
+// of a gathered one.
+__global__ void __launch_bounds__(kGatherThreads) latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table,
+                                                                       int bt_stride, const int* __restrict__ kv_lens,
+                                                                       const int2* __restrict__ plan, int R, int page_size, int rank, int kd, int ko,
+                                                                       __nv_bfloat16* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
+  __shared__ int bad[16];                                  // records whose latent holds an infinity or a NaN
   const int place = blockIdx.x * 16;
   if (place >= plan[R].x) return;
   int row = -1;
@@ -140,9 +151,27 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(const __nv_bfloat16*
   const int key = plan[row].x + place - plan[row].y, live = kv_lens[row] - key;       // records of the 16 that the request holds
   const int page = block_table[(size_t)row * bt_stride + key / page_size];
   const uint4* src = reinterpret_cast<const uint4*>(cache + ((size_t)page * page_size + key % page_size) * kd);
-  uint4* dst = reinterpret_cast<uint4*>(out + (size_t)place * kd);
-  const int per = kd / 8;
-  for (int i = threadIdx.x; i < 16 * per; i += 256) dst[i] = i < live * per ? src[i] : make_uint4(0, 0, 0, 0);
+  uint4* dst = reinterpret_cast<uint4*>(out + (size_t)place * ko);
+  const int per = ko / 8, from = kd / 8, latent = rank / 8;
+  if (threadIdx.x < 16) bad[threadIdx.x] = 0;
+  __syncthreads();
+  uint4 x[kGatherSteps];
+#pragma unroll
+  for (int it = 0; it < kGatherSteps; ++it) {
+    const int i = threadIdx.x + it * kGatherThreads, rec = i / per, c = i - rec * per;
+    x[it] = make_uint4(0, 0, 0, 0);
+    if (rec >= min(16, live) || c >= from) continue;
+    x[it] = src[rec * from + c];
+    if (c < latent && (bf16x2_odd(x[it].x) || bf16x2_odd(x[it].y) || bf16x2_odd(x[it].z) || bf16x2_odd(x[it].w))) bad[rec] = 1;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < kGatherSteps; ++it) {
+    const int i = threadIdx.x + it * kGatherThreads, rec = i / per, c = i - rec * per;
+    if (rec >= 16) break;
+    const uint32_t instead = c < latent ? 0u : 0x7fff7fffu;
+    dst[i] = bad[rec] ? make_uint4(instead, instead, instead, instead) : x[it];
+  }
 }
 
 // What a CTA's roles need to know of one block: 256 queries of one request and one query head.
@@ -189,10 +218,10 @@ struct Block {
 
 constexpr int kWorkReaders = 11;             // who reads a drawn ticket: the two loader warps, the MMA thread, eight softmax warps
 
-// NS: slices of 64 unrotated key numbers, and of values; ROT: a slice of rotated numbers beside them.
-template <int NS, bool ROT>
+// NS: slices of 64 unrotated key numbers, and of values; a slice of rotated numbers stands beside them.
+template <int NS>
 struct Shape {
-  static constexpr int QS = NS + (ROT ? 1 : 0);           // slices of a query or key
+  static constexpr int QS = NS + 1;                       // slices of a query or key
   static constexpr int KG = QS == 3 ? 1 : QS;             // slices of a key stage
   static constexpr int KRING = QS == 3 ? 4 : 2;           // key stages
   static constexpr int GROUPS = QS / KG;                  // key stages that a tile takes
@@ -201,15 +230,15 @@ struct Shape {
   static constexpr size_t SMEM = 2 * (size_t)QTILE + KRING * (size_t)KSTAGE + kVStages * (size_t)VTILE + 1024;
 };
 
-template <int NS, bool ROT>
+template <int NS>
 __global__ void __launch_bounds__(kThreads, 1) latent_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_r,
     const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out, int out_stride, const int* __restrict__ q_indptr,
     const int* __restrict__ kv_lens, const int2* __restrict__ plan, int nq, int qw, int rank, float scale_log2,
-    const __nv_bfloat16* __restrict__ gate, int gate_stride, int window, int nyb, int nblocks, int ticket_slot, int* __restrict__ err) {
+    const __nv_bfloat16* __restrict__ gate, int gate_stride, int window, int nyb, int nblocks, int ticket_slot, int places, int* __restrict__ err) {
   pdl_launch_dependents();
   pdl_wait();
-  typedef Shape<NS, ROT> S_;
+  typedef Shape<NS> S_;
   constexpr int QS = S_::QS, KG = S_::KG, KRING = S_::KRING, GROUPS = S_::GROUPS, HDV = S_::HDV;
   constexpr uint32_t QTILE = S_::QTILE, KSTAGE = S_::KSTAGE, VTILE = S_::VTILE;
   extern __shared__ unsigned char smem_dyn[];
@@ -249,9 +278,6 @@ __global__ void __launch_bounds__(kThreads, 1) latent_prefill_tc_kernel(
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  // Value rows that no load ever fills (beyond the last key) meet P = 0; they must hold numbers
-  for (uint32_t i = threadIdx.x; i < kVStages * VTILE / 16; i += kThreads) reinterpret_cast<uint4*>(v_s)[i] = make_uint4(0, 0, 0, 0);
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   if (warp == kMmaWarp) {
     tmem_alloc(smem_addr(&tmem_base_slot), 512);
     tmem_relinquish();
@@ -322,7 +348,10 @@ __global__ void __launch_bounds__(kThreads, 1) latent_prefill_tc_kernel(
         bool stop = false;
         for (int j = 0; j < blk.ntiles && !stop; ++j) {
           const int key0 = blk.kb + j * BKV + c * 16;
-          const bool on = sl < slices && key0 <= blk.p_last && key0 + 15 >= blk.lo;
+          const bool seen = key0 <= blk.p_last && key0 + 15 >= blk.lo;
+          // Value rows that no query of the block sees meet P = 0, and zero times what an earlier block left there may be NaN: they are
+          // loaded from behind the last place, which fills them with zeros.
+          const bool on = sl < slices && (seen || !keys);
           const int n = __popc(__ballot_sync(0xffffffffu, on));      // boxes of a stage
           for (int g = 0; g < groups; ++g) {
             const int st = issued % ring;
@@ -344,8 +373,8 @@ __global__ void __launch_bounds__(kThreads, 1) latent_prefill_tc_kernel(
             }
             if (on) {
               const int d = g * KG + sl;                    // the key's slice
-              if (!keys) tma_load_2d(smem_addr(v_s + st * VTILE + sl * SUB + c * 2048), &map_v, blk.h * HDV + sl * 64, blk.at + key0, full);
-              else if (ROT && d == NS) tma_load_2d(smem_addr(k_s + st * KSTAGE + sl * SUB + c * 2048), &map_r, rank, blk.at + key0, full);
+              if (!keys) tma_load_2d(smem_addr(v_s + st * VTILE + sl * SUB + c * 2048), &map_v, blk.h * HDV + sl * 64, seen ? blk.at + key0 : places, full);
+              else if (d == NS) tma_load_2d(smem_addr(k_s + st * KSTAGE + sl * SUB + c * 2048), &map_r, rank, blk.at + key0, full);
               else tma_load_2d(smem_addr(k_s + st * KSTAGE + sl * SUB + c * 2048), &map_k, blk.h * HDV + d * 64, blk.at + key0, full);
             }
             ++issued;
@@ -606,12 +635,12 @@ __global__ void __launch_bounds__(kThreads, 1) latent_prefill_tc_kernel(
   if (threadIdx.x == 0 && abort_flag && err) atomicExch(err, 5);
 }
 
-template <int NS, bool ROT>
+template <int NS>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mr, const CUtensorMap& mv, void* out, int out_stride, const int* q_indptr,
            const int* kv_lens, const int* plan, int nq, int qw, int rank, float scale, const void* gate, int gate_stride, int window, int rows,
-           int max_q_len, int* err, cudaStream_t s) {
-  auto kernel = latent_prefill_tc_kernel<NS, ROT>;
-  constexpr size_t smem = Shape<NS, ROT>::SMEM;
+           int max_q_len, int places, int* err, cudaStream_t s) {
+  auto kernel = latent_prefill_tc_kernel<NS>;
+  constexpr size_t smem = Shape<NS>::SMEM;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -629,7 +658,7 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mr, 
   const int ticket_slot = (int)(launches++ % kTicketSlots);
   cudaError_t e = launch_kernel(kernel, dim3(ctas), dim3(kThreads), smem, s, 1, mq, mk, mr, mv, (__nv_bfloat16*)out, out_stride, q_indptr, kv_lens,
                                 (const int2*)plan, nq, qw, rank, scale * 1.4426950408889634f, (const __nv_bfloat16*)gate, gate_stride, window, nyb,
-                                (int)nblocks, ticket_slot, err);
+                                (int)nblocks, ticket_slot, places, err);
   if (e != cudaSuccess) return (int)e;
   return launch_status();
 }
@@ -643,19 +672,22 @@ ARLE_API int arle_latent_plan(const int* q_indptr, const int* kv_lens, int R, in
   return launch_status();
 }
 
-// cache bfloat16 [pages, 1, page_size, kd]; out [places, kd], places a multiple of 16 and at least what the plan counts.
+// cache bfloat16 [pages, 1, page_size, rank + dr]; out [places, rank + max(dr, 8)], places a multiple of 16 and at least what the plan
+// counts.  rank up to 512, dr up to 64, multiples of 8.
 ARLE_API int arle_latent_gather(const void* cache, const int* block_table, int bt_stride, const int* kv_lens, const int* plan, int R, int page_size,
-                                int kd, void* out, int places, cudaStream_t s) {
+                                int rank, int dr, void* out, int places, cudaStream_t s) {
   if (R <= 0 || places <= 0) return 0;
-  if (page_size % 16 || kd % 8 || places % 16 || ((uintptr_t)cache & 15) || ((uintptr_t)out & 15)) return ARLE_E_UNSUPPORTED;
-  launch_kernel(latent_gather_kernel, dim3(places / 16), dim3(256), 0, s, 1, (const __nv_bfloat16*)cache, block_table, bt_stride, kv_lens,
-                (const int2*)plan, R, page_size, kd, (__nv_bfloat16*)out);
+  if (page_size % 16 || rank <= 0 || rank > 512 || rank % 8 || dr < 0 || dr > 64 || dr % 8 || places % 16 || ((uintptr_t)cache & 15) ||
+      ((uintptr_t)out & 15))
+    return ARLE_E_UNSUPPORTED;
+  launch_kernel(latent_gather_kernel, dim3(places / 16), dim3(kGatherThreads), 0, s, 1, (const __nv_bfloat16*)cache, block_table, bt_stride, kv_lens,
+                (const int2*)plan, R, page_size, rank, rank + dr, rank + gathered_tail(dr), (__nv_bfloat16*)out);
   return launch_status();
 }
 
 // q bfloat16 [num_tokens, heads * (dn + dr)] (any row stride that is a multiple of 8): a head's unrotated numbers, then its rotated ones.
-// keys [places, heads * dn] and values [places, heads * dn] (row stride kv_stride), records [places, rank + dr]: the built arrays and the
-// gathered records of the plan.  out [num_tokens, heads * dn] (row stride out_stride): only the plan's rows are written.
+// keys [places, heads * dn] and values [places, heads * dn] (row stride kv_stride), records [places, rank + max(dr, 8)]: the built arrays
+// and the gathered records of the plan.  out [num_tokens, heads * dn] (row stride out_stride): only the plan's rows are written.
 // dn 64 or 128, dr 0 or a multiple of 8 up to 64.
 ARLE_API int arle_latent_prefill_tc(const void* q, int q_stride, int num_tokens, const void* keys, const void* values, int kv_stride,
                                     const void* records, int places, void* out, int out_stride, const int* q_indptr, const int* kv_lens,
@@ -669,16 +701,11 @@ ARLE_API int arle_latent_prefill_tc(const void* q, int q_stride, int num_tokens,
   int rc = tensor_map_2d_bf16(q, num_tokens, heads * (dn + dr), q_stride, BQ, &mq);
   if (!rc) rc = tensor_map_2d_bf16(keys, places, heads * dn, kv_stride, 16, &mk);
   if (!rc) rc = tensor_map_2d_bf16(values, places, heads * dn, kv_stride, 16, &mv);
-  if (!rc) rc = tensor_map_2d_bf16(records, places, rank + dr, rank + dr, 16, &mr);
+  if (!rc) rc = tensor_map_2d_bf16(records, places, rank + gathered_tail(dr), rank + gathered_tail(dr), 16, &mr);
   if (rc) return rc;
-#define ARLE_LATENT(NS, ROT) \
-  return launch<NS, ROT>(mq, mk, mr, mv, out, out_stride, q_indptr, kv_lens, plan, heads, dn + dr, rank, scale, gate, gate_stride, window, rows, \
-                         max_q_len, err, s)
-  if (dn == 128) {
-    if (dr) ARLE_LATENT(2, true);
-    ARLE_LATENT(2, false);
-  }
-  if (dr) ARLE_LATENT(1, true);
-  ARLE_LATENT(1, false);
-#undef ARLE_LATENT
+  if (dn == 128)
+    return launch<2>(mq, mk, mr, mv, out, out_stride, q_indptr, kv_lens, plan, heads, dn + dr, rank, scale, gate, gate_stride, window, rows, max_q_len,
+                     places, err, s);
+  return launch<1>(mq, mk, mr, mv, out, out_stride, q_indptr, kv_lens, plan, heads, dn + dr, rank, scale, gate, gate_stride, window, rows, max_q_len,
+                   places, err, s);
 }

@@ -92,7 +92,7 @@ _SIGNATURES = {
     "arle_latent_prep": [_P, _I, _P, _I, _I, _P, _P, _P, _F, _P, _I, _I, _F, _P, _P, ctypes.c_long, _I, _I, _I, _I, _I, _I, _I, _P],
     "arle_latent_attention_mma": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _I, _P],
     "arle_latent_plan": [_P, _P, _I, _I, _I, _P, _P],
-    "arle_latent_gather": [_P, _P, _I, _P, _P, _I, _I, _I, _P, _I, _P],
+    "arle_latent_gather": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _P, _I, _P],
     "arle_latent_prefill_tc": [_P, _I, _I, _P, _P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _I, _I, _I, _I, _P, _P],
     "arle_latent_attention": [_P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
     "arle_decay_scan": [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _I, _P],
@@ -1356,9 +1356,9 @@ def latent_prefill(q, out, records, batch, block_table, w_ukv, heads: int, place
         plan = batch.ws.get(f"latent_plan_{window}", (R + 1, 2), torch.int32)
         _check(lib.arle_latent_plan(_ptr(batch.q_indptr), _ptr(batch.kv_lens), R, LATENT_BUILT_LEAST, window, _ptr(plan), s), "latent_plan")
         batch.memo[key] = plan
-    lat = batch.ws.get("latent_gathered", (places, kd), q.dtype)
-    _check(lib.arle_latent_gather(_ptr(records), _ptr(block_table), block_table.stride(0), _ptr(batch.kv_lens), _ptr(plan), R, page_size, kd,
-                                  _ptr(lat), places, s), "latent_gather")
+    lat = batch.ws.get("latent_gathered", (places, rank + (dr or 8)), q.dtype)
+    _check(lib.arle_latent_gather(_ptr(records), _ptr(block_table), block_table.stride(0), _ptr(batch.kv_lens), _ptr(plan), R, page_size, rank,
+                                  dr, _ptr(lat), places, s), "latent_gather")
     width = heads * dn
     group = min(heads, max(T * heads // places, LATENT_BUILT_NUMBERS // (places * dn), 1))
     for h0 in range(0, heads, group):

@@ -1,0 +1,64 @@
+"""An infinity or a NaN stays with the tokens that see it: tokens in front of it, tokens whose window has passed it and other requests of the
+step get what they get without it.  (In the kernels on tiles a masked place is a weight of zero, and zero times infinity is not zero.)"""
+import math
+
+import pytest
+import torch
+
+from arle_b200 import ops
+from arle_b200.cache import CacheManager
+from arle_b200.engine import StepEntry
+from arle_b200.engine.batch import StepContext, Workspace
+from arle_b200.parts.base import CacheNeed, StateNeed
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF = torch.bfloat16
+INF = math.inf
+
+
+def _step(need, lens, dtype, page=16):
+    state = isinstance(need, StateNeed)
+    cm = CacheManager([] if state else [need], [need] if state else [], page, sum(-(-n // page) for n in lens) + 2, len(lens) + 1, 4096, dtype, DEV)
+    for i in range(len(lens)):
+        cm.add_request(i)
+    cm.append([(i, n) for i, n in enumerate(lens)])
+    ctx = StepContext(cm, Workspace(DEV)).build([StepEntry(i, [0] * n) for i, n in enumerate(lens)], [0] * len(lens))
+    return cm, ctx
+
+
+def _slots(cm, lens):
+    return [torch.from_numpy(cm.slot_mapping(0, i, 0, n)).long().to(DEV) for i, n in enumerate(lens)]
+
+
+@pytest.mark.parametrize("dn,dr,rank", [(128, 64, 512), (64, 32, 256), (128, 0, 128), (64, 0, 64)])
+@pytest.mark.parametrize("window", [None, 64])
+def test_latent_prefill(dn, dr, rank, window):
+    heads, kd, lens = 40, rank + dr, [300, 200, 270, 70]          # 320 blocks: a CTA runs several requests' blocks
+    g = torch.Generator(device=DEV).manual_seed(dn + dr)
+    cm, ctx = _step(CacheNeed(streams=((1, kd),), window=window), lens, BF)
+    cm.groups[0].arrays[0].normal_(generator=g)
+    view, slots, T = ctx.cache_view(0), _slots(cm, lens), sum(lens)
+    q = torch.empty(T, heads * (dn + dr), device=DEV, dtype=BF).normal_(generator=g)
+    w = torch.empty(2 * heads * dn, rank, device=DEV, dtype=BF).normal_(0.0, rank ** -0.5, generator=g)
+    places = ops.latent_built_places(ctx, q, dn, dr, dn, rank, 16, window)
+
+    def run():
+        out = torch.empty(T, heads * dn, device=DEV, dtype=BF)
+        ops.latent_prefill(q, out, view.streams[0], ctx, view.block_table, w, heads, places, dr, rank, 16, (dn + dr) ** -0.5, window)
+        return out
+
+    clean = run()
+    flat = view.streams[0].view(-1, kd)
+    flat[slots[0][2:], 3] = INF                                    # all but two tokens of the first request
+    flat[slots[1][100], rank - 1] = math.nan
+    flat[slots[2][150], 0] = -INF
+    hit = torch.zeros(T, dtype=torch.bool, device=DEV)
+    reach = window or T
+    hit[2: 300] = True
+    hit[300 + 100: min(300 + 100 + reach, 500)] = True
+    hit[500 + 150: min(500 + 150 + reach, 770)] = True
+    out = run()
+    assert torch.equal(out[~hit], clean[~hit])
+    assert out[hit].isnan().all()
+    ops.check_errors(DEV)
