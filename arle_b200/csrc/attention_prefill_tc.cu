@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out, const int* __restrict__ q_indptr,
     const int* __restrict__ kv_lens, const int* __restrict__ block_table, int bt_stride, int bt_width, int nq, int nkv,
     int page_size, float scale_log2, HeadTail<__nv_bfloat16> tail, int window, int skip_single, int nyb, int nblocks, int ticket_slot, int* __restrict__ err,
-    int keep_arg, float cap_arg, float scale_over_cap, int chunk_arg, const float* __restrict__ pb) {
+    int keep_arg, float cap_arg, float scale_over_cap, int chunk_arg, const float* __restrict__ pb, int row_behind) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr bool EXT = FORM == 1, SIG = FORM == 2;
@@ -242,10 +242,6 @@ __global__ void __launch_bounds__(kThreads, 1) paged_prefill_tc_kernel(
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  // Value rows that no load ever fills (beyond the last key) meet P = 0; they must hold
-  // numbers, not whatever bits shared memory had (later blocks find an earlier tile's values there).
-  for (uint32_t i = threadIdx.x; i < kStages * TILE / 16; i += kThreads) reinterpret_cast<uint4*>(v_s)[i] = make_uint4(0, 0, 0, 0);
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   if (warp == kMmaWarp) {
     tmem_alloc(smem_addr(&tmem_base_slot), 512);
     tmem_relinquish();
@@ -349,6 +345,9 @@ __global__ void __launch_bounds__(kThreads, 1) paged_prefill_tc_kernel(
             const int page = rel < 32 ? from_cur : from_nxt;
             row = (page * nkv + blk.kvh) * page_size + (key0 - pi * page_size);
           }
+          // Value rows that no query of the block sees meet P = 0, and zero times what another request's tile left there may be NaN: they
+          // are loaded from behind the cache's last row, which fills them with zeros.
+          if (!keys && lane < 16 && row < 0) row = row_behind;
           const int n = __popc(__ballot_sync(0xffffffffu, row >= 0)) >> 1;      // pages of this tile
           uint64_t* full = keys ? &k_full[st] : &v_full[st];
           int go = 1;
@@ -731,7 +730,7 @@ ARLE_API int arle_paged_attention_prefill_tc(const void* q, int q_row_stride, in
                                 q_indptr, kv_lens, block_table, bt_stride, bt_width, nq, nkv, page_size,
                                 scale * 1.4426950408889634f, HeadTail<__nv_bfloat16>{sinks, (const __nv_bfloat16*)gate, gate_stride}, window, skip_single, nyb, (int)nblocks, ticket_slot, err,
                                 window > 0 ? keep_first : 0, softcap > 0.f ? softcap * 1.4426950408889634f : 0.f,
-                                softcap > 0.f ? scale / softcap : 0.f, chunk, pb);
+                                softcap > 0.f ? scale / softcap : 0.f, chunk, pb, (int)(cache_rows < 0x7fffffff ? cache_rows : 0x7fffffff));
   if (e != cudaSuccess) return (int)e;
   return launch_status();
 }

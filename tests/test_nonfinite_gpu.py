@@ -62,3 +62,26 @@ def test_latent_prefill(dn, dr, rank, window):
     assert torch.equal(out[~hit], clean[~hit])
     assert out[hit].isnan().all()
     ops.check_errors(DEV)
+
+
+@pytest.mark.parametrize("window", [None, 32])
+def test_prefill_attention_of_another_request(window):
+    nq, nkv, hd, lens = 32, 8, 128, [600, 600, 600, 70, 300, 33]
+    g = torch.Generator(device=DEV).manual_seed(1)
+    cm, ctx = _step(CacheNeed(nkv, hd, window), lens, BF)
+    for a in cm.groups[0].arrays:
+        a.normal_(generator=g)
+    view, slots, T = ctx.cache_view(0), _slots(cm, lens), sum(lens)
+    q = torch.empty(T, nq * hd, device=DEV, dtype=BF).normal_(generator=g)
+
+    def run():
+        out = torch.empty(T, nq * hd, device=DEV, dtype=BF)
+        ops.paged_attention(q, out, view.k, view.v, ctx.positions, ctx.row_of_token, view.block_table, nq, nkv, hd, 16, hd ** -0.5, window, batch=ctx)
+        return out
+
+    clean = run()
+    for s in slots[:3]:
+        view.v[s // 16, :, s % 16] = INF
+    out = run()
+    assert torch.equal(out[1800:], clean[1800:])
+    ops.check_errors(DEV)
