@@ -4,7 +4,7 @@
 // L2.  Here a block takes 32 queries of a row and one head and walks the visible keys in tiles of 64 (boundaries at multiples of 64 of
 // the key's position), which all its queries share in shared memory: 4 x 4 scores a thread, the softmax's maxima and sums by shuffles
 // over the sixteen lanes of a query, 4 queries x hd / 16 columns of the output a thread.  Scores, softmax, P and all sums are float32
-// (FFMA; P is not rounded).  A masked key's weight is exactly zero, so the order of a token's sums depends on its position and its first
+// (FFMA; P is not rounded).  A masked key's weight is exactly zero and its value is not looked at, so the order of a token's sums depends on its position and its first
 // visible key alone.  Rows with fewer than `least` queries are left alone (the general kernel runs them).
 //
 // The next tile's keys are on their way while P . V is formed, its values while the scores are.  What bounds it: the loads from shared
@@ -132,7 +132,30 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float* __
     __syncthreads();                                       // P is there and the keys are used up
     if (j0 + kKeys <= last) load(ks, k_cache, b ^ 1); else cp_commit();
     cp_wait<1>();                                          // the values are here; the next keys are on their way
-    __syncthreads();
+    // A masked key's weight is zero, and zero times infinity is not: where some query does not see some key of the tile, the threads look
+    // at the values they fetched, and a tile with an infinity or a NaN is added up key by key.
+    const bool whole = j0 + kKeys - 1 <= pos0 && (window <= 0 || j0 >= last - window + 1);
+    bool odd = false;
+    if (!whole) {
+#pragma unroll
+      for (int it = 0; it < kKeys * CH / kThreads; ++it) {
+        const int idx = tid + it * kThreads;
+        const float4 x = *reinterpret_cast<const float4*>(vs + idx / CH * PITCH + idx % CH * 4);
+        odd |= !(fabsf(x.x) < INFINITY && fabsf(x.y) < INFINITY && fabsf(x.z) < INFINITY && fabsf(x.w) < INFINITY);
+      }
+    }
+    if (__syncthreads_or(odd)) {
+#pragma unroll 1
+      for (int j = 0; j < kKeys; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int p = pos0 + ty * 4 + i;
+          if (j0 + j > p || (window > 0 && j0 + j < p - window + 1)) continue;
+          const float w = ps[(ty * 4 + i) * PP + j];
+#pragma unroll
+          for (int c = 0; c < NC * 4; ++c) acc[i][c] = fmaf(w, vs[j * PITCH + (c >> 2) * 64 + tx * 4 + (c & 3)], acc[i][c]);
+        }
+    } else {
 #pragma unroll 4
     for (int j = 0; j < kKeys; j += 4) {
       float4 a[4];
@@ -152,6 +175,7 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float* __
             acc[i][4 * c + 3] = fmaf(p, b.w, acc[i][4 * c + 3]);
           }
         }
+    }
     }
     __syncthreads();                                       // the values are used up
   }

@@ -85,3 +85,34 @@ def test_prefill_attention_of_another_request(window):
     out = run()
     assert torch.equal(out[1800:], clean[1800:])
     ops.check_errors(DEV)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window", [None, 40])
+@pytest.mark.parametrize("lens", [[150, 8], [40, 3, 100]], ids=["150-8", "40-3-100"])
+def test_float32_attention(hd, window, lens):
+    nq, nkv = 4, 2
+    g = torch.Generator(device=DEV).manual_seed(hd)
+    cm, ctx = _step(CacheNeed(nkv, hd, window), lens, torch.float32)
+    for a in cm.groups[0].arrays:
+        a.normal_(generator=g)
+    view, slots, T = ctx.cache_view(0), _slots(cm, lens), sum(lens)
+    q = torch.randn(T, nq * hd, generator=g, device=DEV)
+
+    def run(batch):
+        out = torch.empty(T, nq * hd, device=DEV)
+        ops.paged_attention(q, out, view.k, view.v, ctx.positions, ctx.row_of_token, view.block_table, nq, nkv, hd, 16, hd ** -0.5, window, batch=batch)
+        return out
+
+    clean = run(ctx)
+    s = slots[0][[20, 37]]
+    view.v[s[0] // 16, 0, s[0] % 16, 5] = INF
+    view.v[s[1] // 16, 1, s[1] % 16, 7] = math.nan
+    view.k[s[1] // 16, 1, s[1] % 16, 9] = math.nan
+    out, general = run(ctx), run(None)                             # the general kernel takes a token at a time
+    assert torch.equal(out.isfinite(), general.isfinite())
+    hit = torch.zeros(T, dtype=torch.bool, device=DEV)
+    hit[20: min(lens[0], 37 + window if window else T)] = True
+    assert torch.equal(out[~hit], clean[~hit]) and not out[hit].isfinite().all()
+    same = out.isfinite() & hit[:, None]
+    assert torch.equal(out[same], clean[same])
