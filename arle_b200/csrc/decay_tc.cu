@@ -21,7 +21,7 @@
 // by 0.8e-7 to 1.0e-7 (0.6e-7 to 1.1e-7).
 //
 // What bounds it: the chain of chunks of a block (some 9 us each: the tensor cores' legacy path, a third of the time, then the matrix
-// loads and the barriers between the phases), with one block an SM.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 299 us (the
+// loads and the barriers between the phases), with one block an SM.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 306 us (the
 // scan 1,162), 8 heads of 256 x 513 324 us (1,740 to 1,937 as the scan's mean of both).
 #include "common.cuh"
 #include "mma_utils.cuh"
@@ -51,6 +51,36 @@ __device__ __forceinline__ void mma_add(float (&acc)[4], const uint32_t (&a)[4],
   mma_bf16(t, a, b0, b1);
 #pragma unroll
   for (int i = 0; i < 4; ++i) acc[i] += t[i];
+}
+
+// What the products of a tile of 16 weights (in three parts, as the tensor cores take them) with its values come to, row i of the tile
+// with the values up to i alone.  v: the tile's first value in this lane's first column of o0; o1's columns are eight further on.
+template <int VP>
+__device__ __forceinline__ void add_seen(const uint32_t (&pa)[3][4], const __nv_bfloat16* v, int lane, float (&o0)[4], float (&o1)[4]) {
+  const int row = lane >> 2;
+#pragma unroll
+  for (int reg = 0; reg < 4; ++reg) {                      // rows 0 .. 7 and 8 .. 15 of the weights in turn, keys 8 (reg / 2) ..
+    float w[2] = {0.f, 0.f};
+#pragma unroll
+    for (int i = 2; i >= 0; --i) {
+      const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(&pa[i][reg]);
+      w[0] += __low2float(x), w[1] += __high2float(x);
+    }
+    const int half = reg & 1;
+#pragma unroll 1
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float wj = __shfl_sync(0xffffffffu, w[e], (lane & ~3) | s);
+        const int j = (reg >> 1) * 8 + 2 * s + e;
+        if (j > row + 8 * half) continue;
+        const __nv_bfloat16* x = v + j * VP;
+        o0[2 * half] = fmaf(wj, __bfloat162float(x[0]), o0[2 * half]);
+        o0[2 * half + 1] = fmaf(wj, __bfloat162float(x[1]), o0[2 * half + 1]);
+        o1[2 * half] = fmaf(wj, __bfloat162float(x[8]), o1[2 * half]);
+        o1[2 * half + 1] = fmaf(wj, __bfloat162float(x[9]), o1[2 * half + 1]);
+      }
+  }
 }
 
 template <int DIM, int VT>
@@ -162,11 +192,13 @@ __global__ void __launch_bounds__(kThreads, 1) decay_tc_kernel(
         if (lane >= o) sum += y;
       }
       const double total = __shfl_sync(0xffffffffu, sum, 31);
-      cum[2 * lane] = sum - x[1];
+      double first = __shfl_up_sync(0xffffffffu, sum, 1);  // of the tokens before this lane's: a NaN among the decays stays behind them
+      first = (lane ? first : 0.0) + x[0];
+      cum[2 * lane] = first;
       cum[2 * lane + 1] = sum;
       bs[2 * lane] = lb[0];
       bs[2 * lane + 1] = lb[1];
-      ws[2 * lane] = lb[0] * exp2f((float)(total - (sum - x[1])));
+      ws[2 * lane] = lb[0] * exp2f((float)(total - first));
       ws[2 * lane + 1] = lb[1] * exp2f((float)(total - sum));
       if (t0 + kC < end) gates(t0 + kC);
     }
@@ -192,7 +224,12 @@ __global__ void __launch_bounds__(kThreads, 1) decay_tc_kernel(
 #pragma unroll
       for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(wv + i * L::WV + j * VP + c) = s3[i];
     }
-    if (rt * 16 < n) {
+    // In the rows' own tile a value that comes after a row meets a weight of zero, which an infinity or a NaN survives.  So a warp that
+    // finds one among its sums forms them again, with that tile's products added up value by value.
+    const bool rows_here = rt * 16 < n;
+#pragma unroll 1
+    for (int pass = 0; rows_here && pass < 2; ++pass) {
+      uint32_t own[3][4];                                  // second time: the weights of the rows' own tile
       float sc[8][4], o[NT][4], rest[NT][4];               // rest: from the middle and last parts
 #pragma unroll
       for (int i = 0; i < 8; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
@@ -255,6 +292,11 @@ __global__ void __launch_bounds__(kThreads, 1) decay_tc_kernel(
           split3(w[0], w[1], pa[0][2 * hh], pa[1][2 * hh], pa[2][2 * hh]);
           split3(w[2], w[3], pa[0][2 * hh + 1], pa[1][2 * hh + 1], pa[2][2 * hh + 1]);
         }
+        if (pass && jt == rt) {
+#pragma unroll
+          for (int i = 0; i < 12; ++i) own[i / 4][i % 4] = pa[i / 4][i % 4];
+          break;
+        }
 #pragma unroll
         for (int nt = 0; nt < NT; nt += 2) {
           uint32_t b0, b1, b2, b3;
@@ -268,6 +310,18 @@ __global__ void __launch_bounds__(kThreads, 1) decay_tc_kernel(
           mma_add(o[nt + 1], pa[0], b2, b3);
         }
       }
+      float odd = 0.f;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          o[nt][i] += rest[nt][i];
+          odd = fmaf(o[nt][i], 0.f, odd);
+        }
+      if (pass == 0 && __any_sync(0xffffffffu, odd != odd)) continue;
+      if (pass)
+#pragma unroll
+        for (int nt = 0; nt < NT; nt += 2) add_seen<VP>(own, vs + rt * 16 * VP + n_half + nt * 8 + 2 * t4, lane, o[nt], o[nt + 1]);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -275,9 +329,10 @@ __global__ void __launch_bounds__(kThreads, 1) decay_tc_kernel(
           const int i = i0 + half * 8, c = c0 + n_half + nt * 8 + 2 * t4;
           if (i >= n) continue;
           float* op = out + ((size_t)(t0 + i) * H + h) * vcols + c;
-          if (c < vcols) op[0] = o[nt][2 * half] + rest[nt][2 * half];
-          if (c + 1 < vcols) op[1] = o[nt][2 * half + 1] + rest[nt][2 * half + 1];
+          if (c < vcols) op[0] = o[nt][2 * half];
+          if (c + 1 < vcols) op[1] = o[nt][2 * half + 1];
         }
+      break;
     }
     __syncthreads();                                       // the weighted values are there, S_0's parts are used up
     const float whole = exp2f((float)cum[kC - 1]);

@@ -116,3 +116,36 @@ def test_float32_attention(hd, window, lens):
     assert torch.equal(out[~hit], clean[~hit]) and not out[hit].isfinite().all()
     same = out.isfinite() & hit[:, None]
     assert torch.equal(out[same], clean[same])
+
+
+@pytest.mark.parametrize("dim,vdim,ones", [(64, 64, True), (128, 64, False), (256, 32, False)])
+def test_decay_memories(dim, vdim, ones):
+    H, G, lens, vcols = 4, 2, [130, 70], vdim + int(ones)
+    T = sum(lens)
+    g = torch.Generator(device=DEV).manual_seed(dim)
+    _, ctx = _step(StateNeed((H * vcols * dim,), torch.float32), lens, BF)
+    wide = torch.empty(T, 2 * G * dim + H * vdim, device=DEV, dtype=BF).normal_(generator=g)
+    q, k, v = wide.split([G * dim, G * dim, H * vdim], 1)
+    a = 1 - 0.05 * torch.rand(T, H, generator=g, device=DEV)
+    b = torch.rand(T, H, generator=g, device=DEV)
+    state0 = torch.randn(3, H * vcols * dim, generator=g, device=DEV)
+
+    def run(fn):
+        st, out = state0.clone(), torch.empty(T, H, vcols, device=DEV)
+        if fn is ops.decay_scan:
+            fn(q, k, v, a, b, st, ctx.q_indptr, ctx.state_slots, out, H, G, dim, vdim, ones, 0.3)
+        else:
+            fn(q, k, v, a, b, st, ctx, out, H, G, dim, vdim, ones, 0.3)
+        return out, st
+
+    clean, _ = run(ops.decay_memories)
+    v[70 + 9, 3] = INF                                             # head 0, column 3: inside a tile of 16 tokens
+    k[100, dim] = -INF                                             # the second group's heads, every column
+    a[71, 1] = math.nan                                            # head 1, the second token of a pair
+    b[64, 0] = INF
+    (out, st), (scan, scan_st) = run(ops.decay_memories), run(ops.decay_scan)
+    assert torch.equal(out.isfinite(), scan.isfinite())
+    assert torch.equal(st.isfinite(), scan_st.isfinite())
+    ok = out.isfinite()
+    assert torch.equal(out[:64], clean[:64])
+    assert (out[ok] - scan[ok]).norm() <= 1e-5 * scan[ok].norm()
