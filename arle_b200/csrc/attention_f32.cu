@@ -208,12 +208,9 @@ int launch(const float* q, int q_stride, float* out, const float* k_cache, const
            const int* block_table, int bt_stride, int nq, int nkv, int page_size, float scale, int window, HeadTail<float> tail, int rows,
            int max_q_len, int least, cudaStream_t s) {
   constexpr size_t smem = ((size_t)(kQ + 2 * kKeys) * (HD + 4) + kQ * (kKeys + 4)) * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SharedLimit limit;
+  const cudaError_t raised = limit.raise((const void*)attention_f32_kernel<HD>, smem);
+  if (raised != cudaSuccess) return (int)raised;
   launch_kernel(attention_f32_kernel<HD>, dim3((max_q_len + kQ - 1) / kQ, nq, rows), dim3(kThreads), smem, s, 1, q, q_stride, out, k_cache, v_cache,
                 q_indptr, kv_lens, block_table, bt_stride, nq, nkv, page_size, scale, window, tail, least);
   return launch_status();

@@ -289,12 +289,9 @@ int launch_prefill(const void* q, int q_row_stride, void* out, const void* k_cac
   const size_t smem = (size_t)(4 * kTile) * ROW * sizeof(__nv_bfloat16);
   const int form = pb ? 2 : ((window > 0 && keep_first > 0) || softcap > 0.f) ? 1 : 0;
   auto kernel = form == 2 ? paged_prefill_kernel<HD, 2> : form == 1 ? paged_prefill_kernel<HD, 1> : paged_prefill_kernel<HD, 0>;
-  static bool configured[3] = {false, false, false};
-  if (!configured[form]) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured[form] = true;
-  }
+  static SharedLimit limits[3];
+  const cudaError_t raised = limits[form].raise((const void*)kernel, smem);
+  if (raised != cudaSuccess) return (int)raised;
   dim3 grid((max_q_len + kBlockM - 1) / kBlockM, nq, rows);
   launch_kernel(kernel, dim3(grid), dim3(kThreads), smem, s, 1, 
       (const __nv_bfloat16*)q, q_row_stride, (__nv_bfloat16*)out, (const __nv_bfloat16*)k_cache,

@@ -710,12 +710,9 @@ ARLE_API int arle_paged_attention_prefill_tc(const void* q, int q_row_stride, in
   if (pb ? (keep_first > 0 || softcap > 0.f) : chunk > 0) return ARLE_E_UNSUPPORTED;      // the sigmoid form has neither; only it has chunks
   const int form = pb ? 2 : ((window > 0 && keep_first > 0) || softcap > 0.f) ? 1 : 0;
   auto kernel = form == 2 ? paged_prefill_tc_kernel<2> : form == 1 ? paged_prefill_tc_kernel<1> : paged_prefill_tc_kernel<0>;
-  static bool configured[3] = {false, false, false};
-  if (!configured[form]) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured[form] = true;
-  }
+  static SharedLimit limits[3];
+  const cudaError_t raised = limits[form].raise((const void*)kernel, smem);
+  if (raised != cudaSuccess) return (int)raised;
   // CTAs stay resident and draw blocks (a query head, 256 queries of a request) from a counter, the heaviest first
   const int nyb = (max_q_len + BQ2 - 1) / BQ2;
   const long long nblocks = (long long)nq * nyb * rows;

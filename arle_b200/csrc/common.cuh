@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <utility>
 
 #define ARLE_E_UNSUPPORTED (-2)
@@ -172,6 +173,25 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
                                  int cluster, Args&&... args) {
   return launch_kernel_as((pdl_enabled() & 1) != 0, kernel, grid, block, smem, stream, cluster, std::forward<Args>(args)...);
 }
+
+// A kernel's limit of dynamic shared memory is a setting of the device it runs on, and a process may run models on several: a launcher
+// keeps one of these per kernel and raises the limit once on each device.
+class SharedLimit {
+ public:
+  cudaError_t raise(const void* kernel, size_t bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;       // further devices are set every time
+    if (done_.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) done_.fetch_or(bit, std::memory_order_release);
+    return e;
+  }
+
+ private:
+  std::atomic<uint64_t> done_{0};
+};
 
 inline int launch_status() {
   cudaError_t e = cudaGetLastError();

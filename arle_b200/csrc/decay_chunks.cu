@@ -425,13 +425,10 @@ int launch_as(const void* q, const void* k, const void* v, int q_stride, int k_s
   const dim3 grid((vdim + VT - 1) / VT, H, chunks);
   const size_t smem1 = (size_t)(kC * (DP + kPad) + kC * VT + kC) * sizeof(float);
   const size_t smem3 = (size_t)((2 * kC + VT) * (DP + kPad) + (kC + VT) * (kC + kPad) + kC + 4) * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(chunk_own_kernel<T, DP, VT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_kernel<T, DP, VT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SharedLimit own_limit, out_limit;
+  cudaError_t raised = own_limit.raise((const void*)chunk_own_kernel<T, DP, VT, VEC>, smem1);
+  if (raised == cudaSuccess) raised = out_limit.raise((const void*)chunk_out_kernel<T, DP, VT, VEC>, smem3);
+  if (raised != cudaSuccess) return (int)raised;
   launch_kernel(chunk_own_kernel<T, DP, VT, VEC>, grid, dim3(kThreads), smem1, s, 1, (const T*)k, (const T*)v, (long)k_stride, (long)v_stride, decay,
                 plan, R, st, own, H, dim, vdim);
   const long total = (long)H * vdim * dim;

@@ -398,12 +398,9 @@ template <int DIM, int VT>
 int launch(const void* q, const void* k, const void* v, long q_stride, long k_stride, long v_stride, const float* a, const float* b, float* state,
            long slot_stride, const int* q_indptr, const int* state_slots, float* out, int R, int H, int kq_heads, int vdim, int vcols,
            float q_scale, int longest, cudaStream_t s) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(decay_tc_kernel<DIM, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Layout<DIM, VT>::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SharedLimit limit;
+  const cudaError_t raised = limit.raise((const void*)decay_tc_kernel<DIM, VT>, Layout<DIM, VT>::SMEM);
+  if (raised != cudaSuccess) return (int)raised;
   launch_kernel(decay_tc_kernel<DIM, VT>, dim3((vcols + VT - 1) / VT, H, R), dim3(kThreads), Layout<DIM, VT>::SMEM, s, 1, (const __nv_bfloat16*)q,
                 (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, q_stride, k_stride, v_stride, a, b, state, slot_stride, q_indptr, state_slots, out,
                 H, kq_heads, vdim, vcols, q_scale, longest);

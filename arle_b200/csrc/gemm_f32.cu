@@ -259,12 +259,9 @@ __global__ void __launch_bounds__(kRowsN) gemm_f32_rows_kernel(const float* __re
 template <typename TW, int MR>
 static int launch_rows(const float* A, const TW* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
   constexpr size_t smem = sizeof(TW) * kRowsStages * kRowsN * (kRowsK + 16 / sizeof(TW)) + sizeof(float) * kRowsStages * MR * kRowsK;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<TW, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SharedLimit limit;
+  const cudaError_t raised = limit.raise((const void*)gemm_f32_rows_kernel<TW, MR>, smem);
+  if (raised != cudaSuccess) return (int)raised;
   launch_kernel(gemm_f32_rows_kernel<TW, MR>, dim3((N + kRowsN - 1) / kRowsN), dim3(kRowsN), smem, s, 1, A, W, C, M, N, K, lda, ldw, ldc);
   return launch_status();
 }

@@ -312,12 +312,9 @@ int launch(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, i
   if (rc) return rc;
   const size_t smem = (size_t)STAGES * (BM * BK * 2 + BNH * BK * 2) + 1024;
   auto kern = gemm_tcgen05_pair_kernel<STAGES, GATED, OutT>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SharedLimit limit;
+  const cudaError_t raised = limit.raise((const void*)kern, smem);
+  if (raised != cudaSuccess) return (int)raised;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -641,12 +641,9 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mr, 
            int max_q_len, int places, int* err, cudaStream_t s) {
   auto kernel = latent_prefill_tc_kernel<NS>;
   constexpr size_t smem = Shape<NS>::SMEM;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SharedLimit limit;
+  const cudaError_t raised = limit.raise((const void*)kernel, smem);
+  if (raised != cudaSuccess) return (int)raised;
   const int nyb = (max_q_len + BQ2 - 1) / BQ2;
   const long long nblocks = (long long)nq * nyb * rows;
   if (nblocks > 0x3fffffffLL) return ARLE_E_UNSUPPORTED;

@@ -331,13 +331,9 @@ int launch(const void* x, int ldx, int x_rows, const int* rows, const void* W, v
   if (rc) return rc;
   const size_t smem = (size_t)kStages * STAGE + 1024;
   auto kern = rows ? moe_tcgen05_kernel<FINISH, true> : moe_tcgen05_kernel<FINISH, false>;
-  static bool configured[2] = {false, false};
-  cudaError_t e;
-  if (!configured[rows != nullptr]) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured[rows != nullptr] = true;
-  }
+  static SharedLimit limits[2];
+  cudaError_t e = limits[rows != nullptr].raise((const void*)kern, smem);
+  if (e != cudaSuccess) return (int)e;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
