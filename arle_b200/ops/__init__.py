@@ -639,7 +639,8 @@ def paged_attention(q, out, k_cache, v_cache, positions, row_of_token, block_tab
         return
     least = 0
     if (q.dtype == torch.float32 and batch is not None and _KERNEL_SET == "fast" and vd == hd and hd in (64, 128) and batch.max_q_len >= ATTENTION_F32_LEAST
-            and not (keep_first or softcap or chunk) and score_bias is None and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0):
+            and not (keep_first or softcap or chunk) and score_bias is None and q.stride(0) % 4 == 0 and batch.num_rows <= 65535 and nq <= 65535
+            and all(t.data_ptr() % 16 == 0 for t in (q, out, k_cache, v_cache))):
         least = ATTENTION_F32_LEAST
         _check(library().arle_attention_f32(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(batch.q_indptr), _ptr(batch.kv_lens),
                                             _ptr(block_table), block_table.stride(0), nq, nkv, hd, page_size, float(scale),

@@ -78,3 +78,24 @@ def test_result_does_not_depend_on_the_cutting():
         out = torch.empty(b - a, nq * hd, device=DEV)
         ops.paged_attention(q[a:b].contiguous(), out, view.k, view.v, part.positions, part.row_of_token, view.block_table, *args, 70, batch=part)
         assert torch.equal(out, whole[a:b])
+
+
+@pytest.mark.parametrize("which", ["q", "out", "k", "v"])
+def test_arrays_off_their_boundaries_take_the_general_kernel(which):
+    g = torch.Generator(device=DEV).manual_seed(5)
+    nq, nkv, hd, page, n = 4, 2, 64, 16, 70
+    cm, ctx, view = _setup([(n, 0)], nkv, hd, page, None, g)
+
+    def moved(name, t):                                            # the same numbers one float further on
+        if name != which:
+            return t
+        wide = torch.empty(t.numel() + 1, device=DEV)
+        return wide[1:].view(t.shape).copy_(t)
+
+    q = torch.randn(n, nq * hd, generator=g, device=DEV)
+    k, v = moved("k", view.k.contiguous()), moved("v", view.v.contiguous())
+    out, general = moved("out", torch.empty(n, nq * hd, device=DEV)), torch.empty(n, nq * hd, device=DEV)
+    args = (ctx.positions, ctx.row_of_token, view.block_table, nq, nkv, hd, page, hd ** -0.5, None)
+    ops.paged_attention(moved("q", q), out, k, v, *args, batch=ctx)
+    ops.paged_attention(q, general, view.k, view.v, *args)
+    assert torch.equal(out, general)
