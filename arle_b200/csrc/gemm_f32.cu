@@ -292,7 +292,9 @@ static int launch_f32(const float* A, const void* Wv, float* C, int M, int N, in
     const float b = (float)(((long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn) + 147) / 148) * added;
     return alone * alone * alone + b * b * b;
   };
-  const float c0 = cost(64, 128, 70.f, 53.f), c1 = cost(64, 64, 60.f, 29.f), c2 = cost(32, 64, 39.4f, 20.2f), c3 = cost(32, 32, 37.4f, 11.f);
+  const bool low = M <= 65535 * 32;                        // a grid has room for the rows in tiles of 32
+  const float c0 = cost(64, 128, 70.f, 53.f), c1 = cost(64, 64, 60.f, 29.f), c2 = low ? cost(32, 64, 39.4f, 20.2f) : INFINITY,
+              c3 = low ? cost(32, 32, 37.4f, 11.f) : INFINITY;
   const float best = fminf(fminf(c0, c1), fminf(c2, c3));
   if (best == c0) return launch_tiles<TW, 64, 128, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
   if (best == c1) return launch_tiles<TW, 64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);

@@ -23,3 +23,13 @@ def test_same_bits_as_the_general_kernel(wdtype, M, N, K):
     assert torch.equal(got[:M], want) and (got[M] == 7.0).all()
     exact = x.double() @ w.double().t()
     assert ((got[:M].double() - exact).abs() <= K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())).all()
+
+
+def test_as_many_rows_as_the_general_kernel_takes():
+    M, N, K = 65535 * 32 + 1, 3, 8                                     # one more than a grid of tiles of 32 rows holds
+    g = torch.Generator(device=DEV).manual_seed(1)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    got = torch.empty(M, N, device=DEV)
+    ops.gemm(x, w, got)
+    exact = x.double() @ w.double().t()
+    assert ((got.double() - exact).abs() <= K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())).all()
