@@ -1,7 +1,8 @@
 // General paged causal attention: any head size up to 256, any page size, any
 // number of heads and groups, float32 or bfloat16 storage, float32 arithmetic
 // throughout (scores, softmax, P.V; P is not rounded before P.V).  It serves the
-// 32-bit path of the engine and is the yardstick of the tensor-core kernels.
+// 32-bit path of the engine where attention_f32.cu does not (other head sizes, kept
+// first keys, caps, sigmoid weights) and is the yardstick of the tensor-core kernels.
 //
 // One block per (token, query head).  The query at absolute position p of request
 // row r sees keys j in [max(0, p - window + 1), p] (window <= 0: from 0), found
@@ -32,8 +33,7 @@ __global__ void paged_attention_plain_kernel(const T* __restrict__ q, int q_row_
                                              const int* __restrict__ row_of_token,
                                              const int* __restrict__ block_table, int bt_stride, int nq,
                                              int nkv, int hd, int vd, int page_size, float scale, int window,
-                                             HeadTail<T> tail, int keep_first, float softcap, int chunk, const float* __restrict__ pb,
-                                             const int* __restrict__ q_indptr, int shorter_than) {
+                                             HeadTail<T> tail, int keep_first, float softcap, int chunk, const float* __restrict__ pb) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float qs[256];
@@ -43,9 +43,7 @@ __global__ void paged_attention_plain_kernel(const T* __restrict__ q, int q_row_
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = h / (nq / nkv);
   const int pos = positions[t];
-  const int row = row_of_token[t];
-  if (shorter_than > 0 && q_indptr[row + 1] - q_indptr[row] >= shorter_than) return;      // attention_f32.cu runs the long rows
-  const int* bt = block_table + (size_t)row * bt_stride;
+  const int* bt = block_table + (size_t)row_of_token[t] * bt_stride;
   const int lo = first_visible_key(pos, window, chunk);
   const int ka = min(keep_first, lo);                // kept first keys outside the window
   const int nvis = ka + pos - lo + 1;                // visible keys: index i is key i (i < ka) or key lo + i - ka
@@ -133,7 +131,7 @@ ARLE_API int arle_paged_attention_plain(const void* q, int q_row_stride, void* o
                                         const int* row_of_token, const int* block_table, int bt_stride,
                                         int nq, int nkv, int hd, int vd, int page_size, float scale, int window,
                                         const float* sinks, const void* gate, int gate_stride, int keep_first, float softcap, int chunk, const float* pb,
-                                        int num_tokens, const int* q_indptr, int shorter_than, cudaStream_t s) {
+                                        int num_tokens, cudaStream_t s) {
   if (num_tokens <= 0) return 0;
   if (chunk < 0 || (chunk > 0 && window > 0) || (pb && sinks)) return ARLE_E_BADARG;
   if (vd <= 0 || vd > 256) return ARLE_E_UNSUPPORTED;
@@ -145,12 +143,12 @@ ARLE_API int arle_paged_attention_plain(const void* q, int q_row_stride, void* o
     launch_kernel(paged_attention_plain_kernel<float>, dim3(grid), dim3(kAttnWarps * 32), 0, s, 1, 
         (const float*)q, q_row_stride, (float*)out, (const float*)k_cache, (const float*)v_cache, positions,
         row_of_token, block_table, bt_stride, nq, nkv, hd, vd, page_size, scale, window,
-        HeadTail<float>{sinks, (const float*)gate, gate_stride}, keep_first, softcap, chunk, pb, q_indptr, shorter_than);
+        HeadTail<float>{sinks, (const float*)gate, gate_stride}, keep_first, softcap, chunk, pb);
   else if (dtype == 1)
     launch_kernel(paged_attention_plain_kernel<__nv_bfloat16>, dim3(grid), dim3(kAttnWarps * 32), 0, s, 1, 
         (const __nv_bfloat16*)q, q_row_stride, (__nv_bfloat16*)out, (const __nv_bfloat16*)k_cache,
         (const __nv_bfloat16*)v_cache, positions, row_of_token, block_table, bt_stride, nq, nkv, hd, vd,
-        page_size, scale, window, HeadTail<__nv_bfloat16>{sinks, (const __nv_bfloat16*)gate, gate_stride}, keep_first, softcap, chunk, pb, q_indptr, shorter_than);
+        page_size, scale, window, HeadTail<__nv_bfloat16>{sinks, (const __nv_bfloat16*)gate, gate_stride}, keep_first, softcap, chunk, pb);
   else
     return ARLE_E_BADARG;
   return launch_status();

@@ -54,7 +54,8 @@ _SIGNATURES = {
     "arle_attention_prep": [_P, _I, _I, _P, _P, _P, _P, _F, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     "arle_rotary_angles": [_P, _P, _P, _I, _I, _P],
     "arle_attention_f32": [_P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P, _I, _I, _I, _I, _P],
-    "arle_paged_attention_plain": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P, _I, _I, _F, _I, _P, _I, _P, _I, _P],
+    "arle_paged_attention_plain": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P, _I, _I, _F, _I, _P, _I, _P],
+    "arle_attention_f32_short": [_P, _I, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P, _I, _I, _I, _P],
     "arle_attention_prep_post": [_P, _I, _I, _P, _P, _P, _P, _F, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "arle_branch_norm_add": [_P, _P, _I, _P, _P, _I, _I, _I, _F, _P],
     "arle_branch_norm_add_norm": [_P, _P, _I, _P, _P, _P, _I, _I, _I, _F, _F, _P],
@@ -637,27 +638,31 @@ def paged_attention(q, out, k_cache, v_cache, positions, row_of_token, block_tab
                                    page_size, scale, window, splits, part_o, part_ml, counters, sink=sink, keep_first=keep_first,
                                    softcap=softcap, chunk=chunk, score_bias=score_bias, gate=gate)
         return
-    least = 0
-    if (q.dtype == torch.float32 and batch is not None and _KERNEL_SET == "fast" and vd == hd and hd in (64, 128) and batch.max_q_len >= ATTENTION_F32_LEAST
-            and not (keep_first or softcap or chunk) and score_bias is None and q.stride(0) % 4 == 0 and batch.num_rows <= 65535 and nq <= 65535
+    if (q.dtype == torch.float32 and batch is not None and _KERNEL_SET == "fast" and vd == hd and hd in (64, 128) and not (keep_first or softcap or chunk)
+            and score_bias is None and q.stride(0) % 4 == 0 and batch.num_rows <= 65535 and nq <= 65535
             and all(t.data_ptr() % 16 == 0 for t in (q, out, k_cache, v_cache))):
-        least = ATTENTION_F32_LEAST
-        _check(library().arle_attention_f32(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(batch.q_indptr), _ptr(batch.kv_lens),
-                                            _ptr(block_table), block_table.stride(0), nq, nkv, hd, page_size, float(scale),
-                                            int(window) if window else 0, _ptr(sink), gate_p, gate_stride, batch.num_rows, batch.max_q_len, least,
-                                            _stream()), "attention_f32")
-        if min(batch.q_lens) >= least:
-            return
+        # two kernels with one order of sums: which of them runs a row does not show in its numbers
+        w, least = int(window) if window else 0, ATTENTION_F32_LEAST
+        if batch.max_q_len >= least:
+            _check(library().arle_attention_f32(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(batch.q_indptr), _ptr(batch.kv_lens),
+                                                _ptr(block_table), block_table.stride(0), nq, nkv, hd, page_size, float(scale), w, _ptr(sink), gate_p,
+                                                gate_stride, batch.num_rows, batch.max_q_len, least, _stream()), "attention_f32")
+        if min(batch.q_lens) < least:
+            _check(library().arle_attention_f32_short(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(batch.q_indptr),
+                                                      _ptr(positions), _ptr(row_of_token), _ptr(block_table), block_table.stride(0), nq, nkv, hd,
+                                                      page_size, float(scale), w, _ptr(sink), gate_p, gate_stride, T,
+                                                      least if batch.max_q_len >= least else 0, _stream()), "attention_f32_short")
+        return
     _check(library().arle_paged_attention_plain(
         _ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _dt(q), _ptr(positions), _ptr(row_of_token),
         _ptr(block_table), block_table.stride(0), nq, nkv, hd, vd, page_size, float(scale),
         int(window) if window else 0, _ptr(sink), gate_p, gate_stride, keep_first, float(softcap or 0.0), chunk,
-        _ptr(score_bias), T, _ptr(batch.q_indptr) if least else None, least, _stream()),
+        _ptr(score_bias), T, _stream()),
         "paged_attention")
 
 
-# Queries of a float32 row from which it runs on the tiles (attention_f32.cu has the figures): a tile has room for 32, so rows of fewer
-# than 8 win there only while they are few, and many of them fill the machine better as a block a token.
+# Queries of a float32 row from which it runs on the tiles.  A tile has room for 32, so the form by queries is the faster one for a single row
+# of 8 (29 and 60 us behind 512 tokens, 16 heads of 128); the tiles are for many queries (301: 48 us).  The bits are the same.
 ATTENTION_F32_LEAST = 8
 
 

@@ -1,6 +1,6 @@
 """The float32 attention on tiles against float64: rows just below and at the least length, at and past a tile of 32 queries and 64 keys,
 behind contexts, windows shorter and longer than a tile, grouped heads, sinks larger and smaller than the scores, gates, pages that no tile
-boundary falls on; and a token's result does not depend on how its prompt was cut."""
+boundary falls on; and a token's bits do not depend on how its prompt was cut, into single tokens, short rows or long ones."""
 import math
 
 import pytest
@@ -63,21 +63,30 @@ def test_against_float64(nq, nkv, hd, page, rows, window, tail):
         at += n
 
 
-def test_result_does_not_depend_on_the_cutting():
+@pytest.mark.parametrize("window", [None, 70, 1])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("tail", [False, True])
+def test_result_does_not_depend_on_the_cutting(window, hd, tail):
     g = torch.Generator(device=DEV).manual_seed(3)
-    nq, nkv, hd, page, n = 4, 2, 128, 16, 150
+    nq, nkv, page, n = 4, 2, 16, 330
     cm, ctx, view = _setup([(n, 0)], nkv, hd, page, None, g)
     q = torch.randn(n, nq * hd, generator=g, device=DEV)
-    args = (nq, nkv, hd, page, hd ** -0.5)
-    whole = torch.empty(n, nq * hd, device=DEV)
-    ops.paged_attention(q, whole, view.k, view.v, ctx.positions, ctx.row_of_token, view.block_table, *args, 70, batch=ctx)
-    for a, b in ((0, 41), (41, 75), (75, 150)):
+    sink = torch.linspace(-3.0, 9.0, nq, device=DEV) if tail else None
+    gate = torch.randn(n, nq, generator=g, device=DEV) if tail else None
+
+    def run(a, b, c):
+        out = torch.empty(b - a, nq * hd, device=DEV)
+        ops.paged_attention(q[a:b].contiguous(), out, view.k, view.v, c.positions, c.row_of_token, view.block_table, nq, nkv, hd, page, hd ** -0.5,
+                            window, batch=c, sink=sink, gate=gate[a:b] if tail else None)
+        return out
+
+    whole = run(0, n, ctx)
+    ends = [1, 8, 15, 41, 42, 75, 83, 150, 157, 200, 201, 208, 320, 327, n]      # portions of 1 and 7 tokens, of 8 and more
+    for a, b in list(zip([0] + ends, ends)) + [(p, p + 1) for p in (256, 255, 192, 191, 128, 127, 64, 63)]:
         cm.truncate(0, a)
         cm.append([(0, b - a)])
         part = StepContext(cm, Workspace(DEV)).build([StepEntry(0, [0] * (b - a))], [a])
-        out = torch.empty(b - a, nq * hd, device=DEV)
-        ops.paged_attention(q[a:b].contiguous(), out, view.k, view.v, part.positions, part.row_of_token, view.block_table, *args, 70, batch=part)
-        assert torch.equal(out, whole[a:b])
+        assert torch.equal(run(a, b, part), whole[a:b]), (a, b)
 
 
 @pytest.mark.parametrize("which", ["q", "out", "k", "v"])
