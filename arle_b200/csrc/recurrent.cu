@@ -14,7 +14,8 @@
 //    the lanes add their parts of o_t by shuffles; a thread holds one column, or four that share its loads of k and q.
 //    q, k, b v and a of 16 tokens are staged in shared memory, then the 16 steps run from there, while the next 16 tokens'
 //    numbers are already on their way into registers.  The split of a column depends on dim alone, so a token's sums have one order
-//    whatever the cutting or the batch.
+//    whatever the cutting or the batch, as long as the scan runs it: bfloat16 rows of more than 32 tokens take decay_tc.cu, whose
+//    chunks are counted from the row's first token in the step (or, with constant decays, decay_chunks.cu).
 //  * mlstm_gates: the log gates of the matrix LSTM (soft-capped), its running maximum m (carried in the state),
 //    and from them a_t, b_t and exp(-m_t); the gates of 128 tokens are evaluated side by side, the maximum runs
 //    through them in order.

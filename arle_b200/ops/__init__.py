@@ -1448,16 +1448,12 @@ def decay_tc_takes(q, k, v, dim: int, vdim: int, ones_column: bool, max_q_len: i
 
 def decay_memories(q, k, v, a, b, state, batch, out, heads: int, kq_heads: int, dim: int, vdim: int, ones_column: bool, q_scale: float) -> None:
     """``decay_scan`` for decays a in [0, 1] (float32 [T, heads], as the mixers' gates make them): rows of more than DECAY_TC_LONGEST tokens run
-    in chunks of 64 tokens on the tensor cores where ``decay_tc_takes`` allows it, the others on the scan."""
+    in chunks of 64 tokens on the tensor cores where ``decay_tc_takes`` allows it, the others on the scan.  A row's own length decides, so its
+    numbers do not depend on the step's other rows."""
     chunks = decay_tc_takes(q, k, v, dim, vdim, ones_column, batch.max_q_len)
-    longest = DECAY_TC_LONGEST
-    if chunks:
-        short = sum(n <= longest for n in batch.q_lens)
-        if short * heads * -(-vdim // 64) <= 148:       # none, or so few that they run beside the long ones without a launch of their own
-            longest = 0
-    if not chunks or longest:
+    if not chunks or min(batch.q_lens) <= DECAY_TC_LONGEST:
         decay_scan(q, k, v, a, b, state, batch.q_indptr, batch.state_slots, out, heads, kq_heads, dim, vdim, ones_column, q_scale,
-                   **({"longest": longest} if chunks else {}))
+                   **({"longest": DECAY_TC_LONGEST} if chunks else {}))
     if not chunks:
         return
     T, vcols = v.shape[0], vdim + int(bool(ones_column))
@@ -1473,7 +1469,7 @@ def decay_memories(q, k, v, a, b, state, batch, out, heads: int, kq_heads: int, 
         raise KernelError("decay_memories: out must be contiguous float32 [T, heads, vcols]")
     _check(library().arle_decay_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(a), _ptr(b), _ptr(state), state.stride(0),
                                    _ptr(batch.q_indptr), _ptr(batch.state_slots), _ptr(out), batch.num_rows, heads, kq_heads, dim, vdim, vcols,
-                                   float(q_scale), longest, _stream()), "decay_tc")
+                                   float(q_scale), DECAY_TC_LONGEST, _stream()), "decay_tc")
 
 
 DECAY_CHUNK = 64                    # tokens of a chunk

@@ -23,7 +23,9 @@ def _ctx(lens, width, starts=None):
 
 
 @pytest.mark.parametrize("dim,vdim,ones,H,G", [(64, 64, True, 4, 2), (64, 40, False, 3, 3), (128, 64, False, 8, 2), (128, 200, False, 2, 1),
-                                               (128, 128, True, 2, 2), (256, 64, True, 2, 1), (256, 32, False, 3, 3), (128, 64, False, 80, 8)])
+                                               (128, 128, True, 2, 2), (256, 64, True, 2, 1), (256, 32, False, 3, 3), (128, 64, False, 80, 8),
+                                               # tiles of 64 columns: more than 74 blocks of them
+                                               (64, 64, True, 40, 8), (64, 200, False, 20, 4), (128, 128, True, 32, 32)])
 @pytest.mark.parametrize("lens", [[33], [64, 5, 65], [200, 1, 32, 128]], ids=["33", "64-5-65", "200-1-32-128"])
 @pytest.mark.parametrize("kind", ["slow", "wild"])
 def test_against_float64(dim, vdim, ones, H, G, lens, kind):
@@ -63,3 +65,30 @@ def test_against_float64(dim, vdim, ones, H, G, lens, kind):
         # no further from float64 than the scan by more than the order of the sums explains (both 24-bit sums of the same terms)
         assert mine.norm() <= 1.5 * theirs.norm() + 2.0 ** -22 * ref.norm()
         assert mine.abs().max() <= 4 * theirs.abs().max() + 2.0 ** -20 * ref.abs().max()
+
+
+@pytest.mark.parametrize("dim,vdim,ones,H,G", [(64, 64, True, 8, 8), (128, 64, False, 40, 8), (256, 64, True, 8, 2)])
+def test_a_row_does_not_depend_on_the_others(dim, vdim, ones, H, G):
+    """One row alone runs tiles of 32 columns, several together tiles of 64; a short row takes the scan either way."""
+    g = torch.Generator(device=DEV).manual_seed(dim)
+    lens, vcols = [33, 7, 200, 1, 32, 64, 90], vdim + int(ones)
+    T, width = sum(lens), H * vcols * dim
+    wide = torch.randn(T, 2 * G * dim + H * vdim, generator=g, device=DEV).to(torch.bfloat16)
+    a, b = 1 - 0.02 * torch.rand(T, H, generator=g, device=DEV), torch.rand(T, H, generator=g, device=DEV)
+    state0 = torch.randn(len(lens) + 1, width, generator=g, device=DEV)
+
+    def run(ctx, lo, hi, state):
+        q, k, v = wide[lo:hi].split([G * dim, G * dim, H * vdim], 1)
+        out = torch.empty(hi - lo, H, vcols, device=DEV)
+        ops.decay_memories(q, k, v, a[lo:hi].contiguous(), b[lo:hi].contiguous(), state, ctx, out, H, G, dim, vdim, ones, 0.3)
+        return out
+
+    ctx, state = _ctx(lens, width), state0.clone()
+    whole, at = run(ctx, 0, T, state), 0
+    for r, n in enumerate(lens):
+        one, slot = _ctx([n], width), int(ctx.state_slots[r])
+        st = torch.zeros(2, width, device=DEV)
+        st[int(one.state_slots[0])] = state0[slot]
+        assert torch.equal(run(one, at, at + n, st), whole[at: at + n])
+        assert torch.equal(st[int(one.state_slots[0])], state[slot])
+        at += n
