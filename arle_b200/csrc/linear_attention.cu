@@ -102,10 +102,19 @@ template <> struct Raw4<__nv_bfloat16, true> { using type = uint2; };
 // alpha that a thread reads from shared memory serves four columns: with one column a thread the kernel was bound by
 // shared-memory bandwidth.
 // BONUS: the read-out before the update, with the current token weighted by u.
-// GROUPS: some row has eight tokens or more; the form without them, for decoded tokens, is bound by memory and holds few enough registers
-// for five blocks an SM.
-template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool GROUPS>
-__global__ void __launch_bounds__(kScanThreads, DPT == 4 && !GROUPS && !BONUS ? 5 : 1) gla_scan_kernel(
+// LONG: some row has eight tokens or more; with 32 lanes a column these run in groups of eight.  The form for shorter rows, decoded tokens
+// above all, is bound by memory: single numbers instead of pairs, which leaves room for few_blocks() blocks an SM (the most that no form
+// spills for), and loads that the compiler may place.  64 requests, 16 heads of 128 x 128: 30.9 us (31.1 with pairs), 64 heads 129.5
+// (132).  The same cap on prompts of small heads spilled: 512 tokens, bfloat16, 16 heads of 4 258 us with it and 76 without.
+template <typename T, int DPT, int LPC, bool VEC, bool BONUS>
+constexpr int few_blocks() {
+  if (DPT > 8) return BONUS ? 2 : 3;
+  if (DPT > 4) return 4;
+  if (LPC == 1) return 3;
+  return VEC && !BONUS && LPC >= 4 ? 5 : 4;
+}
+template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool LONG>
+__global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LPC, VEC, BONUS>()) gla_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int in_stride,
     const float* __restrict__ alpha, const float* __restrict__ bonus, float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
     const int* __restrict__ state_slots, float* __restrict__ out, int heads, int dim, int vdim, float q_scale) {
@@ -121,7 +130,7 @@ __global__ void __launch_bounds__(kScanThreads, DPT == 4 && !GROUPS && !BONUS ? 
   constexpr int QPT = (QUADS + kScanThreads - 1) / kScanThreads;
   constexpr int VPT = (CHUNK * COLS + kScanThreads - 1) / kScanThreads;
   __shared__ __align__(16) float qs[CHUNK * DPAD], ks[CHUNK * DPAD], as[CHUNK * DPAD];
-  constexpr int VD = LPC >= 4 ? 2 : 1;           // v's numbers stand twice side by side (a factor of both halves of a pair), where there is room
+  constexpr int VD = LONG && LPC >= 4 ? 2 : 1;           // v's numbers stand twice side by side (a factor of both halves of a pair), where there is room
   __shared__ __align__(16) float vs[CHUNK * COLS * VD];
   const int r = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * COLS;
   const int l = threadIdx.x & (LPC - 1), jl = threadIdx.x / LPC;
@@ -175,9 +184,15 @@ __global__ void __launch_bounds__(kScanThreads, DPT == 4 && !GROUPS && !BONUS ? 
       const size_t row = ok ? (size_t)(t0 + tt) : (size_t)t_begin;
       const int cs = ok ? c : 0;
       if constexpr (VEC) {
-        rq[u] = load_now(q + row * in_stride + hq + cs, RawT());
-        rk[u] = load_now(k + row * in_stride + hq + cs, RawT());
-        ra[u] = load_now(alpha + row * a_stride + hq + cs, float4());
+        if constexpr (LONG) {
+          rq[u] = load_now(q + row * in_stride + hq + cs, RawT());
+          rk[u] = load_now(k + row * in_stride + hq + cs, RawT());
+          ra[u] = load_now(alpha + row * a_stride + hq + cs, float4());
+        } else {
+          rq[u] = load_raw4(q + row * in_stride + hq + cs);
+          rk[u] = load_raw4(k + row * in_stride + hq + cs);
+          ra[u] = load_raw4(alpha + row * a_stride + hq + cs);
+        }
       } else {
         float4 fq = make_float4(0.f, 0.f, 0.f, 0.f), fk = fq, fa = fq;
         float* pq = &fq.x; float* pk = &fk.x; float* pa = &fa.x;
@@ -198,7 +213,9 @@ __global__ void __launch_bounds__(kScanThreads, DPT == 4 && !GROUPS && !BONUS ? 
       const int idx = threadIdx.x + u * kScanThreads;
       const int tt = idx / COLS, c = idx - tt * COLS;
       const bool ok = idx < CHUNK * COLS && tt < n && j0 + c < vdim;
-      rv[u] = load_now(v + (ok ? (size_t)(t0 + tt) : (size_t)t_begin) * in_stride + hv + (ok ? j0 + c : 0), T());
+      const T* vp = v + (ok ? (size_t)(t0 + tt) : (size_t)t_begin) * in_stride + hv + (ok ? j0 + c : 0);
+      if constexpr (LONG) rv[u] = load_now(vp, T());
+      else rv[u] = *vp;
     }
   };
   auto stage = [&](int n) {                      // registers to shared memory, widened, q scaled on the way
@@ -236,6 +253,37 @@ __global__ void __launch_bounds__(kScanThreads, DPT == 4 && !GROUPS && !BONUS ? 
     if (t0 + CHUNK < t_end) fetch(t0 + CHUNK, min(CHUNK, t_end - t0 - CHUNK));
     // one token: the memory's step and the thread's part of its columns' sums
     auto token = [&](int tt, float (&o)[CPT]) {
+      if constexpr (!LONG) {                     // single numbers: the same roundings in fewer registers
+        const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT);
+        const float vj[CPT] = {v4.x, v4.y, v4.z, v4.w};
+        const float4* qt = reinterpret_cast<const float4*>(qs + tt * DPAD + l * PAD);
+        const float4* kt = reinterpret_cast<const float4*>(ks + tt * DPAD + l * PAD);
+        const float4* at = reinterpret_cast<const float4*>(as + tt * DPAD + l * PAD);
+        float lo[CPT], hi[CPT];
+#pragma unroll
+        for (int cc = 0; cc < CPT; ++cc) lo[cc] = hi[cc] = 0.f;
+#pragma unroll
+        for (int i = 0; i < DPT / 4; ++i) {
+          const float4 a4 = at[i], k4 = kt[i], q4 = qt[i];
+#pragma unroll
+          for (int cc = 0; cc < CPT; ++cc) {
+            const float s0 = low2(S[cc][2 * i]), s1 = high2(S[cc][2 * i]), s2 = low2(S[cc][2 * i + 1]), s3 = high2(S[cc][2 * i + 1]);
+            const float x0 = k4.x * vj[cc], x1 = k4.y * vj[cc], x2 = k4.z * vj[cc], x3 = k4.w * vj[cc];
+            const float n0 = fmaf(a4.x, s0, x0), n1 = fmaf(a4.y, s1, x1), n2 = fmaf(a4.z, s2, x2), n3 = fmaf(a4.w, s3, x3);
+            S[cc][2 * i] = pair2(n0, n1), S[cc][2 * i + 1] = pair2(n2, n3);
+            if constexpr (BONUS) {
+              lo[cc] = fmaf(fmaf(low2(u2[2 * i + 1]), x2, s2), q4.z, fmaf(fmaf(low2(u2[2 * i]), x0, s0), q4.x, lo[cc]));
+              hi[cc] = fmaf(fmaf(high2(u2[2 * i + 1]), x3, s3), q4.w, fmaf(fmaf(high2(u2[2 * i]), x1, s1), q4.y, hi[cc]));
+            } else {
+              lo[cc] = fmaf(n2, q4.z, fmaf(n0, q4.x, lo[cc]));
+              hi[cc] = fmaf(n3, q4.w, fmaf(n1, q4.y, hi[cc]));
+            }
+          }
+        }
+#pragma unroll
+        for (int cc = 0; cc < CPT; ++cc) o[cc] = lo[cc] + hi[cc];
+        return;
+      }
       f32x2 vj[CPT];
       if constexpr (VD == 2) {
         const ulonglong2 va = *reinterpret_cast<const ulonglong2*>(vs + (tt * COLS + jl * CPT) * 2);
@@ -273,7 +321,7 @@ __global__ void __launch_bounds__(kScanThreads, DPT == 4 && !GROUPS && !BONUS ? 
       for (int cc = 0; cc < CPT; ++cc) o[cc] = low2(o2[cc]) + high2(o2[cc]);
     };
     int first = 0;
-    if constexpr (GROUPS && LPC == 32 && CHUNK % 8 == 0) {
+    if constexpr (LONG && LPC == 32 && CHUNK % 8 == 0) {
       // Eight tokens at a time: their 32 sums over 32 lanes in 31 exchanges, after which lane l holds token l / 4's sum of column
       // l % 4.  A sum's additions are those of a token by itself (lanes 16 apart, then 8, 4, 2, 1).
       for (; first + 8 <= n; first += 8) {
@@ -297,6 +345,8 @@ __global__ void __launch_bounds__(kScanThreads, DPT == 4 && !GROUPS && !BONUS ? 
         if (jb + (l & 3) < vdim) out[(size_t)(t0 + first + (l >> 2)) * heads * vdim + hv + jb + (l & 3)] = x[0];
       }
     }
+    constexpr int kUnroll = LPC < 32 ? 4 : 1;    // 32 lanes: at most seven tokens come here; fewer: all (f32 heads of 64, 512 tokens: 91 -> 86 us)
+#pragma unroll kUnroll
     for (int tt = first; tt < n; ++tt) {
       float o[CPT];
       token(tt, o);
@@ -446,10 +496,8 @@ int scan_launch(const void* q, const void* k, const void* v, int in_stride, cons
   const size_t eb = sizeof(T) * 4;               // bytes of four elements of q or k
   const bool vec = dim % 4 == 0 && in_stride % 4 == 0 && ((uintptr_t)q % eb) == 0 && ((uintptr_t)k % eb) == 0 &&
                    ((uintptr_t)alpha % 16) == 0;
-  constexpr bool G = LPC == 32;
-  const bool groups = G && max_q_len >= 8;
-  auto kernel = groups ? (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, G> : gla_scan_kernel<T, DPT, LPC, false, true, G>)
-                                : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, G> : gla_scan_kernel<T, DPT, LPC, false, false, G>))
+  auto kernel = max_q_len >= 8 ? (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, true> : gla_scan_kernel<T, DPT, LPC, false, true, true>)
+                                        : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, true> : gla_scan_kernel<T, DPT, LPC, false, false, true>))
                        : (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, false> : gla_scan_kernel<T, DPT, LPC, false, true, false>)
                                 : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, false> : gla_scan_kernel<T, DPT, LPC, false, false, false>));
   launch_kernel(kernel, grid, dim3(kScanThreads), 0, s, 1, (const T*)q, (const T*)k, (const T*)v, in_stride, alpha, bonus, state, slot_stride,
