@@ -125,7 +125,8 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
   constexpr int DSPAN = DPT * LPC;               // dim rounded up; channels past dim hold zeros
   constexpr int PAD = DPT == 4 ? 4 : DPT + 4;    // floats a thread's channels take in shared memory: 16-byte rows, spread over the banks
   constexpr int DPAD = PAD * LPC;
-  constexpr int CHUNK = DSPAN >= 512 ? 4 : (DSPAN >= 256 ? 8 : 16);
+  // float32 rows with a bonus, decoded: at 16 tokens a chunk the numbers under way spill at four blocks an SM
+  constexpr int CHUNK = DSPAN >= 512 ? 4 : (DSPAN >= 256 || (!LONG && BONUS && sizeof(T) == 4) ? 8 : 16);
   constexpr int QUADS = CHUNK * DSPAN / 4;       // groups of four channels in a chunk
   constexpr int QPT = (QUADS + kScanThreads - 1) / kScanThreads;
   constexpr int VPT = (CHUNK * COLS + kScanThreads - 1) / kScanThreads;
