@@ -16,11 +16,13 @@
 //    round, and since S^T q = g S_old^T q + u (k . q) the read-out needs no second round.  16 tokens are staged in shared
 //    memory at a time as they are; their unit lengths are three sums a token (q . q, k . k, q . k) and enter as factors
 //    of the two products and of u.  Eight lanes a column (sixteen numbers a lane at dim 128) cost a third of the
-//    instructions of thirty-two lanes with four numbers.  Two numbers are one packed instruction (the same roundings), and the next
-//    chunk's q, k and v are on their way into registers while a chunk's tokens run.  What bounds a long row is the chain of a token: loads
-//    from shared memory, four dependent FMAs, three exchanges, the correction and the update, some 550 cycles.  Rows of 479, 701 and 819
-//    tokens, 32 heads of 128 x 128: 570 us (single numbers, loads waited for at each chunk: 633 to 680); one row of 2,048, 8 heads: 581 (710).  The split of a column depends on dim alone, so a token's sums
-//    have one order whatever the cutting or the batch.
+//    instructions of thirty-two lanes with four numbers.  Two numbers are one packed instruction (the same roundings), and in the form
+//    for long rows (AHEAD, see launch_delta for where) the next chunk's q, k and v are on their way into registers while a chunk's tokens
+//    run.  What bounds one long row is the chain of a token: loads from shared memory, four dependent FMAs, three exchanges, the correction
+//    and the update, some 480 cycles.  Several rows also wait for a place: blocks of 128 or 256 threads, two a SM, taken in the order of the
+//    rows.  One row of 2,048 tokens, 8 heads of 128 x 128: 511 us (single numbers, loads waited for at each chunk: 682); 32 heads 652 (805);
+//    rows of 479, 701 and 819 tokens, 32 heads: 549 (612).  The split of a column depends on dim alone, so a token's sums have one order
+//    whatever the cutting or the batch.
 #include "common.cuh"
 #include "scan_utils.cuh"
 using namespace arle;
@@ -56,12 +58,12 @@ constexpr int kDeltaChunk = 16;
 
 // LONG: the step has rows of many tokens (a chunk's loads asked for at once, a full chunk's tokens unrolled); without it the
 // kernel is the short form for steps of single tokens, which needs fewer registers.
-template <typename T, int EPL, int LPC, bool LONG>
-__global__ void __launch_bounds__(256) delta_scan_kernel(
+template <typename T, int EPL, int LPC, bool LONG, bool AHEAD>
+__global__ void __launch_bounds__(256, LONG && !AHEAD && sizeof(T) == 4 && EPL == 32 ? 2 : 0 /* left to the compiler */) delta_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int q_stride, int k_stride, int v_stride,
     const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ state, long slot_stride,
     const int* __restrict__ q_indptr, const int* __restrict__ state_slots, float* __restrict__ out, int H, int kq_heads, int dim,
-    int vdim, float q_scale, float unit_eps, int ahead) {
+    int vdim, float q_scale, float unit_eps) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
@@ -105,8 +107,8 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
 
   // `ahead` (rows of q and k in whole 16-byte pieces): the next chunk's numbers are on their way into registers while this one's
   // tokens run.  Places past the row's end read its first token and are zeroed when staged.
-  constexpr int PER = 16 / sizeof(T), PIECES = kDeltaChunk * DPAD / PER, MAXP = LONG ? (PIECES + 127) / 128 : 1;
-  constexpr int VPT = LONG ? (kDeltaChunk + LPC - 1) / LPC : 1;
+  constexpr int PER = 16 / sizeof(T), PIECES = kDeltaChunk * DPAD / PER, MAXP = AHEAD ? (PIECES + 127) / 128 : 1;
+  constexpr int VPT = AHEAD ? (kDeltaChunk + LPC - 1) / LPC : 1;
   uint4 rq[MAXP], rk[MAXP];
   T rv[VPT];
   float rg = 0.f, rb = 0.f;
@@ -132,11 +134,11 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
       rb = load_now(beta + t * H + h, 0.f);
     }
   };
-  if (LONG && ahead && beg < end) fetch(beg);
+  if (AHEAD && beg < end) fetch(beg);
   for (int t0 = beg; t0 < end; t0 += kDeltaChunk) {
     const int n = min(kDeltaChunk, end - t0);
     __syncthreads();
-    if (LONG && ahead) {
+    if constexpr (AHEAD) {
 #pragma unroll
       for (int u = 0; u < MAXP; ++u) {
         const int idx = threadIdx.x + u * nthreads, tt = idx / (DPAD / PER), e = idx % (DPAD / PER) * PER;
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
     }
     }
     __syncthreads();
-    if (LONG && ahead && t0 + kDeltaChunk < end) fetch(t0 + kDeltaChunk);
+    if (AHEAD && t0 + kDeltaChunk < end) fetch(t0 + kDeltaChunk);
     {
       float sq = 0.f, sk = 0.f, qk = 0.f;
       if (stt < n)
@@ -280,7 +282,7 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(
 template <typename T, int EPL, int LPC, bool LONG>
 static int launch_delta(const void* q, const void* k, const void* v, int q_stride, int k_stride, int v_stride, const float* beta,
                         const float* decay, float* state, long slot_stride, const int* q_indptr, const int* state_slots, float* out,
-                        int R, int H, int kq_heads, int dim, int vdim, float q_scale, float unit_eps, cudaStream_t s) {
+                        int R, int H, int kq_heads, int dim, int vdim, float q_scale, float unit_eps, int num_tokens, cudaStream_t s) {
   // 128 threads a block while the step's blocks are few; twice the columns share the staging of a head's q and k once the
   // SMs are full
   int threads = 128;
@@ -288,15 +290,23 @@ static int launch_delta(const void* q, const void* k, const void* v, int q_strid
   const int cpb = threads / LPC;
   const size_t smem = ((size_t)2 * kDeltaChunk * (LPC * EPL + 4) + (size_t)kDeltaChunk * cpb + 5 * kDeltaChunk + 3 * 8 * kDeltaChunk) * sizeof(float);
   if (smem > 200 * 1024) return ARLE_E_UNSUPPORTED;
+  const int per = 16 / (int)sizeof(T);
+  // The next chunk's numbers ahead: where some row has several chunks, as far as the counts tell (16 rows of 4 tokens, 32 heads of 64: 21 us
+  // without and 26 with), and not at the price of a block an SM.  float32 heads of 512 would take 244 registers instead of 123, heads of 256
+  // 254 instead of 128: those only while all blocks are resident all the same (16 heads of 256, one row of 512: 252 us and 321 without; 16
+  // rows of 128: 903 and 813).
+  constexpr bool kMay = LONG && !(sizeof(T) == 4 && EPL * LPC == 512), kWide = sizeof(T) == 4 && EPL == 32;
+  const long blocks = (long)((vdim + cpb - 1) / cpb) * H * R;
+  const bool ahead = (num_tokens >= 8L * R || num_tokens - R >= 8 * kDeltaChunk) && (!kWide || blocks * threads <= 148L * 256) && dim % per == 0 && q_stride % per == 0 &&
+                     k_stride % per == 0 && (((uintptr_t)q | (uintptr_t)k) & 15) == 0;
+  auto kernel = kMay && ahead ? delta_scan_kernel<T, EPL, LPC, LONG, kMay> : delta_scan_kernel<T, EPL, LPC, LONG, false>;
   if (smem > 40 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<T, EPL, LPC, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  const int per = 16 / (int)sizeof(T);
-  const int ahead = dim % per == 0 && q_stride % per == 0 && k_stride % per == 0 && (((uintptr_t)q | (uintptr_t)k) & 15) == 0;
   dim3 grid((vdim + cpb - 1) / cpb, H, R);
-  launch_kernel(delta_scan_kernel<T, EPL, LPC, LONG>, dim3(grid), dim3(threads), smem, s, 1, (const T*)q, (const T*)k, (const T*)v, q_stride,
-                k_stride, v_stride, beta, decay, state, slot_stride, q_indptr, state_slots, out, H, kq_heads, dim, vdim, q_scale, unit_eps, ahead);
+  launch_kernel(kernel, dim3(grid), dim3(threads), smem, s, 1, (const T*)q, (const T*)k, (const T*)v, q_stride,
+                k_stride, v_stride, beta, decay, state, slot_stride, q_indptr, state_slots, out, H, kq_heads, dim, vdim, q_scale, unit_eps);
   return launch_status();
 }
 
@@ -312,9 +322,9 @@ ARLE_API int arle_delta_scan(const void* q, const void* k, const void* v, int dt
   const bool long_rows = num_tokens >= 2 * R + kDeltaChunk;       // some row has a full chunk, or nearly
 #define ARLE_DELTA(TT, E, L)                                                                                                           \
   return long_rows ? launch_delta<TT, E, L, true>(q, k, v, q_stride, k_stride, v_stride, beta, decay, state, slot_stride, q_indptr,     \
-                                                  state_slots, out, R, H, kq_heads, dim, vdim, q_scale, unit_eps, s)                    \
+                                                  state_slots, out, R, H, kq_heads, dim, vdim, q_scale, unit_eps, num_tokens, s)                    \
                    : launch_delta<TT, E, L, false>(q, k, v, q_stride, k_stride, v_stride, beta, decay, state, slot_stride, q_indptr,    \
-                                                   state_slots, out, R, H, kq_heads, dim, vdim, q_scale, unit_eps, s)
+                                                   state_slots, out, R, H, kq_heads, dim, vdim, q_scale, unit_eps, num_tokens, s)
 #define ARLE_DELTA_BY_DIM(TT)          \
   if (dim <= 8) ARLE_DELTA(TT, 4, 2);   \
   if (dim <= 32) ARLE_DELTA(TT, 4, 8);  \
