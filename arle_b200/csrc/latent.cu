@@ -111,7 +111,7 @@ template <typename T, int HPW>
 __global__ void latent_attention_kernel(const T* __restrict__ q_abs, T* __restrict__ out, const T* __restrict__ cache,
                                         const int* __restrict__ positions, const int* __restrict__ row_of_token,
                                         const int* __restrict__ block_table, int bt_stride, int H, int rank, int kd,
-                                        int page_size, float scale, int window) {
+                                        int page_size, float scale, int window, const int* __restrict__ q_indptr, int shorter_than) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float sm[];
@@ -123,7 +123,9 @@ __global__ void latent_attention_kernel(const T* __restrict__ q_abs, T* __restri
   const int hb = (blockDim.x >> 5) * HPW;
   const int h0 = blockIdx.y * hb;
   const int pos = positions[t];
-  const int* bt = block_table + (size_t)row_of_token[t] * bt_stride;
+  const int row = row_of_token[t];
+  if (shorter_than > 0 && q_indptr[row + 1] - q_indptr[row] >= shorter_than) return;      // latent_prefill_tc.cu runs the long rows
+  const int* bt = block_table + (size_t)row * bt_stride;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
 
   for (int idx = threadIdx.x; idx < hb * kd; idx += blockDim.x) {
@@ -193,7 +195,7 @@ __global__ void latent_attention_kernel(const T* __restrict__ q_abs, T* __restri
 template <typename T, int HPW>
 static int launch_latent(const void* q_abs, void* out, const void* cache, const int* positions, const int* row_of_token,
                          const int* block_table, int bt_stride, int H, int rank, int kd, int page_size, float scale, int window,
-                         int num_tokens, int warps, cudaStream_t s) {
+                         int num_tokens, int warps, const int* q_indptr, int shorter_than, cudaStream_t s) {
   const int hb = warps * HPW;
   const size_t smem = ((size_t)kLatTile * (kd + 1) + (size_t)hb * kd) * sizeof(float);
   if (smem > 220 * 1024) return ARLE_E_UNSUPPORTED;
@@ -203,7 +205,7 @@ static int launch_latent(const void* q_abs, void* out, const void* cache, const 
   }
   dim3 grid(num_tokens, (H + hb - 1) / hb);
   launch_kernel(latent_attention_kernel<T, HPW>, dim3(grid), dim3(warps * 32), smem, s, 1, (const T*)q_abs, (T*)out, (const T*)cache,
-                positions, row_of_token, block_table, bt_stride, H, rank, kd, page_size, scale, window);
+                positions, row_of_token, block_table, bt_stride, H, rank, kd, page_size, scale, window, q_indptr, shorter_than);
   return launch_status();
 }
 
@@ -452,9 +454,10 @@ ARLE_API int arle_latent_attention_mma(const void* q_abs, void* out, float* part
 }
 
 // q_abs [T, H, kd] (folded queries: rank columns, then the rotated part), out [T, H, rank], cache [pages, 1, page_size, kd].
+// shorter_than > 0: as for the tensor-core form.
 ARLE_API int arle_latent_attention(const void* q_abs, void* out, const void* cache, int dtype, const int* positions,
                                    const int* row_of_token, const int* block_table, int bt_stride, int H, int rank, int kd,
-                                   int page_size, float scale, int window, int num_tokens, cudaStream_t s) {
+                                   int page_size, float scale, int window, int num_tokens, const int* q_indptr, int shorter_than, cudaStream_t s) {
   if (num_tokens <= 0) return 0;
   if (H <= 0 || rank <= 0 || kd < rank || page_size <= 0) return ARLE_E_BADARG;
   if (rank > 32 * kLatMaxD || H > 65535 * 8) return ARLE_E_UNSUPPORTED;
@@ -462,13 +465,13 @@ ARLE_API int arle_latent_attention(const void* q_abs, void* out, const void* cac
   const int warps = two ? 8 : H;
   if (dtype == 0)
     return two ? launch_latent<float, 2>(q_abs, out, cache, positions, row_of_token, block_table, bt_stride, H, rank, kd, page_size,
-                                         scale, window, num_tokens, warps, s)
+                                         scale, window, num_tokens, warps, q_indptr, shorter_than, s)
                : launch_latent<float, 1>(q_abs, out, cache, positions, row_of_token, block_table, bt_stride, H, rank, kd, page_size,
-                                         scale, window, num_tokens, warps, s);
+                                         scale, window, num_tokens, warps, q_indptr, shorter_than, s);
   if (dtype == 1)
     return two ? launch_latent<__nv_bfloat16, 2>(q_abs, out, cache, positions, row_of_token, block_table, bt_stride, H, rank, kd,
-                                                 page_size, scale, window, num_tokens, warps, s)
+                                                 page_size, scale, window, num_tokens, warps, q_indptr, shorter_than, s)
                : launch_latent<__nv_bfloat16, 1>(q_abs, out, cache, positions, row_of_token, block_table, bt_stride, H, rank, kd,
-                                                 page_size, scale, window, num_tokens, warps, s);
+                                                 page_size, scale, window, num_tokens, warps, q_indptr, shorter_than, s);
   return ARLE_E_BADARG;
 }

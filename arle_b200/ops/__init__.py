@@ -95,7 +95,7 @@ _SIGNATURES = {
     "arle_latent_plan": [_P, _P, _I, _I, _I, _P, _P],
     "arle_latent_gather": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _P, _I, _P],
     "arle_latent_prefill_tc": [_P, _I, _I, _P, _P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _I, _I, _I, _I, _P, _P],
-    "arle_latent_attention": [_P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
+    "arle_latent_attention": [_P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P, _I, _P],
     "arle_decay_scan": [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _I, _P],
     "arle_decay_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P],
     "arle_decay_chunk_plan_ints": [_I, _I],
@@ -1283,6 +1283,7 @@ def latent_attention(q_abs, out, cache, positions, row_of_token, block_table, ra
     StepContext, for its scratch buffers) lets the tensor-core kernel run where the shapes allow it; with few tokens in
     the step a token's keys are shared out among several blocks.  ``shorter_than`` > 0 (with ``batch``): the outputs of tokens in rows of
     that many tokens or more need not be written."""
+    long_rows = (_ptr(batch.q_indptr), int(shorter_than)) if shorter_than else (None, 0)
     T, heads, kd = q_abs.shape
     if (not q_abs.is_contiguous() or tuple(out.shape) != (T, heads, rank) or not out.is_contiguous() or out.dtype != q_abs.dtype
             or cache.dtype != q_abs.dtype or tuple(cache.shape[1:]) != (1, page_size, kd) or not cache.is_contiguous()):
@@ -1303,14 +1304,14 @@ def latent_attention(q_abs, out, cache, positions, row_of_token, block_table, ra
         _check(library().arle_latent_attention_mma(_ptr(q_abs), _ptr(out), _ptr(part_o), _ptr(part_ml), _ptr(cache), _ptr(positions),
                                                    _ptr(row_of_token), _ptr(block_table), block_table.stride(0), heads, rank, kd,
                                                    page_size, float(scale), int(window) if window else 0, T, splits,
-                                                   _ptr(batch.q_indptr) if shorter_than else None, int(shorter_than), _stream()),
+                                                   *long_rows, _stream()),
                "latent_attention_mma")
         if splits > 1:
             add_launches(1)
         return
     _check(library().arle_latent_attention(_ptr(q_abs), _ptr(out), _ptr(cache), _dt(q_abs), _ptr(positions), _ptr(row_of_token),
                                            _ptr(block_table), block_table.stride(0), heads, rank, kd, page_size, float(scale),
-                                           int(window) if window else 0, T, _stream()), "latent_attention")
+                                           int(window) if window else 0, T, *long_rows, _stream()), "latent_attention")
 
 
 # Rows of the step for which keys and values are built from the latent records.  A latent attention layer on one row, folded and built (us):

@@ -89,3 +89,27 @@ def test_against_float64(dn, dr, rank, heads, rows, window, monkeypatch):
                 assert (got - ref).abs().max() < 0.1
             at += n
     ops.check_errors(DEV)
+
+
+@pytest.mark.parametrize("rank,dr", [(96, 16), (128, 8), (128, 32)])
+def test_the_folded_form_leaves_long_rows_alone(rank, dr):
+    """On the general kernel (a rank of 96, eight rotated numbers) as on the tensor cores."""
+    heads, kd, lens = 4, rank + dr, [70, 5, 64, 63]
+    cm = CacheManager([CacheNeed(streams=((1, kd),))], [], 16, 20, len(lens), 80, BF, DEV)
+    for i in range(len(lens)):
+        cm.add_request(i)
+    cm.append([(i, n) for i, n in enumerate(lens)])
+    ctx = StepContext(cm, Workspace(DEV)).build([StepEntry(i, [0] * n) for i, n in enumerate(lens)], [0] * len(lens))
+    view, T = ctx.cache_view(0), sum(lens)
+    view.streams[0].normal_()
+    q = torch.randn(T, heads, kd, device=DEV).to(BF)
+    want, out = torch.empty(T, heads, rank, device=DEV, dtype=BF), torch.full((T, heads, rank), 7.0, device=DEV, dtype=BF)
+    args = (view.streams[0], ctx.positions, ctx.row_of_token, view.block_table, rank, 16, kd ** -0.5, None)
+    ops.latent_attention(q, want, *args, batch=ctx)
+    ops.latent_attention(q, out, *args, batch=ctx, shorter_than=64)
+    at = 0
+    for n in lens:
+        assert n >= 64 or torch.equal(out[at: at + n], want[at: at + n])
+        if n >= 64 and not ops.latent_mma_supported(q, rank):
+            assert (out[at: at + n] == 7.0).all()
+        at += n
