@@ -111,7 +111,7 @@ template <typename T, int HPW>
 __global__ void latent_attention_kernel(const T* __restrict__ q_abs, T* __restrict__ out, const T* __restrict__ cache,
                                         const int* __restrict__ positions, const int* __restrict__ row_of_token,
                                         const int* __restrict__ block_table, int bt_stride, int H, int rank, int kd,
-                                        int page_size, float scale, int window, const int* __restrict__ q_indptr, int shorter_than) {
+                                        int page_size, float scale, int window, const int2* __restrict__ built) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float sm[];
@@ -124,7 +124,7 @@ __global__ void latent_attention_kernel(const T* __restrict__ q_abs, T* __restri
   const int h0 = blockIdx.y * hb;
   const int pos = positions[t];
   const int row = row_of_token[t];
-  if (shorter_than > 0 && q_indptr[row + 1] - q_indptr[row] >= shorter_than) return;      // latent_prefill_tc.cu runs the long rows
+  if (built && built[row].y >= 0) return;                  // latent_prefill_tc.cu runs the row
   const int* bt = block_table + (size_t)row * bt_stride;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
 
@@ -195,7 +195,7 @@ __global__ void latent_attention_kernel(const T* __restrict__ q_abs, T* __restri
 template <typename T, int HPW>
 static int launch_latent(const void* q_abs, void* out, const void* cache, const int* positions, const int* row_of_token,
                          const int* block_table, int bt_stride, int H, int rank, int kd, int page_size, float scale, int window,
-                         int num_tokens, int warps, const int* q_indptr, int shorter_than, cudaStream_t s) {
+                         int num_tokens, int warps, const int* built, cudaStream_t s) {
   const int hb = warps * HPW;
   const size_t smem = ((size_t)kLatTile * (kd + 1) + (size_t)hb * kd) * sizeof(float);
   if (smem > 220 * 1024) return ARLE_E_UNSUPPORTED;
@@ -205,7 +205,7 @@ static int launch_latent(const void* q_abs, void* out, const void* cache, const 
   }
   dim3 grid(num_tokens, (H + hb - 1) / hb);
   launch_kernel(latent_attention_kernel<T, HPW>, dim3(grid), dim3(warps * 32), smem, s, 1, (const T*)q_abs, (T*)out, (const T*)cache,
-                positions, row_of_token, block_table, bt_stride, H, rank, kd, page_size, scale, window, q_indptr, shorter_than);
+                positions, row_of_token, block_table, bt_stride, H, rank, kd, page_size, scale, window, (const int2*)built);
   return launch_status();
 }
 
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(128) latent_attention_mma_kernel(
     const __nv_bfloat16* __restrict__ q_abs, __nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
     const __nv_bfloat16* __restrict__ cache, const int* __restrict__ positions, const int* __restrict__ row_of_token,
     const int* __restrict__ block_table, int bt_stride, int H, int kd, int page_size, float scale, int window, int splits,
-    const int* __restrict__ q_indptr, int shorter_than) {
+    const int2* __restrict__ built) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr int rank = 64 * R64;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(128) latent_attention_mma_kernel(
   const int g = lane >> 2, t4 = lane & 3;
   const int pos = positions[t];
   const int row = row_of_token[t];
-  if (shorter_than > 0 && q_indptr[row + 1] - q_indptr[row] >= shorter_than) return;      // latent_prefill_tc.cu runs the long rows
+  if (built && built[row].y >= 0) return;                  // latent_prefill_tc.cu runs the row
   const int* bt = block_table + (size_t)row * bt_stride;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
   const int ntiles = (pos - lo) / kMmaTile + 1;
@@ -416,7 +416,7 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_o, const floa
 template <int R64>
 static int launch_latent_mma(const void* q_abs, void* out, float* part_o, float* part_ml, const void* cache, const int* positions,
                              const int* row_of_token, const int* block_table, int bt_stride, int H, int kd, int page_size, float scale,
-                             int window, int num_tokens, int splits, const int* q_indptr, int shorter_than, cudaStream_t s) {
+                             int window, int num_tokens, int splits, const int* built, cudaStream_t s) {
   const size_t smem = (size_t)(16 + kMmaTile) * (kd + 8) * 2 + 16 * kPPitch * 2 + 64 * sizeof(float);
   if (smem > 220 * 1024) return ARLE_E_UNSUPPORTED;
   cudaError_t e = cudaFuncSetAttribute(latent_attention_mma_kernel<R64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -424,7 +424,7 @@ static int launch_latent_mma(const void* q_abs, void* out, float* part_o, float*
   dim3 grid(num_tokens, (H + 15) / 16, splits);
   launch_kernel(latent_attention_mma_kernel<R64>, dim3(grid), dim3(128), smem, s, 1, (const __nv_bfloat16*)q_abs, (__nv_bfloat16*)out,
                 part_o, part_ml, (const __nv_bfloat16*)cache, positions, row_of_token, block_table, bt_stride, H, kd, page_size, scale,
-                window, splits, q_indptr, shorter_than);
+                window, splits, (const int2*)built);
   if (splits > 1)
     launch_kernel(latent_merge_kernel, dim3(num_tokens * H), dim3(64 * R64 >= 256 ? 256 : 64), 0, s, 1, (const float*)part_o,
                   (const float*)part_ml, (__nv_bfloat16*)out, 64 * R64, splits);
@@ -432,19 +432,19 @@ static int launch_latent_mma(const void* q_abs, void* out, float* part_o, float*
 }
 
 // The tensor-core form: bfloat16, rank 64 / 128 / 256 / 512, kd - rank a multiple of 16.  splits > 1 needs part_o float32
-// [T * H * splits * rank] and part_ml float32 [T * H * splits * 2].  shorter_than > 0: tokens of rows (q_indptr) with that many tokens or
-// more are left alone.
+// [T * H * splits * rank] and part_ml float32 [T * H * splits * 2].  built (or null): the plan of latent_prefill_tc.cu, whose rows are
+// left alone.
 ARLE_API int arle_latent_attention_mma(const void* q_abs, void* out, float* part_o, float* part_ml, const void* cache,
                                        const int* positions, const int* row_of_token, const int* block_table, int bt_stride, int H,
                                        int rank, int kd, int page_size, float scale, int window, int num_tokens, int splits,
-                                       const int* q_indptr, int shorter_than, cudaStream_t s) {
+                                       const int* built, cudaStream_t s) {
   if (num_tokens <= 0) return 0;
   if (H <= 0 || kd < rank || (kd - rank) % 16 || page_size <= 0 || splits < 1 || splits > 65535 || splits > 64 || (H + 15) / 16 > 65535 ||
       (splits > 1 && (!part_o || !part_ml)))
     return ARLE_E_BADARG;
 #define ARLE_LAT(R) \
   return launch_latent_mma<R>(q_abs, out, part_o, part_ml, cache, positions, row_of_token, block_table, bt_stride, H, kd, page_size, \
-                              scale, window, num_tokens, splits, q_indptr, shorter_than, s)
+                              scale, window, num_tokens, splits, built, s)
   if (rank == 64) ARLE_LAT(1);
   if (rank == 128) ARLE_LAT(2);
   if (rank == 256) ARLE_LAT(4);
@@ -454,10 +454,10 @@ ARLE_API int arle_latent_attention_mma(const void* q_abs, void* out, float* part
 }
 
 // q_abs [T, H, kd] (folded queries: rank columns, then the rotated part), out [T, H, rank], cache [pages, 1, page_size, kd].
-// shorter_than > 0: as for the tensor-core form.
+// built: as for the tensor-core form.
 ARLE_API int arle_latent_attention(const void* q_abs, void* out, const void* cache, int dtype, const int* positions,
                                    const int* row_of_token, const int* block_table, int bt_stride, int H, int rank, int kd,
-                                   int page_size, float scale, int window, int num_tokens, const int* q_indptr, int shorter_than, cudaStream_t s) {
+                                   int page_size, float scale, int window, int num_tokens, const int* built, cudaStream_t s) {
   if (num_tokens <= 0) return 0;
   if (H <= 0 || rank <= 0 || kd < rank || page_size <= 0) return ARLE_E_BADARG;
   if (rank > 32 * kLatMaxD || H > 65535 * 8) return ARLE_E_UNSUPPORTED;
@@ -465,13 +465,13 @@ ARLE_API int arle_latent_attention(const void* q_abs, void* out, const void* cac
   const int warps = two ? 8 : H;
   if (dtype == 0)
     return two ? launch_latent<float, 2>(q_abs, out, cache, positions, row_of_token, block_table, bt_stride, H, rank, kd, page_size,
-                                         scale, window, num_tokens, warps, q_indptr, shorter_than, s)
+                                         scale, window, num_tokens, warps, built, s)
                : launch_latent<float, 1>(q_abs, out, cache, positions, row_of_token, block_table, bt_stride, H, rank, kd, page_size,
-                                         scale, window, num_tokens, warps, q_indptr, shorter_than, s);
+                                         scale, window, num_tokens, warps, built, s);
   if (dtype == 1)
     return two ? launch_latent<__nv_bfloat16, 2>(q_abs, out, cache, positions, row_of_token, block_table, bt_stride, H, rank, kd,
-                                                 page_size, scale, window, num_tokens, warps, q_indptr, shorter_than, s)
+                                                 page_size, scale, window, num_tokens, warps, built, s)
                : launch_latent<__nv_bfloat16, 1>(q_abs, out, cache, positions, row_of_token, block_table, bt_stride, H, rank, kd,
-                                                 page_size, scale, window, num_tokens, warps, q_indptr, shorter_than, s);
+                                                 page_size, scale, window, num_tokens, warps, built, s);
   return ARLE_E_BADARG;
 }

@@ -7,7 +7,8 @@
 // they run on tcgen05 with the queries in the rows.  Building costs 2 rank (dn + dv) a head and key, what some 170 queries save.
 //
 //  * latent_plan: for every row of the step with at least `least` queries the first key its queries see (a multiple of 16) and where
-//    its keys start in the built arrays; -1 for the others (the folded kernel runs them).
+//    its keys start in the built arrays; -1 for the others, which the folded kernel runs, and for rows whose context is long beside their
+//    queries.  A row's own lengths decide.  Rows whose records do not fit beside one another are built in groups, one after the other.
 //  * latent_gather: the records of those rows from the pages, side by side, each row's padded to a multiple of 16 with zeros.
 //    The product that builds keys and values is the caller's (a plain matrix product over the gathered latents).
 //    A latent with an infinity or a NaN is gathered as zeros with NaN in the rotated numbers beside it (a record without rotated numbers
@@ -99,31 +100,32 @@ __device__ __forceinline__ unsigned int draw_ticket(int nblocks, int slot) {
   return raw + gridDim.x;
 }
 
-// plan: [R] (first key, place of that key in the built arrays or -1), then the places in all.
+// plan: [R] (first key, place of that key in the built arrays of its group or -1).  A row is built from at most max(most * its queries,
+// floor) records, a group holds at most `room`.
 __global__ void __launch_bounds__(32) latent_plan_kernel(const int* __restrict__ q_indptr, const int* __restrict__ kv_lens, int R, int least,
-                                                         int window, int2* __restrict__ plan) {
+                                                         int most, int floor, int room, int window, int2* __restrict__ plan) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x;
-  int carry = 0;
+  int filled = 0;                                          // places of the group so far
   for (int r0 = 0; r0 < R; r0 += 32) {
     const int r = r0 + lane;
-    int need = 0, first = 0;
+    int need = 0, first = 0, at = -1;
     if (r < R) {
       const int n = q_indptr[r + 1] - q_indptr[r], kv = kv_lens[r];
       first = first_visible_key(kv - n, window, 0) & ~15;
-      if (n >= least) need = (kv - first + 15) & ~15;
+      const int records = (kv - first + 15) & ~15;
+      if (n >= least && records <= max(most * n, floor)) need = records;
     }
-    int sum = need;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, sum, o);
-      if (lane >= o) sum += v;
+    for (int i = 0; i < 32; ++i) {
+      const int x = __shfl_sync(0xffffffffu, need, i);
+      if (x == 0) continue;
+      if (filled + x > room) filled = 0;                   // the next group
+      if (lane == i) at = filled;
+      filled += x;
     }
-    if (r < R) plan[r] = make_int2(first, need ? carry + sum - need : -1);
-    carry += __shfl_sync(0xffffffffu, sum, 31);
+    if (r < R) plan[r] = make_int2(first, at);
   }
-  if (lane == 0) plan[R] = make_int2(carry, carry);
 }
 
 // Numbers of a gathered record behind its latent.
@@ -141,7 +143,6 @@ __global__ void __launch_bounds__(kGatherThreads) latent_gather_kernel(const __n
   pdl_wait();
   __shared__ int bad[16];                                  // records whose latent holds an infinity or a NaN
   const int place = blockIdx.x * 16;
-  if (place >= plan[R].x) return;
   int row = -1;
   for (int r = 0; r < R; ++r) {
     const int at = plan[r].y;
@@ -662,15 +663,16 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mr, 
 
 }  // namespace
 
-// plan: int32 [R + 1][2].
-ARLE_API int arle_latent_plan(const int* q_indptr, const int* kv_lens, int R, int least, int window, int* plan, cudaStream_t s) {
+// plan: int32 [R][2].
+ARLE_API int arle_latent_plan(const int* q_indptr, const int* kv_lens, int R, int least, int most, int floor, int room, int window, int* plan,
+                              cudaStream_t s) {
   if (R <= 0) return 0;
-  launch_kernel(latent_plan_kernel, dim3(1), dim3(32), 0, s, 1, q_indptr, kv_lens, R, least, window, (int2*)plan);
+  launch_kernel(latent_plan_kernel, dim3(1), dim3(32), 0, s, 1, q_indptr, kv_lens, R, least, most, floor, room, window, (int2*)plan);
   return launch_status();
 }
 
-// cache bfloat16 [pages, 1, page_size, rank + dr]; out [places, rank + max(dr, 8)], places a multiple of 16 and at least what the plan
-// counts.  rank up to 512, dr up to 64, multiples of 8.
+// cache bfloat16 [pages, 1, page_size, rank + dr]; out [places, rank + max(dr, 8)], places: a group's, R and the arrays by row: its
+// rows.  rank up to 512, dr up to 64, multiples of 8.
 ARLE_API int arle_latent_gather(const void* cache, const int* block_table, int bt_stride, const int* kv_lens, const int* plan, int R, int page_size,
                                 int rank, int dr, void* out, int places, cudaStream_t s) {
   if (R <= 0 || places <= 0) return 0;
@@ -684,7 +686,7 @@ ARLE_API int arle_latent_gather(const void* cache, const int* block_table, int b
 
 // q bfloat16 [num_tokens, heads * (dn + dr)] (any row stride that is a multiple of 8): a head's unrotated numbers, then its rotated ones.
 // keys [places, heads * dn] and values [places, heads * dn] (row stride kv_stride), records [places, rank + max(dr, 8)]: the built arrays
-// and the gathered records of the plan.  out [num_tokens, heads * dn] (row stride out_stride): only the plan's rows are written.
+// and the gathered records of a group; rows, q_indptr, kv_lens and plan: the group's.  out [num_tokens, heads * dn] (row stride out_stride): only the plan's rows are written.
 // dn 64 or 128, dr 0 or a multiple of 8 up to 64.
 ARLE_API int arle_latent_prefill_tc(const void* q, int q_stride, int num_tokens, const void* keys, const void* values, int kv_stride,
                                     const void* records, int places, void* out, int out_stride, const int* q_indptr, const int* kv_lens,

@@ -91,11 +91,11 @@ _SIGNATURES = {
     "arle_gemm_heads_mma": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, ctypes.c_long, _I, _P, _I, _P],
     "arle_gemm_heads": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, ctypes.c_long, _I, _P],
     "arle_latent_prep": [_P, _I, _P, _I, _I, _P, _P, _P, _F, _P, _I, _I, _F, _P, _P, ctypes.c_long, _I, _I, _I, _I, _I, _I, _I, _P],
-    "arle_latent_attention_mma": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _I, _P],
-    "arle_latent_plan": [_P, _P, _I, _I, _I, _P, _P],
+    "arle_latent_attention_mma": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P],
+    "arle_latent_plan": [_P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "arle_latent_gather": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _P, _I, _P],
     "arle_latent_prefill_tc": [_P, _I, _I, _P, _P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _I, _I, _I, _I, _P, _P],
-    "arle_latent_attention": [_P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P, _I, _P],
+    "arle_latent_attention": [_P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P],
     "arle_decay_scan": [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _I, _P],
     "arle_decay_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P],
     "arle_decay_chunk_plan_ints": [_I, _I],
@@ -1276,14 +1276,14 @@ def latent_mma_supported(q_abs, rank: int) -> bool:
 
 
 def latent_attention(q_abs, out, cache, positions, row_of_token, block_table, rank: int, page_size: int, scale: float, window,
-                     batch=None, shorter_than: int = 0) -> None:
+                     batch=None, but_built: bool = False) -> None:
     """Causal attention of folded queries q_abs [T, heads, kd] over records cache [pages, 1, page_size, kd]: head h's score
     against record j is (q_abs[t, h] . record_j) * scale, its output sum_j softmax_j * record_j[:rank] (out [T, heads,
     rank]).  ``window`` None or <= 0: all keys; W: keys p - W + 1 .. p.  Scores, softmax and sums are float32.  ``batch`` (a
     StepContext, for its scratch buffers) lets the tensor-core kernel run where the shapes allow it; with few tokens in
-    the step a token's keys are shared out among several blocks.  ``shorter_than`` > 0 (with ``batch``): the outputs of tokens in rows of
-    that many tokens or more need not be written."""
-    long_rows = (_ptr(batch.q_indptr), int(shorter_than)) if shorter_than else (None, 0)
+    the step a token's keys are shared out among several blocks.  ``but_built`` (with ``batch``): the outputs of the rows that
+    ``latent_prefill`` runs need not be written."""
+    built = _ptr(_latent_plan(batch, window)) if but_built else None
     T, heads, kd = q_abs.shape
     if (not q_abs.is_contiguous() or tuple(out.shape) != (T, heads, rank) or not out.is_contiguous() or out.dtype != q_abs.dtype
             or cache.dtype != q_abs.dtype or tuple(cache.shape[1:]) != (1, page_size, kd) or not cache.is_contiguous()):
@@ -1304,39 +1304,78 @@ def latent_attention(q_abs, out, cache, positions, row_of_token, block_table, ra
         _check(library().arle_latent_attention_mma(_ptr(q_abs), _ptr(out), _ptr(part_o), _ptr(part_ml), _ptr(cache), _ptr(positions),
                                                    _ptr(row_of_token), _ptr(block_table), block_table.stride(0), heads, rank, kd,
                                                    page_size, float(scale), int(window) if window else 0, T, splits,
-                                                   *long_rows, _stream()),
+                                                   built, _stream()),
                "latent_attention_mma")
         if splits > 1:
             add_launches(1)
         return
     _check(library().arle_latent_attention(_ptr(q_abs), _ptr(out), _ptr(cache), _dt(q_abs), _ptr(positions), _ptr(row_of_token),
                                            _ptr(block_table), block_table.stride(0), heads, rank, kd, page_size, float(scale),
-                                           int(window) if window else 0, T, *long_rows, _stream()), "latent_attention")
+                                           int(window) if window else 0, T, built, _stream()), "latent_attention")
 
 
 # Rows of the step for which keys and values are built from the latent records.  A latent attention layer on one row, folded and built (us):
 # 32 heads of 128 + 64 at rank 512, width 4,096: 64 queries 57 and 48 (behind 2,048 tokens 239 and 114, behind 6,144 599 and 213), 512
 # queries 275 and 90 (4,054 and 281); 16 heads of 64 + 32 at rank 256, width 1,024: 64 queries 35 and 32 (68 and 65; 143 and 131), 512
 # queries 92 and 45 (801 and 145).  With 16 queries the two are equal without a context and the folded form wins behind one.
-LATENT_BUILT_LEAST = 64             # queries of a row from which its keys and values are built
-LATENT_BUILT_MOST = 8               # records that are laid side by side, a token of the step ...
-LATENT_BUILT_PLACES = 1 << 16       # ... or this many, whichever is more: what the step's buffers leave room for
+LATENT_BUILT_LEAST = 64             # queries of a row from which its keys and values are built ...
+LATENT_BUILT_MOST = 8               # ... from at most this many records a query ...
+LATENT_BUILT_PLACES = 1 << 16       # ... or this many, whichever is more; and what is laid side by side at a time, a token or at least
 LATENT_BUILT_NUMBERS = 1 << 25      # keys' numbers that are built at a time, where the step's tokens do not give room for more
 
 
+def latent_scratch_elements(heads: int, dn: int, record: int):
+    """(elements a token, elements at least) of the buffers that ``latent_prefill`` may hold."""
+    return (LATENT_BUILT_MOST * record + 2 * heads * dn,
+            LATENT_BUILT_PLACES * record + 2 * max(LATENT_BUILT_NUMBERS, LATENT_BUILT_PLACES * dn))
+
+
+def _latent_groups(batch, window):
+    """The step's rows whose keys and values are built, by their own lengths alone, in groups of neighbouring rows that are laid side by side:
+    ([(first row, row behind the last, places)], rows that stay folded).  Places: records, each row's padded to a multiple of 16."""
+    key = ("latent_groups", int(window) if window else 0)
+    if key not in batch.memo:
+        groups, folded = [], 0
+        room = max(LATENT_BUILT_MOST * batch.num_tokens, LATENT_BUILT_PLACES)
+        for r, (n, kv) in enumerate(zip(batch.q_lens, batch.kv_lens_host)):
+            first = max(0, kv - n - key[1] + 1) if window else 0
+            need = (kv - first // 16 * 16 + 15) // 16 * 16
+            if n < LATENT_BUILT_LEAST or need > max(LATENT_BUILT_MOST * n, LATENT_BUILT_PLACES):
+                folded += 1
+            elif groups and groups[-1][2] + need <= room:
+                groups[-1] = (groups[-1][0], r + 1, groups[-1][2] + need)
+            else:
+                groups.append((r, r + 1, need))
+        batch.memo[key] = groups, folded
+    return batch.memo[key]
+
+
+def _latent_plan(batch, window):
+    """The same on the device: int32 [rows, 2], a row's first key and its place in its group, -1 for rows that stay folded."""
+    window = int(window) if window else 0
+    key = ("latent_plan", window)
+    if key not in batch.memo:
+        plan = batch.ws.get(f"latent_plan_{window}", (batch.num_rows, 2), torch.int32)
+        room = max(LATENT_BUILT_MOST * batch.num_tokens, LATENT_BUILT_PLACES)
+        _check(library().arle_latent_plan(_ptr(batch.q_indptr), _ptr(batch.kv_lens), batch.num_rows, LATENT_BUILT_LEAST, LATENT_BUILT_MOST,
+                                          LATENT_BUILT_PLACES, room, window, _ptr(plan), _stream()), "latent_plan")
+        batch.memo[key] = plan
+    return batch.memo[key]
+
+
 def latent_built_places(batch, q, dn: int, dr: int, vdim: int, rank: int, page_size: int, window) -> int:
-    """Records (each row's padded to a multiple of 16) that ``latent_prefill`` would build keys and values from for this step's rows of
-    LATENT_BUILT_LEAST tokens and more; 0: none, the folded attention runs every row."""
+    """Records that ``latent_prefill`` would build keys and values from for this step's rows of LATENT_BUILT_LEAST tokens and more; 0: none,
+    the folded attention runs every row."""
     if not (batch.max_q_len >= LATENT_BUILT_LEAST and _KERNEL_SET == "fast" and q.is_cuda and q.dtype == torch.bfloat16 and dn in (64, 128)
             and vdim == dn and dr <= 64 and dr % 8 == 0 and rank % 8 == 0 and page_size % 16 == 0 and q.stride(0) % 8 == 0
             and q.data_ptr() % 16 == 0):
         return 0
-    places = 0
-    for n, kv in zip(batch.q_lens, batch.kv_lens_host):
-        if n >= LATENT_BUILT_LEAST:
-            first = max(0, kv - n - int(window) + 1) if window else 0
-            places += (kv - first // 16 * 16 + 15) // 16 * 16
-    return places if places <= max(LATENT_BUILT_MOST * batch.num_tokens, LATENT_BUILT_PLACES) else 0
+    return sum(places for _, _, places in _latent_groups(batch, window)[0])
+
+
+def latent_all_built(batch, window) -> bool:
+    """Whether ``latent_prefill`` runs every row of the step (where ``latent_built_places`` lets it run at all)."""
+    return _latent_groups(batch, window)[1] == 0
 
 
 def latent_prefill(q, out, records, batch, block_table, w_ukv, heads: int, places: int, dr: int, rank: int, page_size: int, scale: float, window,
@@ -1355,17 +1394,24 @@ def latent_prefill(q, out, records, batch, block_table, w_ukv, heads: int, place
             or q.dtype != out.dtype or places <= 0 or (gate is not None and (gate.shape != out.shape or gate.stride(1) != 1 or gate.dtype != out.dtype))):
         raise KernelError("latent_prefill: q, out, records or the heads' maps do not fit")
     _i32(block_table, "block_table")
-    lib, s = library(), _stream()
-    R, window = batch.num_rows, int(window) if window else 0
-    key = ("latent_plan", window)
-    plan = batch.memo.get(key)
-    if plan is None:
-        plan = batch.ws.get(f"latent_plan_{window}", (R + 1, 2), torch.int32)
-        _check(lib.arle_latent_plan(_ptr(batch.q_indptr), _ptr(batch.kv_lens), R, LATENT_BUILT_LEAST, window, _ptr(plan), s), "latent_plan")
-        batch.memo[key] = plan
+    window = int(window) if window else 0
+    groups, plan = _latent_groups(batch, window)[0], _latent_plan(batch, window)
+    if sum(n for _, _, n in groups) != places:
+        raise KernelError("latent_prefill: places are not the step's")
+    for r0, r1, places in groups:
+        _latent_group(q, out, records, batch, block_table, w_ukv, heads, places, dr, rank, page_size, scale, window, gate, plan, r0, r1)
+
+
+def _latent_group(q, out, records, batch, block_table, w_ukv, heads, places, dr, rank, page_size, scale, window, gate, plan, r0, r1) -> None:
+    lib, s, T = library(), _stream(), q.shape[0]
+    dn = w_ukv.shape[0] // (2 * heads)
+    R, by_row = r1 - r0, 4 * r0
+    indptr, kv_lens, tables = _ptr(batch.q_indptr) + by_row, _ptr(batch.kv_lens) + by_row, _ptr(block_table) + by_row * block_table.stride(0)
+    plan = _ptr(plan) + 2 * by_row
+    max_q_len = max(batch.q_lens[r0:r1])
     lat = batch.ws.get("latent_gathered", (places, rank + (dr or 8)), q.dtype)
-    _check(lib.arle_latent_gather(_ptr(records), _ptr(block_table), block_table.stride(0), _ptr(batch.kv_lens), _ptr(plan), R, page_size, rank,
-                                  dr, _ptr(lat), places, s), "latent_gather")
+    _check(lib.arle_latent_gather(_ptr(records), tables, block_table.stride(0), kv_lens, plan, R, page_size, rank, dr, _ptr(lat), places, s),
+           "latent_gather")
     width = heads * dn
     group = min(heads, max(T * heads // places, LATENT_BUILT_NUMBERS // (places * dn), 1))
     for h0 in range(0, heads, group):
@@ -1378,9 +1424,9 @@ def latent_prefill(q, out, records, batch, block_table, w_ukv, heads: int, place
             gemm(lat[:, :rank], w_ukv[width + h0 * dn: width + (h0 + hg) * dn], built[:, hg * dn:])
         at = h0 * dn * 2
         _check(lib.arle_latent_prefill_tc(_ptr(q) + h0 * (dn + dr) * 2, q.stride(0), T, _ptr(built), _ptr(built) + 2 * hg * dn, 2 * hg * dn,
-                                          _ptr(lat), places, _ptr(out) + at, out.stride(0), _ptr(batch.q_indptr), _ptr(batch.kv_lens), _ptr(plan),
+                                          _ptr(lat), places, _ptr(out) + at, out.stride(0), indptr, kv_lens, plan,
                                           hg, dn, dr, rank, float(scale), _ptr(gate) + at if gate is not None else None,
-                                          gate.stride(0) if gate is not None else 0, window, R, batch.max_q_len, _ptr(error_flag(q.device)), s),
+                                          gate.stride(0) if gate is not None else 0, window, R, max_q_len, _ptr(error_flag(q.device)), s),
                "latent_prefill_tc")
 
 

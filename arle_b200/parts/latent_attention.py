@@ -139,7 +139,11 @@ class LatentAttention(Mixer):
     def scratch_elements_per_token(self):
         s = self.spec
         return self.rows + s.num_heads * (self.record + s.kv_rank + s.value_dim) + s.hidden_size + (self.first + self.q_width if s.q_rank else 0) + (
-            ops.LATENT_BUILT_MOST * self.record + s.num_heads * (s.nope_dim + s.value_dim) if self.w_ukv is not None else 0)
+            ops.latent_scratch_elements(s.num_heads, s.nope_dim, s.kv_rank + (s.rope_dim or 8))[0] if self.w_ukv is not None else 0)
+
+    def scratch_elements_at_least(self):
+        s = self.spec
+        return ops.latent_scratch_elements(s.num_heads, s.nope_dim, s.kv_rank + (s.rope_dim or 8))[1] if self.w_ukv is not None else 0
 
     # ------------------------------------------------------------------ cache
     def cache_need(self):
@@ -169,7 +173,7 @@ class LatentAttention(Mixer):
         records = cache.streams[0]
         stores = cache.writable and s.own_latent
         places = ops.latent_built_places(ctx, q, dn, dr, s.value_dim, rank, cache.page_size, s.window) if self.w_ukv is not None else 0
-        all_built = places > 0 and min(ctx.q_lens) >= ops.LATENT_BUILT_LEAST
+        all_built = places > 0 and ops.latent_all_built(ctx, s.window)
         q_abs = None if all_built else ctx.ws.get("latent_q", (T, H, self.record), x.dtype)
 
         def prepare(into, record, store):
@@ -187,9 +191,9 @@ class LatentAttention(Mixer):
             else:
                 q_abs[:, :, :rank].zero_()
             o_lat = ctx.ws.get("latent_o", (T, H, rank), x.dtype)
-            short = {"shorter_than": ops.LATENT_BUILT_LEAST} if places else {}
+            but = {"but_built": True} if places else {}
             ops.latent_attention(q_abs, o_lat, records, ctx.positions, ctx.row_of_token, cache.block_table, rank, cache.page_size,
-                                 s.scale, s.window, batch=ctx, **short)
+                                 s.scale, s.window, batch=ctx, **but)
             ops.gemm_heads(o_lat, self.w_uv, heads_out, gate=gate)
         if places:
             if dr and not all_built:

@@ -106,10 +106,52 @@ def test_the_folded_form_leaves_long_rows_alone(rank, dr):
     want, out = torch.empty(T, heads, rank, device=DEV, dtype=BF), torch.full((T, heads, rank), 7.0, device=DEV, dtype=BF)
     args = (view.streams[0], ctx.positions, ctx.row_of_token, view.block_table, rank, 16, kd ** -0.5, None)
     ops.latent_attention(q, want, *args, batch=ctx)
-    ops.latent_attention(q, out, *args, batch=ctx, shorter_than=64)
+    ops.latent_attention(q, out, *args, batch=ctx, but_built=True)
     at = 0
     for n in lens:
         assert n >= 64 or torch.equal(out[at: at + n], want[at: at + n])
         if n >= 64 and not ops.latent_mma_supported(q, rank):
             assert (out[at: at + n] == 7.0).all()
         at += n
+
+
+def test_a_row_is_built_by_its_own_lengths(monkeypatch):
+    """Rows whose records do not fit beside one another are built in groups, a row whose context is long beside its queries stays folded, and
+    neither shows in the other rows' numbers."""
+    monkeypatch.setattr(ops, "LATENT_BUILT_PLACES", 400)
+    monkeypatch.setattr(ops, "LATENT_BUILT_MOST", 1)
+    dn, dr, rank, heads = 64, 32, 128, 3
+    kd, rows = rank + dr, [(64, 300), (70, 340), (5, 20), (64, 420), (130, 0), (64, 16), (200, 0), (64, 330)]
+    lens, kvs = [n for n, _ in rows], [n + s for n, s in rows]
+    g = torch.Generator(device=DEV).manual_seed(2)
+    cm = CacheManager([CacheNeed(streams=((1, kd),))], [], 16, sum(-(-k // 16) for k in kvs) + 3, len(rows), max(kvs), BF, DEV)
+    for i, (_, s) in enumerate(rows):
+        cm.add_request(i)
+        if s:
+            cm.append([(i, s)])
+    cm.append([(i, n) for i, n in enumerate(lens)])
+    cm.groups[0].arrays[0].normal_(generator=g)
+    T = sum(lens)
+    q = torch.empty(T, heads * (dn + dr), device=DEV, dtype=BF).normal_(generator=g)
+    w = torch.empty(2 * heads * dn, rank, device=DEV, dtype=BF).normal_(0.0, rank ** -0.5, generator=g)
+
+    def run(idx, lo, hi):
+        ctx = StepContext(cm, Workspace(DEV)).build([StepEntry(i, [0] * lens[i]) for i in idx], [rows[i][1] for i in idx])
+        view, out = ctx.cache_view(0), torch.full((hi - lo, heads * dn), 7.0, device=DEV, dtype=BF)
+        places = ops.latent_built_places(ctx, q[lo:hi], dn, dr, dn, rank, 16, None)
+        if places:
+            ops.latent_prefill(q[lo:hi], out, view.streams[0], ctx, view.block_table, w, heads, places, dr, rank, 16, kd ** -0.5, None)
+        return ctx, out
+
+    ctx, whole = run(range(len(rows)), 0, T)
+    groups, folded = ops._latent_groups(ctx, None)
+    plan = ops._latent_plan(ctx, None).tolist()
+    assert len(groups) >= 2 and folded == 3                          # 5 queries; contexts of 410 and 484 behind 70 and 64 queries
+    at = 0
+    for i, n in enumerate(lens):
+        _, one = run([i], at, at + n)
+        # the product that builds keys and values may take another order of sums for another number of records: bfloat16 roundings apart
+        assert (one.double() - whole[at: at + n].double()).norm() <= 2.0 ** -7 * one.double().norm()
+        assert (plan[i][1] < 0) == bool((one == 7.0).all()) == (i in (1, 2, 3))
+        at += n
+    ops.check_errors(DEV)
