@@ -118,6 +118,10 @@ class Part:
         engine uses to leave memory for them beside the cache)."""
         return 0
 
+    def scratch_elements_at_least(self) -> int:
+        """Activation elements of step buffers that may grow to this size however few tokens a step has (long contexts)."""
+        return 0
+
     # Optional fusion of the norms into the products around them (decode steps of few rows; see
     # ``ops.ResidualSink`` and ``ops.ScaledRows``).  A part that says yes to ``takes_scaled_rows`` may
     # get ``ops.ScaledRows`` as its input instead of a tensor; a part that says yes to ``can_sink`` may

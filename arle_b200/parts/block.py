@@ -45,6 +45,9 @@ class PreNormBlock(Block):
     def weight_bytes(self):
         return sum(p.weight_bytes() for p in self._parts)
 
+    def scratch_elements_at_least(self):
+        return max(p.scratch_elements_at_least() for p in self._parts)
+
     def scratch_elements_per_token(self):
         # the two normalised inputs and the larger of the two branches' buffers
         if self.ffn is None:
@@ -155,6 +158,9 @@ class OutputNormBlock(Block):
     def weight_bytes(self):
         return sum(p.weight_bytes() for p in self._parts)
 
+    def scratch_elements_at_least(self):
+        return max(p.scratch_elements_at_least() for p in self._parts)
+
     def scratch_elements_per_token(self):
         width = self.mixer_norm.scratch_elements_per_token()
         return 2 * width + max(self.mixer.scratch_elements_per_token(), self.ffn.scratch_elements_per_token() if self.ffn is not None else 0)
@@ -226,6 +232,9 @@ class SandwichBlock(Block):
 
     def weight_bytes(self):
         return sum(p.weight_bytes() for p in self._parts)
+
+    def scratch_elements_at_least(self):
+        return max(p.scratch_elements_at_least() for p in self._parts)
 
     def scratch_elements_per_token(self):
         width = self.mixer_norm.scratch_elements_per_token()

@@ -375,7 +375,8 @@ class DecoderModel:
         widest = max((b.scratch_elements_per_token() for b in self.blocks), default=0)
         H = self.spec.hidden_size
         H4 = 8 * H if self.readds_embedding else 4 * H
-        return tokens * (H4 + widest * act) + wanted * (self.spec.vocab_size * 4 + H * act)
+        fixed = max((b.scratch_elements_at_least() for b in self.blocks), default=0) if tokens >= ops.LATENT_BUILT_LEAST else 0
+        return fixed * act + tokens * (H4 + widest * act) + wanted * (self.spec.vocab_size * 4 + H * act)
 
 
 register_model("decoder", DecoderModel)

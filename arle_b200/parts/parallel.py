@@ -107,6 +107,9 @@ class ParallelMixer(Mixer):
     def weight_bytes(self):
         return sum(m.weight_bytes() for m in self.members)
 
+    def scratch_elements_at_least(self):
+        return max(m.scratch_elements_at_least() for m in self.members)
+
     def scratch_elements_per_token(self):
         return sum(m.scratch_elements_per_token() for m in self.members) + (self.w_o.shape[1] if self.w_o is not None else 0)
 
@@ -215,6 +218,9 @@ class ParallelBlock(Block):
 
     def weight_bytes(self):
         return sum(p.weight_bytes() for p in self._parts)
+
+    def scratch_elements_at_least(self):
+        return max(p.scratch_elements_at_least() for p in self._parts)
 
     def scratch_elements_per_token(self):
         return sum(p.scratch_elements_per_token() for p in self._parts) + (self.w_out.shape[1] if self.w_out is not None else 0)
