@@ -90,7 +90,7 @@ __device__ __forceinline__ float finish_pair(float g, float u, float limit, floa
   if (FINISH == kGeluTanh) return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
   g = fminf(g, limit);
   u = fminf(fmaxf(u, -limit), limit);
-  return __fdividef(g, 1.0f + __expf(-alpha * g)) * (u + 1.0f);
+  return g / (1.0f + expf(-alpha * g)) * (u + 1.0f);        // as clamped_glu: the full exponential and division
 }
 
 // The tiles of a product: expert e has cuts[e + 1] - cuts[e] equal token parts.
