@@ -7,12 +7,10 @@
 // expert's c tokens are cut into ceil(c / 256) equal parts, rounded up to a multiple of 32.  Decoded tokens then cost what reading
 // the weights costs, and a prompt's tiles are 84 to 95 % tokens.
 //
-// Operands: the weights (K-major rows) come as 128 x 64 boxes by TMA.  Token rows that stand anywhere in x (row_of_place) come as
-// gathered rows (tile::gather4, four rows of 64 numbers an instruction, one instruction a lane of the producer warp); rows that stand
-// side by side in place order come as boxes of 16 rows.  Gathered rows are slow to fetch (a prompt of 2,048 tokens, 8,192 places of
-// 4,096 numbers against 32 matrices of 6,144 rows: 1,101 us; side by side 491 us), so a caller with room for it copies them side by
-// side first (moe_rows: 14 us there, and no loss at any count: 317.8 us gathered and 312.4 us copied for a whole feed-forward of 32
-// places, 48.0 and 48.6 us at a width of 1,024).  Each CTA of the pair loads half of a tile's tokens.  Places past an expert's last one are computed from whatever row is there and not
+// Operands: the weights (K-major rows) come as 128 x 64 boxes by TMA, the tokens' rows, side by side in place order, as boxes of 16 rows.
+// The caller copies them there first (moe_rows: 14 us for 8,192 places of 4,096 numbers); fetched from where they stand by
+// tile::gather4, four rows an instruction, the product of a prompt of 2,048 tokens with 32 matrices of 6,144 rows took 1,101 us instead of
+// 491, and 32 places gained nothing either.  Each CTA of the pair loads half of a tile's tokens.  Places past an expert's last one are computed from whatever row is there and not
 // stored.
 //
 // Per CTA, by warp (the roles and barriers of gemm_tcgen05_pair.cu): warp 4 producer; warp 5 allocates TMEM and, in the first CTA,
@@ -69,12 +67,6 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
       ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(c0), "r"(c1) : "memory");
 }
-// Four rows of the matrix, 64 numbers each from column c0 on, one below the other.
-__device__ __forceinline__ void tma_gather4_pair(uint32_t dst, const CUtensorMap* map, int c0, int4 rows, uint32_t bar_cluster) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6, "
-      "%7}], [%2];\n" ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(c0), "r"(rows.x), "r"(rows.y), "r"(rows.z), "r"(rows.w) : "memory");
-}
 __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
                ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
@@ -112,9 +104,9 @@ struct Walk {
   }
 };
 
-template <int FINISH, bool GATHER>
+template <int FINISH>
 __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-                                                                  const int* __restrict__ rows, const int* __restrict__ plan, int E,
+                                                                  const int* __restrict__ plan, int E,
                                                                   __nv_bfloat16* __restrict__ out, int ldo, int N, int K,
                                                                   const float* __restrict__ place_scale, float limit, float alpha,
                                                                   int* __restrict__ err) {
@@ -192,14 +184,6 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
       const int half = part >> 1;                          // this CTA's tokens: 16 .. 128
       const int mine = p0 + (int)rank * half;
       const int wrow = walk.expert * N + n_tile * 2 * BM + (int)rank * BM;
-      int4 r4 = make_int4(0, 0, 0, 0);
-      if (GATHER && lane * 4 < half) {
-        const int live = count - (int)rank * half;         // of this CTA's tokens
-        int* r = reinterpret_cast<int*>(&r4);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (lane * 4 + i < live) r[i] = rows[mine + lane * 4 + i];
-      }
       for (int kb = 0; kb < kblocks; ++kb, ++issued) {
         const int s = issued % kStages;
         const bool ok = mbar_wait_bounded(smem_addr(&empty_bar[s]), ((issued / kStages) & 1) ^ 1, aborted);
@@ -216,11 +200,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
           tma_load_2d_pair(a_dst, &map_w, kb * BK, wrow, bar);
         }
         __syncwarp();
-        if (GATHER) {
-          if (lane * 4 < half) tma_gather4_pair(a_dst + A_BYTES + (uint32_t)lane * (4 * BK * 2), &map_x, kb * BK, r4, bar);
-        } else {
-          if (lane * 16 < half) tma_load_2d_pair(a_dst + A_BYTES + (uint32_t)lane * (16 * BK * 2), &map_x, kb * BK, mine + lane * 16, bar);
-        }
+        if (lane * 16 < half) tma_load_2d_pair(a_dst + A_BYTES + (uint32_t)lane * (16 * BK * 2), &map_x, kb * BK, mine + lane * 16, bar);
       }
     }
   } else if (warp == 5) {
@@ -322,17 +302,17 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
 }
 
 template <int FINISH>
-int launch(const void* x, int ldx, int x_rows, const int* rows, const void* W, void* out, int ldo, const int* plan, int E, int pairs, int N, int K,
+int launch(const void* x, int ldx, int x_rows, const void* W, void* out, int ldo, const int* plan, int E, int pairs, int N, int K,
            const float* place_scale, float limit, float alpha, int* err, cudaStream_t s) {
   CUtensorMap mx, mw;
-  int rc = tensor_map_2d_bf16(x, x_rows, K, ldx, rows ? 1 : 16, &mx);
+  int rc = tensor_map_2d_bf16(x, x_rows, K, ldx, 16, &mx);
   if (rc) return rc;
   rc = tensor_map_2d_bf16(W, (long long)E * N, K, K, BM, &mw);
   if (rc) return rc;
   const size_t smem = (size_t)kStages * STAGE + 1024;
-  auto kern = rows ? moe_tcgen05_kernel<FINISH, true> : moe_tcgen05_kernel<FINISH, false>;
-  static SharedLimit limits[2];
-  cudaError_t e = limits[rows != nullptr].raise((const void*)kern, smem);
+  auto kern = moe_tcgen05_kernel<FINISH>;
+  static SharedLimit limit_of;
+  cudaError_t e = limit_of.raise((const void*)kern, smem);
   if (e != cudaSuccess) return (int)e;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -341,7 +321,7 @@ int launch(const void* x, int ldx, int x_rows, const int* rows, const void* W, v
   const long long most = ((long long)pairs / BNMAX + (pairs < E ? pairs : E)) * ((N + 2 * BM - 1) / (2 * BM));
   long long grid_pairs = sms / 2;
   if (most < grid_pairs) grid_pairs = most;
-  e = launch_kernel(kern, dim3((unsigned)(2 * grid_pairs)), dim3(kThreads), smem, s, 2, mx, mw, rows, plan, E, (__nv_bfloat16*)out, ldo, N, K,
+  e = launch_kernel(kern, dim3((unsigned)(2 * grid_pairs)), dim3(kThreads), smem, s, 2, mx, mw, plan, E, (__nv_bfloat16*)out, ldo, N, K,
                     place_scale, limit, alpha, err);
   if (e != cudaSuccess) return (int)e;
   return launch_status();
@@ -367,21 +347,21 @@ ARLE_API int arle_moe_rows(const void* x, int ldx, const int* rows, void* dst, i
   return launch_status();
 }
 
-// x bfloat16 [x_rows, K] (rows != null: the place's row of x; null: x is in place order), W bfloat16 [E][N][K] contiguous,
+// x bfloat16 [x_rows, K] in place order, W bfloat16 [E][N][K] contiguous,
 // out bfloat16 [pairs, N], or [pairs, N / 2] for the gated finishes (W's rows 2i and 2i + 1: gate_i and up_i).
 // finish: 0 none, 1 square of relu, 2 silu gate, 3 gelu (tanh) gate, 4 clamped gate (limit, alpha).  Needs K and ldx multiples of 8
 // and 16-byte aligned x and W.  err: set to 4 if a bounded wait ran out.
-ARLE_API int arle_moe_gemm_tcgen05(const void* x, int ldx, int x_rows, const int* rows, const void* W, void* out, int ldo, const int* plan, int E,
+ARLE_API int arle_moe_gemm_tcgen05(const void* x, int ldx, int x_rows, const void* W, void* out, int ldo, const int* plan, int E,
                                    int pairs, int N, int K, const float* place_scale, int finish, float limit, float alpha, int* err,
                                    cudaStream_t s) {
   if (pairs <= 0 || N <= 0) return 0;
   if (K <= 0 || E <= 0 || finish < 0 || finish > 4 || x_rows <= 0 || (finish >= 2 && N % 2)) return ARLE_E_BADARG;
   if (E > kMaxExperts || K % 8 || ldx % 8 || ((uintptr_t)x & 15) || ((uintptr_t)W & 15) || (long long)E * N > 0x7fffffffll) return ARLE_E_UNSUPPORTED;
   switch (finish) {
-    case kNone: return launch<kNone>(x, ldx, x_rows, rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
-    case kSquareRelu: return launch<kSquareRelu>(x, ldx, x_rows, rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
-    case kSilu: return launch<kSilu>(x, ldx, x_rows, rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
-    case kGeluTanh: return launch<kGeluTanh>(x, ldx, x_rows, rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
-    default: return launch<kClamped>(x, ldx, x_rows, rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
+    case kNone: return launch<kNone>(x, ldx, x_rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
+    case kSquareRelu: return launch<kSquareRelu>(x, ldx, x_rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
+    case kSilu: return launch<kSilu>(x, ldx, x_rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
+    case kGeluTanh: return launch<kGeluTanh>(x, ldx, x_rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
+    default: return launch<kClamped>(x, ldx, x_rows, W, out, ldo, plan, E, pairs, N, K, place_scale, limit, alpha, err, s);
   }
 }

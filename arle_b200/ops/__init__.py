@@ -111,7 +111,7 @@ _SIGNATURES = {
     "arle_moe_plan": [_P, _I, _I, _I, _P, _P, _P, _P, _P, _P],
     "arle_moe_gemm": [_P, _I, _P, _P, _I, ctypes.c_long, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _P, _I, _P],
     "arle_moe_rows": [_P, _I, _P, _P, _I, _I, _P],
-    "arle_moe_gemm_tcgen05": [_P, _I, _I, _P, _P, _P, _I, _P, _I, _I, _I, _I, _P, _I, _F, _F, _P, _P],
+    "arle_moe_gemm_tcgen05": [_P, _I, _I, _P, _P, _I, _P, _I, _I, _I, _I, _P, _I, _F, _F, _P, _P],
     "arle_layernorm": [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P],
     "arle_branch_layernorm_add": [_P, _P, _I, _P, _P, _I, _I, _I, _F, _P, _I, _P, ctypes.c_long, _P, _P, _P],
     "arle_input_conv": [_P, _P, _P, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
@@ -1768,7 +1768,11 @@ def _moe_tcgen05_takes(x, w, pairs: int, experts: int) -> bool:
 
 
 def _moe_gemm_tcgen05(x, rows, w, out, plan, experts, place_scale, finish: int, limit: float, alpha: float) -> None:
-    _check(library().arle_moe_gemm_tcgen05(_ptr(x), x.stride(0), x.shape[0], _ptr(rows), _ptr(w), _ptr(out), out.stride(0), _ptr(plan), experts,
+    if rows is not None:                                    # the kernel reads its rows side by side (the engine has copied them: ``moe_rows``)
+        side = torch.empty((out.shape[0], x.shape[1]), dtype=x.dtype, device=x.device)
+        moe_rows(x, rows, side)
+        x = side
+    _check(library().arle_moe_gemm_tcgen05(_ptr(x), x.stride(0), x.shape[0], _ptr(w), _ptr(out), out.stride(0), _ptr(plan), experts,
                                            out.shape[0], w.shape[1], x.shape[1], _ptr(place_scale), finish, limit, alpha,
                                            _ptr(error_flag(x.device)), _stream()), "moe_gemm_tcgen05")
 
