@@ -1,8 +1,9 @@
 // A causal convolution of four taps per channel over the tokens of every row, several tokens a thread: the four inputs of a token
 // slide through registers, so a row of x is read once (and the three before a thread's first token once more) instead of four times,
 // VEC channels an access.  Sums in the order of the kernels that take a token a thread (causal_conv, conv_silu): the same bits.
-// What bounds it: memory.  2,048 tokens of 10,240 channels, bfloat16: 57 us (a token a
-// thread: 172); 1,999 tokens of 8,192 55 us (135).
+// What bounds it: a thread's chain of four loads ahead, the sums, the exponentials and divisions of silu; memory is at a quarter of its rate
+// (2,048 tokens of 10,240 channels, bfloat16, 84 MB: 57 us with the launch that brings the state up to date; a token a thread took 172;
+// 1,999 tokens of 8,192 55 us, 135).
 #pragma once
 #include "common.cuh"
 

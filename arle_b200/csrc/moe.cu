@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(256) moe_gemv_kernel(const __nv_bfloat16* __re
 
 // dtype: type of A and C; w_dtype: type of W [E][N][K] (an expert every w_expert elements).  pairs: places in all.
 // place_scale float32 [pairs] or null, act 0 none / 1 square of relu: see finish_sum.
-// fast: few pairs of bfloat16 operands with aligned rows take the dot products (many take moe_tcgen05.cu).
+// fast: few pairs of bfloat16 operands with aligned rows take the dot products (from 24 pairs on the caller takes moe_tcgen05.cu).
 ARLE_API int arle_moe_gemm(const void* A, int lda, const int* rows, const void* W, int ldw, long w_expert, void* C, int ldc,
                            int dtype, int w_dtype, const int* plan, int E, int pairs, int N, int K, int fast,
                            const float* place_scale, int act, cudaStream_t s) {
