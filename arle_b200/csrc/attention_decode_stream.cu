@@ -523,10 +523,12 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(
 #pragma unroll
             for (int e = 0; e < 4; ++e) s[nn][e] += s2[nn][e];
           float mx0 = -INFINITY, mx1 = -INFINITY;
+          uint32_t keep[2];                                    // of a pair of values, those of keys in range: see below
 #pragma unroll
           for (int nn = 0; nn < 2; ++nn) {
             const int kj = kbeg + 8 * nn + 2 * tq;
             const bool in0 = kj < kv_len && kj >= lo, in1 = kj + 1 < kv_len && kj + 1 >= lo;
+            keep[nn] = (in0 ? 0xffffu : 0u) | (in1 ? 0xffff0000u : 0u);
             s[nn][0] = in0 ? s[nn][0] * scale_log2 : -INFINITY;
             s[nn][1] = in1 ? s[nn][1] * scale_log2 : -INFINITY;
             s[nn][2] = in0 ? s[nn][2] * scale_log2 : -INFINITY;
@@ -571,8 +573,9 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(
             uint32_t b0, b1, b2, b3;
             ldsm_x4_t(vt + (j >> 3) * (16 * 128) + (uint32_t)(((lane >> 3) & 1) * 8 + (lane & 7)) * 128 + (((j & 7) ^ sw) << 4),
                       b0, b1, b2, b3);
-            mma_bf16(o[2 * dn], pa, b0, b1);
-            mma_bf16(o[2 * dn + 1], pa, b2, b3);
+            // a slot out of range holds what another request or an older token left: its weight is zero, but zero times infinity is not
+            mma_bf16(o[2 * dn], pa, b0 & keep[0], b1 & keep[1]);
+            mma_bf16(o[2 * dn + 1], pa, b2 & keep[0], b3 & keep[1]);
           }
         }
         __syncwarp();

@@ -149,3 +149,35 @@ def test_decay_memories(dim, vdim, ones):
     ok = out.isfinite()
     assert torch.equal(out[:64], clean[:64])
     assert (out[ok] - scan[ok]).norm() <= 1e-5 * scan[ok].norm()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("page", [16, 32])
+@pytest.mark.parametrize("window", [None, 40])
+@pytest.mark.parametrize("rows", [[(1, 70), (1, 300), (1, 0), (1, 31)], [(1, 517)]], ids=["four", "one"])
+def test_decoded_tokens_do_not_see_other_slots_of_a_page(hd, page, window, rows):
+    """What a page's former owner left behind the last token, and what lies in front of the window."""
+    nq, nkv, kvs = 8, 2, [n + s for n, s in rows]
+    cm = CacheManager([CacheNeed(nkv, hd, window)], [], page, sum(-(-k // page) for k in kvs) + 2, len(rows), max(kvs), BF, DEV)
+    for i, (n, s) in enumerate(rows):
+        cm.add_request(i)
+        if s:
+            cm.append([(i, s)])
+    cm.append([(i, 1) for i in range(len(rows))])
+    ctx = StepContext(cm, Workspace(DEV)).build([StepEntry(i, [0]) for i in range(len(rows))], [s for _, s in rows])
+    view, g = ctx.cache_view(0), torch.Generator(device=DEV).manual_seed(2)
+    q = torch.empty(len(rows), nq * hd, device=DEV, dtype=BF).normal_(generator=g)
+    new = [[torch.empty(k, nkv, hd, device=DEV, dtype=BF).normal_(generator=g) for _ in range(2)] for k in kvs]
+    outs = []
+    for fill in (0.0, INF, math.nan):
+        for a, which in ((view.k, 0), (view.v, 1)):
+            a.fill_(fill)
+            for i, k in enumerate(kvs):
+                first = max(0, k - window) if window else 0
+                s = torch.from_numpy(cm.slot_mapping(0, i, 0, k)).long().to(DEV)[first:]
+                a.permute(0, 2, 1, 3)[s // page, s % page] = new[i][which][first:]
+        outs.append(torch.empty(len(rows), nq * hd, device=DEV, dtype=BF))
+        ops.paged_attention(q, outs[-1], view.k, view.v, ctx.positions, ctx.row_of_token, view.block_table, nq, nkv, hd, page, hd ** -0.5, window,
+                            batch=ctx)
+    assert outs[0].isfinite().all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    ops.check_errors(DEV)
