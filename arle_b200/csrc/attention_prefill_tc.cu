@@ -138,6 +138,7 @@ struct Block {
   int r, h, kvh, t0, mbeg;
   int rows_x[2], pf_x[2], pl_x[2], jlo_x[2], jhi_x[2];
   int kb, ntiles, lo, p_last;
+  int kv_end;        // keys of the request
   int nk, keep;      // key tiles of kept first keys in front of the window's tiles (tile j < nk starts at key j * BKV), and how many keys are kept
   // false: the block is beyond the request's queries (or the request is one that the decode kernel serves)
   __device__ bool init(int b, int nq, int nkv, int nyb, const int* q_indptr, const int* kv_lens, int window, int skip_single,
@@ -153,6 +154,7 @@ struct Block {
     if (mbeg >= qlen || (skip_single && qlen == 1)) return false;
     const int kv_len = kv_lens[r];
     const int pos0 = kv_len - qlen;
+    kv_end = kv_len;
     kvh = h / (nq / nkv);
     // The two query tiles: rows, positions of the first and last row, first key, tiles [jlo, jhi) of
     // the block's sequence of key tiles (which starts at kb, a multiple of 128).
@@ -197,7 +199,8 @@ __global__ void __launch_bounds__(kThreads, 1) paged_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out, const int* __restrict__ q_indptr,
     const int* __restrict__ kv_lens, const int* __restrict__ block_table, int bt_stride, int bt_width, int nq, int nkv,
     int page_size, float scale_log2, HeadTail<__nv_bfloat16> tail, int window, int skip_single, int nyb, int nblocks, int ticket_slot, int* __restrict__ err,
-    int keep_arg, float cap_arg, float scale_over_cap, int chunk_arg, const float* __restrict__ pb, int row_behind) {
+    int keep_arg, float cap_arg, float scale_over_cap, int chunk_arg, const float* __restrict__ pb, const __nv_bfloat16* __restrict__ v_cache,
+    int row_behind) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr bool EXT = FORM == 1, SIG = FORM == 2;
@@ -348,21 +351,42 @@ __global__ void __launch_bounds__(kThreads, 1) paged_prefill_tc_kernel(
           // Value rows that no query of the block sees meet P = 0, and zero times what another request's tile left there may be NaN: they
           // are loaded from behind the cache's last row, which fills them with zeros.
           if (!keys && lane < 16 && row < 0) row = row_behind;
-          const int n = __popc(__ballot_sync(0xffffffffu, row >= 0)) >> 1;      // pages of this tile
+          // The slots of a page behind the request's last token hold what the page's former owner left, which no weight of zero makes
+          // harmless either: where the request ends inside the block's last box of values, the warp copies the box itself, with zeros
+          // behind the end.
+          const int tile0 = blk.template tile_key<EXT>(j), cut = !keys && (blk.p_last ^ (blk.kv_end - 1)) < 16 ? blk.kv_end & 15 : 0;
+          const int cut_box = (blk.p_last - tile0) >> 4;                        // of the tile's eight, if it is one of them
+          const int cut_row = __shfl_sync(0xffffffffu, row, 2 * (cut_box & 7));
+          const bool own = cut && cut_box >= 0 && cut_box < 8;
+          if (own && lane < 16 && c == cut_box) row = -1;
+          const int n = __popc(__ballot_sync(0xffffffffu, row >= 0)) >> 1;      // pages of this tile that TMA brings
           uint64_t* full = keys ? &k_full[st] : &v_full[st];
           int go = 1;
           if (lane == 0) {
             if (!mbar_wait_bounded(smem_addr(keys ? &k_empty[st] : &v_empty[st]), par ^ 1, aborted)) {
               abort_flag = 1;
               go = 0;
-            } else {
+            } else if (!own) {
               mbar_expect_tx(smem_addr(full), (uint32_t)n * 4096u);
             }
           }
           go = __shfl_sync(0xffffffffu, go, 0);
-          if (!go || *aborted) {
+          if (__any_sync(0xffffffffu, !go || *aborted)) {
             stop = true;
             break;
+          }
+          if (own) {
+            const uint4* src = reinterpret_cast<const uint4*>(v_cache + (size_t)cut_row * HD);
+#pragma unroll 4
+            for (int i = lane; i < 16 * 16; i += 32) {                          // 16 rows of 16 pieces of 16 bytes, swizzled as TMA does
+              const int r = i >> 4, piece = i & 15;
+              *reinterpret_cast<uint4*>(tile_s + st * TILE + (piece >> 3) * SUB + (cut_box * 16 + r) * 128 + (((piece & 7) ^ (r & 7)) << 4)) =
+                  r < cut ? src[i] : make_uint4(0, 0, 0, 0);
+            }
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_expect_tx(smem_addr(full), (uint32_t)n * 4096u);
+            __syncwarp();
           }
           if (row >= 0) tma_load_2d(smem_addr(tile_s + st * TILE + half * SUB + c * 2048), map, half * 64, row, smem_addr(full));
           ++issued;
@@ -727,7 +751,7 @@ ARLE_API int arle_paged_attention_prefill_tc(const void* q, int q_row_stride, in
                                 q_indptr, kv_lens, block_table, bt_stride, bt_width, nq, nkv, page_size,
                                 scale * 1.4426950408889634f, HeadTail<__nv_bfloat16>{sinks, (const __nv_bfloat16*)gate, gate_stride}, window, skip_single, nyb, (int)nblocks, ticket_slot, err,
                                 window > 0 ? keep_first : 0, softcap > 0.f ? softcap * 1.4426950408889634f : 0.f,
-                                softcap > 0.f ? scale / softcap : 0.f, chunk, pb, (int)(cache_rows < 0x7fffffff ? cache_rows : 0x7fffffff));
+                                softcap > 0.f ? scale / softcap : 0.f, chunk, pb, (const __nv_bfloat16*)v_cache, (int)(cache_rows < 0x7fffffff ? cache_rows : 0x7fffffff));
   if (e != cudaSuccess) return (int)e;
   return launch_status();
 }

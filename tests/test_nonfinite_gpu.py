@@ -157,27 +157,47 @@ def test_decay_memories(dim, vdim, ones):
 @pytest.mark.parametrize("rows", [[(1, 70), (1, 300), (1, 0), (1, 31)], [(1, 517)]], ids=["four", "one"])
 def test_decoded_tokens_do_not_see_other_slots_of_a_page(hd, page, window, rows):
     """What a page's former owner left behind the last token, and what lies in front of the window."""
+    _other_slots(hd, page, window, rows, window)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("page,window", [(16, None), (32, 40), (64, 300)])
+@pytest.mark.parametrize("rows", [[(70, 0), (300, 5), (33, 0), (256, 0)], [(1, 70), (45, 3), (16, 0), (2, 126)], [(513, 130)]], ids=["rows", "mixed", "one"])
+@pytest.mark.parametrize("form", ["softmax", "cap", "kept", "sigmoid"])
+def test_prompts_do_not_see_other_slots_of_a_page(hd, page, window, rows, form):
+    """What a page's former owner left behind the last token."""
+    if form == "kept" and not window:
+        return
+    extra = {"softmax": {}, "cap": {"softcap": 20.0}, "kept": {"keep_first": 5},
+             "sigmoid": {"score_bias": torch.zeros(8, device=DEV)}}[form]
+    _other_slots(hd, page, window, rows, None, **extra)
+
+
+def _other_slots(hd, page, window, rows, held, **extra):
+    """held: the last keys of a request that hold numbers (None: all)."""
     nq, nkv, kvs = 8, 2, [n + s for n, s in rows]
-    cm = CacheManager([CacheNeed(nkv, hd, window)], [], page, sum(-(-k // page) for k in kvs) + 2, len(rows), max(kvs), BF, DEV)
+    cm = CacheManager([CacheNeed(nkv, hd, window, keep_first=extra.get("keep_first", 0))], [], page, sum(-(-k // page) for k in kvs) + 2, len(rows), max(kvs),
+                      BF, DEV)
     for i, (n, s) in enumerate(rows):
         cm.add_request(i)
         if s:
             cm.append([(i, s)])
-    cm.append([(i, 1) for i in range(len(rows))])
-    ctx = StepContext(cm, Workspace(DEV)).build([StepEntry(i, [0]) for i in range(len(rows))], [s for _, s in rows])
+    cm.append([(i, n) for i, (n, _) in enumerate(rows)])
+    ctx = StepContext(cm, Workspace(DEV)).build([StepEntry(i, [0] * n) for i, (n, _) in enumerate(rows)], [s for _, s in rows])
+    T = sum(n for n, _ in rows)
     view, g = ctx.cache_view(0), torch.Generator(device=DEV).manual_seed(2)
-    q = torch.empty(len(rows), nq * hd, device=DEV, dtype=BF).normal_(generator=g)
+    q = torch.empty(T, nq * hd, device=DEV, dtype=BF).normal_(generator=g)
     new = [[torch.empty(k, nkv, hd, device=DEV, dtype=BF).normal_(generator=g) for _ in range(2)] for k in kvs]
     outs = []
     for fill in (0.0, INF, math.nan):
         for a, which in ((view.k, 0), (view.v, 1)):
             a.fill_(fill)
             for i, k in enumerate(kvs):
-                first = max(0, k - window) if window else 0
+                first = max(0, k - held) if held else 0
                 s = torch.from_numpy(cm.slot_mapping(0, i, 0, k)).long().to(DEV)[first:]
                 a.permute(0, 2, 1, 3)[s // page, s % page] = new[i][which][first:]
-        outs.append(torch.empty(len(rows), nq * hd, device=DEV, dtype=BF))
+        outs.append(torch.empty(T, nq * hd, device=DEV, dtype=BF))
         ops.paged_attention(q, outs[-1], view.k, view.v, ctx.positions, ctx.row_of_token, view.block_table, nq, nkv, hd, page, hd ** -0.5, window,
-                            batch=ctx)
+                            batch=ctx, **extra)
     assert outs[0].isfinite().all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     ops.check_errors(DEV)
