@@ -1,19 +1,20 @@
 // A causal convolution of four taps per channel over the tokens of every row, several tokens a thread: the four inputs of a token
 // slide through registers, so a row of x is read once (and the three before a thread's first token once more) instead of four times,
 // VEC channels an access.  Sums in the order of the kernels that take a token a thread (causal_conv, conv_silu): the same bits.
-// What bounds it: a thread's chain of four loads ahead, the sums, the exponentials and divisions of silu; memory is at a quarter of its rate
-// (2,048 tokens of 10,240 channels, bfloat16, 84 MB: 57 us with the launch that brings the state up to date; a token a thread took 172;
-// 1,999 tokens of 8,192 55 us, 135).
+// What bounds it: instructions, the exponentials and divisions of silu above all (37 an element, and a division has a branch of its own, so that
+// the next one waits); memory is at a third of its rate.  Four channels a thread leave room for six blocks an SM: 2,048 tokens of 10,240
+// channels, bfloat16, 84 MB 42.6 us, 1,999 tokens of 8,192 35 us, 300 of 2,304 14.6 (eight channels a thread, three blocks an SM: 57.7, 53 and
+// 20.8; five blocks 51; eight blocks spill, 45; two channels 52; 32 tokens a thread 45).
 #pragma once
 #include "common.cuh"
 
 namespace arle {
 
-constexpr int kConvTokens = 16, kConvAhead = 4, kConvThreads = 128;
+constexpr int kConvTokens = 16, kConvAhead = 4, kConvThreads = 128, kConvVec = 4;
 
 // in_bias is added to a row's inputs (not to what the state holds); act 1: silu.
 template <typename TI, typename TO, int VEC>
-__global__ void __launch_bounds__(kConvThreads) conv_window_kernel(const TI* __restrict__ x, int x_stride, const float* __restrict__ in_bias,
+__global__ void __launch_bounds__(kConvThreads, 6) conv_window_kernel(const TI* __restrict__ x, int x_stride, const float* __restrict__ in_bias,
                                                                    const float* __restrict__ w, const float* __restrict__ out_bias, int act,
                                                                    const float* __restrict__ state, long slot_stride, long conv_off,
                                                                    const int* __restrict__ q_indptr, const int* __restrict__ row_of_token,
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(kConvThreads) conv_window_kernel(const TI* __r
 // Whether it takes these arrays: four taps, several tokens a row, channels in whole groups on their boundaries.
 template <typename TI, typename TO>
 inline bool conv_window_takes(const void* x, int x_stride, const float* w, const void* out, int out_stride, int T, int R, int C, int taps) {
-  constexpr int VEC = sizeof(TI) == 2 ? 8 : 4;
+  constexpr int VEC = kConvVec;
   return taps == 4 && T >= 4 * R && T >= 32 && C % VEC == 0 && x_stride % VEC == 0 && out_stride % VEC == 0 && vec_aligned<VEC>(x, sizeof(TI)) &&
          vec_aligned<VEC>(out, sizeof(TO)) && ((uintptr_t)w & 15) == 0 && (T + kConvTokens - 1) / kConvTokens <= 65535;
 }
@@ -94,7 +95,7 @@ template <typename TI, typename TO>
 inline void launch_conv_window(const void* x, int x_stride, const float* in_bias, const float* w, const float* out_bias, int act, const float* state,
                                long slot_stride, long conv_off, const int* q_indptr, const int* row_of_token, const int* state_slots, void* out,
                                int out_stride, int T, int C, cudaStream_t s) {
-  constexpr int VEC = sizeof(TI) == 2 ? 8 : 4;
+  constexpr int VEC = kConvVec;
   const dim3 grid((C / VEC + kConvThreads - 1) / kConvThreads, (T + kConvTokens - 1) / kConvTokens);
   launch_kernel(conv_window_kernel<TI, TO, VEC>, grid, dim3(kConvThreads), 0, s, 1, (const TI*)x, x_stride, in_bias, w, out_bias, act, state,
                 slot_stride, conv_off, q_indptr, row_of_token, state_slots, (TO*)out, out_stride, T, C);

@@ -44,6 +44,11 @@ def test_convolution_window_gives_the_same_bits(dtype, lens, C):
         assert torch.equal(o1, o2) and torch.equal(s1, s2)
 
 
+@pytest.mark.parametrize("C", [4, 260])                          # groups of four channels, of which eight do not make whole ones
+def test_convolution_window_of_channels_in_fours(C):
+    test_convolution_window_gives_the_same_bits(torch.bfloat16, [37, 1, 2, 80, 3], C)
+
+
 @pytest.mark.parametrize("inner,parts,skip", [(1024, 1, True), (8192, 1, True), (8192, 2, False), (4160, 1, True), (2048 * 3, 3, True)])
 def test_gated_group_norm(inner, parts, skip):
     g = torch.Generator(device=DEV).manual_seed(inner)
