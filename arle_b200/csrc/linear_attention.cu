@@ -105,6 +105,58 @@ __device__ __forceinline__ float4 widen4(uint2 u) {
 template <typename T, bool VEC> struct Raw4 { using type = float4; };
 template <> struct Raw4<__nv_bfloat16, true> { using type = uint2; };
 
+// A long row as segments that are scanned side by side, each from an empty memory but the first; gla_join then forms the memory in front of
+// every segment (S <- diag(D) S + what the segment alone leaves, D the product of its decays), and gla_carry adds what the segment's tokens read
+// from it, o_t += (D_t q_t) S with D_t the product of the segment's decays up to t.  One scan of 2,048 tokens, 16 heads of 128 x 128, keeps a
+// single warp on each scheduler (37 % of the issue slots); sixteen segments keep three.  SEGMENT_FIGURES
+// A row's own length decides how it is cut: from kSegFrom tokens on (below, the two further launches cost what the shorter chain gains), in
+// parts of kSegTokens and more, sixteen at most, which bounds the memories between them.
+constexpr int kSegTokens = 128, kSegFrom = 384, kMostSegs = 16;
+struct Segments {
+  float* left;                                   // [cut][head][vdim][dim]: the memory that a segment leaves
+  float* decay;                                  // [cut][head][dim]: the product of its decays
+  float* q_decayed;                              // [tokens][head][dim]: D_t q_t, scaled; written for all segments but a row's first
+  int rows;
+};
+__device__ __forceinline__ int segment_tokens(int n) {
+  if (n < kSegFrom) return n > 0 ? n : 1;
+  const int parts = min(kMostSegs, n / kSegTokens);
+  return ((n + parts - 1) / parts + 15) / 16 * 16;
+}
+// The row and the segment of a slot (all of a warp's lanes together), false if there is no such slot.  Slots are counted over all segments of
+// all rows (ALL), or over those of rows in several segments; `cut` is the slot's number among the latter.
+template <bool ALL>
+__device__ __forceinline__ bool segment_of(int slot, const int* q_indptr, int rows, int& row, int& seg, int& parts, int& cut) {
+  const int lane = threadIdx.x & 31;
+  int before = 0, cut_before = 0;
+  for (int r0 = 0; r0 < rows; r0 += 32) {
+    int n = 0;
+    if (r0 + lane < rows) {
+      const int tokens = q_indptr[r0 + lane + 1] - q_indptr[r0 + lane], len = segment_tokens(tokens);
+      n = max(1, (tokens + len - 1) / len);
+    }
+    const int n_cut = n > 1 ? n : 0, mine = ALL ? n : n_cut;
+    int sum = mine, cut_sum = n_cut;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, sum, o), z = __shfl_up_sync(0xffffffffu, cut_sum, o);
+      if (lane >= o) sum += y, cut_sum += z;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, slot < before + sum);
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      row = r0 + src;
+      parts = __shfl_sync(0xffffffffu, n, src);
+      seg = slot - before - __shfl_sync(0xffffffffu, sum - mine, src);
+      cut = cut_before + __shfl_sync(0xffffffffu, cut_sum - n_cut, src) + seg;
+      return true;
+    }
+    before += __shfl_sync(0xffffffffu, sum, 31);
+    cut_before += __shfl_sync(0xffffffffu, cut_sum, 31);
+  }
+  return false;
+}
+
 // DPT: consecutive key channels that a thread keeps of each of its kScanCpt columns of the state (4 up to 128
 // channels, then 8, 16).  LPC: lanes that share a column (a power of two; LPC * DPT >= dim).  VEC: four channels
 // at a time can be fetched with one aligned load.  A chunk of CHUNK tokens is staged in shared memory; while it is
@@ -123,11 +175,12 @@ constexpr int few_blocks() {
   if (LPC == 1) return 3;
   return VEC && !BONUS && LPC >= 4 ? 5 : 4;
 }
-template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool LONG>
-__global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LPC, VEC, BONUS>()) gla_scan_kernel(
+// SEGS: a row in segments, see Segments above.
+template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool LONG, bool SEGS>
+__global__ void __launch_bounds__(kScanThreads, SEGS ? 3 : LONG ? 1 : few_blocks<T, DPT, LPC, VEC, BONUS>()) gla_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int in_stride,
     const float* __restrict__ alpha, const float* __restrict__ bonus, float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
-    const int* __restrict__ state_slots, float* __restrict__ out, int heads, int dim, int vdim, float q_scale) {
+    const int* __restrict__ state_slots, float* __restrict__ out, int heads, int dim, int vdim, float q_scale, Segments sg) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr int CPT = kScanCpt;
@@ -143,10 +196,23 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
   __shared__ __align__(16) float qs[CHUNK * DPAD], ks[CHUNK * DPAD], as[CHUNK * DPAD];
   constexpr int VD = LONG && LPC >= 4 ? 2 : 1;           // v's numbers stand twice side by side (a factor of both halves of a pair), where there is room
   __shared__ __align__(16) float vs[CHUNK * COLS * VD];
-  const int r = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * COLS;
+  const int h = blockIdx.y, j0 = blockIdx.x * COLS;
   const int l = threadIdx.x & (LPC - 1), jl = threadIdx.x / LPC;
   const int jb = j0 + jl * CPT;                  // this thread's first column
-  const int t_begin = q_indptr[r], t_end = q_indptr[r + 1];
+  int r = blockIdx.z, seg = 0, parts = 1, cut = 0;
+  if constexpr (SEGS) {
+    if (!segment_of<true>(blockIdx.z, q_indptr, sg.rows, r, seg, parts, cut)) return;
+  }
+  int t_begin = q_indptr[r], t_end = q_indptr[r + 1];
+  if constexpr (SEGS) {
+    const int len = segment_tokens(t_end - t_begin);
+    t_begin += seg * len;
+    t_end = min(t_end, t_begin + len);
+  }
+  const bool leads = SEGS && seg > 0 && blockIdx.x == 0 && threadIdx.x < 32;   // the warp that writes D_t q_t
+  f32x2 prod[SEGS ? DPT / 2 : 1];
+#pragma unroll
+  for (int i = 0; i < (SEGS ? DPT / 2 : 1); ++i) prod[i] = pair2(1.f, 1.f);
   // the state of a head is kept as [vdim][dim]: a thread's channels of a column are contiguous
   float* S_g = state + (size_t)state_slots[r] * slot_stride + ((size_t)h * vdim) * dim + l * DPT;
   const bool vec_state = (dim & 3) == 0 && (slot_stride & 3) == 0 && ((uintptr_t)state & 15) == 0;
@@ -161,7 +227,7 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
   f32x2 S[CPT][DPT / 2];                         // channels 2i and 2i + 1 of a column
 #pragma unroll
   for (int cc = 0; cc < CPT; ++cc) {
-    const bool col_ok = jb + cc < vdim;
+    const bool col_ok = jb + cc < vdim && seg == 0;
     const float* sp = S_g + (size_t)(col_ok ? jb + cc : 0) * dim;
 #pragma unroll
     for (int i = 0; i < DPT; i += 4) {
@@ -313,6 +379,14 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
 #pragma unroll
       for (int i = 0; i < DPT / 4; ++i) {
         const ulonglong2 a4 = at[i], k4 = kt[i], q4 = qt[i];
+        if constexpr (SEGS) {
+          if (leads) {
+            prod[2 * i] = mul2(prod[2 * i], a4.x), prod[2 * i + 1] = mul2(prod[2 * i + 1], a4.y);
+            if (l * DPT + 4 * i < dim)
+              *reinterpret_cast<ulonglong2*>(sg.q_decayed + (size_t)(t0 + tt) * a_stride + hq + l * DPT + 4 * i) =
+                  make_ulonglong2(mul2(q4.x, prod[2 * i]), mul2(q4.y, prod[2 * i + 1]));
+          }
+        }
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
           const f32x2 kv0 = mul2(k4.x, vj[cc]), kv1 = mul2(k4.y, vj[cc]);
@@ -386,6 +460,19 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
       }
     }
   }
+  bool vec_left = vec_state;
+  if constexpr (SEGS) {
+    if (parts > 1) {
+      S_g = sg.left + ((size_t)cut * heads + h) * vdim * dim + l * DPT;
+      vec_left = true;                           // dim is a multiple of four here, and the buffer starts on 16 bytes
+    }
+    if (leads) {
+#pragma unroll
+      for (int i = 0; i < DPT; i += 4)
+        if (l * DPT + i < dim)
+          *reinterpret_cast<ulonglong2*>(sg.decay + ((size_t)cut * heads + h) * dim + l * DPT + i) = make_ulonglong2(prod[i / 2], prod[i / 2 + 1]);
+    }
+  }
 #pragma unroll
   for (int cc = 0; cc < CPT; ++cc) {
     const bool col_ok = jb + cc < vdim;
@@ -393,13 +480,122 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
 #pragma unroll
     for (int i = 0; i < DPT; i += 4) {
       const int c = l * DPT + i;
-      if (vec_state) {
+      if (vec_left) {
         if (col_ok && c < dim)
           *reinterpret_cast<ulonglong2*>(sp + i) = make_ulonglong2(S[cc][i / 2], S[cc][i / 2 + 1]);
       } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
           if (col_ok && c + e < dim) sp[i + e] = e & 1 ? high2(S[cc][(i + e) / 2]) : low2(S[cc][(i + e) / 2]);
+      }
+    }
+  }
+}
+
+// left[i] of a row in segments becomes the memory behind its segment i; the last one's goes to the row's slot.  A thread has four channels of a
+// column and runs through the segments, all of whose numbers it asks for first.
+__global__ void __launch_bounds__(256) gla_join_kernel(float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
+                                                       const int* __restrict__ state_slots, int heads, int dim, int vdim, Segments sg) {
+  pdl_launch_dependents();
+  pdl_wait();
+  int r, seg, parts, cut;
+  if (!segment_of<false>(blockIdx.z, q_indptr, sg.rows, r, seg, parts, cut) || seg) return;
+  const int h = blockIdx.y, idx = blockIdx.x * 256 + threadIdx.x, quads = dim / 4;
+  if (idx >= vdim * quads) return;
+  const int e = idx % quads * 4;
+  const size_t step = (size_t)heads * vdim * dim, d_step = (size_t)heads * dim;
+  float* left = sg.left + ((size_t)cut * heads + h) * vdim * dim + (size_t)idx * 4;
+  const float* decay = sg.decay + ((size_t)cut * heads + h) * dim + e;
+  float4 x[kMostSegs], d[kMostSegs];
+#pragma unroll
+  for (int i = 0; i < kMostSegs; ++i)
+    if (i < parts) {
+      x[i] = *reinterpret_cast<const float4*>(left + i * step);
+      d[i] = i ? *reinterpret_cast<const float4*>(decay + i * d_step) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  float4 S = x[0];
+#pragma unroll
+  for (int i = 1; i < kMostSegs; ++i)
+    if (i < parts) {
+      S = make_float4(fmaf(d[i].x, S.x, x[i].x), fmaf(d[i].y, S.y, x[i].y), fmaf(d[i].z, S.z, x[i].z), fmaf(d[i].w, S.w, x[i].w));
+      if (i + 1 < parts) *reinterpret_cast<float4*>(left + i * step) = S;
+    }
+  float* sp = state + (size_t)state_slots[r] * slot_stride + (size_t)h * vdim * dim + (size_t)idx * 4;
+  sp[0] = S.x, sp[1] = S.y, sp[2] = S.z, sp[3] = S.w;
+}
+
+// o_t[j] += sum over d of q_decayed[t][d] left[j][d] for the tokens of every segment but a row's first; left: of the segment in front.  A block
+// has 128 columns and runs through the segment 64 tokens at a time; a thread eight tokens and four columns, two channels to a packed FMA, and
+// sums of 32 channels at a time, so that they are rounded as often as the scan's.
+constexpr int kCarryTokens = 64, kCarryCols = 128, kCarryPitch = 132;   // floats a row: eight rows' 16 bytes fall on different banks
+constexpr size_t kCarrySmem = (size_t)(kCarryTokens + kCarryCols) * kCarryPitch * sizeof(float);
+__global__ void __launch_bounds__(256, 2) gla_carry_kernel(const int* __restrict__ q_indptr, float* __restrict__ out, int heads, int dim, int vdim,
+                                                           Segments sg) {
+  pdl_launch_dependents();
+  pdl_wait();
+  int r, seg, parts, cut;
+  if (!segment_of<false>(blockIdx.z, q_indptr, sg.rows, r, seg, parts, cut) || seg == 0) return;
+  extern __shared__ __align__(16) float sm[];
+  float* qs = sm;                                // [tokens][pitch], zeros past dim
+  float* ms = qs + kCarryTokens * kCarryPitch;   // [columns][pitch]
+  const int h = blockIdx.y, j0 = blockIdx.x * kCarryCols, tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+  const int beg = q_indptr[r], end = q_indptr[r + 1], len = segment_tokens(end - beg);
+  const int t_begin = beg + seg * len, t_end = min(end, t_begin + len);
+  const float* left = sg.left + ((size_t)(cut - 1) * heads + h) * vdim * dim;
+  for (int i = tid; i < kCarryCols * 32; i += 256) {
+    const int j = i >> 5, e = (i & 31) * 4;
+    const float4 x = (j0 + j < vdim && e < dim) ? *reinterpret_cast<const float4*>(left + (size_t)(j0 + j) * dim + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(ms + j * kCarryPitch + e) = x;
+  }
+  for (int t0 = t_begin; t0 < t_end; t0 += kCarryTokens) {
+    __syncthreads();
+    for (int i = tid; i < kCarryTokens * 32; i += 256) {
+      const int t = t0 + (i >> 5), e = (i & 31) * 4;
+      const float4 x = (t < t_end && e < dim) ? *reinterpret_cast<const float4*>(sg.q_decayed + ((size_t)t * heads + h) * dim + e)
+                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(qs + (i >> 5) * kCarryPitch + e) = x;
+    }
+    __syncthreads();
+    float sum[8][4];
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) sum[a][b] = 0.f;
+#pragma unroll 1
+    for (int e0 = 0; e0 < dim; e0 += 32) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {     // four tokens at a time: the packed sums of eight would not fit in registers
+        f32x2 acc[4][4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) acc[a][b] = 0;
+#pragma unroll 2
+        for (int e = 0; e < 32; e += 4) {
+          ulonglong2 m[4];
+#pragma unroll
+          for (int b = 0; b < 4; ++b) m[b] = *reinterpret_cast<const ulonglong2*>(ms + (tx + 32 * b) * kCarryPitch + e0 + e);
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(qs + (ty * 8 + half * 4 + a) * kCarryPitch + e0 + e);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) acc[a][b] = fma2(x.y, m[b].y, fma2(x.x, m[b].x, acc[a][b]));
+          }
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) sum[half * 4 + a][b] += low2(acc[a][b]) + high2(acc[a][b]);
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const int t = t0 + ty * 8 + a;
+      if (t >= t_end) break;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int j = j0 + tx + 32 * b;
+        if (j < vdim) out[((size_t)t * heads + h) * vdim + j] += sum[a][b];
       }
     }
   }
@@ -507,12 +703,12 @@ int scan_launch(const void* q, const void* k, const void* v, int in_stride, cons
   const size_t eb = sizeof(T) * 4;               // bytes of four elements of q or k
   const bool vec = dim % 4 == 0 && in_stride % 4 == 0 && ((uintptr_t)q % eb) == 0 && ((uintptr_t)k % eb) == 0 &&
                    ((uintptr_t)alpha % 16) == 0;
-  auto kernel = max_q_len >= 8 ? (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, true> : gla_scan_kernel<T, DPT, LPC, false, true, true>)
-                                        : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, true> : gla_scan_kernel<T, DPT, LPC, false, false, true>))
-                       : (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, false> : gla_scan_kernel<T, DPT, LPC, false, true, false>)
-                                : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, false> : gla_scan_kernel<T, DPT, LPC, false, false, false>));
+  auto kernel = max_q_len >= 8 ? (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, true, false> : gla_scan_kernel<T, DPT, LPC, false, true, true, false>)
+                                        : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, true, false> : gla_scan_kernel<T, DPT, LPC, false, false, true, false>))
+                       : (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, false, false> : gla_scan_kernel<T, DPT, LPC, false, true, false, false>)
+                                : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, false, false> : gla_scan_kernel<T, DPT, LPC, false, false, false, false>));
   launch_kernel(kernel, grid, dim3(kScanThreads), 0, s, 1, (const T*)q, (const T*)k, (const T*)v, in_stride, alpha, bonus, state, slot_stride,
-                q_indptr, state_slots, out, heads, dim, vdim, q_scale);
+                q_indptr, state_slots, out, heads, dim, vdim, q_scale, Segments{});
   return launch_status();
 }
 
@@ -549,6 +745,45 @@ ARLE_API int arle_gla_scan(const void* q, const void* k, const void* v, int dtyp
   if (dtype == 1)
     return scan_dispatch<__nv_bfloat16>(q, k, v, in_stride, alpha, bonus, state, slot_stride, q_indptr, state_slots, out, rows, heads, dim, vdim, q_scale, max_q_len, s);
   return ARLE_E_BADARG;
+}
+
+// How many float32 numbers of scratch arle_gla_scan_segments wants for num_tokens tokens of `rows` rows; 0: it does not take them (arle_gla_scan
+// does).  bfloat16, dim over 64 and up to 128 in groups of four, some row long enough to be cut.
+ARLE_API long arle_gla_segments_scratch(int num_tokens, int rows, int heads, int dim, int vdim, int max_q_len) {
+  if (rows <= 0 || heads <= 0 || vdim <= 0 || dim <= 64 || dim > 128 || dim % 4 || max_q_len < kSegFrom || rows + num_tokens / kSegTokens > 65535) return 0;
+  const long slots = num_tokens / kSegTokens;
+  return slots * heads * ((long)vdim * dim + dim) + (long)num_tokens * heads * dim;
+}
+
+// arle_gla_scan for steps with long rows (arle_gla_segments_scratch above zero, no bonus).  q, k, alpha and scratch on 16-byte boundaries (q and k
+// on 8), in_stride a multiple of 4.
+ARLE_API int arle_gla_scan_segments(const void* q, const void* k, const void* v, int in_stride, const float* alpha, float* state, long slot_stride,
+                                    const int* q_indptr, const int* state_slots, float* out, float* scratch, int num_tokens, int rows, int heads,
+                                    int dim, int vdim, float q_scale, int max_q_len, cudaStream_t s) {
+  if (rows <= 0 || num_tokens <= 0) return 0;
+  if (heads <= 0 || dim <= 0 || vdim <= 0 || max_q_len <= 0 || slot_stride < (long)heads * vdim * dim || !scratch) return ARLE_E_BADARG;
+  if (arle_gla_segments_scratch(num_tokens, rows, heads, dim, vdim, max_q_len) == 0 || heads > 65535 || in_stride % 4 ||
+      (((uintptr_t)q | (uintptr_t)k) & 7) || (((uintptr_t)alpha | (uintptr_t)scratch) & 15))
+    return ARLE_E_UNSUPPORTED;
+  const int slots = num_tokens / kSegTokens;     // of rows in several segments: none has fewer tokens
+  Segments sg;
+  sg.left = scratch;
+  sg.decay = sg.left + (size_t)slots * heads * vdim * dim;
+  sg.q_decayed = sg.decay + (size_t)slots * heads * dim;
+  sg.rows = rows;
+  constexpr int COLS = kScanThreads / 32 * kScanCpt;
+  static SharedLimit limit;
+  const cudaError_t raised = limit.raise((const void*)gla_carry_kernel, kCarrySmem);
+  if (raised != cudaSuccess) return (int)raised;
+  typedef __nv_bfloat16 T;
+  launch_kernel(gla_scan_kernel<T, 4, 32, true, false, true, true>, dim3((vdim + COLS - 1) / COLS, heads, rows + slots), dim3(kScanThreads), 0, s, 1,
+                (const T*)q, (const T*)k, (const T*)v, in_stride, alpha, (const float*)nullptr, state, slot_stride, q_indptr, state_slots, out, heads,
+                dim, vdim, q_scale, sg);
+  launch_kernel(gla_join_kernel, dim3((vdim * (dim / 4) + 255) / 256, heads, slots), dim3(256), 0, s, 1, state, slot_stride, q_indptr, state_slots,
+                heads, dim, vdim, sg);
+  launch_kernel(gla_carry_kernel, dim3((vdim + kCarryCols - 1) / kCarryCols, heads, slots), dim3(256), kCarrySmem, s, 1, q_indptr, out, heads, dim,
+                vdim, sg);
+  return launch_status();
 }
 
 ARLE_API int arle_gla_out(const float* o, const void* gate, int dtype, int gate_stride, const float* weight, float eps,
