@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256, LONG && !AHEAD && sizeof(T) == 4 && EPL =
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int q_stride, int k_stride, int v_stride,
     const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ state, long slot_stride,
     const int* __restrict__ q_indptr, const int* __restrict__ state_slots, float* __restrict__ out, int H, int kq_heads, int dim,
-    int vdim, float q_scale, float unit_eps) {
+    int vdim, float q_scale, float unit_eps, int longest) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(256, LONG && !AHEAD && sizeof(T) == 4 && EPL =
   const int g = h / (H / kq_heads);
   const int cl = threadIdx.x / LPC, part = threadIdx.x % LPC;
   const int beg = q_indptr[r], end = q_indptr[r + 1];
+  if (longest > 0 && end - beg > longest) return;        // another kernel's row
   const bool col_live = c0 + cl < vdim;
   float* sp = state + (size_t)state_slots[r] * slot_stride + (size_t)h * vdim * dim + (size_t)(c0 + cl) * dim;
   const bool vec_state = dim % 4 == 0 && ((uintptr_t)sp & 15) == 0;
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(256, LONG && !AHEAD && sizeof(T) == 4 && EPL =
 template <typename T, int EPL, int LPC, bool LONG>
 static int launch_delta(const void* q, const void* k, const void* v, int q_stride, int k_stride, int v_stride, const float* beta,
                         const float* decay, float* state, long slot_stride, const int* q_indptr, const int* state_slots, float* out,
-                        int R, int H, int kq_heads, int dim, int vdim, float q_scale, float unit_eps, int num_tokens, cudaStream_t s) {
+                        int R, int H, int kq_heads, int dim, int vdim, float q_scale, float unit_eps, int longest, int num_tokens, cudaStream_t s) {
   // 128 threads a block while the step's blocks are few; twice the columns share the staging of a head's q and k once the
   // SMs are full
   int threads = 128;
@@ -306,25 +307,26 @@ static int launch_delta(const void* q, const void* k, const void* v, int q_strid
   }
   dim3 grid((vdim + cpb - 1) / cpb, H, R);
   launch_kernel(kernel, dim3(grid), dim3(threads), smem, s, 1, (const T*)q, (const T*)k, (const T*)v, q_stride,
-                k_stride, v_stride, beta, decay, state, slot_stride, q_indptr, state_slots, out, H, kq_heads, dim, vdim, q_scale, unit_eps);
+                k_stride, v_stride, beta, decay, state, slot_stride, q_indptr, state_slots, out, H, kq_heads, dim, vdim, q_scale, unit_eps, longest);
   return launch_status();
 }
 
 // q, k [T, kq_heads*dim] and v [T, H*vdim] in the activation type (row strides given); beta, decay float32 [T, H]; state:
-// float32, a slot every slot_stride numbers, [H][vdim][dim] at its start; out float32 [T, H, vdim]; num_tokens: T, all rows'.
+// float32, a slot every slot_stride numbers, [H][vdim][dim] at its start; out float32 [T, H, vdim]; num_tokens: T, all rows'.  longest > 0:
+// rows of more tokens are left alone (arle_delta_tc runs them).
 ARLE_API int arle_delta_scan(const void* q, const void* k, const void* v, int dtype, int q_stride, int k_stride, int v_stride,
                              const float* beta, const float* decay, float* state, long slot_stride, const int* q_indptr,
                              const int* state_slots, float* out, int num_tokens, int R, int H, int kq_heads, int dim, int vdim,
-                             float q_scale, float unit_eps, cudaStream_t s) {
+                             float q_scale, float unit_eps, int longest, cudaStream_t s) {
   if (R <= 0 || num_tokens <= 0) return 0;
   if (H <= 0 || kq_heads <= 0 || H % kq_heads || dim <= 0 || vdim <= 0 || H > 65535 || R > 65535) return ARLE_E_BADARG;
   if (dim > 512) return ARLE_E_UNSUPPORTED;
   const bool long_rows = num_tokens >= 2 * R + kDeltaChunk;       // some row has a full chunk, or nearly
 #define ARLE_DELTA(TT, E, L)                                                                                                           \
   return long_rows ? launch_delta<TT, E, L, true>(q, k, v, q_stride, k_stride, v_stride, beta, decay, state, slot_stride, q_indptr,     \
-                                                  state_slots, out, R, H, kq_heads, dim, vdim, q_scale, unit_eps, num_tokens, s)                    \
+                                                  state_slots, out, R, H, kq_heads, dim, vdim, q_scale, unit_eps, longest, num_tokens, s)                    \
                    : launch_delta<TT, E, L, false>(q, k, v, q_stride, k_stride, v_stride, beta, decay, state, slot_stride, q_indptr,    \
-                                                   state_slots, out, R, H, kq_heads, dim, vdim, q_scale, unit_eps, num_tokens, s)
+                                                   state_slots, out, R, H, kq_heads, dim, vdim, q_scale, unit_eps, longest, num_tokens, s)
 #define ARLE_DELTA_BY_DIM(TT)          \
   if (dim <= 8) ARLE_DELTA(TT, 4, 2);   \
   if (dim <= 32) ARLE_DELTA(TT, 4, 8);  \

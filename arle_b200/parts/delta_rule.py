@@ -93,7 +93,9 @@ class GatedDeltaRule(Mixer):
         return sum(t.numel() * t.element_size() for t in (self.w_in, self.w_gates, self.w_o))
 
     def scratch_elements_per_token(self):
-        return 2 * (self.channels + self.inner) + 4 * self.inner + 8 * self.spec.num_heads + self.spec.hidden_size
+        # with long prompts of heads of 128 what a chunk's heads keep: 7,936 float32 numbers, 32 tokens a chunk at the least
+        chunks = 2 * 7936 // 32 * self.spec.num_heads if self.spec.key_dim == 128 else 0
+        return 2 * (self.channels + self.inner) + 4 * self.inner + 8 * self.spec.num_heads + self.spec.hidden_size + chunks
 
     def state_need(self):
         n = self.conv_offset + self.channels * (self.spec.conv_taps - 1)
@@ -113,8 +115,11 @@ class GatedDeltaRule(Mixer):
         beta, decay = (ctx.ws.get(n, (T, H), torch.float32) for n in ("delta_beta", "delta_decay"))
         ops.delta_gates(pre, self.a_log, self.dt_bias, beta, decay)
         o = ctx.ws.get("delta_o", (T, H, s.value_dim), torch.float32)
-        ops.delta_scan(qkv[:, :dqk], qkv[:, dqk: 2 * dqk], qkv[:, 2 * dqk:], beta, decay, state, ctx.q_indptr, ctx.state_slots, o,
-                       H, s.num_kq_heads, s.key_dim, s.value_dim, float(s.key_dim) ** -0.5, s.unit_eps)
+        q, k, v = qkv[:, :dqk], qkv[:, dqk: 2 * dqk], qkv[:, 2 * dqk:]
+        n = ops.delta_scan_scratch(q, k, v, o, ctx.state_slots.numel(), H, s.key_dim, s.value_dim, ctx.max_q_len)
+        chunks = dict(max_q_len=ctx.max_q_len, scratch=ctx.ws.get("delta_chunks", (n,), torch.float32)) if n else {}
+        ops.delta_scan(q, k, v, beta, decay, state, ctx.q_indptr, ctx.state_slots, o, H, s.num_kq_heads, s.key_dim, s.value_dim,
+                       float(s.key_dim) ** -0.5, s.unit_eps, **chunks)
         gated = ctx.ws.get("delta_gated", (T, inner), x.dtype)
         ops.gla_out(o.view(T, inner), proj[:, C:], self.norm, s.norm_eps, 1.0, gated, H, s.value_dim)
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)

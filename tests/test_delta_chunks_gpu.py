@@ -1,0 +1,97 @@
+"""The gated delta rule in chunks on the tensor cores against float64: lengths around the first row that runs in chunks and around a chunk's
+end, long rows beside short ones, columns that do not fill a block, shared q/k heads; no further off than the scan of whole rows; a row's
+bits do not depend on what stands beside it; decays of zero, and an overflow that stays with the tokens behind it."""
+import pytest
+import torch
+
+from arle_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV, DIM = "cuda", 128
+
+
+def _inputs(lens, H, kq, vdim):
+    g = torch.Generator(device=DEV).manual_seed(vdim + sum(lens))
+    T = sum(lens)
+    wide = torch.nn.functional.silu(torch.randn(T, 2 * kq * DIM + H * vdim, generator=g, device=DEV) * 0.7).to(torch.bfloat16)
+    q, k, v = wide.split([kq * DIM, kq * DIM, H * vdim], 1)
+    beta = torch.sigmoid(torch.randn(T, H, generator=g, device=DEV))
+    decay = torch.exp(-torch.rand(T, H, generator=g, device=DEV) * 0.3)
+    return q, k, v, beta, decay, torch.randn(len(lens) + 1, H * vdim * DIM + 8, generator=g, device=DEV)
+
+
+def _run(q, k, v, beta, decay, state, lens, H, kq, vdim, chunks=True, slots=None):
+    at = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0).to(torch.int32)
+    out = torch.full((q.shape[0] + 1, H, vdim), 7.0, device=DEV)
+    state, n = state.clone(), ops.delta_scan_scratch(q, k, v, out, len(lens), H, DIM, vdim, max(lens))
+    assert n > 0
+    scratch = torch.full((n + 4,), float("nan"), device=DEV)
+    slots = torch.tensor(slots or list(range(len(lens))), dtype=torch.int32, device=DEV)
+    ops.delta_scan(q, k, v, beta, decay, state, at, slots, out[:-1], H, kq, DIM, vdim, DIM ** -0.5, 1e-6,
+                   **(dict(max_q_len=max(lens), scratch=scratch[:n]) if chunks else {}))
+    assert (out[-1] == 7.0).all() and scratch[n:].isnan().all()
+    return out[:-1], state
+
+
+def _exact(q, k, v, beta, decay, state, lens, H, kq, vdim):
+    def unit(x):
+        x = x.double().view(-1, kq, DIM)
+        return (x * torch.rsqrt(x.square().sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // kq, 1)
+
+    qq, kk, vv = unit(q) * DIM ** -0.5, unit(k), v.double().view(-1, H, vdim)
+    S, outs, t = state[:, : H * vdim * DIM].double().view(-1, H, vdim, DIM).clone(), [], 0
+    for r, n in enumerate(lens):
+        for _ in range(n):
+            S[r] *= decay[t].double()[:, None, None]
+            u = beta[t].double()[:, None] * (vv[t] - torch.einsum("hvd,hd->hv", S[r], kk[t]))
+            S[r] += u[..., None] * kk[t][:, None]
+            outs.append(torch.einsum("hvd,hd->hv", S[r], qq[t]))
+            t += 1
+    return torch.stack(outs), S.reshape(S.shape[0], -1)
+
+
+@pytest.mark.parametrize("lens", [[64], [65], [128], [1000], [5, 200, 1, 63, 64, 333], [1] * 40 + [190]])
+@pytest.mark.parametrize("H,kq,vdim", [(2, 2, 128), (4, 2, 40), (1, 1, 8)])
+def test_chunks(lens, H, kq, vdim):
+    x = _inputs(lens, H, kq, vdim)
+    want, want_s = _exact(*x, lens, H, kq, vdim)
+    got, got_s = _run(*x, lens, H, kq, vdim)
+    whole, whole_s = _run(*x, lens, H, kq, vdim, chunks=False)
+    used = H * vdim * DIM
+    for a, b, w in ((got, whole, want), (got_s[:, :used], whole_s[:, :used], want_s)):
+        off, ref = ((y.double() - w).norm() / w.norm() for y in (a, b))
+        assert off < 4e-7 and off < 1.3 * ref + 2e-8           # the float32 sums of both come in different orders
+    assert torch.equal(got_s[:, used:], x[-1][:, used:])
+    t = 0
+    for r, n in enumerate(lens):                                # a row by itself: the same bits
+        if n < 64:
+            assert torch.equal(got[t: t + n], whole[t: t + n])
+        else:
+            alone, s = _run(*(y[t: t + n] for y in x[:-1]), x[-1], [n], H, kq, vdim, slots=[r])
+            assert torch.equal(alone, got[t: t + n]) and torch.equal(s[r], got_s[r])
+        t += n
+
+
+def test_decays_of_zero_and_overflow():
+    lens, H, kq, vdim = [150], 2, 1, 48
+    q, k, v, beta, decay, state = _inputs(lens, H, kq, vdim)
+    decay[::13] = 0.0
+    decay[5::17, 0] = 1e-30
+    want, want_s = _exact(q, k, v, beta, decay, state, lens, H, kq, vdim)
+    got, got_s = _run(q, k, v, beta, decay, state, lens, H, kq, vdim)
+    assert (got.double() - want).norm() < 4e-7 * want.norm()
+    assert (got_s[0, : want_s.shape[1]].double() - want_s[0]).norm() < 4e-7 * want_s[0].norm()
+    decay[:] = 0.97
+    clean, _ = _run(q, k, v, beta, decay, state, lens, H, kq, vdim)
+    bad = v.clone()
+    bad[75, 3] = float("inf")                                   # one head's column, in the middle of a tile
+    odd, _ = _run(q, k, bad, beta, decay, state, lens, H, kq, vdim)
+    close = dict(rtol=1e-5, atol=1e-6)
+    assert torch.allclose(odd[:75], clean[:75], **close) and not odd[75:, 0, 3].isfinite().any()
+    assert torch.equal(odd[:, 1], clean[:, 1])
+    odd[:, 0, 3] = clean[:, 0, 3]
+    assert torch.allclose(odd, clean, **close)                  # the other columns as they were
+    worse = k.clone()
+    worse[75, 4] = float("nan")
+    odd, _ = _run(q, worse, v, beta, decay, state, lens, H, kq, vdim)
+    assert torch.allclose(odd[:75], clean[:75], **close) and not odd[75:].isfinite().any()
