@@ -58,6 +58,9 @@ constexpr uint32_t kSpinLimit = 1u << 22;    // polls of an mbarrier before givi
 constexpr int kSsSlots = 192;                // slots of a sum-of-squares table (one per CTA or cluster of the product that fills it)
 constexpr int kSsRows = 16;                  // rows of x a slot covers
 
+constexpr long long kDirectMost = 8 << 20;   // elements of W
+constexpr long long kDirectWarps = 4096;
+
 // The optional fusions (see the top of the file).  All pointers null: a plain product.
 struct Fusion {
   const float* in_ss;          // [kSsRows][kSsSlots]: sums of squares of the rows of x, a row's slots to be added up (a row is
@@ -426,6 +429,161 @@ __global__ void __launch_bounds__(kThreads, 1) skinny_gemm_kernel(
   if (timed_out && err) atomicExch(err, 1);
 }
 
+// Small products (up to 8 rows of x), where the ring above takes longer to start and to drain than its bytes need: nothing is staged.  A block
+// has NR rows of W, its warps shares of K; a lane asks for 16 bytes of a row at a time, eight neighbouring elements of K, which are two of the
+// tensor cores' K steps in an order of their own (x is read in the same order, so the sums are the same products).  With 128 elements of K a
+// warp all of a block's loads are under way before the first is used; the warps' sums are added in warp order.  What bounds it: a launch, one
+// round trip to memory and the sums, some 3 us, and the bytes on top.  DIRECT_FIGURES
+__device__ __forceinline__ uint4 ld_weights(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_rows(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+template <int NR, int WARPS, typename OutT>
+__global__ void __launch_bounds__(WARPS * 32) direct_gemm_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ W,
+                                                                 int ldw, OutT* __restrict__ out, int ldo, int M, int N, int K, int gated,
+                                                                 Fusion fu) {
+  constexpr int U = 4, HALVES = NR / 8;                    // blocks of 32 elements of K under way; rows g and g + 8 of the tile
+  __shared__ float red[WARPS][NR * 8];
+  __shared__ float row_scale[8];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int r0 = blockIdx.x * NR;
+  // what is needed last is asked for first: loads issued behind the weights would wait for all their bytes
+  float ss[kSsSlots / 32], r_old = 0.f, gain = 0.f;
+  if (fu.in_ss && warp < M) {
+#pragma unroll
+    for (int i = 0; i < kSsSlots / 32; ++i) ss[i] = __ldcg(fu.in_ss + warp * kSsSlots + lane + 32 * i);
+  }
+  const int row = tid % NR, m = tid / NR, n = r0 + row;    // of the first NR * 8 threads: the sum they finish
+  const bool valid = tid < NR * 8 && m < M && n < N;
+  if (fu.resid && valid) {
+    r_old = __ldcg(fu.resid + (size_t)m * fu.ldr + n);
+    if (fu.extra) r_old += __ldcg(fu.extra + (size_t)m * fu.ldr + n);
+    gain = __ldg(fu.gamma + n);
+  }
+  const int blocks = K / 32, per = (blocks + WARPS - 1) / WARPS;
+  const int b0 = warp * per, b1 = min(blocks, b0 + per);
+  const __nv_bfloat16* wp[HALVES];
+#pragma unroll
+  for (int h = 0; h < HALVES; ++h) wp[h] = W + (size_t)min(r0 + h * 8 + g, N - 1) * ldw + t * 8;
+  const __nv_bfloat16* xp = x + (size_t)(g < M ? g : 0) * ldx + t * 8;
+  float acc[2][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[0][i] = acc[1][i] = 0.f;
+  for (int b = b0; b < b1; b += U) {
+    uint4 wv[U][HALVES], xv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {                          // places behind the share's end read its first block and are left out
+      const size_t at = (size_t)(b + u < b1 ? b + u : b) * 32;
+      xv[u] = ld_rows(xp + at);
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) wv[u][h] = ld_weights(wp[h] + at);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (b + u >= b1) break;
+      if (g >= M) xv[u] = make_uint4(0, 0, 0, 0);
+      const uint4 lo = wv[u][0], hi = HALVES > 1 ? wv[u][HALVES - 1] : make_uint4(0, 0, 0, 0);
+      const uint32_t a[4] = {lo.x, hi.x, lo.y, hi.y}, c[4] = {lo.z, hi.z, lo.w, hi.w};
+      mma_bf16(acc[0], a, xv[u].x, xv[u].y);
+      mma_bf16(acc[1], c, xv[u].z, xv[u].w);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2 * HALVES; ++i) red[warp][(2 * t + (i & 1)) * NR + g + (i >> 1) * 8] = acc[0][i] + acc[1][i];
+  if (warp < 8) {
+    float f = 1.f;
+    if (fu.in_ss && warp < M) {
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < kSsSlots / 32; ++i) s += ss[i];
+      f = rsqrtf(warp_sum(s) * fu.inv_width + fu.eps);
+    }
+    if (lane == 0) row_scale[warp] = f;
+  }
+  __syncthreads();
+  if (tid < NR * 8) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) s += red[w][tid];
+    s *= row_scale[m];
+    if (gated) {
+      const float up = __shfl_down_sync(0xffffffffu, s, 1);
+      if (!(row & 1) && valid)
+        store_out<OutT>(out + (size_t)m * ldo + (n >> 1),
+                        (gated == 2 ? 0.5f * s * (1.0f + tanhf(0.7978845608028654f * (s + 0.044715f * s * s * s))) : s / (1.0f + expf(-s))) * up);
+    } else if (fu.resid) {
+      float r = 0.f;
+      if (valid) {
+        r = fmaf(fu.branch_scale, s, r_old);
+        fu.resid[(size_t)m * fu.ldr + n] = r;
+        fu.xs[(size_t)m * fu.ldxs + n] = __float2bfloat16_rn(r * gain);
+      }
+      float q = r * r;
+#pragma unroll
+      for (int o = NR / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+      if (row == 0) {
+        fu.out_ss[m * kSsSlots + blockIdx.x] = q;
+        fu.out_ss[(8 + m) * kSsSlots + blockIdx.x] = 0.f;
+      }
+    } else if (valid) {
+      if (fu.act) {
+        s = fmaxf(s, 0.f);
+        s *= s;
+      }
+      store_out<OutT>(out + (size_t)m * ldo + n, s);
+    }
+  }
+  if (fu.resid && blockIdx.x == 0) {                       // the slots that no block has
+    const int used = gridDim.x, left = kSsSlots - used;
+    for (int i = tid; i < kSsRows * left; i += WARPS * 32) fu.out_ss[(i / left) * kSsSlots + used + i % left] = 0.f;
+  }
+}
+
+// Whether a product is one of those, and how it is cut.  DIRECT_RULE
+struct DirectPlan {
+  int rows, warps;                                         // of a block; rows 0: the ring
+};
+inline DirectPlan plan_direct(int M, int N, int K, bool sink) {
+  DirectPlan p{0, 8};
+  if (M > 8 || (long long)N * K > kDirectMost) return p;
+  p.warps = K <= 1024 ? 8 : K <= 2048 ? 16 : K <= 3072 ? 24 : 32;
+  p.rows = (long long)(N + 7) / 8 * p.warps <= kDirectWarps ? 8 : 16;
+  if (sink && (N + p.rows - 1) / p.rows > kSsSlots) p.rows = 0;
+  return p;
+}
+
+template <int NR, int WARPS, typename OutT>
+int launch_direct(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, int M, int N, int K, int gated, const Fusion& fu,
+                  cudaStream_t s) {
+  const cudaError_t e = launch_kernel_as((pdl_enabled() & 3) != 0, direct_gemm_kernel<NR, WARPS, OutT>, dim3((N + NR - 1) / NR), dim3(WARPS * 32), 0, s,
+                                         1, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W, ldw, (OutT*)out, ldo, M, N, K, gated, fu);
+  return e != cudaSuccess ? (int)e : launch_status();
+}
+template <typename OutT>
+int run_direct(const DirectPlan& p, const void* x, int ldx, const void* W, int ldw, void* out, int ldo, int M, int N, int K, int gated,
+               const Fusion& fu, cudaStream_t s) {
+#define ARLE_DIRECT(R, C) \
+  if (p.rows == R && p.warps == C) return launch_direct<R, C, OutT>(x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, s)
+  ARLE_DIRECT(8, 8);
+  ARLE_DIRECT(8, 16);
+  ARLE_DIRECT(8, 24);
+  ARLE_DIRECT(8, 32);
+  ARLE_DIRECT(16, 8);
+  ARLE_DIRECT(16, 16);
+  ARLE_DIRECT(16, 24);
+  ARLE_DIRECT(16, 32);
+#undef ARLE_DIRECT
+  return ARLE_E_BADARG;
+}
+
 template <int NT>
 size_t smem_bytes(int KS, int KC, int S, int csize) {
   size_t n = ((size_t)NT * 8 * (KS + kXPad) * 2 + 127) / 128 * 128;
@@ -535,6 +693,11 @@ int skinny_entry(const void* x, int ldx, const void* W, int ldw, void* out, int 
   if (gated && N % 2 != 0) return ARLE_E_BADARG;
   if (fu.resid && (gated || !fu.gamma || !fu.xs || !fu.out_ss)) return ARLE_E_BADARG;
   if (!fu.resid && !out) return ARLE_E_BADARG;
+  const DirectPlan direct = plan_direct(M, N, K, fu.resid != nullptr);
+  if (direct.rows) {
+    if (out_dtype == 0) return run_direct<float>(direct, x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, s);
+    if (out_dtype == 1) return run_direct<__nv_bfloat16>(direct, x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, s);
+  }
   if (M <= 8) {
     if (out_dtype == 0) return plan_and_launch<1, float>(x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, err, s);
     if (out_dtype == 1) return plan_and_launch<1, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, err, s);

@@ -542,6 +542,7 @@ __global__ void __launch_bounds__(256, 2) gla_carry_kernel(const int* __restrict
   const int beg = q_indptr[r], end = q_indptr[r + 1], len = segment_tokens(end - beg);
   const int t_begin = beg + seg * len, t_end = min(end, t_begin + len);
   const float* left = sg.left + ((size_t)(cut - 1) * heads + h) * vdim * dim;
+#pragma unroll 8
   for (int i = tid; i < kCarryCols * 32; i += 256) {
     const int j = i >> 5, e = (i & 31) * 4;
     const float4 x = (j0 + j < vdim && e < dim) ? *reinterpret_cast<const float4*>(left + (size_t)(j0 + j) * dim + e) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -549,6 +550,7 @@ __global__ void __launch_bounds__(256, 2) gla_carry_kernel(const int* __restrict
   }
   for (int t0 = t_begin; t0 < t_end; t0 += kCarryTokens) {
     __syncthreads();
+#pragma unroll
     for (int i = tid; i < kCarryTokens * 32; i += 256) {
       const int t = t0 + (i >> 5), e = (i & 31) * 4;
       const float4 x = (t < t_end && e < dim) ? *reinterpret_cast<const float4*>(sg.q_decayed + ((size_t)t * heads + h) * dim + e)
@@ -556,11 +558,15 @@ __global__ void __launch_bounds__(256, 2) gla_carry_kernel(const int* __restrict
       *reinterpret_cast<float4*>(qs + (i >> 5) * kCarryPitch + e) = x;
     }
     __syncthreads();
+    // what the segment alone gave, asked for before the products: a load behind a store to the same array would wait for it
     float sum[8][4];
 #pragma unroll
     for (int a = 0; a < 8; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) sum[a][b] = 0.f;
+      for (int b = 0; b < 4; ++b) {
+        const int t = t0 + ty * 8 + a, j = j0 + tx + 32 * b;
+        sum[a][b] = t < t_end && j < vdim ? out[((size_t)t * heads + h) * vdim + j] : 0.f;
+      }
 #pragma unroll 1
     for (int e0 = 0; e0 < dim; e0 += 32) {
 #pragma unroll
@@ -595,7 +601,7 @@ __global__ void __launch_bounds__(256, 2) gla_carry_kernel(const int* __restrict
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
         const int j = j0 + tx + 32 * b;
-        if (j < vdim) out[((size_t)t * heads + h) * vdim + j] += sum[a][b];
+        if (j < vdim) out[((size_t)t * heads + h) * vdim + j] = sum[a][b];
       }
     }
   }
