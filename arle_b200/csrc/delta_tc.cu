@@ -90,11 +90,12 @@ struct ChunkSmem {
   float A[kC][kC + 4], T[kC][kC + 4];
   float W[3][16][17];                                      // products on their way into a tile of T
   double cum[kC];
-  float beta[kC], iq[kC], ik[kC];
+  double iq[kC], ik[kC];                                   // q_scale / |q|, 1 / |k|
+  float beta[kC];
 };
 
 // 256 threads a chunk and head.
-__global__ void __launch_bounds__(256) delta_chunks_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, long q_stride,
+__global__ void __launch_bounds__(256, 3) delta_chunks_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, long q_stride,
                                                            long k_stride, const float* __restrict__ beta, const float* __restrict__ decay,
                                                            const int* __restrict__ q_indptr, int rows, int longest, int H, int kq_heads,
                                                            float q_scale, float unit_eps, uint32_t* __restrict__ chunks) {
@@ -154,8 +155,8 @@ __global__ void __launch_bounds__(256) delta_chunks_kernel(const __nv_bfloat16* 
       sk += __shfl_xor_sync(0xffffffffu, sk, o);
     }
     if (part == 0) {
-      sm.iq[j] = q_scale / sqrtf(sq + unit_eps);
-      sm.ik[j] = 1.0f / sqrtf(sk + unit_eps);
+      sm.iq[j] = q_scale / sqrt((double)sq + unit_eps);
+      sm.ik[j] = 1.0 / sqrt((double)sk + unit_eps);
     }
   }
   __syncthreads();
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(256) delta_chunks_kernel(const __nv_bfloat16* 
     }
     const int i0 = rt * 16 + (lane >> 2);
     const double cu[2] = {sm.cum[i0], sm.cum[i0 + 8]};
-    const float fr[2] = {is_q ? sm.iq[i0] : sm.beta[i0] * sm.ik[i0], is_q ? sm.iq[i0 + 8] : sm.beta[i0 + 8] * sm.ik[i0 + 8]};
+    const double fr[2] = {is_q ? sm.iq[i0] : sm.beta[i0] * sm.ik[i0], is_q ? sm.iq[i0 + 8] : sm.beta[i0 + 8] * sm.ik[i0 + 8]};
 #pragma unroll
     for (int jt = 0; jt < 4; ++jt) {
       if (jt > rt) break;
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(256) delta_chunks_kernel(const __nv_bfloat16* 
         for (int i = 0; i < 4; ++i) {
           const int j = jt * 16 + hh * 8 + 2 * (lane & 3) + (i & 1), row = i0 + (i >> 1) * 8;
           const bool seen = is_q ? j <= row : j < row;
-          w[hh * 4 + i] = seen ? sc[2 * jt + hh][i] * (fr[i >> 1] * (sm.ik[j] * exp2f((float)(cu[i >> 1] - sm.cum[j])))) : 0.f;
+          w[hh * 4 + i] = seen ? (float)(sc[2 * jt + hh][i] * (fr[i >> 1] * (sm.ik[j] * exp2(cu[i >> 1] - sm.cum[j])))) : 0.f;
         }
       if (is_q) {
         split_tile(w, to + (kTiles + rt * (rt + 1) / 2 + jt) * kTileWords, lane);
@@ -204,12 +205,12 @@ __global__ void __launch_bounds__(256) delta_chunks_kernel(const __nv_bfloat16* 
   }
   if (tid < kC) {
     const double c = sm.cum[tid];
-    const float d = exp2f((float)c);
+    const double d = exp2(c);
     float* s = reinterpret_cast<float*>(to + 2 * kTiles * kTileWords);
-    s[tid] = d * sm.ik[tid];
-    s[kC + tid] = d * sm.iq[tid];
-    s[2 * kC + tid] = exp2f((float)(sm.cum[kC - 1] - c)) * sm.ik[tid];
-    if (tid == kC - 1) s[3 * kC] = d;
+    s[tid] = (float)(d * sm.ik[tid]);
+    s[kC + tid] = (float)(d * sm.iq[tid]);
+    s[2 * kC + tid] = (float)(exp2(sm.cum[kC - 1] - c) * sm.ik[tid]);
+    if (tid == kC - 1) s[3 * kC] = (float)d;
   }
   __syncthreads();
   if (tid < kC) {                                          // the tiles on the diagonal: a thread has a column
@@ -502,14 +503,14 @@ __global__ void __launch_bounds__(128 * G, 1) delta_tc_kernel(const __nv_bfloat1
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) sum[nt][i] = o[nt][i], rest[nt][i] = 0.f;
+          for (int i = 0; i < 4; ++i) sum[nt][i] = rest[nt][i] = 0.f;
         tiles_times<VP>(w, rt - pass, smem_u32(us), L::V, lane, sum, rest);
         float odd = 0.f;
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            sum[nt][i] += rest[nt][i];
+            sum[nt][i] = o[nt][i] + (sum[nt][i] + rest[nt][i]);
             odd = fmaf(sum[nt][i], 0.f, odd);
           }
         if (pass) seen_alone<VP>(tiles + (kTiles + rt * (rt + 1) / 2 + rt) * kTileWords, us + rt * 16 * VP, L::V, lane, sum);
@@ -525,13 +526,13 @@ __global__ void __launch_bounds__(128 * G, 1) delta_tc_kernel(const __nv_bfloat1
         }
     }
     const float whole = num[3 * kC];
-    float rest[2][2][4];
+    float more[2][2][4], rest[2][2][4];                    // the chunk's own sums, so that S is rounded once a chunk
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
       for (int nn = 0; nn < 2; ++nn)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) S[m][nn][i] *= whole, rest[m][nn][i] = 0.f;
+        for (int i = 0; i < 4; ++i) more[m][nn][i] = rest[m][nn][i] = 0.f;
 #pragma unroll
     for (int kk = 0; kk < kC / 16; ++kk) {
       uint32_t ka[2][4];
@@ -549,8 +550,8 @@ __global__ void __launch_bounds__(128 * G, 1) delta_tc_kernel(const __nv_bfloat1
             mma_bf16(rest[m][0], ka[m], b0, b1);
             mma_bf16(rest[m][1], ka[m], b2, b3);
           } else {
-            mma_add(S[m][0], ka[m], b0, b1);
-            mma_add(S[m][1], ka[m], b2, b3);
+            mma_add(more[m][0], ka[m], b0, b1);
+            mma_add(more[m][1], ka[m], b2, b3);
           }
         }
       }
@@ -560,7 +561,7 @@ __global__ void __launch_bounds__(128 * G, 1) delta_tc_kernel(const __nv_bfloat1
 #pragma unroll
       for (int nn = 0; nn < 2; ++nn)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) S[m][nn][i] += rest[m][nn][i];
+        for (int i = 0; i < 4; ++i) S[m][nn][i] = fmaf(S[m][nn][i], whole, more[m][nn][i] + rest[m][nn][i]);
   }
 #pragma unroll
   for (int m = 0; m < 2; ++m)
@@ -618,8 +619,9 @@ ARLE_API int arle_delta_tc(const void* q, const void* k, const void* v, int q_st
   if (raised != cudaSuccess) return (int)raised;
   launch_kernel(delta_chunks_kernel, dim3(slots, H), dim3(256), sizeof(ChunkSmem), s, 1, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
                 (long)q_stride, (long)k_stride, beta, decay, q_indptr, R, longest, H, kq_heads, q_scale, unit_eps, chunks);
-#ifndef GSEL
-#define GSEL 2
-#endif
-  return launch<GSEL>(q, k, v, q_stride, k_stride, v_stride, chunks, state, slot_stride, q_indptr, state_slots, out, R, H, kq_heads, vdim, longest, s);
+  // Groups of 16 columns by themselves while every block finds an SM (8 heads of 128, one row of 2,048: 134 us, 171 with two to a block, 265
+  // with four), two to a block beyond (32 heads: 309, 208 and 299; rows of 819, 701 and 479 tokens 298, 210 and 202).  The same bits.
+  if ((long)((vdim + 15) / 16) * H * R <= 148)
+    return launch<1>(q, k, v, q_stride, k_stride, v_stride, chunks, state, slot_stride, q_indptr, state_slots, out, R, H, kq_heads, vdim, longest, s);
+  return launch<2>(q, k, v, q_stride, k_stride, v_stride, chunks, state, slot_stride, q_indptr, state_slots, out, R, H, kq_heads, vdim, longest, s);
 }

@@ -58,9 +58,6 @@ constexpr uint32_t kSpinLimit = 1u << 22;    // polls of an mbarrier before givi
 constexpr int kSsSlots = 192;                // slots of a sum-of-squares table (one per CTA or cluster of the product that fills it)
 constexpr int kSsRows = 16;                  // rows of x a slot covers
 
-constexpr long long kDirectMost = 8 << 20;   // elements of W
-constexpr long long kDirectWarps = 4096;
-
 // The optional fusions (see the top of the file).  All pointers null: a plain product.
 struct Fusion {
   const float* in_ss;          // [kSsRows][kSsSlots]: sums of squares of the rows of x, a row's slots to be added up (a row is
@@ -433,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, 1) skinny_gemm_kernel(
 // has NR rows of W, its warps shares of K; a lane asks for 16 bytes of a row at a time, eight neighbouring elements of K, which are two of the
 // tensor cores' K steps in an order of their own (x is read in the same order, so the sums are the same products).  With 128 elements of K a
 // warp all of a block's loads are under way before the first is used; the warps' sums are added in warp order.  What bounds it: a launch, one
-// round trip to memory and the sums, some 3 us, and the bytes on top.  DIRECT_FIGURES
+// round trip to memory and the sums, some 3 us, and the bytes on top.  plan_direct has the figures.
 __device__ __forceinline__ uint4 ld_weights(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -547,16 +544,24 @@ __global__ void __launch_bounds__(WARPS * 32) direct_gemm_kernel(const __nv_bflo
   }
 }
 
-// Whether a product is one of those, and how it is cut.  DIRECT_RULE
+// Whether a product is one of those, and how it is cut: as many warps as are resident together (31 an SM at 64 registers), no more than two
+// blocks of 32 elements of K leave work for; eight rows a block where sixteen would leave SMs without one.  Above 2^24 elements the ring
+// keeps more bytes in flight.  One row of x in a graph, weights not in L2, us (the ring's in brackets): 1,024 x 2,048 3.5 (4.9), 4,096 x 1,024
+// 4.0 (5.1), 1,024 x 3,072 4.1 (5.5), 6,144 x 1,024 4.8 (6.5), 64 x 4,096 3.3 (5.6), 8,192 x 1,024 7.1 (7.3), 4,096 x 4,096 8.6 (9.1), 6,144 x
+// 4,096 12.1 (11.9), 16,384 x 1,024 10.3 (9.8); eight rows the same to 0.3 us more.  1,024 x 4,096 with 32, 16 and 8 warps of 8 rows: 4.5, 5.9,
+// 9.0, with 32 of 16 rows 5.0; 2,048 x 4,096 with 32 warps of 16 rows 5.8, 16 of 8 6.6.
 struct DirectPlan {
   int rows, warps;                                         // of a block; rows 0: the ring
 };
 inline DirectPlan plan_direct(int M, int N, int K, bool sink) {
-  DirectPlan p{0, 8};
-  if (M > 8 || (long long)N * K > kDirectMost) return p;
-  p.warps = K <= 1024 ? 8 : K <= 2048 ? 16 : K <= 3072 ? 24 : 32;
-  p.rows = (long long)(N + 7) / 8 * p.warps <= kDirectWarps ? 8 : 16;
-  if (sink && (N + p.rows - 1) / p.rows > kSsSlots) p.rows = 0;
+  constexpr long long kMostElements = 1ll << 24;
+  constexpr int kMostWarps = 4608;
+  DirectPlan p{0, 0};
+  if (M > 8 || (long long)N * K > kMostElements) return p;
+  const int rows = N <= 1152 ? 8 : 16, tiles = (N + rows - 1) / rows;
+  for (int w = 8; w <= 32; w += 8)
+    if ((w == 8 || w * 64 <= K) && (long long)tiles * w <= kMostWarps) p.warps = w;
+  if (p.warps && !(sink && tiles > kSsSlots)) p.rows = rows;
   return p;
 }
 

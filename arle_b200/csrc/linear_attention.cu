@@ -111,7 +111,11 @@ template <> struct Raw4<__nv_bfloat16, true> { using type = uint2; };
 // single warp on each scheduler (37 % of the issue slots); sixteen segments keep three.  SEGMENT_FIGURES
 // A row's own length decides how it is cut: from kSegFrom tokens on (below, the two further launches cost what the shorter chain gains), in
 // parts of kSegTokens and more, sixteen at most, which bounds the memories between them.
-constexpr int kSegTokens = 128, kSegFrom = 384, kMostSegs = 16;
+#ifndef SEGCPT
+#define SEGCPT 8
+#define SEGN 128
+#endif
+constexpr int kSegTokens = SEGN, kSegFrom = 384, kMostSegs = 16;
 struct Segments {
   float* left;                                   // [cut][head][vdim][dim]: the memory that a segment leaves
   float* decay;                                  // [cut][head][dim]: the product of its decays
@@ -176,14 +180,13 @@ constexpr int few_blocks() {
   return VEC && !BONUS && LPC >= 4 ? 5 : 4;
 }
 // SEGS: a row in segments, see Segments above.
-template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool LONG, bool SEGS>
-__global__ void __launch_bounds__(kScanThreads, SEGS ? 3 : LONG ? 1 : few_blocks<T, DPT, LPC, VEC, BONUS>()) gla_scan_kernel(
+template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool LONG, bool SEGS, int CPT = kScanCpt>
+__global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks<T, DPT, LPC, VEC, BONUS>()) gla_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int in_stride,
     const float* __restrict__ alpha, const float* __restrict__ bonus, float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
     const int* __restrict__ state_slots, float* __restrict__ out, int heads, int dim, int vdim, float q_scale, Segments sg) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int CPT = kScanCpt;
   constexpr int COLS = kScanThreads / LPC * CPT; // columns a block takes
   constexpr int DSPAN = DPT * LPC;               // dim rounded up; channels past dim hold zeros
   constexpr int PAD = DPT == 4 ? 4 : DPT + 4;    // floats a thread's channels take in shared memory: 16-byte rows, spread over the banks
@@ -194,7 +197,7 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 3 : LONG ? 1 : few_blocks
   constexpr int QPT = (QUADS + kScanThreads - 1) / kScanThreads;
   constexpr int VPT = (CHUNK * COLS + kScanThreads - 1) / kScanThreads;
   __shared__ __align__(16) float qs[CHUNK * DPAD], ks[CHUNK * DPAD], as[CHUNK * DPAD];
-  constexpr int VD = LONG && LPC >= 4 ? 2 : 1;           // v's numbers stand twice side by side (a factor of both halves of a pair), where there is room
+  constexpr int VD = LONG && LPC >= 4 && CPT == 4 ? 2 : 1;           // v's numbers stand twice side by side (a factor of both halves of a pair), where there is room
   __shared__ __align__(16) float vs[CHUNK * COLS * VD];
   const int h = blockIdx.y, j0 = blockIdx.x * COLS;
   const int l = threadIdx.x & (LPC - 1), jl = threadIdx.x / LPC;
@@ -330,7 +333,7 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 3 : LONG ? 1 : few_blocks
     if (t0 + CHUNK < t_end) fetch(t0 + CHUNK, min(CHUNK, t_end - t0 - CHUNK));
     // one token: the memory's step and the thread's part of its columns' sums
     auto token = [&](int tt, float (&o)[CPT]) {
-      if constexpr (!LONG) {                     // single numbers: the same roundings in fewer registers
+      if constexpr (!LONG && CPT == 4) {         // single numbers: the same roundings in fewer registers
         const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT);
         const float vj[CPT] = {v4.x, v4.y, v4.z, v4.w};
         const float4* qt = reinterpret_cast<const float4*>(qs + tt * DPAD + l * PAD);
@@ -367,8 +370,11 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 3 : LONG ? 1 : few_blocks
         const ulonglong2 vb = *reinterpret_cast<const ulonglong2*>(vs + (tt * COLS + jl * CPT) * 2 + 4);
         vj[0] = va.x, vj[1] = va.y, vj[2] = vb.x, vj[3] = vb.y;
       } else {
-        const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT);
-        vj[0] = pair2(v4.x, v4.x), vj[1] = pair2(v4.y, v4.y), vj[2] = pair2(v4.z, v4.z), vj[3] = pair2(v4.w, v4.w);
+#pragma unroll
+        for (int cc = 0; cc < CPT; cc += 4) {
+          const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT + cc);
+          vj[cc] = pair2(v4.x, v4.x), vj[cc + 1] = pair2(v4.y, v4.y), vj[cc + 2] = pair2(v4.z, v4.z), vj[cc + 3] = pair2(v4.w, v4.w);
+        }
       }
       const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(qs + tt * DPAD + l * PAD);
       const ulonglong2* kt = reinterpret_cast<const ulonglong2*>(ks + tt * DPAD + l * PAD);
@@ -406,13 +412,14 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 3 : LONG ? 1 : few_blocks
       for (int cc = 0; cc < CPT; ++cc) o[cc] = low2(o2[cc]) + high2(o2[cc]);
     };
     int first = 0;
-    if constexpr (LONG && LPC == 32 && CHUNK % 8 == 0) {
-      // Eight tokens at a time: their 32 sums over 32 lanes in 31 exchanges, after which lane l holds token l / 4's sum of column
-      // l % 4.  A sum's additions are those of a token by itself (lanes 16 apart, then 8, 4, 2, 1).
-      for (; first + 8 <= n; first += 8) {
+    constexpr int GROUP = 32 / CPT;              // tokens whose sums of CPT columns are 32
+    if constexpr (LONG && LPC == 32 && CHUNK % GROUP == 0) {
+      // A group of tokens at a time: their 32 sums over 32 lanes in 31 exchanges, after which lane l holds token l / CPT's sum of column
+      // l % CPT.  A sum's additions are those of a token by itself (lanes 16 apart, then 8, 4, 2, 1).
+      for (; first + GROUP <= n; first += GROUP) {
         float x[32];
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
+        for (int g = 0; g < GROUP; ++g) {
           float o[CPT];
           token(first + g, o);
 #pragma unroll
@@ -427,7 +434,7 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 3 : LONG ? 1 : few_blocks
             x[i] = (up ? x[i + w] : x[i]) + got;
           }
         }
-        if (jb + (l & 3) < vdim) out[(size_t)(t0 + first + (l >> 2)) * heads * vdim + hv + jb + (l & 3)] = x[0];
+        if (jb + (l & (CPT - 1)) < vdim) out[(size_t)(t0 + first + l / CPT) * heads * vdim + hv + jb + (l & (CPT - 1))] = x[0];
       }
     }
     constexpr int kUnroll = LPC < 32 ? 4 : 1;    // 32 lanes: at most seven tokens come here; fewer: all (f32 heads of 64, 512 tokens: 91 -> 86 us)
@@ -438,7 +445,7 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 3 : LONG ? 1 : few_blocks
       // the four columns' sums over the LPC lanes: two exchanges halve what a lane holds, then a butterfly
       int mine = 0;                              // the column whose sum this lane ends up with
       float b;
-      if (LPC >= 4) {
+      if constexpr (LPC >= 4 && CPT == 4) {
         const bool up = (l & (LPC / 2)) != 0, up2 = (l & (LPC / 4)) != 0;
         const float r0 = __shfl_xor_sync(0xffffffffu, up ? o[0] : o[2], LPC / 2);
         const float r1 = __shfl_xor_sync(0xffffffffu, up ? o[1] : o[3], LPC / 2);
@@ -494,32 +501,35 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 3 : LONG ? 1 : few_blocks
 
 // left[i] of a row in segments becomes the memory behind its segment i; the last one's goes to the row's slot.  A thread has four channels of a
 // column and runs through the segments, all of whose numbers it asks for first.
-__global__ void __launch_bounds__(256) gla_join_kernel(float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
+__global__ void __launch_bounds__(128) gla_join_kernel(float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
                                                        const int* __restrict__ state_slots, int heads, int dim, int vdim, Segments sg) {
   pdl_launch_dependents();
   pdl_wait();
   int r, seg, parts, cut;
   if (!segment_of<false>(blockIdx.z, q_indptr, sg.rows, r, seg, parts, cut) || seg) return;
-  const int h = blockIdx.y, idx = blockIdx.x * 256 + threadIdx.x, quads = dim / 4;
+  const int h = blockIdx.y, idx = blockIdx.x * 128 + threadIdx.x, quads = dim / 4;
   if (idx >= vdim * quads) return;
   const int e = idx % quads * 4;
   const size_t step = (size_t)heads * vdim * dim, d_step = (size_t)heads * dim;
   float* left = sg.left + ((size_t)cut * heads + h) * vdim * dim + (size_t)idx * 4;
   const float* decay = sg.decay + ((size_t)cut * heads + h) * dim + e;
-  float4 x[kMostSegs], d[kMostSegs];
+  float4 S = *reinterpret_cast<const float4*>(left);
+#pragma unroll 1
+  for (int i0 = 1; i0 < parts; i0 += 5) {        // five segments' numbers at a time, all asked for before the first is used
+    float4 x[5], d[5];
 #pragma unroll
-  for (int i = 0; i < kMostSegs; ++i)
-    if (i < parts) {
-      x[i] = *reinterpret_cast<const float4*>(left + i * step);
-      d[i] = i ? *reinterpret_cast<const float4*>(decay + i * d_step) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  float4 S = x[0];
+    for (int u = 0; u < 5; ++u)
+      if (i0 + u < parts) {
+        x[u] = *reinterpret_cast<const float4*>(left + (i0 + u) * step);
+        d[u] = *reinterpret_cast<const float4*>(decay + (i0 + u) * d_step);
+      }
 #pragma unroll
-  for (int i = 1; i < kMostSegs; ++i)
-    if (i < parts) {
-      S = make_float4(fmaf(d[i].x, S.x, x[i].x), fmaf(d[i].y, S.y, x[i].y), fmaf(d[i].z, S.z, x[i].z), fmaf(d[i].w, S.w, x[i].w));
-      if (i + 1 < parts) *reinterpret_cast<float4*>(left + i * step) = S;
-    }
+    for (int u = 0; u < 5; ++u)
+      if (i0 + u < parts) {
+        S = make_float4(fmaf(d[u].x, S.x, x[u].x), fmaf(d[u].y, S.y, x[u].y), fmaf(d[u].z, S.z, x[u].z), fmaf(d[u].w, S.w, x[u].w));
+        if (i0 + u + 1 < parts) *reinterpret_cast<float4*>(left + (i0 + u) * step) = S;
+      }
+  }
   float* sp = state + (size_t)state_slots[r] * slot_stride + (size_t)h * vdim * dim + (size_t)idx * 4;
   sp[0] = S.x, sp[1] = S.y, sp[2] = S.z, sp[3] = S.w;
 }
@@ -558,15 +568,11 @@ __global__ void __launch_bounds__(256, 2) gla_carry_kernel(const int* __restrict
       *reinterpret_cast<float4*>(qs + (i >> 5) * kCarryPitch + e) = x;
     }
     __syncthreads();
-    // what the segment alone gave, asked for before the products: a load behind a store to the same array would wait for it
     float sum[8][4];
 #pragma unroll
     for (int a = 0; a < 8; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int t = t0 + ty * 8 + a, j = j0 + tx + 32 * b;
-        sum[a][b] = t < t_end && j < vdim ? out[((size_t)t * heads + h) * vdim + j] : 0.f;
-      }
+      for (int b = 0; b < 4; ++b) sum[a][b] = 0.f;
 #pragma unroll 1
     for (int e0 = 0; e0 < dim; e0 += 32) {
 #pragma unroll
@@ -594,16 +600,22 @@ __global__ void __launch_bounds__(256, 2) gla_carry_kernel(const int* __restrict
           for (int b = 0; b < 4; ++b) sum[half * 4 + a][b] += low2(acc[a][b]) + high2(acc[a][b]);
       }
     }
+    // what the segment alone gave, all asked for before the first store: a load behind a store to the same array would wait for it
+    float alone[8][4];
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const int t = t0 + ty * 8 + a;
-      if (t >= t_end) break;
+    for (int a = 0; a < 8; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const int j = j0 + tx + 32 * b;
-        if (j < vdim) out[((size_t)t * heads + h) * vdim + j] = sum[a][b];
+        const int t = t0 + ty * 8 + a, j = j0 + tx + 32 * b;
+        alone[a][b] = t < t_end && j < vdim ? out[((size_t)t * heads + h) * vdim + j] : 0.f;
       }
-    }
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int t = t0 + ty * 8 + a, j = j0 + tx + 32 * b;
+        if (t < t_end && j < vdim) out[((size_t)t * heads + h) * vdim + j] = alone[a][b] + sum[a][b];
+      }
   }
 }
 
@@ -777,15 +789,15 @@ ARLE_API int arle_gla_scan_segments(const void* q, const void* k, const void* v,
   sg.decay = sg.left + (size_t)slots * heads * vdim * dim;
   sg.q_decayed = sg.decay + (size_t)slots * heads * dim;
   sg.rows = rows;
-  constexpr int COLS = kScanThreads / 32 * kScanCpt;
+  constexpr int CPT = SEGCPT, COLS = kScanThreads / 32 * CPT;
   static SharedLimit limit;
   const cudaError_t raised = limit.raise((const void*)gla_carry_kernel, kCarrySmem);
   if (raised != cudaSuccess) return (int)raised;
   typedef __nv_bfloat16 T;
-  launch_kernel(gla_scan_kernel<T, 4, 32, true, false, true, true>, dim3((vdim + COLS - 1) / COLS, heads, rows + slots), dim3(kScanThreads), 0, s, 1,
+  launch_kernel(gla_scan_kernel<T, 4, 32, true, false, true, true, CPT>, dim3((vdim + COLS - 1) / COLS, heads, rows + slots), dim3(kScanThreads), 0, s, 1,
                 (const T*)q, (const T*)k, (const T*)v, in_stride, alpha, (const float*)nullptr, state, slot_stride, q_indptr, state_slots, out, heads,
                 dim, vdim, q_scale, sg);
-  launch_kernel(gla_join_kernel, dim3((vdim * (dim / 4) + 255) / 256, heads, slots), dim3(256), 0, s, 1, state, slot_stride, q_indptr, state_slots,
+  launch_kernel(gla_join_kernel, dim3((vdim * (dim / 4) + 127) / 128, heads, slots), dim3(128), 0, s, 1, state, slot_stride, q_indptr, state_slots,
                 heads, dim, vdim, sg);
   launch_kernel(gla_carry_kernel, dim3((vdim + kCarryCols - 1) / kCarryCols, heads, slots), dim3(256), kCarrySmem, s, 1, q_indptr, out, heads, dim,
                 vdim, sg);

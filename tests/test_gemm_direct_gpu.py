@@ -1,0 +1,48 @@
+"""Products of up to 8 rows that read their weights straight from memory, against float64: each way of cutting them (8 and 16 rows a block, 8 to
+32 warps), sizes at which a block's rows and a warp's share of K do not come out whole, and the sizes on both sides of the rule; with and without
+the rows' norm factors, as a gated pair and into a residual."""
+import pytest
+import torch
+
+from arle_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 32), (8, 9, 96), (3, 1152, 1056), (5, 1147, 1600), (2, 1151, 2080), (7, 1153, 2048), (1, 2303, 1568), (8, 4608, 1056),
+                                   (4, 9215, 64), (6, 9217, 64), (8, 4096, 4096), (2, 4097, 4096)])
+def test_direct_products(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    wide = torch.randn(M, K + 8, generator=g, device=DEV).to(torch.bfloat16)
+    x, w = wide[:, :K], (torch.randn(N, K + 8, generator=g, device=DEV) * K ** -0.5).to(torch.bfloat16)[:, :K]
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    room = K * 2.0 ** -24 * size                                # float32 sums of exact products, whatever their order
+    for dtype, unit in ((torch.float32, 2.0 ** -24), (torch.bfloat16, 2.0 ** -8)):
+        out = torch.full((M + 1, N + 8), 7.0, device=DEV, dtype=dtype)
+        ops.gemm(x, w, out[:M, :N])
+        assert ((out[:M, :N].double() - want).abs() <= room + unit * want.abs()).all() and (out[M] == 7.0).all() and (out[:, N:] == 7.0).all()
+    rows = ops.ScaledRows(x, torch.rand(ops.SS_TABLE_SHAPE, generator=g, device=DEV), 1e-6)
+    f = torch.rsqrt(rows.ss[:M].double().sum(1, keepdim=True) / K + 1e-6)
+    out = torch.empty(M, N, device=DEV)
+    ops.gemm(rows, w, out)
+    assert ((out.double() - want * f).abs() <= (room + 1e-6 * want.abs()) * f).all()
+    if N % 2 == 0:
+        out = torch.empty(M, N // 2, device=DEV, dtype=torch.float32)
+        ops.gemm_silu_mul(rows, w, torch.empty(M, N, device=DEV, dtype=torch.bfloat16), out)
+        gate, up = (want * f)[:, 0::2], (want * f)[:, 1::2]
+        near = (room * f)[:, 0::2] * 1.1 * up.abs() + (room * f)[:, 1::2] * gate.abs() + 2e-6 * (gate * up).abs() + 1e-12
+        assert ((out.double() - gate * torch.sigmoid(gate) * up).abs() <= near).all()
+    resid0, gain = torch.randn(M, N, generator=g, device=DEV), torch.rand(N, generator=g, device=DEV)
+    got = []
+    for _ in range(2):
+        sink = ops.ResidualSink(resid0.clone(), gain, 1e-6, torch.empty(M, N, device=DEV, dtype=torch.bfloat16), torch.full(ops.SS_TABLE_SHAPE, 7.0, device=DEV), 0.5)
+        assert ops.gemm(x, w, None, sink=sink)
+        got.append(sink)
+    r = got[0].resid.double()
+    assert ((r - resid0.double() - 0.5 * want).abs() <= room + 2.0 ** -23 * (resid0.double().abs() + want.abs())).all()
+    assert ((got[0].xs.double() - r * gain.double()).abs() <= 2.0 ** -8 * (r * gain.double()).abs()).all()
+    ss = got[0].ss.double()
+    assert (ss[M:] == 0).all() and ((ss[:M].sum(1) - r.square().sum(1)).abs() <= 1e-5 * r.square().sum(1)).all()
+    assert torch.equal(got[0].resid, got[1].resid) and torch.equal(got[0].ss, got[1].ss)
+    ops.check_errors(DEV)
