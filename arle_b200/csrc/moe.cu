@@ -96,11 +96,14 @@ __global__ void moe_select_kernel(const float* __restrict__ z, int z_stride, con
   }
 }
 
-// The same without groups and softmax over all experts, for the usual sizes: a warp per token, a lane keeps the choice scores of
-// the experts lane, lane + 32, ...; the largest is found by exchanges, ties to the lower index.
+// The same without softmax over all experts, for the usual sizes: a warp per token, a lane keeps the choice scores of
+// the experts lane, lane + 32, ...; the largest is found by exchanges, ties to the lower index.  With groups a lane forms one group's score
+// from shared memory.  Bound by its chain of exchanges (the kernel above runs a thread's whole token through memory): 32 experts in 4 groups, 64
+// tokens 4.6 us (12.2 there), 2,048 tokens 5.1 (14.3).
+constexpr int kSelectWarps = 4;
 template <int PER>
-__global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride, const float* __restrict__ correction, int E, int top, float scale,
-                                       int mode, int* __restrict__ ids, float* __restrict__ wts, int num_tokens) {
+__global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride, const float* __restrict__ correction, int E, int top, int groups,
+                                       int keep, float scale, int mode, int* __restrict__ ids, float* __restrict__ wts, int num_tokens) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -113,6 +116,46 @@ __global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride
     const int e = lane + 32 * i;
     zv[i] = e < E ? zr[e] : 0.f;
     ch[i] = ((mode & 4) ? zv[i] : 1.0f / (1.0f + expf(-zv[i]))) + (correction && e < E ? correction[e] : 0.f);
+  }
+  if (keep < groups) {
+    __shared__ float scores[kSelectWarps][32 * PER];
+    float* sc = scores[threadIdx.x >> 5];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) sc[lane + 32 * i] = ch[i];
+    __syncwarp();
+    const int per = E / groups;
+    float gs = -INFINITY;                               // of group `lane`
+    if (lane < groups) {
+      float b1 = -INFINITY, b2 = -INFINITY;
+      for (int i = 0; i < per; ++i) {
+        const float v = sc[lane * per + i];
+        if (v > b1) {
+          b2 = b1;
+          b1 = v;
+        } else if (v > b2) {
+          b2 = v;
+        }
+      }
+      gs = (per > 1 && !(mode & 2)) ? b1 + b2 : b1;
+    }
+    unsigned kept = 0;
+    for (int it = 0; it < keep; ++it) {
+      float bv = gs;
+      int bi = lane < groups && !((kept >> lane) & 1) ? lane : 0x7fffffff;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (oi != 0x7fffffff && (bi == 0x7fffffff || ov > bv || (ov == bv && oi < bi))) {
+          bv = ov;
+          bi = oi;
+        }
+      }
+      kept |= 1u << __shfl_sync(0xffffffffu, bi, 0);    // one lane's word for all: a NaN may leave them apart
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (lane + 32 * i < E && !((kept >> ((lane + 32 * i) / per)) & 1)) ch[i] = -INFINITY;
   }
   unsigned taken = 0;                                   // this lane's experts that are chosen, or not experts at all
 #pragma unroll
@@ -139,6 +182,8 @@ __global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride
         bi = oi;
       }
     }
+    bi = __shfl_sync(0xffffffffu, bi, 0);
+    bz = __shfl_sync(0xffffffffu, bz, 0);
     if ((bi & 31) == lane) taken |= 1u << (bi >> 5);
     if (it == 0) cm = bz;
     const float w = (mode & 4) ? expf(bz - cm) : scale / (1.0f + expf(-bz));
@@ -156,10 +201,10 @@ ARLE_API int arle_moe_select(const float* z, int z_stride, const float* correcti
                              int keep, float scale, int mode, int* ids, float* wts, int num_tokens, cudaStream_t s) {
   if (num_tokens <= 0) return 0;
   if (E <= 0 || top <= 0 || groups <= 0 || E % groups || keep <= 0 || keep > groups || top > keep * (E / groups)) return ARLE_E_BADARG;
-  if (groups == 1 && !(mode & 1) && E <= 256 && !((mode & 4) && correction)) {
+  if (groups <= 32 && !(mode & 1) && E <= 256 && !((mode & 4) && correction)) {
     auto kernel = E <= 32 ? moe_select_warp_kernel<1> : E <= 64 ? moe_select_warp_kernel<2> : moe_select_warp_kernel<8>;
-    const int warps = num_tokens <= 592 ? 1 : 4;
-    launch_kernel(kernel, dim3((num_tokens + warps - 1) / warps), dim3(32 * warps), 0, s, 1, z, z_stride, correction, E, top, scale, mode, ids, wts,
+    const int warps = num_tokens <= 592 ? 1 : kSelectWarps;
+    launch_kernel(kernel, dim3((num_tokens + warps - 1) / warps), dim3(32 * warps), 0, s, 1, z, z_stride, correction, E, top, groups, keep, scale, mode, ids, wts,
                   num_tokens);
     return launch_status();
   }
