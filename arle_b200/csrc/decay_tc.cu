@@ -22,8 +22,9 @@
 // by 0.8e-7 to 1.0e-7 (0.6e-7 to 1.1e-7).
 //
 // What bounds it: the chain of chunks of a block (some 9 us each: the tensor cores' legacy path, a third of the time, then the matrix
-// loads and the barriers between the phases), with one block an SM.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 306 us (the
-// scan 1,162), 8 heads of 256 x 513 324 us (1,740 to 1,937 as the scan's mean of both).
+// loads and the barriers between the phases), with one block an SM.  A scheduler has two warps; one takes an early tile of rows and the other a
+// late one, which sees more keys.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 284 us (306 with two early or two late ones, the
+// scan 1,162), 8 heads of 256 x 513 324 us before (1,740 to 1,937 as the scan's mean of both).
 #include "common.cuh"
 #include "mma_utils.cuh"
 using namespace arle;
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(kThreads, 1) decay_tc_kernel(
   const int g = h / (H / kq_heads);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, t4 = lane & 3;
-  const int rt = warp & 3, n_half = (warp >> 2) * (VT / 2);
+  const int rt = warp < 4 ? warp : 7 - warp, n_half = (warp >> 2) * (VT / 2);      // a scheduler's two warps take early and late rows
   const int um = (SPLIT_N ? (warp & 3) : warp * MT) * 16, un = SPLIT_N ? n_half : 0;
   float* sp = state + (size_t)state_slots[r] * slot_stride + (size_t)h * vcols * DIM;
 
