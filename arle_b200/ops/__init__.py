@@ -2056,7 +2056,7 @@ def delta_gates(pre, a_log, dt_bias, beta, decay) -> None:
 
 def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: int, kq_heads: int, dim: int, vdim: int,
                q_scale: float, unit_eps: float, max_q_len: int = 0, scratch=None) -> None:
-    """``scratch`` (float32, ``delta_scan_scratch`` numbers, or None): the rows of 64 tokens and more run in chunks on the tensor cores.
+    """``scratch`` (float32, ``delta_scan_scratch`` numbers, or None): the rows of 80 tokens and more run in chunks on the tensor cores.
     The gated delta rule over the tokens of every row of the step, from and into state[state_slots[r]]: with q and k brought
     to unit length per head (x / sqrt(sum x^2 + unit_eps); q also times q_scale), S <- decay_t S; u = beta_t (v_t - S^T k_t);
     S <- S + k_t u^T; o_t = S^T q_t.  q, k [T, kq_heads*dim] (head h reads head h // (heads / kq_heads)), v [T, heads*vdim], in
@@ -2093,12 +2093,13 @@ def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: i
                                      dim, vdim, float(q_scale), float(unit_eps), longest, _stream()), "delta_scan")
 
 
-# Rows of the delta rule up to this length are scanned, also where longer rows run in chunks: a row's own length decides.  DELTA_RULE_LINE
-DELTA_SCAN_LONGEST = 63
+# Rows of the delta rule up to this length are scanned, also where longer rows run in chunks: a row's own length decides.  One row, 8 heads of 128:
+# 64 tokens 21 us scanned and 24 in chunks, 128 tokens 37 and 27; 32 heads 25 and 24, four rows of 80 83 and 63.
+DELTA_SCAN_LONGEST = 79
 
 
 def delta_scan_scratch(q, k, v, out, rows: int, heads: int, dim: int, vdim: int, max_q_len: int) -> int:
-    """How many float32 numbers of scratch let ``delta_scan`` run the step's rows of 64 tokens and more in chunks on the tensor cores; 0: all
+    """How many float32 numbers of scratch let ``delta_scan`` run the step's rows of 80 tokens and more in chunks on the tensor cores; 0: all
     rows are scanned (short rows, other types and sizes, arrays off their boundaries)."""
     if (_KERNEL_SET != "fast" or not q.is_cuda or q.dtype != torch.bfloat16 or dim != 128 or vdim % 8 or max_q_len <= DELTA_SCAN_LONGEST
             or heads > 65535 or rows > 65535 or any(t.stride(0) % 8 or t.data_ptr() % 16 for t in (q, k, v)) or out.data_ptr() % 8):
