@@ -105,62 +105,6 @@ __device__ __forceinline__ float4 widen4(uint2 u) {
 template <typename T, bool VEC> struct Raw4 { using type = float4; };
 template <> struct Raw4<__nv_bfloat16, true> { using type = uint2; };
 
-// A long row as segments that are scanned side by side, each from an empty memory but the first; gla_join then forms the memory in front of
-// every segment (S <- diag(D) S + what the segment alone leaves, D the product of its decays), and gla_carry adds what the segment's tokens read
-// from it, o_t += (D_t q_t) S with D_t the product of the segment's decays up to t.  One scan of 2,048 tokens, 16 heads of 128 x 128, keeps a
-// single warp on each scheduler (37 % of the issue slots); sixteen segments keep three.  SEGMENT_FIGURES
-// A row's own length decides how it is cut: from kSegFrom tokens on (below, the two further launches cost what the shorter chain gains), in
-// parts of kSegTokens and more, sixteen at most, which bounds the memories between them.
-#ifndef SEGCPT
-#define SEGCPT 8
-#define SEGN 128
-#endif
-constexpr int kSegTokens = SEGN, kSegFrom = 384, kMostSegs = 16;
-struct Segments {
-  float* left;                                   // [cut][head][vdim][dim]: the memory that a segment leaves
-  float* decay;                                  // [cut][head][dim]: the product of its decays
-  float* q_decayed;                              // [tokens][head][dim]: D_t q_t, scaled; written for all segments but a row's first
-  int rows;
-};
-__device__ __forceinline__ int segment_tokens(int n) {
-  if (n < kSegFrom) return n > 0 ? n : 1;
-  const int parts = min(kMostSegs, n / kSegTokens);
-  return ((n + parts - 1) / parts + 15) / 16 * 16;
-}
-// The row and the segment of a slot (all of a warp's lanes together), false if there is no such slot.  Slots are counted over all segments of
-// all rows (ALL), or over those of rows in several segments; `cut` is the slot's number among the latter.
-template <bool ALL>
-__device__ __forceinline__ bool segment_of(int slot, const int* q_indptr, int rows, int& row, int& seg, int& parts, int& cut) {
-  const int lane = threadIdx.x & 31;
-  int before = 0, cut_before = 0;
-  for (int r0 = 0; r0 < rows; r0 += 32) {
-    int n = 0;
-    if (r0 + lane < rows) {
-      const int tokens = q_indptr[r0 + lane + 1] - q_indptr[r0 + lane], len = segment_tokens(tokens);
-      n = max(1, (tokens + len - 1) / len);
-    }
-    const int n_cut = n > 1 ? n : 0, mine = ALL ? n : n_cut;
-    int sum = mine, cut_sum = n_cut;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, sum, o), z = __shfl_up_sync(0xffffffffu, cut_sum, o);
-      if (lane >= o) sum += y, cut_sum += z;
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, slot < before + sum);
-    if (hit) {
-      const int src = __ffs(hit) - 1;
-      row = r0 + src;
-      parts = __shfl_sync(0xffffffffu, n, src);
-      seg = slot - before - __shfl_sync(0xffffffffu, sum - mine, src);
-      cut = cut_before + __shfl_sync(0xffffffffu, cut_sum - n_cut, src) + seg;
-      return true;
-    }
-    before += __shfl_sync(0xffffffffu, sum, 31);
-    cut_before += __shfl_sync(0xffffffffu, cut_sum, 31);
-  }
-  return false;
-}
-
 // DPT: consecutive key channels that a thread keeps of each of its kScanCpt columns of the state (4 up to 128
 // channels, then 8, 16).  LPC: lanes that share a column (a power of two; LPC * DPT >= dim).  VEC: four channels
 // at a time can be fetched with one aligned load.  A chunk of CHUNK tokens is staged in shared memory; while it is
@@ -179,14 +123,14 @@ constexpr int few_blocks() {
   if (LPC == 1) return 3;
   return VEC && !BONUS && LPC >= 4 ? 5 : 4;
 }
-// SEGS: a row in segments, see Segments above.
-template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool LONG, bool SEGS, int CPT = kScanCpt>
-__global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks<T, DPT, LPC, VEC, BONUS>()) gla_scan_kernel(
+template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool LONG>
+__global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LPC, VEC, BONUS>()) gla_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int in_stride,
     const float* __restrict__ alpha, const float* __restrict__ bonus, float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
-    const int* __restrict__ state_slots, float* __restrict__ out, int heads, int dim, int vdim, float q_scale, Segments sg) {
+    const int* __restrict__ state_slots, float* __restrict__ out, int heads, int dim, int vdim, float q_scale) {
   pdl_launch_dependents();
   pdl_wait();
+  constexpr int CPT = kScanCpt;
   constexpr int COLS = kScanThreads / LPC * CPT; // columns a block takes
   constexpr int DSPAN = DPT * LPC;               // dim rounded up; channels past dim hold zeros
   constexpr int PAD = DPT == 4 ? 4 : DPT + 4;    // floats a thread's channels take in shared memory: 16-byte rows, spread over the banks
@@ -197,25 +141,12 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
   constexpr int QPT = (QUADS + kScanThreads - 1) / kScanThreads;
   constexpr int VPT = (CHUNK * COLS + kScanThreads - 1) / kScanThreads;
   __shared__ __align__(16) float qs[CHUNK * DPAD], ks[CHUNK * DPAD], as[CHUNK * DPAD];
-  constexpr int VD = LONG && LPC >= 4 && CPT == 4 ? 2 : 1;           // v's numbers stand twice side by side (a factor of both halves of a pair), where there is room
+  constexpr int VD = LONG && LPC >= 4 ? 2 : 1;           // v's numbers stand twice side by side (a factor of both halves of a pair), where there is room
   __shared__ __align__(16) float vs[CHUNK * COLS * VD];
-  const int h = blockIdx.y, j0 = blockIdx.x * COLS;
+  const int r = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * COLS;
   const int l = threadIdx.x & (LPC - 1), jl = threadIdx.x / LPC;
   const int jb = j0 + jl * CPT;                  // this thread's first column
-  int r = blockIdx.z, seg = 0, parts = 1, cut = 0;
-  if constexpr (SEGS) {
-    if (!segment_of<true>(blockIdx.z, q_indptr, sg.rows, r, seg, parts, cut)) return;
-  }
-  int t_begin = q_indptr[r], t_end = q_indptr[r + 1];
-  if constexpr (SEGS) {
-    const int len = segment_tokens(t_end - t_begin);
-    t_begin += seg * len;
-    t_end = min(t_end, t_begin + len);
-  }
-  const bool leads = SEGS && seg > 0 && blockIdx.x == 0 && threadIdx.x < 32;   // the warp that writes D_t q_t
-  f32x2 prod[SEGS ? DPT / 2 : 1];
-#pragma unroll
-  for (int i = 0; i < (SEGS ? DPT / 2 : 1); ++i) prod[i] = pair2(1.f, 1.f);
+  const int t_begin = q_indptr[r], t_end = q_indptr[r + 1];
   // the state of a head is kept as [vdim][dim]: a thread's channels of a column are contiguous
   float* S_g = state + (size_t)state_slots[r] * slot_stride + ((size_t)h * vdim) * dim + l * DPT;
   const bool vec_state = (dim & 3) == 0 && (slot_stride & 3) == 0 && ((uintptr_t)state & 15) == 0;
@@ -230,7 +161,7 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
   f32x2 S[CPT][DPT / 2];                         // channels 2i and 2i + 1 of a column
 #pragma unroll
   for (int cc = 0; cc < CPT; ++cc) {
-    const bool col_ok = jb + cc < vdim && seg == 0;
+    const bool col_ok = jb + cc < vdim;
     const float* sp = S_g + (size_t)(col_ok ? jb + cc : 0) * dim;
 #pragma unroll
     for (int i = 0; i < DPT; i += 4) {
@@ -333,7 +264,7 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
     if (t0 + CHUNK < t_end) fetch(t0 + CHUNK, min(CHUNK, t_end - t0 - CHUNK));
     // one token: the memory's step and the thread's part of its columns' sums
     auto token = [&](int tt, float (&o)[CPT]) {
-      if constexpr (!LONG && CPT == 4) {         // single numbers: the same roundings in fewer registers
+      if constexpr (!LONG) {                     // single numbers: the same roundings in fewer registers
         const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT);
         const float vj[CPT] = {v4.x, v4.y, v4.z, v4.w};
         const float4* qt = reinterpret_cast<const float4*>(qs + tt * DPAD + l * PAD);
@@ -370,11 +301,8 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
         const ulonglong2 vb = *reinterpret_cast<const ulonglong2*>(vs + (tt * COLS + jl * CPT) * 2 + 4);
         vj[0] = va.x, vj[1] = va.y, vj[2] = vb.x, vj[3] = vb.y;
       } else {
-#pragma unroll
-        for (int cc = 0; cc < CPT; cc += 4) {
-          const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT + cc);
-          vj[cc] = pair2(v4.x, v4.x), vj[cc + 1] = pair2(v4.y, v4.y), vj[cc + 2] = pair2(v4.z, v4.z), vj[cc + 3] = pair2(v4.w, v4.w);
-        }
+        const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT);
+        vj[0] = pair2(v4.x, v4.x), vj[1] = pair2(v4.y, v4.y), vj[2] = pair2(v4.z, v4.z), vj[3] = pair2(v4.w, v4.w);
       }
       const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(qs + tt * DPAD + l * PAD);
       const ulonglong2* kt = reinterpret_cast<const ulonglong2*>(ks + tt * DPAD + l * PAD);
@@ -385,14 +313,6 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
 #pragma unroll
       for (int i = 0; i < DPT / 4; ++i) {
         const ulonglong2 a4 = at[i], k4 = kt[i], q4 = qt[i];
-        if constexpr (SEGS) {
-          if (leads) {
-            prod[2 * i] = mul2(prod[2 * i], a4.x), prod[2 * i + 1] = mul2(prod[2 * i + 1], a4.y);
-            if (l * DPT + 4 * i < dim)
-              *reinterpret_cast<ulonglong2*>(sg.q_decayed + (size_t)(t0 + tt) * a_stride + hq + l * DPT + 4 * i) =
-                  make_ulonglong2(mul2(q4.x, prod[2 * i]), mul2(q4.y, prod[2 * i + 1]));
-          }
-        }
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
           const f32x2 kv0 = mul2(k4.x, vj[cc]), kv1 = mul2(k4.y, vj[cc]);
@@ -412,14 +332,13 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
       for (int cc = 0; cc < CPT; ++cc) o[cc] = low2(o2[cc]) + high2(o2[cc]);
     };
     int first = 0;
-    constexpr int GROUP = 32 / CPT;              // tokens whose sums of CPT columns are 32
-    if constexpr (LONG && LPC == 32 && CHUNK % GROUP == 0) {
-      // A group of tokens at a time: their 32 sums over 32 lanes in 31 exchanges, after which lane l holds token l / CPT's sum of column
-      // l % CPT.  A sum's additions are those of a token by itself (lanes 16 apart, then 8, 4, 2, 1).
-      for (; first + GROUP <= n; first += GROUP) {
+    if constexpr (LONG && LPC == 32 && CHUNK % 8 == 0) {
+      // Eight tokens at a time: their 32 sums over 32 lanes in 31 exchanges, after which lane l holds token l / 4's sum of column
+      // l % 4.  A sum's additions are those of a token by itself (lanes 16 apart, then 8, 4, 2, 1).
+      for (; first + 8 <= n; first += 8) {
         float x[32];
 #pragma unroll
-        for (int g = 0; g < GROUP; ++g) {
+        for (int g = 0; g < 8; ++g) {
           float o[CPT];
           token(first + g, o);
 #pragma unroll
@@ -434,7 +353,7 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
             x[i] = (up ? x[i + w] : x[i]) + got;
           }
         }
-        if (jb + (l & (CPT - 1)) < vdim) out[(size_t)(t0 + first + l / CPT) * heads * vdim + hv + jb + (l & (CPT - 1))] = x[0];
+        if (jb + (l & 3) < vdim) out[(size_t)(t0 + first + (l >> 2)) * heads * vdim + hv + jb + (l & 3)] = x[0];
       }
     }
     constexpr int kUnroll = LPC < 32 ? 4 : 1;    // 32 lanes: at most seven tokens come here; fewer: all (f32 heads of 64, 512 tokens: 91 -> 86 us)
@@ -445,7 +364,7 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
       // the four columns' sums over the LPC lanes: two exchanges halve what a lane holds, then a butterfly
       int mine = 0;                              // the column whose sum this lane ends up with
       float b;
-      if constexpr (LPC >= 4 && CPT == 4) {
+      if (LPC >= 4) {
         const bool up = (l & (LPC / 2)) != 0, up2 = (l & (LPC / 4)) != 0;
         const float r0 = __shfl_xor_sync(0xffffffffu, up ? o[0] : o[2], LPC / 2);
         const float r1 = __shfl_xor_sync(0xffffffffu, up ? o[1] : o[3], LPC / 2);
@@ -467,19 +386,6 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
       }
     }
   }
-  bool vec_left = vec_state;
-  if constexpr (SEGS) {
-    if (parts > 1) {
-      S_g = sg.left + ((size_t)cut * heads + h) * vdim * dim + l * DPT;
-      vec_left = true;                           // dim is a multiple of four here, and the buffer starts on 16 bytes
-    }
-    if (leads) {
-#pragma unroll
-      for (int i = 0; i < DPT; i += 4)
-        if (l * DPT + i < dim)
-          *reinterpret_cast<ulonglong2*>(sg.decay + ((size_t)cut * heads + h) * dim + l * DPT + i) = make_ulonglong2(prod[i / 2], prod[i / 2 + 1]);
-    }
-  }
 #pragma unroll
   for (int cc = 0; cc < CPT; ++cc) {
     const bool col_ok = jb + cc < vdim;
@@ -487,7 +393,7 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
 #pragma unroll
     for (int i = 0; i < DPT; i += 4) {
       const int c = l * DPT + i;
-      if (vec_left) {
+      if (vec_state) {
         if (col_ok && c < dim)
           *reinterpret_cast<ulonglong2*>(sp + i) = make_ulonglong2(S[cc][i / 2], S[cc][i / 2 + 1]);
       } else {
@@ -496,126 +402,6 @@ __global__ void __launch_bounds__(kScanThreads, SEGS ? 2 : LONG ? 1 : few_blocks
           if (col_ok && c + e < dim) sp[i + e] = e & 1 ? high2(S[cc][(i + e) / 2]) : low2(S[cc][(i + e) / 2]);
       }
     }
-  }
-}
-
-// left[i] of a row in segments becomes the memory behind its segment i; the last one's goes to the row's slot.  A thread has four channels of a
-// column and runs through the segments, all of whose numbers it asks for first.
-__global__ void __launch_bounds__(128) gla_join_kernel(float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
-                                                       const int* __restrict__ state_slots, int heads, int dim, int vdim, Segments sg) {
-  pdl_launch_dependents();
-  pdl_wait();
-  int r, seg, parts, cut;
-  if (!segment_of<false>(blockIdx.z, q_indptr, sg.rows, r, seg, parts, cut) || seg) return;
-  const int h = blockIdx.y, idx = blockIdx.x * 128 + threadIdx.x, quads = dim / 4;
-  if (idx >= vdim * quads) return;
-  const int e = idx % quads * 4;
-  const size_t step = (size_t)heads * vdim * dim, d_step = (size_t)heads * dim;
-  float* left = sg.left + ((size_t)cut * heads + h) * vdim * dim + (size_t)idx * 4;
-  const float* decay = sg.decay + ((size_t)cut * heads + h) * dim + e;
-  float4 S = *reinterpret_cast<const float4*>(left);
-#pragma unroll 1
-  for (int i0 = 1; i0 < parts; i0 += 5) {        // five segments' numbers at a time, all asked for before the first is used
-    float4 x[5], d[5];
-#pragma unroll
-    for (int u = 0; u < 5; ++u)
-      if (i0 + u < parts) {
-        x[u] = *reinterpret_cast<const float4*>(left + (i0 + u) * step);
-        d[u] = *reinterpret_cast<const float4*>(decay + (i0 + u) * d_step);
-      }
-#pragma unroll
-    for (int u = 0; u < 5; ++u)
-      if (i0 + u < parts) {
-        S = make_float4(fmaf(d[u].x, S.x, x[u].x), fmaf(d[u].y, S.y, x[u].y), fmaf(d[u].z, S.z, x[u].z), fmaf(d[u].w, S.w, x[u].w));
-        if (i0 + u + 1 < parts) *reinterpret_cast<float4*>(left + (i0 + u) * step) = S;
-      }
-  }
-  float* sp = state + (size_t)state_slots[r] * slot_stride + (size_t)h * vdim * dim + (size_t)idx * 4;
-  sp[0] = S.x, sp[1] = S.y, sp[2] = S.z, sp[3] = S.w;
-}
-
-// o_t[j] += sum over d of q_decayed[t][d] left[j][d] for the tokens of every segment but a row's first; left: of the segment in front.  A block
-// has 128 columns and runs through the segment 64 tokens at a time; a thread eight tokens and four columns, two channels to a packed FMA, and
-// sums of 32 channels at a time, so that they are rounded as often as the scan's.
-constexpr int kCarryTokens = 64, kCarryCols = 128, kCarryPitch = 132;   // floats a row: eight rows' 16 bytes fall on different banks
-constexpr size_t kCarrySmem = (size_t)(kCarryTokens + kCarryCols) * kCarryPitch * sizeof(float);
-__global__ void __launch_bounds__(256, 2) gla_carry_kernel(const int* __restrict__ q_indptr, float* __restrict__ out, int heads, int dim, int vdim,
-                                                           Segments sg) {
-  pdl_launch_dependents();
-  pdl_wait();
-  int r, seg, parts, cut;
-  if (!segment_of<false>(blockIdx.z, q_indptr, sg.rows, r, seg, parts, cut) || seg == 0) return;
-  extern __shared__ __align__(16) float sm[];
-  float* qs = sm;                                // [tokens][pitch], zeros past dim
-  float* ms = qs + kCarryTokens * kCarryPitch;   // [columns][pitch]
-  const int h = blockIdx.y, j0 = blockIdx.x * kCarryCols, tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-  const int beg = q_indptr[r], end = q_indptr[r + 1], len = segment_tokens(end - beg);
-  const int t_begin = beg + seg * len, t_end = min(end, t_begin + len);
-  const float* left = sg.left + ((size_t)(cut - 1) * heads + h) * vdim * dim;
-#pragma unroll 8
-  for (int i = tid; i < kCarryCols * 32; i += 256) {
-    const int j = i >> 5, e = (i & 31) * 4;
-    const float4 x = (j0 + j < vdim && e < dim) ? *reinterpret_cast<const float4*>(left + (size_t)(j0 + j) * dim + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-    *reinterpret_cast<float4*>(ms + j * kCarryPitch + e) = x;
-  }
-  for (int t0 = t_begin; t0 < t_end; t0 += kCarryTokens) {
-    __syncthreads();
-#pragma unroll
-    for (int i = tid; i < kCarryTokens * 32; i += 256) {
-      const int t = t0 + (i >> 5), e = (i & 31) * 4;
-      const float4 x = (t < t_end && e < dim) ? *reinterpret_cast<const float4*>(sg.q_decayed + ((size_t)t * heads + h) * dim + e)
-                                              : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(qs + (i >> 5) * kCarryPitch + e) = x;
-    }
-    __syncthreads();
-    float sum[8][4];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) sum[a][b] = 0.f;
-#pragma unroll 1
-    for (int e0 = 0; e0 < dim; e0 += 32) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {     // four tokens at a time: the packed sums of eight would not fit in registers
-        f32x2 acc[4][4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] = 0;
-#pragma unroll 2
-        for (int e = 0; e < 32; e += 4) {
-          ulonglong2 m[4];
-#pragma unroll
-          for (int b = 0; b < 4; ++b) m[b] = *reinterpret_cast<const ulonglong2*>(ms + (tx + 32 * b) * kCarryPitch + e0 + e);
-#pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(qs + (ty * 8 + half * 4 + a) * kCarryPitch + e0 + e);
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = fma2(x.y, m[b].y, fma2(x.x, m[b].x, acc[a][b]));
-          }
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) sum[half * 4 + a][b] += low2(acc[a][b]) + high2(acc[a][b]);
-      }
-    }
-    // what the segment alone gave, all asked for before the first store: a load behind a store to the same array would wait for it
-    float alone[8][4];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int t = t0 + ty * 8 + a, j = j0 + tx + 32 * b;
-        alone[a][b] = t < t_end && j < vdim ? out[((size_t)t * heads + h) * vdim + j] : 0.f;
-      }
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int t = t0 + ty * 8 + a, j = j0 + tx + 32 * b;
-        if (t < t_end && j < vdim) out[((size_t)t * heads + h) * vdim + j] = alone[a][b] + sum[a][b];
-      }
   }
 }
 
@@ -721,12 +507,12 @@ int scan_launch(const void* q, const void* k, const void* v, int in_stride, cons
   const size_t eb = sizeof(T) * 4;               // bytes of four elements of q or k
   const bool vec = dim % 4 == 0 && in_stride % 4 == 0 && ((uintptr_t)q % eb) == 0 && ((uintptr_t)k % eb) == 0 &&
                    ((uintptr_t)alpha % 16) == 0;
-  auto kernel = max_q_len >= 8 ? (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, true, false> : gla_scan_kernel<T, DPT, LPC, false, true, true, false>)
-                                        : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, true, false> : gla_scan_kernel<T, DPT, LPC, false, false, true, false>))
-                       : (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, false, false> : gla_scan_kernel<T, DPT, LPC, false, true, false, false>)
-                                : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, false, false> : gla_scan_kernel<T, DPT, LPC, false, false, false, false>));
+  auto kernel = max_q_len >= 8 ? (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, true> : gla_scan_kernel<T, DPT, LPC, false, true, true>)
+                                        : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, true> : gla_scan_kernel<T, DPT, LPC, false, false, true>))
+                       : (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, false> : gla_scan_kernel<T, DPT, LPC, false, true, false>)
+                                : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, false> : gla_scan_kernel<T, DPT, LPC, false, false, false>));
   launch_kernel(kernel, grid, dim3(kScanThreads), 0, s, 1, (const T*)q, (const T*)k, (const T*)v, in_stride, alpha, bonus, state, slot_stride,
-                q_indptr, state_slots, out, heads, dim, vdim, q_scale, Segments{});
+                q_indptr, state_slots, out, heads, dim, vdim, q_scale);
   return launch_status();
 }
 
@@ -763,45 +549,6 @@ ARLE_API int arle_gla_scan(const void* q, const void* k, const void* v, int dtyp
   if (dtype == 1)
     return scan_dispatch<__nv_bfloat16>(q, k, v, in_stride, alpha, bonus, state, slot_stride, q_indptr, state_slots, out, rows, heads, dim, vdim, q_scale, max_q_len, s);
   return ARLE_E_BADARG;
-}
-
-// How many float32 numbers of scratch arle_gla_scan_segments wants for num_tokens tokens of `rows` rows; 0: it does not take them (arle_gla_scan
-// does).  bfloat16, dim over 64 and up to 128 in groups of four, some row long enough to be cut.
-ARLE_API long arle_gla_segments_scratch(int num_tokens, int rows, int heads, int dim, int vdim, int max_q_len) {
-  if (rows <= 0 || heads <= 0 || vdim <= 0 || dim <= 64 || dim > 128 || dim % 4 || max_q_len < kSegFrom || rows + num_tokens / kSegTokens > 65535) return 0;
-  const long slots = num_tokens / kSegTokens;
-  return slots * heads * ((long)vdim * dim + dim) + (long)num_tokens * heads * dim;
-}
-
-// arle_gla_scan for steps with long rows (arle_gla_segments_scratch above zero, no bonus).  q, k, alpha and scratch on 16-byte boundaries (q and k
-// on 8), in_stride a multiple of 4.
-ARLE_API int arle_gla_scan_segments(const void* q, const void* k, const void* v, int in_stride, const float* alpha, float* state, long slot_stride,
-                                    const int* q_indptr, const int* state_slots, float* out, float* scratch, int num_tokens, int rows, int heads,
-                                    int dim, int vdim, float q_scale, int max_q_len, cudaStream_t s) {
-  if (rows <= 0 || num_tokens <= 0) return 0;
-  if (heads <= 0 || dim <= 0 || vdim <= 0 || max_q_len <= 0 || slot_stride < (long)heads * vdim * dim || !scratch) return ARLE_E_BADARG;
-  if (arle_gla_segments_scratch(num_tokens, rows, heads, dim, vdim, max_q_len) == 0 || heads > 65535 || in_stride % 4 ||
-      (((uintptr_t)q | (uintptr_t)k) & 7) || (((uintptr_t)alpha | (uintptr_t)scratch) & 15))
-    return ARLE_E_UNSUPPORTED;
-  const int slots = num_tokens / kSegTokens;     // of rows in several segments: none has fewer tokens
-  Segments sg;
-  sg.left = scratch;
-  sg.decay = sg.left + (size_t)slots * heads * vdim * dim;
-  sg.q_decayed = sg.decay + (size_t)slots * heads * dim;
-  sg.rows = rows;
-  constexpr int CPT = SEGCPT, COLS = kScanThreads / 32 * CPT;
-  static SharedLimit limit;
-  const cudaError_t raised = limit.raise((const void*)gla_carry_kernel, kCarrySmem);
-  if (raised != cudaSuccess) return (int)raised;
-  typedef __nv_bfloat16 T;
-  launch_kernel(gla_scan_kernel<T, 4, 32, true, false, true, true, CPT>, dim3((vdim + COLS - 1) / COLS, heads, rows + slots), dim3(kScanThreads), 0, s, 1,
-                (const T*)q, (const T*)k, (const T*)v, in_stride, alpha, (const float*)nullptr, state, slot_stride, q_indptr, state_slots, out, heads,
-                dim, vdim, q_scale, sg);
-  launch_kernel(gla_join_kernel, dim3((vdim * (dim / 4) + 127) / 128, heads, slots), dim3(128), 0, s, 1, state, slot_stride, q_indptr, state_slots,
-                heads, dim, vdim, sg);
-  launch_kernel(gla_carry_kernel, dim3((vdim + kCarryCols - 1) / kCarryCols, heads, slots), dim3(256), kCarrySmem, s, 1, q_indptr, out, heads, dim,
-                vdim, sg);
-  return launch_status();
 }
 
 ARLE_API int arle_gla_out(const float* o, const void* gate, int dtype, int gate_stride, const float* weight, float eps,

@@ -38,7 +38,7 @@ def add_launches(n: int) -> None:
 
 
 _P, _I, _F = c_void_p, c_int, c_float
-_SIZES = {"arle_gla_segments_scratch": 6, "arle_delta_tc_scratch": 4}               # how much scratch an entry wants: whole numbers in, a size out
+_SIZES = {"arle_delta_tc_scratch": 4}               # how much scratch an entry wants: whole numbers in, a size out
 
 _SIGNATURES = {
     "arle_embedding": [_P, _P, _I, _P, _I, _I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _P],
@@ -51,7 +51,6 @@ _SIGNATURES = {
     "arle_weighted_sum": [_P, _F, _P, _F, _P, _I, ctypes.c_longlong, _P],
     "arle_logit_cap": [_P, _F, ctypes.c_longlong, _P],
     "arle_gla_decay": [_P, _I, _I, _P, _P, _F, _P, _I, _I, _I, _I, _P],
-    "arle_gla_scan_segments": [_P, _P, _P, _I, _P, _P, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
     "arle_gla_scan": [_P, _P, _P, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _F, _I, _P],
     "arle_gla_out": [_P, _P, _I, _I, _P, _F, _F, _P, _I, _I, _I, _I, _I, _I, _P],
     "arle_attention_prep": [_P, _I, _I, _P, _P, _P, _P, _F, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P],
@@ -1131,8 +1130,8 @@ def gla_decay(low, w2t, bias, tau: float, alpha, form: str = "sigmoid_root") -> 
 
 
 def gla_scan(q, k, v, alpha, state, q_indptr, state_slots, out, heads: int, dim: int, vdim: int, q_scale: float,
-             max_q_len: int, bonus=None, scratch=None) -> None:
-    """``scratch`` (float32, ``gla_scan_scratch`` numbers, or None): rows of several hundred tokens run as segments side by side.  ``bonus`` (float32 [heads*dim]): the read-out comes before the update, o_t = (S + diag(bonus) k_t v_t^T)^T (q_t *
+             max_q_len: int, bonus=None) -> None:
+    """``bonus`` (float32 [heads*dim]): the read-out comes before the update, o_t = (S + diag(bonus) k_t v_t^T)^T (q_t *
     q_scale).  Without it: the recurrence S <- diag(alpha_t) S + k_t v_t^T, o_t = S^T (q_t * q_scale) over the tokens of every row of
     the step (row r owns tokens q_indptr[r] .. q_indptr[r+1]-1), from and into state[state_slots[r]].
     q, k [T, heads*dim] and v [T, heads*vdim]: slices of one wider buffer (same row stride, unit inner stride);
@@ -1157,27 +1156,9 @@ def gla_scan(q, k, v, alpha, state, q_indptr, state_slots, out, heads: int, dim:
     _i32(q_indptr, "q_indptr"), _i32(state_slots, "state_slots")
     if q_indptr.numel() != R + 1:
         raise KernelError("gla_scan: q_indptr must have one entry more than state_slots")
-    if scratch is not None:
-        need = gla_scan_scratch(q, k, alpha, R, heads, dim, vdim, max_q_len)
-        if (bonus is not None or need == 0 or scratch.dtype != torch.float32 or not scratch.is_contiguous() or scratch.numel() < need
-                or scratch.data_ptr() % 16):
-            raise KernelError("gla_scan: scratch is for steps that gla_scan_scratch has a size for, float32, contiguous, on 16 bytes")
-        _check(library().arle_gla_scan_segments(_ptr(q), _ptr(k), _ptr(v), q.stride(0), _ptr(alpha), _ptr(state), state.stride(0), _ptr(q_indptr),
-                                                _ptr(state_slots), _ptr(out), _ptr(scratch), T, R, heads, dim, vdim, float(q_scale),
-                                                int(max_q_len), _stream()), "gla_scan_segments")
-        return
     _check(library().arle_gla_scan(_ptr(q), _ptr(k), _ptr(v), _dt(q), q.stride(0), _ptr(alpha), _ptr(bonus), _ptr(state),
                                    state.stride(0), _ptr(q_indptr), _ptr(state_slots), _ptr(out), R, heads, dim, vdim, float(q_scale), int(max_q_len), _stream()),
            "gla_scan")
-
-
-def gla_scan_scratch(q, k, alpha, rows: int, heads: int, dim: int, vdim: int, max_q_len: int) -> int:
-    """How many float32 numbers of scratch let ``gla_scan`` (without a bonus) cut the step's long rows into segments that run side by side; 0:
-    it runs row by row (short rows, other types and sizes, arrays off their boundaries)."""
-    if (_KERNEL_SET != "fast" or not q.is_cuda or q.dtype != torch.bfloat16 or q.stride(0) % 4 or q.data_ptr() % 8 or k.data_ptr() % 8
-            or alpha.data_ptr() % 16 or heads > 65535):
-        return 0
-    return int(library().arle_gla_segments_scratch(q.shape[0], int(rows), int(heads), int(dim), int(vdim), int(max_q_len)))
 
 
 def gla_out(o, gate, weight, eps: float, scale: float, out, heads: int, vdim: int, gate_act: str = "silu") -> None:

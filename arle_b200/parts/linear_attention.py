@@ -95,9 +95,7 @@ class GatedLinearAttention(Mixer):
     def scratch_elements_per_token(self):
         s = self.spec
         # the packed projection and the gated output in the activation type; alpha and o in float32 (two elements each)
-        # ; of long prompts the decayed queries, and a memory for every 128 tokens
-        segments = 2 * s.num_heads * (s.key_dim + -(-(s.value_dim + 1) * s.key_dim // 128))
-        return self.rows + s.num_heads * s.value_dim + 2 * s.num_heads * (s.key_dim + s.value_dim) + s.hidden_size + segments
+        return self.rows + s.num_heads * s.value_dim + 2 * s.num_heads * (s.key_dim + s.value_dim) + s.hidden_size
 
     # ------------------------------------------------------------------ state
     def state_need(self):
@@ -127,10 +125,8 @@ class GatedLinearAttention(Mixer):
         alpha = ctx.ws.get("gla_alpha", (T, H * dk), torch.float32)
         ops.gla_decay(proj[:, at["low"]: at["low"] + s.decay_rank], self.w_decay, self.decay_bias, s.tau, alpha)
         o = ctx.ws.get("gla_o", (T, H * dv), torch.float32)
-        q, k, v = (proj[:, at[n]: at[n] + H * d] for n, d in (("q", dk), ("k", dk), ("v", dv)))
-        n = ops.gla_scan_scratch(q, k, alpha, ctx.state_slots.numel(), H, dk, dv, ctx.max_q_len)
-        segments = dict(scratch=ctx.ws.get("gla_segments", (n,), torch.float32)) if n else {}
-        ops.gla_scan(q, k, v, alpha, state, ctx.q_indptr, ctx.state_slots, o, H, dk, dv, self.q_scale, ctx.max_q_len, **segments)
+        ops.gla_scan(proj[:, at["q"]: at["q"] + H * dk], proj[:, at["k"]: at["k"] + H * dk], proj[:, at["v"]: at["v"] + H * dv],
+                     alpha, state, ctx.q_indptr, ctx.state_slots, o, H, dk, dv, self.q_scale, ctx.max_q_len)
         ops.gla_out(o, proj[:, at["gate"]: at["gate"] + H * dv], self.norm, s.norm_eps, scale, into, H, dv)
 
     def forward(self, x, ctx, cache, state, sink=None):
