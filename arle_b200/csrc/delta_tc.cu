@@ -28,6 +28,11 @@
 #include "mma_utils.cuh"
 using namespace arle;
 
+ARLE_API int arle_delta_scan(const void* q, const void* k, const void* v, int dtype, int q_stride, int k_stride, int v_stride, const float* beta,
+                             const float* decay, float* state, long slot_stride, const int* q_indptr, const int* state_slots, float* out,
+                             int num_tokens, int R, int H, int kq_heads, int dim, int vdim, float q_scale, float unit_eps, int longest,
+                             cudaStream_t s);
+
 namespace {
 
 constexpr int kC = 64, kDim = 128, kQP = kDim + 8;
@@ -601,25 +606,26 @@ int most_chunks(int num_tokens, int R, int longest) {      // of rows of more th
 
 }  // namespace
 
-// How many float32 numbers of scratch arle_delta_tc wants.
-ARLE_API long arle_delta_tc_scratch(int num_tokens, int R, int H, int longest) {
-  return (long)most_chunks(num_tokens, R, longest) * H * (long)kChunkWords;
-}
-
-// Rows of more than `longest` tokens (the others are left alone).  q, k bfloat16 [T, kq_heads*128], v bfloat16 [T, H*vdim] (row strides multiples
+// Rows of more than `longest` tokens; the others, where there may be any (`short_rows`), go to arle_delta_scan.  q, k bfloat16 [T, kq_heads*128], v bfloat16 [T, H*vdim] (row strides multiples
 // of 8, 16-byte aligned), beta, decay float32 [T, H]; state: float32, a slot every slot_stride numbers, [H][vdim][128] at its start; out float32
-// [T, H, vdim], 8-byte aligned; vdim a multiple of 8; scratch: arle_delta_tc_scratch numbers, 16-byte aligned.
+// [T, H, vdim], 8-byte aligned; vdim a multiple of 8; scratch: 7,936 float32 numbers for each head and chunk, 16-byte aligned, for as many chunks
+// as such rows can have (num_tokens / 64 + min(R, num_tokens / (longest + 1)), whole numbers).
 ARLE_API int arle_delta_tc(const void* q, const void* k, const void* v, int q_stride, int k_stride, int v_stride, const float* beta,
                            const float* decay, float* state, long slot_stride, const int* q_indptr, const int* state_slots, float* out,
                            float* scratch, int num_tokens, int R, int H, int kq_heads, int vdim, float q_scale, float unit_eps, int longest,
-                           cudaStream_t s) {
+                           int short_rows, cudaStream_t s) {
   if (R <= 0 || num_tokens <= 0) return 0;
   if (H <= 0 || kq_heads <= 0 || H % kq_heads || vdim <= 0 || longest < 0 || !scratch) return ARLE_E_BADARG;
   if (vdim % 8 || q_stride % 8 || k_stride % 8 || v_stride % 8 || H > 65535 || R > 65535 ||
       (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)scratch) & 15) || ((uintptr_t)out & 7))
     return ARLE_E_UNSUPPORTED;
   const int slots = most_chunks(num_tokens, R, longest);
-  if (slots == 0) return 0;
+  if (slots == 0) short_rows = 1;
+  if (short_rows) {
+    const int e = arle_delta_scan(q, k, v, 1, q_stride, k_stride, v_stride, beta, decay, state, slot_stride, q_indptr, state_slots, out, num_tokens, R, H,
+                                  kq_heads, kDim, vdim, q_scale, unit_eps, longest, s);
+    if (e || slots == 0) return e;
+  }
   uint32_t* chunks = reinterpret_cast<uint32_t*>(scratch);
   static SharedLimit limit;
   const cudaError_t raised = limit.raise((const void*)delta_chunks_kernel, sizeof(ChunkSmem));

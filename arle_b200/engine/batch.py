@@ -31,14 +31,18 @@ class Workspace:
     def __init__(self, device):
         self.device = torch.device(device)
         self._bufs: Dict[Tuple[str, torch.dtype], torch.Tensor] = {}
+        self._views: Dict[Tuple[str, torch.dtype], Tuple[Tuple[int, ...], torch.Tensor]] = {}     # the shape asked for last, and its view
         self.frozen = False
         self.generation = 0            # counts (re)allocations: addresses handed out earlier may be stale after one
 
     def get(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+        key = (name, dtype)
+        last = self._views.get(key)
+        if last is not None and last[0] == shape:
+            return last[1]
         n = 1
         for s in shape:
             n *= int(s)
-        key = (name, dtype)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < n:
             if self.frozen:
@@ -46,15 +50,20 @@ class Workspace:
             buf = torch.empty(max(n, 1), dtype=dtype, device=self.device)
             self._bufs[key] = buf
             self.generation += 1
-        return buf[:n].view(shape)
+        view = buf[:n].view(shape)
+        self._views[key] = (tuple(shape), view)
+        return view
 
     def get_zeroed(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         """Like ``get``, but the buffer is zero when it is first handed out (and after it
         had to grow).  For flags and counters that kernels leave at zero."""
+        key = (name, dtype)
+        last = self._views.get(key)
+        if last is not None and last[0] == shape:
+            return last[1]
         n = 1
         for s in shape:
             n *= int(s)
-        key = (name, dtype)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < n:
             if self.frozen:
@@ -62,7 +71,9 @@ class Workspace:
             buf = torch.zeros(max(n, 1), dtype=dtype, device=self.device)
             self._bufs[key] = buf
             self.generation += 1
-        return buf[:n].view(shape)
+        view = buf[:n].view(shape)
+        self._views[key] = (tuple(shape), view)
+        return view
 
     def nbytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._bufs.values())

@@ -38,8 +38,6 @@ def add_launches(n: int) -> None:
 
 
 _P, _I, _F = c_void_p, c_int, c_float
-_SIZES = {"arle_delta_tc_scratch": 4}               # how much scratch an entry wants: whole numbers in, a size out
-
 _SIGNATURES = {
     "arle_embedding": [_P, _P, _I, _P, _I, _I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _P],
     "arle_rmsnorm": [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _F, _P, _P],
@@ -68,7 +66,7 @@ _SIGNATURES = {
     "arle_rglru_scan": [_P, _P, _P, _I, _I, _P, _P, _P, _P, _F, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "arle_delta_gates": [_P, _I, _P, _P, _P, _P, _I, _I, _P],
     "arle_delta_scan": [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _I, _P],
-    "arle_delta_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _P],
+    "arle_delta_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _I, _P],
     "arle_clamped_glu": [_P, _P, _I, _I, _I, _I, _F, _F, _P],
     "arle_paged_attention_decode": [_P, _I, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P],
     "arle_paged_attention_decode_stream": [_P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I,
@@ -139,10 +137,6 @@ def library() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.argtypes = args
             fn.restype = c_int
-        for name, n in _SIZES.items():
-            fn = getattr(lib, name)
-            fn.argtypes = [_I] * n
-            fn.restype = ctypes.c_long
         _LIB = lib
     return _LIB
 
@@ -2037,8 +2031,8 @@ def delta_gates(pre, a_log, dt_bias, beta, decay) -> None:
 
 def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: int, kq_heads: int, dim: int, vdim: int,
                q_scale: float, unit_eps: float, max_q_len: int = 0, scratch=None) -> None:
-    """``scratch`` (float32, ``delta_scan_scratch`` numbers, or None): the rows of 80 tokens and more run in chunks on the tensor cores.
-    The gated delta rule over the tokens of every row of the step, from and into state[state_slots[r]]: with q and k brought
+    """``scratch`` (float32, ``delta_scan_scratch`` numbers, or None; see ``delta_scan_takes_chunks``): the rows of 80 tokens and more run in
+    chunks on the tensor cores.  The gated delta rule over the tokens of every row of the step, from and into state[state_slots[r]]: with q and k brought
     to unit length per head (x / sqrt(sum x^2 + unit_eps); q also times q_scale), S <- decay_t S; u = beta_t (v_t - S^T k_t);
     S <- S + k_t u^T; o_t = S^T q_t.  q, k [T, kq_heads*dim] (head h reads head h // (heads / kq_heads)), v [T, heads*vdim], in
     the activation type (views of wider rows are fine); beta, decay float32 [T, heads]; state float32 [slots, n] whose first
@@ -2058,20 +2052,18 @@ def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: i
     _i32(q_indptr, "q_indptr"), _i32(state_slots, "state_slots")
     if q_indptr.numel() != R + 1:
         raise KernelError("delta_scan: q_indptr must have one entry more than state_slots")
-    longest = 0
     if scratch is not None:
-        need = delta_scan_scratch(q, k, v, out, R, heads, dim, vdim, max_q_len)
-        if need == 0 or scratch.dtype != torch.float32 or not scratch.is_contiguous() or scratch.numel() < need or scratch.data_ptr() % 16:
-            raise KernelError("delta_scan: scratch is for steps that delta_scan_scratch has a size for, float32, contiguous, on 16 bytes")
-        longest = DELTA_SCAN_LONGEST
+        if (q.dtype != torch.bfloat16 or dim != 128 or scratch.dtype != torch.float32 or not scratch.is_contiguous()
+                or scratch.numel() < delta_scan_scratch(T, R, heads)):
+            raise KernelError("delta_scan: scratch is for bfloat16 heads of 128, contiguous float32 of delta_scan_scratch numbers")
+        short = T - (R - 1) * max_q_len <= DELTA_SCAN_LONGEST    # else the shortest row is a long one too
         _check(library().arle_delta_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(beta), _ptr(decay), _ptr(state),
                                        state.stride(0), _ptr(q_indptr), _ptr(state_slots), _ptr(out), _ptr(scratch), T, R, heads, kq_heads,
-                                       vdim, float(q_scale), float(unit_eps), longest, _stream()), "delta_tc")
-        if T - (R - 1) * max_q_len > longest:                    # the shortest row is a long one too
-            return
+                                       vdim, float(q_scale), float(unit_eps), DELTA_SCAN_LONGEST, int(short), _stream()), "delta_tc")
+        return
     _check(library().arle_delta_scan(_ptr(q), _ptr(k), _ptr(v), _dt(q), q.stride(0), k.stride(0), v.stride(0), _ptr(beta), _ptr(decay),
                                      _ptr(state), state.stride(0), _ptr(q_indptr), _ptr(state_slots), _ptr(out), T, R, heads, kq_heads,
-                                     dim, vdim, float(q_scale), float(unit_eps), longest, _stream()), "delta_scan")
+                                     dim, vdim, float(q_scale), float(unit_eps), 0, _stream()), "delta_scan")
 
 
 # Rows of the delta rule up to this length are scanned, also where longer rows run in chunks: a row's own length decides.  One row, 8 heads of 128:
@@ -2079,13 +2071,15 @@ def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: i
 DELTA_SCAN_LONGEST = 79
 
 
-def delta_scan_scratch(q, k, v, out, rows: int, heads: int, dim: int, vdim: int, max_q_len: int) -> int:
-    """How many float32 numbers of scratch let ``delta_scan`` run the step's rows of 80 tokens and more in chunks on the tensor cores; 0: all
-    rows are scanned (short rows, other types and sizes, arrays off their boundaries)."""
-    if (_KERNEL_SET != "fast" or not q.is_cuda or q.dtype != torch.bfloat16 or dim != 128 or vdim % 8 or max_q_len <= DELTA_SCAN_LONGEST
-            or heads > 65535 or rows > 65535 or any(t.stride(0) % 8 or t.data_ptr() % 16 for t in (q, k, v)) or out.data_ptr() % 8):
-        return 0
-    return int(library().arle_delta_tc_scratch(v.shape[0], int(rows), int(heads), DELTA_SCAN_LONGEST))
+def delta_scan_takes_chunks(q, vdim: int, dim: int, max_q_len: int) -> bool:
+    """Whether ``delta_scan`` takes ``scratch`` for such a step (q, k and v on 16-byte boundaries, as rows of one buffer of the activation type
+    are): some row of 80 tokens and more, bfloat16 heads of 128, the fast kernel set."""
+    return max_q_len > DELTA_SCAN_LONGEST and dim == 128 and vdim % 8 == 0 and q.dtype == torch.bfloat16 and _KERNEL_SET == "fast" and q.is_cuda
+
+
+def delta_scan_scratch(tokens: int, rows: int, heads: int) -> int:
+    """How many float32 numbers of scratch the chunks of a step's long rows want: 7,936 for each chunk of 64 tokens and head."""
+    return (tokens // 64 + min(rows, tokens // (DELTA_SCAN_LONGEST + 1))) * heads * 7936
 
 
 def gate_mul(x, gate, out) -> None:

@@ -23,8 +23,8 @@ def _inputs(lens, H, kq, vdim):
 def _run(q, k, v, beta, decay, state, lens, H, kq, vdim, chunks=True, slots=None):
     at = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0).to(torch.int32)
     out = torch.full((q.shape[0] + 1, H, vdim), 7.0, device=DEV)
-    state, n = state.clone(), ops.delta_scan_scratch(q, k, v, out, len(lens), H, DIM, vdim, max(lens))
-    assert n > 0
+    state, n = state.clone(), ops.delta_scan_scratch(q.shape[0], len(lens), H)
+    assert n > 0 and ops.delta_scan_takes_chunks(q, vdim, DIM, max(lens))
     scratch = torch.full((n + 4,), float("nan"), device=DEV)
     slots = torch.tensor(slots or list(range(len(lens))), dtype=torch.int32, device=DEV)
     ops.delta_scan(q, k, v, beta, decay, state, at, slots, out[:-1], H, kq, DIM, vdim, DIM ** -0.5, 1e-6,
