@@ -24,7 +24,7 @@
 // What bounds it: the chain of chunks of a block (some 9 us each: the tensor cores' legacy path, a third of the time, then the matrix
 // loads and the barriers between the phases), with one block an SM.  A scheduler has two warps; one takes an early tile of rows and the other a
 // late one, which sees more keys.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 284 us (306 with two early or two late ones, the
-// scan 1,162), 8 heads of 256 x 513 324 us before (1,740 to 1,937 as the scan's mean of both).
+// scan 1,162), 8 heads of 256 x 513 305 us (326; 1,740 to 1,937 as the scan's mean of both).
 #include "common.cuh"
 #include "mma_utils.cuh"
 using namespace arle;

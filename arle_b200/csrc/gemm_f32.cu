@@ -9,16 +9,18 @@
 // kernel set runs it for every projection, so that a bfloat16 discrepancy can be put
 // down to the fast kernels or to the arithmetic.
 //
-// float32 A runs on one of three kernels, all with that order of sums, so all with the same bits:
+// float32 A runs on one of four kernels, all with that order of sums, so all with the same bits:
 //  * gemm_f32_rows (up to 16 rows): a thread per column of C, W staged by cp.async.  Bound by W's bytes for one row, by the loads from
 //    shared memory for more.
-//  * gemm_f32_tiles: tiles of 64 x 128 to 32 x 32, 8 x 4 or 4 x 4 sums a thread, the next 16 numbers of k on their way while the present
+//  * gemm_f32_stages: tiles of 32 x 32 and 64 x 64, stages of 32 numbers of k as they lie in memory on their way by cp.async, three ahead.  For
+//    the products of short prompts, whose few tiles an SM are bound by how long memory takes to answer (gemm_f32_tiles asks one stage ahead).
+//  * gemm_f32_tiles: tiles of 64 x 128, 8 x 4 sums a thread, the next 16 numbers of k on their way while the present
 //    ones are multiplied; two neighbouring sums are one packed instruction (fma.rn.f32x2: each half the same rounded fused product).
-//    Bound by the loads from shared memory and, since no sum may be split along k, by how few tiles there are: the launcher takes the
-//    tile that leaves the busiest SM the least.
+//    Bound by instructions, half of FFMA's rate.  No sum may be split along k, so the launcher takes the tile that leaves the busiest SM the least.
 //  * gemm_f32 (rows that are not on 16-byte boundaries, and bfloat16 A): the general one, tiles of 64 x 64.
-// Measured, the general kernel and these (us): 301 rows, 4,096 x 1,024 168 and 98, 1,024 x 2,048 150 and 89, 6,144 x 1,024 222 and 117,
-// 1,024 x 3,072 224 and 130; 1,024 rows of 24,576 x 4,096 8,726 and 4,420 (47 TFLOP/s); one row, 151,936 x 1,024 880 and 58 (5.3 TB/s),
+// Measured, the general kernel, gemm_f32_tiles at its best tile of 64 x 128 to 32 x 32, and these (us, W bfloat16): 301 rows, 4,096 x 1,024 168, 97
+// and 86; 1,024 x 2,048 150, 88 and 62; 6,144 x 1,024 222, 117 and 117; 1,024 x 3,072 224, 130 and 90; 40 rows, 1,024 x 2,048 72 and 31; 120
+// rows, 6,144 x 1,024 68 and 60; 1,024 rows of 24,576 x 4,096 8,726 and 4,420 (47 TFLOP/s); one row, 151,936 x 1,024 880 and 58 (5.3 TB/s),
 // 4,096 x 1,024 76 and 12; 8 rows 883 and 117.
 #include "common.cuh"
 #include "mma_utils.cuh"
@@ -188,6 +190,104 @@ __global__ void __launch_bounds__((BM_ / TM) * (BN_ / TN)) gemm_f32_tiles_kernel
   }
 }
 
+// TM, TN: rows and columns of C a thread holds, BM / TM and BN / TN apart (neighbouring threads' rows of a stage are 16 bytes more than whole
+// rounds of the banks apart).  A stage is 32 numbers of k of the tile's rows of A and W as they lie in memory, brought by cp.async three stages
+// ahead: a thread reads four (A) or sixteen bytes of (W) numbers of k at once and runs through them in order.
+constexpr int kTileK = 32, kTileStages = 4;
+template <typename TW, int BM_, int BN_>
+struct TileSmem {
+  static constexpr int AP = kTileK + 4, WP = kTileK + 16 / (int)sizeof(TW);      // numbers from row to row
+  static constexpr size_t A = (size_t)BM_ * AP * sizeof(float), W = (size_t)BN_ * WP * sizeof(TW), BYTES = kTileStages * (A + W);
+};
+// Number kk (0 .. 3) of k of a column from sixteen bytes of them.
+__device__ __forceinline__ float nth(const uint4& v, int kk, float) { return __uint_as_float(kk == 0 ? v.x : kk == 1 ? v.y : kk == 2 ? v.z : v.w); }
+__device__ __forceinline__ float nth(const uint4& v, int kk, __nv_bfloat16) {
+  const uint32_t u = kk < 2 ? v.x : kk < 4 ? v.y : kk < 6 ? v.z : v.w;
+  return __uint_as_float(kk & 1 ? u & 0xffff0000u : u << 16);
+}
+
+template <typename TW, int BM_, int BN_, int TM, int TN>
+__global__ void __launch_bounds__((BM_ / TM) * (BN_ / TN)) gemm_f32_stages_kernel(const float* __restrict__ A, const TW* __restrict__ W,
+                                                                                 float* __restrict__ C, int M, int N, int K, int lda,
+                                                                                 int ldw, int ldc) {
+  pdl_launch_dependents();
+  pdl_wait();
+  typedef TileSmem<TW, BM_, BN_> L;
+  constexpr int THREADS = (BM_ / TM) * (BN_ / TN), TX = BN_ / TN, TY = BM_ / TM;
+  constexpr int PER = 16 / sizeof(TW), AC = kTileK / 4, WC = kTileK / PER;       // numbers of W in 16 bytes; pieces of a row
+  static_assert(BM_ * AC % THREADS == 0 && BN_ * WC % THREADS == 0, "staging");
+  extern __shared__ __align__(16) unsigned char tile_sm[];
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  const int m0 = blockIdx.y * BM_, n0 = blockIdx.x * BN_;
+  const int nk = (K + kTileK - 1) / kTileK;
+  auto load = [&](int kt) {
+    float* as = reinterpret_cast<float*>(tile_sm + (kt % kTileStages) * (L::A + L::W));
+    TW* ws = reinterpret_cast<TW*>(reinterpret_cast<unsigned char*>(as) + L::A);
+    const int k0 = kt * kTileK;
+#pragma unroll
+    for (int i = 0; i < BM_ * AC / THREADS; ++i) {
+      const int idx = tid + i * THREADS, r = idx / AC, k = idx % AC * 4;
+      const bool ok = m0 + r < M && k0 + k < K;
+      cp_async16(smem_u32(as + r * L::AP + k), ok ? A + (size_t)(m0 + r) * lda + k0 + k : A, ok ? 16 : 0);
+    }
+#pragma unroll
+    for (int i = 0; i < BN_ * WC / THREADS; ++i) {
+      const int idx = tid + i * THREADS, r = idx / WC, k = idx % WC * PER;
+      const bool ok = n0 + r < N && k0 + k < K;
+      cp_async16(smem_u32(ws + r * L::WP + k), ok ? W + (size_t)(n0 + r) * ldw + k0 + k : W, ok ? 16 : 0);
+    }
+  };
+  float acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+#pragma unroll
+  for (int kt = 0; kt < kTileStages - 1; ++kt) {
+    if (kt < nk) load(kt);
+    cp_commit();
+  }
+  for (int kt = 0; kt < nk; ++kt) {
+    cp_wait<kTileStages - 2>();
+    __syncthreads();                                         // the stage is here, and the one that is loaded next was used up
+    if (kt + kTileStages - 1 < nk) load(kt + kTileStages - 1);
+    cp_commit();
+    const float* as = reinterpret_cast<const float*>(tile_sm + (kt % kTileStages) * (L::A + L::W)) + ty * L::AP;
+    const TW* ws = reinterpret_cast<const TW*>(tile_sm + (kt % kTileStages) * (L::A + L::W) + L::A) + tx * L::WP;
+#pragma unroll
+    for (int k0 = 0; k0 < kTileK; k0 += PER) {
+      uint4 w[TN];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const uint4*>(ws + j * TX * L::WP + k0);
+#pragma unroll
+      for (int k4 = 0; k4 < PER; k4 += 4) {
+        float a[TM][4];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) load_vec<float, 4>(as + i * TY * L::AP + k0 + k4, a[i]);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) {
+            const float wj = nth(w[j], k4 + kk, TW());
+#pragma unroll
+            for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i][kk], wj, acc[i][j]);
+          }
+      }
+    }
+  }
+  cp_wait<0>();
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int gm = m0 + ty + i * TY;
+    if (gm >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int gn = n0 + tx + j * TX;
+      if (gn < N) C[(size_t)gm * ldc + gn] = acc[i][j];
+    }
+  }
+}
+
 // Up to 16 rows of A: a thread holds one column of C for all rows.  A block stages 128 rows of W, 64 numbers of k at a time, three
 // stages; a staged row is 16 bytes longer than its numbers, so that eight lanes' 16-byte reads fall on different banks.
 constexpr int kRowsN = 128, kRowsK = 64, kRowsStages = 3;
@@ -274,6 +374,19 @@ static int launch_tiles(const float* A, const TW* W, float* C, int M, int N, int
   return launch_status();
 }
 
+template <typename TW, int BM_, int BN_, int TM, int TN>
+static int launch_stages(const float* A, const TW* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+  dim3 grid((N + BN_ - 1) / BN_, (M + BM_ - 1) / BM_);
+  if (grid.y > 65535) return ARLE_E_UNSUPPORTED;
+  constexpr size_t smem = TileSmem<TW, BM_, BN_>::BYTES;
+  static SharedLimit limit;
+  auto kernel = gemm_f32_stages_kernel<TW, BM_, BN_, TM, TN>;
+  const cudaError_t raised = limit.raise((const void*)kernel, smem);
+  if (raised != cudaSuccess) return (int)raised;
+  launch_kernel(kernel, grid, dim3((BM_ / TM) * (BN_ / TN)), smem, s, 1, A, W, C, M, N, K, lda, ldw, ldc);
+  return launch_status();
+}
+
 template <typename TW>
 static int launch_f32(const float* A, const void* Wv, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
   const TW* W = (const TW*)Wv;
@@ -287,19 +400,16 @@ static int launch_f32(const float* A, const void* Wv, float* C, int M, int N, in
     return launch_rows<TW, 16>(A, W, C, M, N, K, lda, ldw, ldc, s);
   }
   // Microseconds per 1,024 of k: what a tile takes by itself on an SM, and what it adds to an SM that is full of them; in between the
-  // cube root of the sum of cubes is within a tenth of what was measured at 1,024 to 24,576 columns and 12 to 1,024 rows.
+  // cube root of the sum of cubes is within a tenth of what was measured at 1,024 to 6,144 columns and 40 to 1,024 rows.
   auto cost = [&](int bm, int bn, float alone, float added) {
     const float b = (float)(((long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn) + 147) / 148) * added;
     return alone * alone * alone + b * b * b;
   };
   const bool low = M <= 65535 * 32;                        // a grid has room for the rows in tiles of 32
-  const float c0 = cost(64, 128, 70.f, 53.f), c1 = cost(64, 64, 60.f, 29.f), c2 = low ? cost(32, 64, 39.4f, 20.2f) : INFINITY,
-              c3 = low ? cost(32, 32, 37.4f, 11.f) : INFINITY;
-  const float best = fminf(fminf(c0, c1), fminf(c2, c3));
-  if (best == c0) return launch_tiles<TW, 64, 128, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
-  if (best == c1) return launch_tiles<TW, 64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
-  if (best == c2) return launch_tiles<TW, 32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
-  return launch_tiles<TW, 32, 32, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  const float c0 = cost(64, 128, 70.f, 53.f), c1 = cost(64, 64, 36.f, 30.f), c2 = low ? cost(32, 32, 15.6f, 9.2f) : INFINITY;
+  if (c2 <= fminf(c0, c1)) return launch_stages<TW, 32, 32, 4, 2>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  if (c1 <= c0) return launch_stages<TW, 64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  return launch_tiles<TW, 64, 128, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
 }
 
 ARLE_API int arle_gemm_f32(const float* A, const void* W, int w_dtype, float* C, int M, int N, int K, int lda,
