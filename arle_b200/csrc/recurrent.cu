@@ -544,10 +544,12 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const T* __
   }
 }
 
-// The same with the part's numbers kept in registers between the sum and the result, eight an access: parts of up to ITS x 2,048 numbers.
-// Bound by memory: 2,048 rows of 8,192 46 us (168 MB: 3.7 TB/s); read twice number by number it was 110 us.
-template <typename T, int ITS>
-__global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* __restrict__ y, const T* __restrict__ x, int x_stride,
+// The same with the part's numbers kept in registers between the sum and the result, eight an access: parts of up to ITS x THREADS x 8 numbers.
+// Bound by instructions (exponentials and divisions, one after the other) and memory.  2,048 rows of 8,192, 168 MB: 35 us with 512 threads a row
+// and three rows an SM (256 threads, which hold twice the numbers: 44; 1,024 37; four rows spill, 35; read twice number by number 110), 64 rows
+// 6.5 (8.5); of 4,096 16.7 with 256 threads, 18.7 with 512.
+template <typename T, int ITS, int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS) gated_group_norm_vec_kernel(const float* __restrict__ y, const T* __restrict__ x, int x_stride,
                                                                    const float* __restrict__ skip, int vdim, const T* __restrict__ z, int z_stride,
                                                                    const float* __restrict__ weight, float eps, T* __restrict__ out,
                                                                    int out_stride, int inner, int width) {
@@ -559,7 +561,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
   float ss = 0.f;
 #pragma unroll
   for (int it = 0; it < ITS; ++it) {
-    const int i = (it * 256 + threadIdx.x) * 8, c = c0 + i;
+    const int i = (it * THREADS + threadIdx.x) * 8, c = c0 + i;
 #pragma unroll
     for (int g = 0; g < 8; ++g) val[it][g] = 0.f;
     if (i >= width) continue;
@@ -582,7 +584,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
   const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)width + eps);
 #pragma unroll
   for (int it = 0; it < ITS; ++it) {
-    const int i = (it * 256 + threadIdx.x) * 8, c = c0 + i;
+    const int i = (it * THREADS + threadIdx.x) * 8, c = c0 + i;
     if (i >= width) continue;
     float wv[8];
     load_vec<float, 4>(weight + c, reinterpret_cast<float(&)[4]>(wv[0]));
@@ -603,9 +605,9 @@ ARLE_API int arle_gated_group_norm(const float* y, const void* x, int dtype, int
   if (dtype == 1 && width >= 1024 && width <= 8192 && width % 8 == 0 && vdim % 8 == 0 && z_stride % 8 == 0 && out_stride % 8 == 0 &&
       (!skip || x_stride % 8 == 0) &&
       (((uintptr_t)y | (uintptr_t)z | (uintptr_t)out | (uintptr_t)weight | (skip ? (uintptr_t)x : 0)) & 15) == 0) {
-    auto kernel = width <= 2048 ? gated_group_norm_vec_kernel<__nv_bfloat16, 1>
-                  : width <= 4096 ? gated_group_norm_vec_kernel<__nv_bfloat16, 2> : gated_group_norm_vec_kernel<__nv_bfloat16, 4>;
-    launch_kernel(kernel, dim3(num_tokens, parts), dim3(256), 0, s, 1, y, (const __nv_bfloat16*)x, x_stride, skip, vdim, (const __nv_bfloat16*)z,
+    auto kernel = width <= 2048 ? gated_group_norm_vec_kernel<__nv_bfloat16, 1, 256, 1>
+                  : width <= 4096 ? gated_group_norm_vec_kernel<__nv_bfloat16, 2, 256, 1> : gated_group_norm_vec_kernel<__nv_bfloat16, 2, 512, 3>;
+    launch_kernel(kernel, dim3(num_tokens, parts), dim3(width <= 4096 ? 256 : 512), 0, s, 1, y, (const __nv_bfloat16*)x, x_stride, skip, vdim, (const __nv_bfloat16*)z,
                   z_stride, weight, eps, (__nv_bfloat16*)out, out_stride, inner, width);
     return launch_status();
   }
