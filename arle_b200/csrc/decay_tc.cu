@@ -26,64 +26,12 @@
 // late one, which sees more keys.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 284 us (306 with two early or two late ones, the
 // scan 1,162), 8 heads of 256 x 513 305 us (326; 1,740 to 1,937 as the scan's mean of both).
 #include "common.cuh"
-#include "mma_utils.cuh"
+#include "chunk_parts.cuh"
 using namespace arle;
 
 namespace {
 
-constexpr int kC = 64, kThreads = 256;
-
-// x = hi + mid + lo to 24 bits; an infinity stays one (hi alone).
-__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-  float rx = x - __low2float(h), ry = y - __high2float(h);
-  rx = fabsf(rx) <= fabsf(x) ? rx : 0.f;
-  ry = fabsf(ry) <= fabsf(y) ? ry : 0.f;
-  const __nv_bfloat162 m = __floats2bfloat162_rn(rx, ry);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(rx - __low2float(m), ry - __high2float(m));
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  mid = *reinterpret_cast<const uint32_t*>(&m);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-
-// acc += a . b with the sum of the sixteen products rounded once on its own: the tensor core cuts off what an accumulator cannot hold, and
-// over a chain of products that is a few times the error of a float32 sum.
-__device__ __forceinline__ void mma_add(float (&acc)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  float t[4] = {0.f, 0.f, 0.f, 0.f};
-  mma_bf16(t, a, b0, b1);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) acc[i] += t[i];
-}
-
-// What the products of a tile of 16 weights (in three parts, as the tensor cores take them) with its values come to, row i of the tile
-// with the values up to i alone.  v: the tile's first value in this lane's first column of o0; o1's columns are eight further on.
-template <int VP>
-__device__ __forceinline__ void add_seen(const uint32_t (&pa)[3][4], const __nv_bfloat16* v, int lane, float (&o0)[4], float (&o1)[4]) {
-  const int row = lane >> 2;
-#pragma unroll
-  for (int reg = 0; reg < 4; ++reg) {                      // rows 0 .. 7 and 8 .. 15 of the weights in turn, keys 8 (reg / 2) ..
-    float w[2] = {0.f, 0.f};
-#pragma unroll
-    for (int i = 2; i >= 0; --i) {
-      const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(&pa[i][reg]);
-      w[0] += __low2float(x), w[1] += __high2float(x);
-    }
-    const int half = reg & 1;
-#pragma unroll 1
-    for (int s = 0; s < 4; ++s)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const float wj = __shfl_sync(0xffffffffu, w[e], (lane & ~3) | s);
-        const int j = (reg >> 1) * 8 + 2 * s + e;
-        if (j > row + 8 * half) continue;
-        const __nv_bfloat16* x = v + j * VP;
-        o0[2 * half] = fmaf(wj, __bfloat162float(x[0]), o0[2 * half]);
-        o0[2 * half + 1] = fmaf(wj, __bfloat162float(x[1]), o0[2 * half + 1]);
-        o1[2 * half] = fmaf(wj, __bfloat162float(x[8]), o1[2 * half]);
-        o1[2 * half + 1] = fmaf(wj, __bfloat162float(x[9]), o1[2 * half + 1]);
-      }
-  }
-}
+constexpr int kThreads = 256;
 
 template <int DIM, int VT>
 struct Layout {

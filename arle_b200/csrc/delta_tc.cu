@@ -25,7 +25,7 @@
 // cores' legacy path about half of the time); delta_chunks takes some 20 us of a step of 2,000 tokens.  Rows of 819, 701 and 479 tokens, 32 heads
 // of 128 x 128: 219 us (the scan 530); one row of 2,048 218 (651), with 8 heads 138 (515); 300 tokens, 8 heads 37 (81).
 #include "common.cuh"
-#include "mma_utils.cuh"
+#include "chunk_parts.cuh"
 using namespace arle;
 
 ARLE_API int arle_delta_scan(const void* q, const void* k, const void* v, int dtype, int q_stride, int k_stride, int v_stride, const float* beta,
@@ -35,67 +35,10 @@ ARLE_API int arle_delta_scan(const void* q, const void* k, const void* v, int dt
 
 namespace {
 
-constexpr int kC = 64, kDim = 128, kQP = kDim + 8;
-constexpr int kTileWords = 3 * 32 * 4;                     // a tile of 16 x 16 in three parts, as the tensor cores take it: [part][lane][4]
+constexpr int kDim = 128, kQP = kDim + 8;
 constexpr int kTiles = 10;                                 // tiles on and below the diagonal of a chunk
 constexpr int kScalars = 256;                              // a chunk's numbers: [64] D_i / |k_i|, [64] q_scale D_i / |q_i|, [64] D_nj / |k_j|, D_n
 constexpr size_t kChunkWords = 2 * kTiles * kTileWords + kScalars;   // of one head: T, P, numbers
-
-__device__ __forceinline__ int row_chunks(int n, int longest) { return n > longest ? (n + kC - 1) / kC : 0; }
-
-// The row and the chunk of a slot (a warp's lanes together); false: no such slot.
-__device__ __forceinline__ bool chunk_of(int slot, const int* q_indptr, int rows, int longest, int& row, int& chunk) {
-  const int lane = threadIdx.x & 31;
-  int before = 0;
-  for (int r0 = 0; r0 < rows; r0 += 32) {
-    const int mine = r0 + lane < rows ? row_chunks(q_indptr[r0 + lane + 1] - q_indptr[r0 + lane], longest) : 0;
-    int sum = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, sum, o);
-      if (lane >= o) sum += y;
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, slot < before + sum);
-    if (hit) {
-      const int src = __ffs(hit) - 1;
-      row = r0 + src;
-      chunk = slot - before - __shfl_sync(0xffffffffu, sum - mine, src);
-      return true;
-    }
-    before += __shfl_sync(0xffffffffu, sum, 31);
-  }
-  return false;
-}
-
-// x = hi + mid + lo to 24 bits; an infinity stays one (hi alone).
-__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-  float rx = x - __low2float(h), ry = y - __high2float(h);
-  rx = fabsf(rx) <= fabsf(x) ? rx : 0.f;
-  ry = fabsf(ry) <= fabsf(y) ? ry : 0.f;
-  const __nv_bfloat162 m = __floats2bfloat162_rn(rx, ry);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(rx - __low2float(m), ry - __high2float(m));
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  mid = *reinterpret_cast<const uint32_t*>(&m);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-
-// acc += a . b with the sum of the sixteen products rounded once on its own (decay_tc.cu says why).
-__device__ __forceinline__ void mma_add(float (&acc)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  float t[4] = {0.f, 0.f, 0.f, 0.f};
-  mma_bf16(t, a, b0, b1);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) acc[i] += t[i];
-}
-
-__device__ __forceinline__ void split_tile(const float (&w)[8], uint32_t* to, int lane) {
-  // w: (row g, columns 2t, 2t+1), (g+8, same), (g, 2t+8, 2t+9), (g+8, same)
-  uint32_t p[3][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) split3(w[2 * i], w[2 * i + 1], p[0][i], p[1][i], p[2][i]);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(to + (i * 32 + lane) * 4) = make_uint4(p[i][0], p[i][1], p[i][2], p[i][3]);
-}
 
 struct ChunkSmem {
   __nv_bfloat16 q[kC][kQP], k[kC][kQP];
