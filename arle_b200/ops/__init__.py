@@ -1516,9 +1516,25 @@ def decay_memories(q, k, v, a, b, state, batch, out, heads: int, kq_heads: int, 
         raise KernelError(f"decay_memories: state {tuple(state.shape)} must be float32 [slots, >= {heads * vcols * dim}]")
     if out.dtype != torch.float32 or tuple(out.shape) != (T, heads, vcols) or not out.is_contiguous():
         raise KernelError("decay_memories: out must be contiguous float32 [T, heads, vcols]")
+    n = decay_rows_chunks(batch, dim, ones_column)
+    if n:
+        scratch = batch.ws.get("decay_tiles", (n * heads * 4096,), torch.float32)
+        _check(library().arle_decay_rows_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(a), _ptr(b), _ptr(state),
+                                            state.stride(0), _ptr(batch.q_indptr), _ptr(batch.state_slots), _ptr(out), _ptr(scratch), n,
+                                            batch.num_rows, heads, kq_heads, vdim, float(q_scale), DECAY_TC_LONGEST, _stream()), "decay_rows_tc")
+        return
     _check(library().arle_decay_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(a), _ptr(b), _ptr(state), state.stride(0),
                                    _ptr(batch.q_indptr), _ptr(batch.state_slots), _ptr(out), batch.num_rows, heads, kq_heads, dim, vdim, vcols,
                                    float(q_scale), DECAY_TC_LONGEST, _stream()), "decay_tc")
+
+
+def decay_rows_chunks(batch, dim: int, ones_column: bool) -> int:
+    """The chunks of 64 tokens of a step's long rows, where ``decay_memories`` forms their scores side by side (4,096 float32 numbers of scratch a
+    chunk and head; 32 tokens a chunk at the least, which the mixers count); 0: one launch does it all.  The same bits either way."""
+    if dim != 128 or ones_column:
+        return 0
+    n = sum(-(-t // DECAY_CHUNK) for t in batch.q_lens if t > DECAY_TC_LONGEST)
+    return n if 32 * n <= batch.num_tokens else 0
 
 
 DECAY_CHUNK = 64                    # tokens of a chunk

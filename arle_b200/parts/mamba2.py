@@ -90,7 +90,9 @@ class Mamba2(Mixer):
         return sum(t.numel() * t.element_size() for t in (self.w_in, self.w_o))
 
     def scratch_elements_per_token(self):
-        return self.main_rows + self.channels + 3 * self.inner + 6 * self.spec.num_heads + self.spec.hidden_size
+        # with long prompts and 128 keys what a chunk's heads keep: 4,096 float32 numbers, 32 tokens a chunk at the least
+        chunks = 2 * 4096 // 32 * self.spec.num_heads if self.spec.state_dim == 128 else 0
+        return self.main_rows + self.channels + 3 * self.inner + 6 * self.spec.num_heads + self.spec.hidden_size + chunks
 
     def state_need(self):
         n = self.conv_offset + self.channels * (self.spec.conv_taps - 1)
