@@ -1530,8 +1530,9 @@ def decay_memories(q, k, v, a, b, state, batch, out, heads: int, kq_heads: int, 
 
 def decay_rows_chunks(batch, dim: int, ones_column: bool) -> int:
     """The chunks of 64 tokens of a step's long rows, where ``decay_memories`` forms their scores side by side (4,096 float32 numbers of scratch a
-    chunk and head; 32 tokens a chunk at the least, which the mixers count); 0: one launch does it all.  The same bits either way."""
-    if dim != 128 or ones_column:
+    chunk and head; 32 tokens a chunk at the least, which the mixers count); 0: one launch does it all.  The same bits either way, so the longest
+    row may decide: from three full chunks on the shorter chain gains more than the second launch costs."""
+    if dim != 128 or ones_column or batch.max_q_len < 3 * DECAY_CHUNK:
         return 0
     n = sum(-(-t // DECAY_CHUNK) for t in batch.q_lens if t > DECAY_TC_LONGEST)
     return n if 32 * n <= batch.num_tokens else 0
