@@ -1,0 +1,37 @@
+"""Memories with a scalar decay and 128 keys: the scores of all chunks formed side by side and the chain behind them give the bits of the one launch
+that does both, for rows around a chunk's end, short rows beside long ones, heads in fours and by themselves, columns that do not fill a block, one
+group of columns a block and four, decays of zero, and values that overflow."""
+import pytest
+import torch
+
+from arle_b200 import ops
+from test_decay_tc_gpu import DEV, _ctx
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,G,vdim", [(8, 2, 64), (3, 3, 40), (2, 1, 200), (80, 8, 64)])
+@pytest.mark.parametrize("lens", [[192], [257], [300, 1, 33, 128, 20]], ids=["192", "257", "300-1-33-128-20"])
+@pytest.mark.parametrize("kind", ["slow", "wild", "odd"])
+def test_the_bits_of_the_one_launch(monkeypatch, H, G, vdim, lens, kind):
+    g = torch.Generator(device=DEV).manual_seed(H + vdim + len(lens))
+    T, dim = sum(lens), 128
+    wide = torch.randn(T, 2 * G * dim + H * vdim + 8, generator=g, device=DEV).to(torch.bfloat16)
+    q, k, v = wide[:, : G * dim], wide[:, G * dim: 2 * G * dim], wide[:, 2 * G * dim: 2 * G * dim + H * vdim]
+    u, b = (torch.rand(T, H, generator=g, device=DEV) for _ in range(2))
+    a = 1.0 - 0.05 * u if kind == "slow" else torch.where(u < 0.1, torch.zeros_like(u), torch.where(u < 0.3, u * 1e-30, 1 - 1e-3 * u))
+    if kind == "odd":
+        v[T // 2, 1], v[T // 3, vdim // 2] = float("inf"), float("nan")
+    ctx, width = _ctx(lens, H * vdim * dim + 4), H * vdim * dim + 4
+    state0 = torch.randn(len(lens) + 1, width, generator=g, device=DEV)
+    assert ops.decay_rows_chunks(ctx, dim, False) > 0 and ops.decay_rows_chunks(ctx, dim, True) == 0
+    got = []
+    for split in (True, False):
+        if not split:
+            monkeypatch.setattr(ops, "decay_rows_chunks", lambda *_: 0)
+        state, out = state0.clone(), torch.full((T + 1, H, vdim), 7.0, device=DEV)
+        ops.decay_memories(q, k, v, a, b, state, ctx, out[:T], H, G, dim, vdim, False, 0.3)
+        got.append((out, state))
+    for x, y in zip(*got):
+        assert torch.equal(x.nan_to_num(5.0, 3e38, -3e38), y.nan_to_num(5.0, 3e38, -3e38)) and torch.equal(x.isnan(), y.isnan())
+    assert (got[0][0][T] == 7.0).all()
