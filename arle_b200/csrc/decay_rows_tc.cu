@@ -1,7 +1,8 @@
 // The recurrence of decay_tc.cu in two launches, for memories of 128 x vdim without a column of ones: what does not need the memory is formed for
 // all chunks and heads side by side (decay_tiles: the weighted scores D_ij b_j (q_i . k_j), cut into three bfloat16 numbers, and the chunk's
 // decays), and the chain of a row's chunks (decay_rows_tc) is left with S_0^T q, the weighted scores times v and the update.  Every sum has the
-// order it has there: the same bits, so that a step may take either.
+// order it has there: the same bits, so that a step may take either.  (Beside an infinity or a NaN in v, whose tile is added up value by value, the
+// columns of the same warp differ in the last bits: 16 here, up to 32 there.)
 //
 // decay_rows_tc: a block has a head and 16 G columns of v for a whole row, four warps 16 columns; the groups share the chunk's q and k and
 // nothing else.  A warp forms the rows of a tile of 16 tokens and holds 32 rows of S.  A chunk has one barrier for the block and one for the group.
