@@ -133,7 +133,7 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 
 // Bit 0: every kernel is launched with programmatic stream serialisation allowed; bit 1:
 // the weight-streaming products only (they fill their weight ring while the kernel before
-// them finishes).  Off by default.
+// them finishes).  Off by default.  (The small products of gemm_skinny.cu are always launched so.)
 inline int& pdl_enabled() {
   static int on = 0;
   return on;

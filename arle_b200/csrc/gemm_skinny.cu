@@ -32,6 +32,7 @@
 //  * "row scale": the product reads such a table, forms 1 / sqrt(sum r^2 / width + eps)
 //    per row of x, and multiplies its sums by it, which is the same as having normalised
 //    x before (the factor is one number per row, the product is linear in x).
+// Products of few elements do without the ring: direct_gemm_kernel, below.
 // Every wait on an mbarrier is bounded: after kSpinLimit polls the kernel raises
 // the error flag and carries on to its end instead of hanging.
 //
@@ -430,7 +431,12 @@ __global__ void __launch_bounds__(kThreads, 1) skinny_gemm_kernel(
 // has NR rows of W, its warps shares of K; a lane asks for 16 bytes of a row at a time, eight neighbouring elements of K, which are two of the
 // tensor cores' K steps in an order of their own (x is read in the same order, so the sums are the same products).  With 128 elements of K a
 // warp all of a block's loads are under way before the first is used; the warps' sums are added in warp order.  What bounds it: a launch, one
-// round trip to memory and the sums, some 3 us, and the bytes on top.  plan_direct has the figures.
+// round trip to memory and the sums, some 3 us, and the bytes on top.  So it is launched as soon as the kernel in front has started its last
+// block (programmatic launch), and its blocks, small enough to stand beside those of another such product, ask L2 for their first weights before they
+// wait for that kernel: a 0.6B layer's four products one behind the other 12.7 us in a graph (14.6 without the prefetch, 15.4 launched in stream order,
+// 20.8 on the ring); a decode step of 28 such layers 787 us (799 in stream order), of 8 layers behind 100 tokens 265 (285).  Weights are read
+// behind the wait alone, since a program may write them in the kernel in front (read ahead of it, into registers: 13.4).  plan_direct has the
+// figures by size, in stream order.
 __device__ __forceinline__ uint4 ld_weights(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -441,18 +447,34 @@ __device__ __forceinline__ uint4 ld_rows(const void* p) {
   asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
-template <int NR, int WARPS, typename OutT>
-__global__ void __launch_bounds__(WARPS * 32) direct_gemm_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ W,
-                                                                 int ldw, OutT* __restrict__ out, int ldo, int M, int N, int K, int gated,
-                                                                 Fusion fu) {
-  constexpr int U = 4, HALVES = NR / 8;                    // blocks of 32 elements of K under way; rows g and g + 8 of the tile
+template <int NR, int WARPS, int U, typename OutT>
+__global__ void __launch_bounds__(WARPS * 32, WARPS > 16 ? 1 : WARPS == 16 ? 2 : NR == 16 && U == 4 ? 3 : 4) direct_gemm_kernel(
+    const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ W, int ldw, OutT* __restrict__ out, int ldo, int M, int N, int K,
+    int gated, Fusion fu) {
+  constexpr int HALVES = NR / 8;                           // rows g and g + 8 of the tile; U: blocks of 32 elements of K under way
   __shared__ float red[WARPS][NR * 8];
   __shared__ float row_scale[8];
   pdl_launch_dependents();
-  pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int r0 = blockIdx.x * NR;
-  // what is needed last is asked for first: loads issued behind the weights would wait for all their bytes
+  const int blocks = K / 32, per = (blocks + WARPS - 1) / WARPS;
+  const int b0 = warp * per, b1 = min(blocks, b0 + per);
+  const __nv_bfloat16* wp[HALVES];
+#pragma unroll
+  for (int h = 0; h < HALVES; ++h) wp[h] = W + (size_t)min(r0 + h * 8 + g, N - 1) * ldw + t * 8;
+  uint4 wv[U][HALVES], xv[U];
+  auto weights = [&](int b) {                              // places behind the share's end read its first block and are left out
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) wv[u][h] = ld_weights(wp[h] + (size_t)(b + u < b1 ? b + u : b) * 32);
+  };
+  // The weights' lines are asked into L2 before the kernel in front has ended; they are read after it, since it may have written them.
+  if (b0 < b1 && t * 2 < U && (b0 + t * 2 < b1)) {
+#pragma unroll
+    for (int h = 0; h < HALVES; ++h) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(wp[h] - t * 8 + (size_t)(b0 + t * 2) * 32));
+  }
+  pdl_wait();
   float ss[kSsSlots / 32], r_old = 0.f, gain = 0.f;
   if (fu.in_ss && warp < M) {
 #pragma unroll
@@ -465,24 +487,14 @@ __global__ void __launch_bounds__(WARPS * 32) direct_gemm_kernel(const __nv_bflo
     if (fu.extra) r_old += __ldcg(fu.extra + (size_t)m * fu.ldr + n);
     gain = __ldg(fu.gamma + n);
   }
-  const int blocks = K / 32, per = (blocks + WARPS - 1) / WARPS;
-  const int b0 = warp * per, b1 = min(blocks, b0 + per);
-  const __nv_bfloat16* wp[HALVES];
-#pragma unroll
-  for (int h = 0; h < HALVES; ++h) wp[h] = W + (size_t)min(r0 + h * 8 + g, N - 1) * ldw + t * 8;
   const __nv_bfloat16* xp = x + (size_t)(g < M ? g : 0) * ldx + t * 8;
   float acc[2][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) acc[0][i] = acc[1][i] = 0.f;
   for (int b = b0; b < b1; b += U) {
-    uint4 wv[U][HALVES], xv[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {                          // places behind the share's end read its first block and are left out
-      const size_t at = (size_t)(b + u < b1 ? b + u : b) * 32;
-      xv[u] = ld_rows(xp + at);
-#pragma unroll
-      for (int h = 0; h < HALVES; ++h) wv[u][h] = ld_weights(wp[h] + at);
-    }
+    for (int u = 0; u < U; ++u) xv[u] = ld_rows(xp + (size_t)(b + u < b1 ? b + u : b) * 32);
+    weights(b);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (b + u >= b1) break;
@@ -568,8 +580,11 @@ inline DirectPlan plan_direct(int M, int N, int K, bool sink) {
 template <int NR, int WARPS, typename OutT>
 int launch_direct(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, int M, int N, int K, int gated, const Fusion& fu,
                   cudaStream_t s) {
-  const cudaError_t e = launch_kernel_as((pdl_enabled() & 3) != 0, direct_gemm_kernel<NR, WARPS, OutT>, dim3((N + NR - 1) / NR), dim3(WARPS * 32), 0, s,
-                                         1, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W, ldw, (OutT*)out, ldo, M, N, K, gated, fu);
+  // two blocks of K a warp need half of the registers, with which twice the blocks find a place
+  auto kernel = K <= 64 * WARPS ? direct_gemm_kernel<NR, WARPS, 2, OutT> : direct_gemm_kernel<NR, WARPS, 4, OutT>;
+  // Launched as soon as the kernel in front has started its last block (programmatic launch): what a block asks for ahead of pdl_wait is weights.
+  const cudaError_t e = launch_kernel_as(true, kernel, dim3((N + NR - 1) / NR), dim3(WARPS * 32), 0, s, 1, (const __nv_bfloat16*)x, ldx,
+                                         (const __nv_bfloat16*)W, ldw, (OutT*)out, ldo, M, N, K, gated, fu);
   return e != cudaSuccess ? (int)e : launch_status();
 }
 template <typename OutT>
