@@ -15,6 +15,7 @@
 //
 // Per chunk, eight warps: scores 16 rows x 64 (two warps each, half the columns of v), read-out of S_0 from its three parts in
 // shared memory, weighted scores times v, and the update, where a warp holds 16 (or 32) rows of S.
+// With 128 keys and no column of ones, steps with rows of three chunks and more take decay_rows_tc.cu, which has the same bits.
 // Rows of up to `longest` tokens are left alone (the scan runs them).  A token's sums have one order for its place in its row, whatever
 // else is in the step; where a prompt is cut shows in the last bits.
 //
