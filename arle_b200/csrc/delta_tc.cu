@@ -109,9 +109,9 @@ __global__ void __launch_bounds__(256, 3) delta_chunks_kernel(const __nv_bfloat1
       sq += __shfl_xor_sync(0xffffffffu, sq, o);
       sk += __shfl_xor_sync(0xffffffffu, sk, o);
     }
-    if (part == 0) {
-      sm.iq[j] = q_scale / sqrt((double)sq + unit_eps);
-      sm.ik[j] = 1.0 / sqrt((double)sk + unit_eps);
+    if (part == 0) {                                       // behind the row's end zeros: with a unit_eps of zero the factors would be infinities
+      sm.iq[j] = j < n ? q_scale / sqrt((double)sq + unit_eps) : 0.0;
+      sm.ik[j] = j < n ? 1.0 / sqrt((double)sk + unit_eps) : 0.0;
     }
   }
   __syncthreads();

@@ -20,23 +20,23 @@ def _inputs(lens, H, kq, vdim):
     return q, k, v, beta, decay, torch.randn(len(lens) + 1, H * vdim * DIM + 8, generator=g, device=DEV)
 
 
-def _run(q, k, v, beta, decay, state, lens, H, kq, vdim, chunks=True, slots=None):
+def _run(q, k, v, beta, decay, state, lens, H, kq, vdim, chunks=True, slots=None, eps=1e-6):
     at = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0).to(torch.int32)
     out = torch.full((q.shape[0] + 1, H, vdim), 7.0, device=DEV)
     state, n = state.clone(), ops.delta_scan_scratch(q.shape[0], len(lens), H)
     assert n > 0 and ops.delta_scan_takes_chunks(q, vdim, DIM, max(lens))
     scratch = torch.full((n + 4,), float("nan"), device=DEV)
     slots = torch.tensor(slots or list(range(len(lens))), dtype=torch.int32, device=DEV)
-    ops.delta_scan(q, k, v, beta, decay, state, at, slots, out[:-1], H, kq, DIM, vdim, DIM ** -0.5, 1e-6,
+    ops.delta_scan(q, k, v, beta, decay, state, at, slots, out[:-1], H, kq, DIM, vdim, DIM ** -0.5, eps,
                    **(dict(max_q_len=max(lens), scratch=scratch[:n]) if chunks else {}))
     assert (out[-1] == 7.0).all() and scratch[n:].isnan().all()
     return out[:-1], state
 
 
-def _exact(q, k, v, beta, decay, state, lens, H, kq, vdim):
+def _exact(q, k, v, beta, decay, state, lens, H, kq, vdim, eps=1e-6):
     def unit(x):
         x = x.double().view(-1, kq, DIM)
-        return (x * torch.rsqrt(x.square().sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // kq, 1)
+        return (x * torch.rsqrt(x.square().sum(-1, keepdim=True) + eps)).repeat_interleave(H // kq, 1)
 
     qq, kk, vv = unit(q) * DIM ** -0.5, unit(k), v.double().view(-1, H, vdim)
     S, outs, t = state[:, : H * vdim * DIM].double().view(-1, H, vdim, DIM).clone(), [], 0
@@ -95,3 +95,17 @@ def test_decays_of_zero_and_overflow():
     worse[75, 4] = float("nan")
     odd, _ = _run(q, worse, v, beta, decay, state, lens, H, kq, vdim)
     assert torch.allclose(odd[:75], clean[:75], **close) and not odd[75:].isfinite().any()
+
+
+@pytest.mark.parametrize("lens", [[81], [128], [100, 5, 229]])
+def test_lengths_without_an_epsilon(lens):
+    """The places behind a row's end have q and k of zeros, whose length has no inverse: they stay out of the memory all the same."""
+    H, kq, vdim = 3, 1, 40
+    x = _inputs(lens, H, kq, vdim)
+    want, want_s = _exact(*x, lens, H, kq, vdim, eps=0.0)
+    got, got_s = _run(*x, lens, H, kq, vdim, eps=0.0)
+    whole, whole_s = _run(*x, lens, H, kq, vdim, chunks=False, eps=0.0)
+    used = H * vdim * DIM
+    for a, b, w in ((got, whole, want), (got_s[:-1, :used], whole_s[:-1, :used], want_s[:-1])):
+        off, ref = ((y.double() - w).norm() / w.norm() for y in (a, b))
+        assert off < 4e-7 and off < 1.3 * ref + 2e-8
