@@ -2048,13 +2048,15 @@ def delta_gates(pre, a_log, dt_bias, beta, decay) -> None:
 
 
 def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: int, kq_heads: int, dim: int, vdim: int,
-               q_scale: float, unit_eps: float, max_q_len: int = 0, scratch=None) -> None:
-    """``scratch`` (float32, ``delta_scan_scratch`` numbers, or None; see ``delta_scan_takes_chunks``): the rows of 80 tokens and more run in
-    chunks on the tensor cores.  The gated delta rule over the tokens of every row of the step, from and into state[state_slots[r]]: with q and k brought
-    to unit length per head (x / sqrt(sum x^2 + unit_eps); q also times q_scale), S <- decay_t S; u = beta_t (v_t - S^T k_t);
+               q_scale: float, unit_eps: float, max_q_len: int = 0, scratch=None, q_lens=None) -> None:
+    """The gated delta rule over the tokens of every row of the step, from and into state[state_slots[r]]: with q and k brought to unit length per head (x / sqrt(sum x^2 + unit_eps); q also times q_scale), S <- decay_t S; u = beta_t (v_t - S^T k_t);
     S <- S + k_t u^T; o_t = S^T q_t.  q, k [T, kq_heads*dim] (head h reads head h // (heads / kq_heads)), v [T, heads*vdim], in
     the activation type (views of wider rows are fine); beta, decay float32 [T, heads]; state float32 [slots, n] whose first
-    heads * vdim * dim numbers are the memories, a head's transposed ([heads][vdim][dim]); out float32 [T, heads, vdim]."""
+    heads * vdim * dim numbers are the memories, a head's transposed ([heads][vdim][dim]); out float32 [T, heads, vdim].
+
+    With ``scratch`` (float32, ``delta_scan_scratch`` numbers; where ``delta_scan_takes_chunks`` says so) rows of 80 tokens and more run in chunks
+    on the tensor cores, for beta and decays in [0, 1] as ``delta_gates`` makes them.  Every row runs whatever the other two say: ``q_lens``, the rows' lengths on the host,
+    spares the launch for short rows where there are none; a ``max_q_len`` of 1 to 79 sends all rows to the scan."""
     T = v.shape[0]
     R = state_slots.numel()
     if (q.shape != (T, kq_heads * dim) or k.shape != q.shape or v.shape != (T, heads * vdim) or q.dtype != k.dtype
@@ -2070,11 +2072,13 @@ def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: i
     _i32(q_indptr, "q_indptr"), _i32(state_slots, "state_slots")
     if q_indptr.numel() != R + 1:
         raise KernelError("delta_scan: q_indptr must have one entry more than state_slots")
-    if scratch is not None:
+    if scratch is not None and not 0 < max_q_len <= DELTA_SCAN_LONGEST:
         if (q.dtype != torch.bfloat16 or dim != 128 or scratch.dtype != torch.float32 or not scratch.is_contiguous()
                 or scratch.numel() < delta_scan_scratch(T, R, heads)):
             raise KernelError("delta_scan: scratch is for bfloat16 heads of 128, contiguous float32 of delta_scan_scratch numbers")
-        short = T - (R - 1) * max_q_len <= DELTA_SCAN_LONGEST    # else the shortest row is a long one too
+        if q_lens is not None and (len(q_lens) != R or sum(q_lens) > T):
+            raise KernelError("delta_scan: q_lens must have the lengths of q_indptr's rows")
+        short = q_lens is None or (R > 0 and min(q_lens) <= DELTA_SCAN_LONGEST)
         _check(library().arle_delta_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(beta), _ptr(decay), _ptr(state),
                                        state.stride(0), _ptr(q_indptr), _ptr(state_slots), _ptr(out), _ptr(scratch), T, R, heads, kq_heads,
                                        vdim, float(q_scale), float(unit_eps), DELTA_SCAN_LONGEST, int(short), _stream()), "delta_tc")

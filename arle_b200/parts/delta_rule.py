@@ -119,7 +119,7 @@ class GatedDeltaRule(Mixer):
         chunks = {}
         if ops.delta_scan_takes_chunks(q, s.value_dim, s.key_dim, ctx.max_q_len):
             n = ops.delta_scan_scratch(T, ctx.state_slots.numel(), H)
-            chunks = dict(max_q_len=ctx.max_q_len, scratch=ctx.ws.get("delta_chunks", (n,), torch.float32))
+            chunks = dict(q_lens=ctx.q_lens, scratch=ctx.ws.get("delta_chunks", (n,), torch.float32))
         ops.delta_scan(q, k, v, beta, decay, state, ctx.q_indptr, ctx.state_slots, o, H, s.num_kq_heads, s.key_dim, s.value_dim,
                        float(s.key_dim) ** -0.5, s.unit_eps, **chunks)
         gated = ctx.ws.get("delta_gated", (T, inner), x.dtype)

@@ -109,3 +109,31 @@ def test_lengths_without_an_epsilon(lens):
     for a, b, w in ((got, whole, want), (got_s[:-1, :used], whole_s[:-1, :used], want_s[:-1])):
         off, ref = ((y.double() - w).norm() / w.norm() for y in (a, b))
         assert off < 4e-7 and off < 1.3 * ref + 2e-8
+
+
+@pytest.mark.parametrize("lens,spare", [([100, 5], 0), ([300, 5], 1), ([81], 3), ([2, 79, 64], 0), ([100, 90, 229], 0)])
+@pytest.mark.parametrize("say", [dict(), dict(max_q_len=200), dict(max_q_len=40), "q_lens"], ids=str)
+def test_every_row_runs(lens, spare, say):
+    """Whatever is said about the rows' lengths, short rows beside long ones run, also where the arrays have more rows than q_indptr ends at."""
+    H, kq, vdim = 2, 1, 64
+    *x, state = _inputs(lens + [spare] if spare else lens, H, kq, vdim)
+    T, n = sum(lens), ops.delta_scan_scratch(sum(lens) + spare, len(lens), H)
+    at = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0).to(torch.int32)
+    slots = torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    got = []
+    for kw in (dict(scratch=torch.empty(n, device=DEV), **(dict(q_lens=lens) if say == "q_lens" else say)), {}):
+        s, out = state.clone(), torch.full((T + spare, H, vdim), 7.0, device=DEV)
+        ops.delta_scan(*x, s, at, slots, out, H, kq, DIM, vdim, DIM ** -0.5, 1e-6, **kw)
+        got.append((out, s))
+    (a, sa), (b, sb) = got
+    assert (a[T:] == 7.0).all() and not (a[:T] == 7.0).any()
+    assert (a - b).norm() < 1e-6 * b.norm() and (sa - sb).norm() < 1e-6 * sb.norm()
+
+
+def test_lengths_that_are_not_the_rows():
+    *x, state = _inputs([100, 5], 1, 1, 8)
+    at, slots = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ([0, 100, 105], [0, 1]))
+    for lens in ([105], [100, 6]):
+        with pytest.raises(ops.KernelError):
+            ops.delta_scan(*x, state, at, slots, torch.empty(105, 1, 8, device=DEV), 1, 1, DIM, 8, DIM ** -0.5, 1e-6,
+                           scratch=torch.empty(ops.delta_scan_scratch(105, 2, 1), device=DEV), q_lens=lens)
