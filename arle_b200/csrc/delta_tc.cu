@@ -549,24 +549,28 @@ int most_chunks(int num_tokens, int R, int longest) {      // of rows of more th
 
 }  // namespace
 
-// Rows of more than `longest` tokens; the others, where there may be any (`short_rows`), go to arle_delta_scan.  q, k bfloat16 [T, kq_heads*128], v bfloat16 [T, H*vdim] (row strides multiples
-// of 8, 16-byte aligned), beta, decay float32 [T, H]; state: float32, a slot every slot_stride numbers, [H][vdim][128] at its start; out float32
-// [T, H, vdim], 8-byte aligned; vdim a multiple of 8; scratch: 7,936 float32 numbers for each head and chunk, 16-byte aligned, for as many chunks
-// as such rows can have (num_tokens / 64 + min(R, num_tokens / (longest + 1)), whole numbers).
+// Rows of more than `longest` tokens; the others go to arle_delta_scan.  long_rows, long_tokens: how many such rows there are and their tokens
+// together, where the host knows them (long_rows below zero: it does not); what is launched goes by the rows that run there.  q, k bfloat16
+// [T, kq_heads*128], v bfloat16 [T, H*vdim] (row strides multiples of 8, 16-byte aligned), beta, decay float32 [T, H]; state: float32, a slot
+// every slot_stride numbers, [H][vdim][128] at its start; out float32 [T, H, vdim], 8-byte aligned; vdim a multiple of 8; scratch: 7,936 float32
+// numbers for each head and chunk, 16-byte aligned, for as many chunks as such rows can have (num_tokens / 64 + min(R, num_tokens / (longest +
+// 1)), whole numbers).
 ARLE_API int arle_delta_tc(const void* q, const void* k, const void* v, int q_stride, int k_stride, int v_stride, const float* beta,
                            const float* decay, float* state, long slot_stride, const int* q_indptr, const int* state_slots, float* out,
                            float* scratch, int num_tokens, int R, int H, int kq_heads, int vdim, float q_scale, float unit_eps, int longest,
-                           int short_rows, cudaStream_t s) {
+                           int long_rows, int long_tokens, cudaStream_t s) {
   if (R <= 0 || num_tokens <= 0) return 0;
   if (H <= 0 || kq_heads <= 0 || H % kq_heads || vdim <= 0 || longest < 0 || !scratch) return ARLE_E_BADARG;
   if (vdim % 8 || q_stride % 8 || k_stride % 8 || v_stride % 8 || H > 65535 || R > 65535 ||
       (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)scratch) & 15) || ((uintptr_t)out & 7))
     return ARLE_E_UNSUPPORTED;
-  const int slots = most_chunks(num_tokens, R, longest);
-  if (slots == 0) short_rows = 1;
-  if (short_rows) {
-    const int e = arle_delta_scan(q, k, v, 1, q_stride, k_stride, v_stride, beta, decay, state, slot_stride, q_indptr, state_slots, out, num_tokens, R, H,
-                                  kq_heads, kDim, vdim, q_scale, unit_eps, longest, s);
+  const bool known = long_rows >= 0;
+  const int slots = known && long_rows == 0 ? 0 : most_chunks(num_tokens, R, longest);
+  if (slots == 0 || !known || long_rows < R) {
+    // the scan's form goes by the tokens of the rows that it runs (63 of one token beside one of 128, 32 heads: 125 us, 159 in the form for prompts)
+    const int short_tokens = known ? num_tokens - long_tokens + long_rows : num_tokens;
+    const int e = arle_delta_scan(q, k, v, 1, q_stride, k_stride, v_stride, beta, decay, state, slot_stride, q_indptr, state_slots, out,
+                                  short_tokens, R, H, kq_heads, kDim, vdim, q_scale, unit_eps, longest, s);
     if (e || slots == 0) return e;
   }
   uint32_t* chunks = reinterpret_cast<uint32_t*>(scratch);
@@ -575,9 +579,11 @@ ARLE_API int arle_delta_tc(const void* q, const void* k, const void* v, int q_st
   if (raised != cudaSuccess) return (int)raised;
   launch_kernel(delta_chunks_kernel, dim3(slots, H), dim3(256), sizeof(ChunkSmem), s, 1, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
                 (long)q_stride, (long)k_stride, beta, decay, q_indptr, R, longest, H, kq_heads, q_scale, unit_eps, chunks);
-  // Groups of 16 columns by themselves while every block finds an SM (8 heads of 128, one row of 2,048: 134 us, 171 with two to a block, 265
-  // with four), two to a block beyond (32 heads: 309, 208 and 299; rows of 819, 701 and 479 tokens 298, 210 and 202).  The same bits.
-  if ((long)((vdim + 15) / 16) * H * R <= 148)
+  // Groups of 16 columns by themselves while every block that has a row to run finds an SM (8 heads of 128, one row of 2,048: 134 us, 171 with two
+  // to a block, 265 with four), two to a block beyond (32 heads: 309, 208 and 299; rows of 819, 701 and 479 tokens 298, 210 and 202).  The same bits.
+  // Rows that are scanned don't count (8 heads, one row of 2,048 beside 8 decoded tokens: 143 us, 177 when they did).
+  const int most = num_tokens / (longest + 1), rows = known ? long_rows : most < R ? most : R;
+  if ((long)((vdim + 15) / 16) * H * rows <= 148)
     return launch<1>(q, k, v, q_stride, k_stride, v_stride, chunks, state, slot_stride, q_indptr, state_slots, out, R, H, kq_heads, vdim, longest, s);
   return launch<2>(q, k, v, q_stride, k_stride, v_stride, chunks, state, slot_stride, q_indptr, state_slots, out, R, H, kq_heads, vdim, longest, s);
 }

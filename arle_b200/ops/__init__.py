@@ -66,7 +66,7 @@ _SIGNATURES = {
     "arle_rglru_scan": [_P, _P, _P, _I, _I, _P, _P, _P, _P, _F, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "arle_delta_gates": [_P, _I, _P, _P, _P, _P, _I, _I, _P],
     "arle_delta_scan": [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _I, _P],
-    "arle_delta_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _I, _P],
+    "arle_delta_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _I, _I, _I, _P],
     "arle_clamped_glu": [_P, _P, _I, _I, _I, _I, _F, _F, _P],
     "arle_paged_attention_decode": [_P, _I, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P],
     "arle_paged_attention_decode_stream": [_P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I,
@@ -2078,10 +2078,11 @@ def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: i
             raise KernelError("delta_scan: scratch is for bfloat16 heads of 128, contiguous float32 of delta_scan_scratch numbers")
         if q_lens is not None and (len(q_lens) != R or sum(q_lens) > T):
             raise KernelError("delta_scan: q_lens must have the lengths of q_indptr's rows")
-        short = q_lens is None or (R > 0 and min(q_lens) <= DELTA_SCAN_LONGEST)
+        long = [n for n in q_lens if n > DELTA_SCAN_LONGEST] if q_lens is not None else None
         _check(library().arle_delta_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(beta), _ptr(decay), _ptr(state),
                                        state.stride(0), _ptr(q_indptr), _ptr(state_slots), _ptr(out), _ptr(scratch), T, R, heads, kq_heads,
-                                       vdim, float(q_scale), float(unit_eps), DELTA_SCAN_LONGEST, int(short), _stream()), "delta_tc")
+                                       vdim, float(q_scale), float(unit_eps), DELTA_SCAN_LONGEST, -1 if long is None else len(long),
+                                       sum(long or ()), _stream()), "delta_tc")
         return
     _check(library().arle_delta_scan(_ptr(q), _ptr(k), _ptr(v), _dt(q), q.stride(0), k.stride(0), v.stride(0), _ptr(beta), _ptr(decay),
                                      _ptr(state), state.stride(0), _ptr(q_indptr), _ptr(state_slots), _ptr(out), T, R, heads, kq_heads,
