@@ -370,11 +370,11 @@ int launch(const void* q, const void* k, const void* v, long q_stride, long k_st
 
 }  // namespace
 
-// What arle_decay_tc does with dim 128 and vcols == vdim (vdim a multiple of 8), out on 8-byte boundaries.  num_chunks: of 64 tokens, of the rows of
-// more than `longest` tokens; scratch: 4,096 float32 numbers for each of them and each head, 16-byte aligned.
+// What arle_decay_tc does with dim 128 and vcols == vdim (vdim a multiple of 8), out on 8-byte boundaries.  num_chunks: of 64 tokens, of the
+// long_rows rows of more than `longest` tokens; scratch: 4,096 float32 numbers for each of them and each head, 16-byte aligned.
 ARLE_API int arle_decay_rows_tc(const void* q, const void* k, const void* v, int q_stride, int k_stride, int v_stride, const float* a, const float* b,
                                 float* state, long slot_stride, const int* q_indptr, const int* state_slots, float* out, float* scratch,
-                                int num_chunks, int R, int H, int kq_heads, int vdim, float q_scale, int longest, cudaStream_t s) {
+                                int num_chunks, int long_rows, int R, int H, int kq_heads, int vdim, float q_scale, int longest, cudaStream_t s) {
   if (R <= 0 || num_chunks <= 0) return 0;
   if (H <= 0 || kq_heads <= 0 || H % kq_heads || vdim <= 0 || longest < 0 || !scratch) return ARLE_E_BADARG;
   if (vdim % 8 || q_stride % 8 || k_stride % 8 || v_stride % 8 || H > 65535 || R > 65535 ||
@@ -388,9 +388,9 @@ ARLE_API int arle_decay_rows_tc(const void* q, const void* k, const void* v, int
   const int heads = H / kq_heads % kMostHeads == 0 ? kMostHeads : 1;
   launch_kernel(decay_tiles_kernel, dim3(num_chunks, H / heads), dim3(128), sizeof(TilesSmem), s, 1, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
                 (long)q_stride, (long)k_stride, a, b, q_indptr, R, longest, H, kq_heads, heads, q_scale, chunks);
-  // one group a block while two of them an SM hold all columns (32 heads of 64 columns, 2,048 tokens: 84 us, with four groups 179), four beyond
-  // (128 heads: 226 with one or two groups, 199)
-  if ((long)((vdim + 15) / 16) * H * R <= 296)
+  // one group a block while two of them an SM hold all columns of the rows that run here (32 heads of 64 columns, 2,048 tokens: 84 us, with four
+  // groups 179), four beyond (128 heads: 226 with one or two groups, 199)
+  if ((long)((vdim + 15) / 16) * H * long_rows <= 296)
     return launch<1>(q, k, v, q_stride, k_stride, v_stride, chunks, state, slot_stride, q_indptr, state_slots, out, R, H, kq_heads, vdim, longest, s);
   return launch<4>(q, k, v, q_stride, k_stride, v_stride, chunks, state, slot_stride, q_indptr, state_slots, out, R, H, kq_heads, vdim, longest, s);
 }

@@ -98,7 +98,7 @@ _SIGNATURES = {
     "arle_latent_prefill_tc": [_P, _I, _I, _P, _P, _I, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _I, _I, _I, _I, _P, _P],
     "arle_latent_attention": [_P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P],
     "arle_decay_scan": [_P, _P, _P, _I, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _I, _P],
-    "arle_decay_rows_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
+    "arle_decay_rows_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P],
     "arle_decay_tc": [_P, _P, _P, _I, _I, _I, _P, _P, _P, ctypes.c_long, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P],
     "arle_decay_chunk_plan_ints": [_I, _I],
     "arle_decay_chunk_tokens": [],
@@ -1521,7 +1521,7 @@ def decay_memories(q, k, v, a, b, state, batch, out, heads: int, kq_heads: int, 
         scratch = batch.ws.get("decay_tiles", (n * heads * 4096,), torch.float32)
         _check(library().arle_decay_rows_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(a), _ptr(b), _ptr(state),
                                             state.stride(0), _ptr(batch.q_indptr), _ptr(batch.state_slots), _ptr(out), _ptr(scratch), n,
-                                            batch.num_rows, heads, kq_heads, vdim, float(q_scale), DECAY_TC_LONGEST, _stream()), "decay_rows_tc")
+                                            sum(t > DECAY_TC_LONGEST for t in batch.q_lens), batch.num_rows, heads, kq_heads, vdim, float(q_scale), DECAY_TC_LONGEST, _stream()), "decay_rows_tc")
         return
     _check(library().arle_decay_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(a), _ptr(b), _ptr(state), state.stride(0),
                                    _ptr(batch.q_indptr), _ptr(batch.state_slots), _ptr(out), batch.num_rows, heads, kq_heads, dim, vdim, vcols,

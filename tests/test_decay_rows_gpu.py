@@ -1,6 +1,8 @@
 """Memories with a scalar decay and 128 keys: the scores of all chunks formed side by side and the chain behind them give the bits of the one launch
 that does both, for rows around a chunk's end, short rows beside long ones, heads in fours and by themselves, columns that do not fill a block, one
 group of columns a block and four, and decays of zero; with values that overflow the same to the last bits."""
+import re
+
 import pytest
 import torch
 
@@ -38,3 +40,21 @@ def test_the_bits_of_the_one_launch(monkeypatch, H, G, vdim, lens, kind):
         else:
             assert torch.equal(x, y)
     assert (got[0][0][T] == 7.0).all()
+
+
+@pytest.mark.parametrize("H,n", [(32, 2048), (8, 192)])
+def test_the_chain_goes_by_the_rows_that_it_runs(H, n):
+    """A long row beside decoded tokens takes the chain's kernel that it takes by itself (as many groups of columns a block)."""
+    dim, vdim, names = 128, 64, []
+    for lens in ([n], [n] + [1] * 40):
+        T = sum(lens)
+        q, k, v = (torch.zeros(T, w, device=DEV, dtype=torch.bfloat16) for w in (dim, dim, H * vdim))
+        a, b = (torch.ones(T, H, device=DEV) for _ in range(2))
+        ctx, state, out = _ctx(lens, H * vdim * dim), torch.zeros(len(lens) + 1, H * vdim * dim, device=DEV), torch.empty(T, H, vdim, device=DEV)
+        ops.decay_memories(q, k, v, a, b, state, ctx, out, H, 1, dim, vdim, False, 1.0)
+        torch.cuda.synchronize()
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
+            ops.decay_memories(q, k, v, a, b, state, ctx, out, H, 1, dim, vdim, False, 1.0)
+            torch.cuda.synchronize()
+        names.append({m.group(0) for m in (re.search(r"decay_rows_tc_kernel<\d+>", e.name) for e in p.events()) if m})
+    assert len(names[0]) == 1 and names[0] == names[1]
