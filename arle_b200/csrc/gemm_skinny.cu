@@ -437,9 +437,11 @@ __global__ void __launch_bounds__(kThreads, 1) skinny_gemm_kernel(
 // 20.8 on the ring); a decode step of 28 such layers 787 us (799 in stream order), of 8 layers behind 100 tokens 265 (285).  Weights are read
 // behind the wait alone, since a program may write them in the kernel in front (read ahead of it, into registers: 13.4).  plan_direct has the
 // figures by size, in stream order.
+// Plain loads: the non-coherent path (ld.global.nc, __ldg) is for memory that nobody writes while a kernel lives, and this one lives beside the
+// kernel in front, which may write the weights; pdl_wait orders plain loads alone.
 __device__ __forceinline__ uint4 ld_weights(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ uint4 ld_rows(const void* p) {
@@ -485,7 +487,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 16 ? 1 : WARPS == 16 ? 2 :
   if (fu.resid && valid) {
     r_old = __ldcg(fu.resid + (size_t)m * fu.ldr + n);
     if (fu.extra) r_old += __ldcg(fu.extra + (size_t)m * fu.ldr + n);
-    gain = __ldg(fu.gamma + n);
+    gain = __ldcg(fu.gamma + n);
   }
   const __nv_bfloat16* xp = x + (size_t)(g < M ? g : 0) * ldx + t * 8;
   float acc[2][4];

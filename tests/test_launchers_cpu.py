@@ -1,5 +1,6 @@
 """What the launchers keep between calls, read from their sources: a kernel's limit of dynamic shared memory belongs to a device, so no
-launcher may remember for the whole process that it was raised (a model on the process's second device would fail at its first launch)."""
+launcher may remember for the whole process that it was raised (a model on the process's second device would fail at its first launch).  And
+what a kernel that lives beside the one in front of it may not do."""
 import pathlib
 import re
 
@@ -22,3 +23,13 @@ def test_the_limit_is_kept_per_device():
     text = (CSRC / "common.cuh").read_text()
     body = text[text.index("class SharedLimit"):]
     assert "cudaGetDevice(&dev)" in body[: body.index("};")]
+
+
+def test_kernels_that_always_start_early_read_plainly():
+    """The non-coherent load path is for memory that nobody writes while the kernel lives, and a kernel launched programmatically lives beside
+    the one in front of it, which may write its weights: waiting for that kernel orders plain loads alone."""
+    text = (CSRC / "gemm_skinny.cu").read_text()
+    first, last = text.index("uint4 ld_weights("), text.index("struct DirectPlan")
+    body = re.sub(r"//[^\n]*", "", text[first:last])
+    assert "direct_gemm_kernel(" in body and "pdl_wait();" in body
+    assert not re.search(r"\.nc\b|__ldg\(", body)
