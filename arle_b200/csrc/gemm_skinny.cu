@@ -559,23 +559,29 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 16 ? 1 : WARPS == 16 ? 2 :
 }
 
 // Whether a product is one of those, and how it is cut: as many warps as are resident together (31 an SM at 64 registers), no more than two
-// blocks of 32 elements of K leave work for; eight rows a block where sixteen would leave SMs without one.  Above 2^24 elements the ring
-// keeps more bytes in flight.  One row of x in a graph, weights not in L2, us (the ring's in brackets): 1,024 x 2,048 3.5 (4.9), 4,096 x 1,024
-// 4.0 (5.1), 1,024 x 3,072 4.1 (5.5), 6,144 x 1,024 4.8 (6.5), 64 x 4,096 3.3 (5.6), 8,192 x 1,024 7.1 (7.3), 4,096 x 4,096 8.6 (9.1), 6,144 x
-// 4,096 12.1 (11.9), 16,384 x 1,024 10.3 (9.8); eight rows the same to 0.3 us more.  1,024 x 4,096 with 32, 16 and 8 warps of 8 rows: 4.5, 5.9,
-// 9.0, with 32 of 16 rows 5.0; 2,048 x 4,096 with 32 warps of 16 rows 5.8, 16 of 8 6.6.
+// blocks of 32 elements of K leave work for; eight rows a block while every block finds an SM of its own.  Above 2^24 elements the ring keeps
+// more bytes in flight, and so it does with few rows of W and a long K, which it takes apart over a cluster, where each block of 32 elements
+// more is 0.4 us for a warp here (8 rows of x: 12,288 elements of K 7.0 us at 64 to 512 rows of W, the ring 7.2 to 7.7; 16,384 8.9 at 64 and at
+// 512 rows, 7.4 and 8.2; at 700 and 1,024 9.3 and 9.6, 10.0 and 10.5; 128 x 32,768 15.9 and 8.1).
+// One row of x in a graph, weights not in L2, us (the ring's in brackets): 1,024 x 2,048 3.5 (4.9), 4,096 x 1,024 4.0 (5.1), 1,024 x 3,072 4.1
+// (5.5), 6,144 x 1,024 4.8 (6.5), 64 x 4,096 3.3 (5.6), 8,192 x 1,024 7.1 (7.3), 4,096 x 4,096 8.6 (9.1), 6,144 x 4,096 12.1 (11.9), 16,384 x
+// 1,024 10.3 (9.8); eight rows the same to 0.3 us more.  1,024 x 4,096 with 32, 16 and 8 warps of 8 rows: 4.5, 5.9, 9.0, with 32 of 16 rows 5.0;
+// 2,048 x 4,096 with 32 warps of 16 rows 5.8, 16 of 8 6.6.
 struct DirectPlan {
   int rows, warps;                                         // of a block; rows 0: the ring
+  bool last;                                               // only where the ring does not take it
 };
 inline DirectPlan plan_direct(int M, int N, int K, bool sink) {
   constexpr long long kMostElements = 1ll << 24;
   constexpr int kMostWarps = 4608;
-  DirectPlan p{0, 0};
+  DirectPlan p{0, 0, false};
   if (M > 8 || (long long)N * K > kMostElements) return p;
   const int rows = N <= 1152 ? 8 : 16, tiles = (N + rows - 1) / rows;
   for (int w = 8; w <= 32; w += 8)
     if ((w == 8 || w * 64 <= K) && (long long)tiles * w <= kMostWarps) p.warps = w;
   if (p.warps && !(sink && tiles > kSsSlots)) p.rows = rows;
+  const int share = p.warps ? (K / 32 + p.warps - 1) / p.warps : 0;
+  p.last = share > 16 || (share > 12 && N <= 640);
   return p;
 }
 
@@ -715,19 +721,16 @@ int skinny_entry(const void* x, int ldx, const void* W, int ldw, void* out, int 
   if (gated && N % 2 != 0) return ARLE_E_BADARG;
   if (fu.resid && (gated || !fu.gamma || !fu.xs || !fu.out_ss)) return ARLE_E_BADARG;
   if (!fu.resid && !out) return ARLE_E_BADARG;
+  if (out_dtype != 0 && out_dtype != 1) return ARLE_E_BADARG;
   const DirectPlan direct = plan_direct(M, N, K, fu.resid != nullptr);
-  if (direct.rows) {
-    if (out_dtype == 0) return run_direct<float>(direct, x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, s);
-    if (out_dtype == 1) return run_direct<__nv_bfloat16>(direct, x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, s);
-  }
-  if (M <= 8) {
-    if (out_dtype == 0) return plan_and_launch<1, float>(x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, err, s);
-    if (out_dtype == 1) return plan_and_launch<1, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, err, s);
-  } else {
-    if (out_dtype == 0) return plan_and_launch<2, float>(x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, err, s);
-    if (out_dtype == 1) return plan_and_launch<2, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, err, s);
-  }
-  return ARLE_E_BADARG;
+  auto run = [&](auto type) {
+    typedef decltype(type) OutT;
+    if (direct.rows && !direct.last) return run_direct<OutT>(direct, x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, s);
+    const int e = M <= 8 ? plan_and_launch<1, OutT>(x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, err, s)
+                         : plan_and_launch<2, OutT>(x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, err, s);
+    return e == ARLE_E_UNSUPPORTED && direct.rows ? run_direct<OutT>(direct, x, ldx, W, ldw, out, ldo, M, N, K, gated, fu, s) : e;
+  };
+  return out_dtype == 0 ? run(float()) : run(__nv_bfloat16());
 }
 
 }  // namespace

@@ -46,3 +46,21 @@ def test_direct_products(M, N, K):
     assert (ss[M:] == 0).all() and ((ss[:M].sum(1) - r.square().sum(1)).abs() <= 1e-5 * r.square().sum(1)).all()
     assert torch.equal(got[0].resid, got[1].resid) and torch.equal(got[0].ss, got[1].ss)
     ops.check_errors(DEV)
+
+
+@pytest.mark.parametrize("M,N,K,direct", [(8, 512, 12288, True), (1, 40, 12320, False), (8, 512, 16384, False), (3, 700, 16384, True), (1, 700, 16416, False),
+                                          (8, 128, 32768, False), (1, 200, 65536, True)])
+def test_long_shares_go_to_the_ring(M, N, K, direct):
+    """Few rows of a long K would leave a warp one block of K after the other; the ring takes K apart over a cluster (up to what it holds)."""
+    x, w = (torch.randn(m, K, device=DEV).to(torch.bfloat16) for m in (M, N))
+    out = torch.empty(M, N, device=DEV)
+    ops.gemm(x, w, out)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
+        ops.gemm(x, w, out)
+        torch.cuda.synchronize()
+    names = [e.name for e in p.events()]
+    assert any(("direct_gemm_kernel" if direct else "skinny_gemm_kernel") in n for n in names), names
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert ((out.double() - want).abs() <= K * 2.0 ** -24 * size).all()
+    ops.check_errors(DEV)
