@@ -547,7 +547,9 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const T* __
 // The same with the part's numbers kept in registers between the sum and the result, eight an access: parts of up to ITS x THREADS x 8 numbers.
 // Bound by instructions (exponentials and divisions, one after the other) and memory.  2,048 rows of 8,192, 168 MB: 35 us with 512 threads a row
 // and three rows an SM (256 threads, which hold twice the numbers: 44; 1,024 37; four rows spill, 35; read twice number by number 110), 64 rows
-// 6.5 (8.5); of 4,096 16.7 with 256 threads, 18.7 with 512.
+// 4.8 (6.8); of 6,144 26.2 us with 384 threads and four rows an SM (256 32.9; 512 29.6, and 592 rows of 4,104 8.9 instead of 6.6, a second wave); of
+// 4,096 14.9 with 256 threads, 18.7 with 512.  BLOCKS: rows an SM that the registers leave room for; 0: the compiler's choice, which the narrow
+// rows are left to (asked for one at the least it takes 48 registers instead of 40: 16.1 us).
 template <typename T, int ITS, int THREADS, int BLOCKS>
 __global__ void __launch_bounds__(THREADS, BLOCKS) gated_group_norm_vec_kernel(const float* __restrict__ y, const T* __restrict__ x, int x_stride,
                                                                    const float* __restrict__ skip, int vdim, const T* __restrict__ z, int z_stride,
@@ -605,9 +607,10 @@ ARLE_API int arle_gated_group_norm(const float* y, const void* x, int dtype, int
   if (dtype == 1 && width >= 1024 && width <= 8192 && width % 8 == 0 && vdim % 8 == 0 && z_stride % 8 == 0 && out_stride % 8 == 0 &&
       (!skip || x_stride % 8 == 0) &&
       (((uintptr_t)y | (uintptr_t)z | (uintptr_t)out | (uintptr_t)weight | (skip ? (uintptr_t)x : 0)) & 15) == 0) {
-    auto kernel = width <= 2048 ? gated_group_norm_vec_kernel<__nv_bfloat16, 1, 256, 1>
-                  : width <= 4096 ? gated_group_norm_vec_kernel<__nv_bfloat16, 2, 256, 1> : gated_group_norm_vec_kernel<__nv_bfloat16, 2, 512, 3>;
-    launch_kernel(kernel, dim3(num_tokens, parts), dim3(width <= 4096 ? 256 : 512), 0, s, 1, y, (const __nv_bfloat16*)x, x_stride, skip, vdim, (const __nv_bfloat16*)z,
+    auto kernel = width <= 2048   ? gated_group_norm_vec_kernel<__nv_bfloat16, 1, 256, 0>
+                  : width <= 4096 ? gated_group_norm_vec_kernel<__nv_bfloat16, 2, 256, 0>
+                  : width <= 6144 ? gated_group_norm_vec_kernel<__nv_bfloat16, 2, 384, 4> : gated_group_norm_vec_kernel<__nv_bfloat16, 2, 512, 3>;
+    launch_kernel(kernel, dim3(num_tokens, parts), dim3(width <= 4096 ? 256 : width <= 6144 ? 384 : 512), 0, s, 1, y, (const __nv_bfloat16*)x, x_stride, skip, vdim, (const __nv_bfloat16*)z,
                   z_stride, weight, eps, (__nv_bfloat16*)out, out_stride, inner, width);
     return launch_status();
   }

@@ -62,3 +62,8 @@ def test_gated_group_norm(inner, parts, skip):
     val = val.view(T, parts, -1)
     want = (val * torch.rsqrt(val.square().mean(-1, keepdim=True) + 1e-5)).reshape(T, inner) * w.double()
     assert ((out[:T].double() - want).abs() <= (2.0 ** -8 + 1e-5) * want.abs() + 1e-6).all() and (out[T] == 7.0).all()
+
+
+@pytest.mark.parametrize("inner,parts", [(4104, 1), (6144, 1), (6152, 1), (12288, 2)])
+def test_gated_group_norm_of_six_thousand(inner, parts):         # parts of 4,097 to 6,144 numbers have threads of their own number
+    test_gated_group_norm(inner, parts, True)
