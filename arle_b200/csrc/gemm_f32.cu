@@ -14,9 +14,9 @@
 //    shared memory for more.
 //  * gemm_f32_stages: tiles of 32 x 32 and 64 x 64, stages of 32 numbers of k as they lie in memory on their way by cp.async, three ahead.  For
 //    the products of short prompts, whose few tiles an SM are bound by how long memory takes to answer (gemm_f32_tiles asks one stage ahead).
-//  * gemm_f32_tiles: tiles of 64 x 128, 8 x 4 sums a thread, the next 16 numbers of k on their way while the present
-//    ones are multiplied; two neighbouring sums are one packed instruction (fma.rn.f32x2: each half the same rounded fused product).
-//    Bound by instructions, half of FFMA's rate.  No sum may be split along k, so the launcher takes the tile that leaves the busiest SM the least.
+//  * gemm_f32_tiles: tiles of 64 x 128, and of 64 x 64 where a bfloat16 W's fill an SM, 8 x 4 sums a thread, the next 16 numbers of k on their
+//    way while the present ones are multiplied; two neighbouring sums are one packed instruction (fma.rn.f32x2: each half the same rounded
+//    fused product).  Bound by instructions, half of FFMA's rate.  No sum may be split along k, so the launcher takes the tile that leaves the busiest SM the least.
 //  * gemm_f32 (rows that are not on 16-byte boundaries, and bfloat16 A): the general one, tiles of 64 x 64.
 // Measured, the general kernel, gemm_f32_tiles at its best tile of 64 x 128 to 32 x 32, and these (us, W bfloat16): 301 rows, 4,096 x 1,024 168, 97
 // and 86; 1,024 x 2,048 150, 88 and 62; 6,144 x 1,024 222, 117 and 117; 1,024 x 3,072 224, 130 and 90; 40 rows, 1,024 x 2,048 72 and 31; 120
@@ -407,6 +407,14 @@ static int launch_f32(const float* A, const void* Wv, float* C, int M, int N, in
   };
   const bool low = M <= 65535 * 32;                        // a grid has room for the rows in tiles of 32
   const float c0 = cost(64, 128, 70.f, 53.f), c1 = cost(64, 64, 36.f, 30.f), c2 = low ? cost(32, 32, 15.6f, 9.2f) : INFINITY;
+  if constexpr (sizeof(TW) == 2) {
+    // Full SMs don't wait for memory, and gemm_f32_tiles widens a number of W once for all threads: 1,024 rows of 5,120 x 1,024 262 us, in stages 272;
+    // 700 of 4,096 x 1,024 150 and 155 (of a float32 W 148 and 146); 640 of 4,096 x 12,288 1,772 and 1,796.  But a W that L2 does not hold comes
+    // from DRAM once more for the tiles beyond the five an SM that are resident: 301 rows of 12,288 x 4,096 857 to 895, in stages 830.
+    const float c3 = cost(64, 64, 60.f, 29.f);
+    const bool once = (long long)N * K <= 40ll << 20 || (long long)((M + 63) / 64) * ((N + 63) / 64) <= 5 * 148;
+    if (once && c3 < fminf(c0, fminf(c1, c2))) return launch_tiles<TW, 64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
+  }
   if (c2 <= fminf(c0, c1)) return launch_stages<TW, 32, 32, 4, 2>(A, W, C, M, N, K, lda, ldw, ldc, s);
   if (c1 <= c0) return launch_stages<TW, 64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
   return launch_tiles<TW, 64, 128, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);

@@ -1,12 +1,11 @@
 """Memories with a scalar decay and 128 keys: the scores of all chunks formed side by side and the chain behind them give the bits of the one launch
 that does both, for rows around a chunk's end, short rows beside long ones, heads in fours and by themselves, columns that do not fill a block, one
 group of columns a block and four, and decays of zero; with values that overflow the same to the last bits."""
-import re
-
 import pytest
 import torch
 
 from arle_b200 import ops
+from launched import launched
 from test_decay_tc_gpu import DEV, _ctx
 
 pytestmark = pytest.mark.gpu
@@ -51,10 +50,5 @@ def test_the_chain_goes_by_the_rows_that_it_runs(H, n):
         q, k, v = (torch.zeros(T, w, device=DEV, dtype=torch.bfloat16) for w in (dim, dim, H * vdim))
         a, b = (torch.ones(T, H, device=DEV) for _ in range(2))
         ctx, state, out = _ctx(lens, H * vdim * dim), torch.zeros(len(lens) + 1, H * vdim * dim, device=DEV), torch.empty(T, H, vdim, device=DEV)
-        ops.decay_memories(q, k, v, a, b, state, ctx, out, H, 1, dim, vdim, False, 1.0)
-        torch.cuda.synchronize()
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
-            ops.decay_memories(q, k, v, a, b, state, ctx, out, H, 1, dim, vdim, False, 1.0)
-            torch.cuda.synchronize()
-        names.append({m.group(0) for m in (re.search(r"decay_rows_tc_kernel<\d+>", e.name) for e in p.events()) if m})
+        names.append(launched(lambda: ops.decay_memories(q, k, v, a, b, state, ctx, out, H, 1, dim, vdim, False, 1.0), r"decay_rows_tc_kernel<\d+>"))
     assert len(names[0]) == 1 and names[0] == names[1]

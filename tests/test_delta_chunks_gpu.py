@@ -1,12 +1,11 @@
 """The gated delta rule in chunks on the tensor cores against float64: lengths around the first row that runs in chunks and around a chunk's
 end, long rows beside short ones, columns that do not fill a block, shared q/k heads; no further off than the scan of whole rows; a row's
 bits do not depend on what stands beside it; decays of zero, and an overflow that stays with the tokens behind it."""
-import re
-
 import pytest
 import torch
 
 from arle_b200 import ops
+from launched import launched
 
 pytestmark = pytest.mark.gpu
 DEV, DIM = "cuda", 128
@@ -141,17 +140,6 @@ def test_lengths_that_are_not_the_rows():
                            scratch=torch.empty(ops.delta_scan_scratch(105, 2, 1), device=DEV), q_lens=lens)
 
 
-def _kernels(run):
-    """The delta rule's kernels that ``run`` launches, with their template arguments."""
-    run()
-    torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
-        run()
-        torch.cuda.synchronize()
-    names = [re.search(r"delta_\w+_kernel(<.*?>(?=\())?", e.name) for e in p.events()]
-    return {m.group(0) for m in names if m}
-
-
 @pytest.mark.parametrize("H,vdim,n", [(8, 128, 2048), (32, 128, 300), (1, 16, 80)])
 def test_launches_go_by_the_rows_that_they_run(H, vdim, n):
     """A long row beside decoded tokens takes the chunks' kernel that it takes by itself, and the decoded tokens the scan that they take by
@@ -161,7 +149,7 @@ def test_launches_go_by_the_rows_that_they_run(H, vdim, n):
         at = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0).to(torch.int32)
         slots, out = torch.arange(len(lens), dtype=torch.int32, device=DEV), torch.empty(sum(lens), H, vdim, device=DEV)
         kw = dict(scratch=torch.empty(ops.delta_scan_scratch(sum(lens), len(lens), H), device=DEV), q_lens=lens) if max(lens) >= 80 else {}
-        return _kernels(lambda: ops.delta_scan(*x, state, at, slots, out, H, H, DIM, vdim, DIM ** -0.5, 1e-6, **kw))
+        return launched(lambda: ops.delta_scan(*x, state, at, slots, out, H, H, DIM, vdim, DIM ** -0.5, 1e-6, **kw), r"delta_\w+_kernel(<.*?>(?=\())?")
 
     alone, decoded, both = step([n]), step([1] * 12), step([n] + [1] * 12)
     assert len(alone) == 2 and len(decoded) == 1 and both == alone | decoded

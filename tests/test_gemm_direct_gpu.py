@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from arle_b200 import ops
+from launched import launched
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -54,13 +55,7 @@ def test_long_shares_go_to_the_ring(M, N, K, direct):
     """Few rows of a long K would leave a warp one block of K after the other; the ring takes K apart over a cluster (up to what it holds)."""
     x, w = (torch.randn(m, K, device=DEV).to(torch.bfloat16) for m in (M, N))
     out = torch.empty(M, N, device=DEV)
-    ops.gemm(x, w, out)
-    torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
-        ops.gemm(x, w, out)
-        torch.cuda.synchronize()
-    names = [e.name for e in p.events()]
-    assert any(("direct_gemm_kernel" if direct else "skinny_gemm_kernel") in n for n in names), names
+    assert launched(lambda: ops.gemm(x, w, out), r"\w+_gemm_kernel") == {"direct_gemm_kernel" if direct else "skinny_gemm_kernel"}
     want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     assert ((out.double() - want).abs() <= K * 2.0 ** -24 * size).all()
     ops.check_errors(DEV)
