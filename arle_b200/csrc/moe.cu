@@ -4,9 +4,9 @@
 //    stand in `groups` equal groups of neighbours, a group's score is the sum of its two largest choice scores (its one
 //    score when a group is a single expert), only experts of the `keep` best groups can be chosen (the others count as
 //    minus infinity); the `top` largest choice scores are chosen and weighted with s * scale (no renormalisation).
-//    Ties go to the lower index.  One thread per token (a warp per token where there are no groups), everything float32.  `mode` bit 0: the scores are a softmax
-//    over all experts instead of sigmoids; bit 1: a group's score is its largest choice score alone; bit 2: the sums z
-//    themselves are the choice scores and the weights are the softmax over the chosen sums alone (times scale).
+//    Ties go to the lower index.  A warp per token for up to 256 experts and 32 groups (a thread per token beyond, and for a softmax over all
+//    experts), everything float32.  `mode` bit 0: the scores are a softmax over all experts instead of sigmoids; bit 1: a group's score is its
+//    largest choice score alone; bit 2: the sums z themselves are the choice scores and the weights are the softmax over the chosen sums alone (times scale).
 //  * moe_plan: sorts the step's (token, choice) pairs by expert (counts, offsets, a place for every pair) and lists
 //    the tiles of 64 places that the grouped product runs, one block of 1,024 threads; nothing goes through the host,
 //    so the step can be captured in a graph.  The order of the pairs inside an expert's run is whatever the
@@ -97,11 +97,12 @@ __global__ void moe_select_kernel(const float* __restrict__ z, int z_stride, con
 }
 
 // The same without softmax over all experts, for the usual sizes: a warp per token, a lane keeps the choice scores of
-// the experts lane, lane + 32, ...; the largest is found by exchanges, ties to the lower index.  With groups a lane forms one group's score
-// from shared memory.  Bound by its chain of exchanges (the kernel above runs a thread's whole token through memory): 32 experts in 4 groups, 64
-// tokens 4.6 us (12.2 there), 2,048 tokens 5.1 (14.3).
+// the experts lane, lane + 32, ...; the largest is found by exchanges, ties to the lower index.  A score that is NaN counts as minus infinity.
+// GROUPS: some are not kept; a lane forms one group's score from shared memory.  (With that code behind a branch 128 experts without groups take 6.4
+// us for 300 tokens, 6.2 without it.)  Bound by its chain of exchanges (the kernel above runs a thread's whole token through memory): 32 experts
+// in 4 groups, 64 tokens 4.1 us (12.6 there), 2,048 tokens 4.8 (14.1).
 constexpr int kSelectWarps = 4;
-template <int PER>
+template <int PER, bool GROUPS>
 __global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride, const float* __restrict__ correction, int E, int top, int groups,
                                        int keep, float scale, int mode, int* __restrict__ ids, float* __restrict__ wts, int num_tokens) {
   pdl_launch_dependents();
@@ -116,8 +117,9 @@ __global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride
     const int e = lane + 32 * i;
     zv[i] = e < E ? zr[e] : 0.f;
     ch[i] = ((mode & 4) ? zv[i] : 1.0f / (1.0f + expf(-zv[i]))) + (correction && e < E ? correction[e] : 0.f);
+    ch[i] = ch[i] == ch[i] ? ch[i] : -INFINITY;         // a NaN would leave the lanes apart
   }
-  if (keep < groups) {
+  if constexpr (GROUPS) {
     __shared__ float scores[kSelectWarps][32 * PER];
     float* sc = scores[threadIdx.x >> 5];
 #pragma unroll
@@ -137,6 +139,7 @@ __global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride
         }
       }
       gs = (per > 1 && !(mode & 2)) ? b1 + b2 : b1;
+      gs = gs == gs ? gs : -INFINITY;
     }
     unsigned kept = 0;
     for (int it = 0; it < keep; ++it) {
@@ -151,7 +154,7 @@ __global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride
           bi = oi;
         }
       }
-      kept |= 1u << __shfl_sync(0xffffffffu, bi, 0);    // one lane's word for all: a NaN may leave them apart
+      kept |= 1u << bi;
     }
 #pragma unroll
     for (int i = 0; i < PER; ++i)
@@ -182,8 +185,6 @@ __global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride
         bi = oi;
       }
     }
-    bi = __shfl_sync(0xffffffffu, bi, 0);
-    bz = __shfl_sync(0xffffffffu, bz, 0);
     if ((bi & 31) == lane) taken |= 1u << (bi >> 5);
     if (it == 0) cm = bz;
     const float w = (mode & 4) ? expf(bz - cm) : scale / (1.0f + expf(-bz));
@@ -202,7 +203,8 @@ ARLE_API int arle_moe_select(const float* z, int z_stride, const float* correcti
   if (num_tokens <= 0) return 0;
   if (E <= 0 || top <= 0 || groups <= 0 || E % groups || keep <= 0 || keep > groups || top > keep * (E / groups)) return ARLE_E_BADARG;
   if (groups <= 32 && !(mode & 1) && E <= 256 && !((mode & 4) && correction)) {
-    auto kernel = E <= 32 ? moe_select_warp_kernel<1> : E <= 64 ? moe_select_warp_kernel<2> : moe_select_warp_kernel<8>;
+    auto kernel = keep < groups ? (E <= 32 ? moe_select_warp_kernel<1, true> : E <= 64 ? moe_select_warp_kernel<2, true> : moe_select_warp_kernel<8, true>)
+                                : (E <= 32 ? moe_select_warp_kernel<1, false> : E <= 64 ? moe_select_warp_kernel<2, false> : moe_select_warp_kernel<8, false>);
     const int warps = num_tokens <= 592 ? 1 : kSelectWarps;
     launch_kernel(kernel, dim3((num_tokens + warps - 1) / warps), dim3(32 * warps), 0, s, 1, z, z_stride, correction, E, top, groups, keep, scale, mode, ids, wts,
                   num_tokens);
