@@ -60,6 +60,7 @@ class GatedDeltaRule(Mixer):
         self.channels = 2 * self.dqk + self.inner               # what the convolution runs over: q | k | v
         self.conv_offset = spec.num_heads * spec.value_dim * spec.key_dim
         self.w_in = self.w_gates = self.w_o = self.conv = self.a_log = self.dt_bias = self.norm = None
+        self.in_chunks = False                                  # whether long prompts run in chunks, which keep something in step buffers
 
     def _name(self, role: str) -> str:
         return self.spec.prefix + self.names[role]
@@ -78,6 +79,7 @@ class GatedDeltaRule(Mixer):
         def kept(*ts):
             return dtype if dtype == torch.bfloat16 else (torch.float32 if any(t.dtype == torch.float32 for t in ts) else torch.bfloat16)
 
+        self.in_chunks = dtype == torch.bfloat16 and self.spec.key_dim == 128 and self.spec.value_dim % 8 == 0
         main = [tensors[self._name(n)] for n in ("q", "k", "v", "gate")]
         self.w_in = torch.cat([m.to(device=device, dtype=kept(*main)) for m in main], dim=0).contiguous()
         small = [tensors[self._name(n)] for n in ("beta", "a")]
@@ -93,8 +95,8 @@ class GatedDeltaRule(Mixer):
         return sum(t.numel() * t.element_size() for t in (self.w_in, self.w_gates, self.w_o))
 
     def scratch_elements_per_token(self):
-        # with long prompts of heads of 128 what a chunk's heads keep: 7,936 float32 numbers, 32 tokens a chunk at the least
-        chunks = 2 * 7936 // 32 * self.spec.num_heads if self.spec.key_dim == 128 else 0
+        # what a chunk's heads keep: 7,936 float32 numbers, 32 tokens a chunk at the least
+        chunks = 2 * 7936 // 32 * self.spec.num_heads if self.in_chunks else 0
         return 2 * (self.channels + self.inner) + 4 * self.inner + 8 * self.spec.num_heads + self.spec.hidden_size + chunks
 
     def state_need(self):

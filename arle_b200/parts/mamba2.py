@@ -61,6 +61,7 @@ class Mamba2(Mixer):
         self.main_rows = self.inner + self.channels          # z, x, B, C
         self.conv_offset = spec.num_heads * spec.head_dim * spec.state_dim
         self.w_in = self.w_o = self.conv = self.conv_bias = self.dt_bias = self.a_log = self.skip = self.norm = None
+        self.in_chunks = False                               # whether long prompts' chunks keep something in step buffers
 
     def _name(self, role: str) -> str:
         return self.spec.prefix + self.names[role]
@@ -79,6 +80,7 @@ class Mamba2(Mixer):
         def kept(t):
             return dtype if dtype == torch.bfloat16 else (torch.float32 if t.dtype == torch.float32 else torch.bfloat16)
 
+        self.in_chunks = dtype == torch.bfloat16 and self.spec.state_dim == 128 and self.spec.head_dim % 8 == 0
         w, o = tensors[self._name("in")], tensors[self._name("o")]
         self.w_in = w.to(device=device, dtype=kept(w)).contiguous()
         self.w_o = o.to(device=device, dtype=kept(o)).contiguous()
@@ -90,8 +92,8 @@ class Mamba2(Mixer):
         return sum(t.numel() * t.element_size() for t in (self.w_in, self.w_o))
 
     def scratch_elements_per_token(self):
-        # with long prompts and 128 keys what a chunk's heads keep: 4,096 float32 numbers, 32 tokens a chunk at the least
-        chunks = 2 * 4096 // 32 * self.spec.num_heads if self.spec.state_dim == 128 else 0
+        # what a chunk's heads keep: 4,096 float32 numbers, 32 tokens a chunk at the least
+        chunks = 2 * 4096 // 32 * self.spec.num_heads if self.in_chunks else 0
         return self.main_rows + self.channels + 3 * self.inner + 6 * self.spec.num_heads + self.spec.hidden_size + chunks
 
     def state_need(self):
