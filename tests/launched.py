@@ -1,15 +1,40 @@
-"""Which kernels of the package a call launches, for tests of what a launcher chooses."""
+"""Which kernels of the package a call launches, for tests of what a launcher chooses: the call is captured in a graph, whose nodes are read."""
+import ctypes
 import re
 
 import torch
 
 
+def _shown(mangled: bytes) -> str:
+    demangle = ctypes.CDLL("libstdc++.so.6").__cxa_demangle
+    demangle.restype = ctypes.c_void_p
+    at = demangle(ctypes.c_char_p(mangled), None, None, ctypes.byref(ctypes.c_int()))
+    return ctypes.string_at(at).decode() if at else mangled.decode()
+
+
 def launched(run, pattern):
-    """The parts of the launched kernels' names (template arguments included) that ``pattern`` matches, after a first call by itself."""
+    """The parts of the kernels' names (template arguments included) that ``pattern`` matches, after a first call by itself."""
+    from cuda.bindings import driver
+
+    def ok(res):
+        assert res[0] == driver.CUresult.CUDA_SUCCESS, res[0]
+        return res[1]
+
     run()
     torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as p:
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
         run()
-        torch.cuda.synchronize()
-    found = (re.search(pattern, e.name) for e in p.events())
-    return {m.group(0) for m in found if m}
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    err, _, count = driver.cuGraphGetNodes(raw)
+    assert err == driver.CUresult.CUDA_SUCCESS
+    found = set()
+    for node in ok(driver.cuGraphGetNodes(raw, count))[:count]:
+        if ok(driver.cuGraphNodeGetType(node)) != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            continue
+        p = ok(driver.cuGraphKernelNodeGetParams(node))
+        name = ok(driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern))
+        m = re.search(pattern, _shown(name))
+        if m:
+            found.add(m.group(0))
+    return found

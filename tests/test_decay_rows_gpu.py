@@ -52,3 +52,9 @@ def test_the_chain_goes_by_the_rows_that_it_runs(H, n):
         ctx, state, out = _ctx(lens, H * vdim * dim), torch.zeros(len(lens) + 1, H * vdim * dim, device=DEV), torch.empty(T, H, vdim, device=DEV)
         names.append(launched(lambda: ops.decay_memories(q, k, v, a, b, state, ctx, out, H, 1, dim, vdim, False, 1.0), r"decay_rows_tc_kernel<\d+>"))
     assert len(names[0]) == 1 and names[0] == names[1]
+
+
+@pytest.mark.parametrize("H,G,vdim", [(128, 8, 40), (24, 6, 200)])      # four groups of columns a block: one block part full, and a last one with one group
+@pytest.mark.parametrize("lens", [[192], [300, 1, 33, 128, 20]], ids=["192", "300-1-33-128-20"])
+def test_four_groups_with_columns_left_over(monkeypatch, H, G, vdim, lens):
+    test_the_bits_of_the_one_launch(monkeypatch, H, G, vdim, lens, "wild")

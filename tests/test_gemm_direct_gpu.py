@@ -59,3 +59,61 @@ def test_long_shares_go_to_the_ring(M, N, K, direct):
     want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     assert ((out.double() - want).abs() <= K * 2.0 ** -24 * size).all()
     ops.check_errors(DEV)
+
+
+# (rows, warps, blocks of K under way): (16, 8, 4), (16, 16, 2), (16, 24, 2), (8, 8, 4), (8, 16, 2), (8, 24, 2); shares of 5 and 6 blocks, of which a second
+# round has one and two, and one whose last warp has fewer
+@pytest.mark.parametrize("M,N,K", [(2, 6144, 1024), (3, 4096, 1024), (1, 3000, 1536), (8, 1152, 544), (4, 1000, 1024), (5, 1000, 1536), (2, 6144, 1344), (8, 1000, 5088)])
+def test_further_cuts(M, N, K):
+    test_direct_products(M, N, K)
+
+
+@pytest.mark.parametrize("M,H,F", [(1, 1024, 3072), (5, 1024, 3072), (8, 256, 4608)])
+def test_products_behind_one_another(M, H, F):
+    """Products that start beside the one in front of them read what it wrote: into a residual, out of its norm factors, a gated pair and into the residual
+    again, with weights that the kernel in front has just written; in stream order, with a wait behind each, and in a graph, over and over."""
+    g = torch.Generator(device=DEV).manual_seed(M + H)
+    x0 = torch.randn(M, F, generator=g, device=DEV).to(torch.bfloat16)
+    w_new = [(torch.randn(*s, generator=g, device=DEV) * s[1] ** -0.5).to(torch.bfloat16) for s in ((H, F), (2 * F, H), (H, F))]
+    gain, r0 = torch.rand(H, generator=g, device=DEV), torch.randn(M, H, generator=g, device=DEV)
+    bf = dict(device=DEV, dtype=torch.bfloat16)
+    ws, gains = [torch.empty_like(w) for w in w_new], torch.empty_like(gain)
+    resid, mid, pair = torch.empty(M, H, device=DEV), torch.empty(M, F, **bf), torch.empty(M, 2 * F, **bf)
+    sinks = [ops.ResidualSink(resid, gains, 1e-6, torch.empty(M, H, **bf), torch.empty(ops.SS_TABLE_SHAPE, device=DEV), 1.0) for _ in range(2)]
+
+    def chain(wait):
+        for t in ws:
+            t.fill_(float("nan"))
+        gains.fill_(float("nan"))
+        resid.copy_(r0)
+        x = x0
+        for i in range(3):
+            gains.copy_(gain)
+            ws[0].copy_(w_new[0])                                # by a kernel that the product stands right behind
+            assert ops.gemm(x, ws[0], None, sink=sinks[0])
+            wait()
+            ws[1].copy_(w_new[1])
+            ops.gemm_silu_mul(ops.ScaledRows(sinks[0].xs, sinks[0].ss, 1e-6), ws[1], pair, mid)
+            wait()
+            ws[2].copy_(w_new[2])
+            assert ops.gemm(mid, ws[2], None, sink=sinks[1])
+            wait()
+            x = mid
+        return [t.clone() for t in (resid, sinks[1].xs, sinks[1].ss, mid)]
+
+    want = chain(torch.cuda.synchronize)
+    assert torch.isfinite(want[0]).all()
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(want, chain(lambda: None)))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        chain(lambda: None)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(lambda: None)
+    for _ in range(20):
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
+    ops.check_errors(DEV)
