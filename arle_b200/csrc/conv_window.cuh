@@ -14,12 +14,11 @@ constexpr int kConvTokens = 16, kConvAhead = 4, kConvThreads = 128, kConvVec = 4
 
 // in_bias is added to a row's inputs (not to what the state holds); act 1: silu.
 template <typename TI, typename TO, int VEC>
-__global__ void __launch_bounds__(kConvThreads, sizeof(TI) + sizeof(TO) == 4 ? 6 : 5) conv_window_kernel(const TI* __restrict__ x, int x_stride, const float* __restrict__ in_bias,
-                                                                   const float* __restrict__ w, const float* __restrict__ out_bias, int act,
-                                                                   const float* __restrict__ state, long slot_stride, long conv_off,
-                                                                   const int* __restrict__ q_indptr, const int* __restrict__ row_of_token,
-                                                                   const int* __restrict__ state_slots, TO* __restrict__ out, int out_stride, int T,
-                                                                   int C) {
+__global__ void __launch_bounds__(kConvThreads, sizeof(TI) + sizeof(TO) == 4 ? 6 : 5)
+    conv_window_kernel(const TI* __restrict__ x, int x_stride, const float* __restrict__ in_bias, const float* __restrict__ w,
+                       const float* __restrict__ out_bias, int act, const float* __restrict__ state, long slot_stride, long conv_off,
+                       const int* __restrict__ q_indptr, const int* __restrict__ row_of_token, const int* __restrict__ state_slots,
+                       TO* __restrict__ out, int out_stride, int T, int C) {
   pdl_launch_dependents();
   pdl_wait();
   const int c = (blockIdx.x * kConvThreads + threadIdx.x) * VEC;

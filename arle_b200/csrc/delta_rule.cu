@@ -21,8 +21,9 @@
 //    run.  What bounds one long row is the chain of a token: loads from shared memory, four dependent FMAs, three exchanges, the correction
 //    and the update, some 480 cycles.  Several rows also wait for a place: blocks of 128 or 256 threads, two a SM, taken in the order of the
 //    rows.  One row of 2,048 tokens, 8 heads of 128 x 128: 511 us (single numbers, loads waited for at each chunk: 682); 32 heads 652 (805);
-//    rows of 479, 701 and 819 tokens, 32 heads: 549 (612).  The split of a column depends on dim alone, so a token's sums have one order
-//    whatever the cutting or the batch.  bfloat16 rows of 80 tokens and more with heads of 128 run in delta_tc.cu.
+//    rows of 479, 701 and 819 tokens, 32 heads: 549 (612).  The split of a column depends on dim alone, so a token's sums over the memory
+//    have one order whatever the cutting or the batch; its lengths are added up by as many threads as a block has, 128 or 256, which goes by
+//    the step's rows.  bfloat16 rows of 80 tokens and more with heads of 128 run in delta_tc.cu.
 #include "common.cuh"
 #include "scan_utils.cuh"
 using namespace arle;
@@ -298,8 +299,8 @@ static int launch_delta(const void* q, const void* k, const void* v, int q_strid
   // rows of 128: 903 and 813).
   constexpr bool kMay = LONG && !(sizeof(T) == 4 && EPL * LPC == 512), kWide = sizeof(T) == 4 && EPL == 32;
   const long blocks = (long)((vdim + cpb - 1) / cpb) * H * R;
-  const bool ahead = (num_tokens >= 8L * R || num_tokens - R >= 8 * kDeltaChunk) && (!kWide || blocks * threads <= 148L * 256) && dim % per == 0 && q_stride % per == 0 &&
-                     k_stride % per == 0 && (((uintptr_t)q | (uintptr_t)k) & 15) == 0;
+  const bool ahead = (num_tokens >= 8L * R || num_tokens - R >= 8 * kDeltaChunk) && (!kWide || blocks * threads <= 148L * 256) && dim % per == 0 &&
+                     q_stride % per == 0 && k_stride % per == 0 && (((uintptr_t)q | (uintptr_t)k) & 15) == 0;
   auto kernel = kMay && ahead ? delta_scan_kernel<T, EPL, LPC, LONG, kMay> : delta_scan_kernel<T, EPL, LPC, LONG, false>;
   if (smem > 40 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -312,8 +313,8 @@ static int launch_delta(const void* q, const void* k, const void* v, int q_strid
 }
 
 // q, k [T, kq_heads*dim] and v [T, H*vdim] in the activation type (row strides given); beta, decay float32 [T, H]; state:
-// float32, a slot every slot_stride numbers, [H][vdim][dim] at its start; out float32 [T, H, vdim]; num_tokens: T, all rows'.  longest > 0:
-// rows of more tokens are left alone (arle_delta_tc runs them).
+// float32, a slot every slot_stride numbers, [H][vdim][dim] at its start; out float32 [T, H, vdim].  longest > 0: rows of more
+// tokens are left alone (arle_delta_tc runs them).  num_tokens: of the rows that run here, and one for each of the others; the form goes by it.
 ARLE_API int arle_delta_scan(const void* q, const void* k, const void* v, int dtype, int q_stride, int k_stride, int v_stride,
                              const float* beta, const float* decay, float* state, long slot_stride, const int* q_indptr,
                              const int* state_slots, float* out, int num_tokens, int R, int H, int kq_heads, int dim, int vdim,

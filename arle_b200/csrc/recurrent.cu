@@ -610,8 +610,9 @@ ARLE_API int arle_gated_group_norm(const float* y, const void* x, int dtype, int
     auto kernel = width <= 2048   ? gated_group_norm_vec_kernel<__nv_bfloat16, 1, 256, 0>
                   : width <= 4096 ? gated_group_norm_vec_kernel<__nv_bfloat16, 2, 256, 0>
                   : width <= 6144 ? gated_group_norm_vec_kernel<__nv_bfloat16, 2, 384, 4> : gated_group_norm_vec_kernel<__nv_bfloat16, 2, 512, 3>;
-    launch_kernel(kernel, dim3(num_tokens, parts), dim3(width <= 4096 ? 256 : width <= 6144 ? 384 : 512), 0, s, 1, y, (const __nv_bfloat16*)x, x_stride, skip, vdim, (const __nv_bfloat16*)z,
-                  z_stride, weight, eps, (__nv_bfloat16*)out, out_stride, inner, width);
+    const int width_threads = width <= 4096 ? 256 : width <= 6144 ? 384 : 512;
+    launch_kernel(kernel, dim3(num_tokens, parts), dim3(width_threads), 0, s, 1, y, (const __nv_bfloat16*)x, x_stride, skip, vdim,
+                  (const __nv_bfloat16*)z, z_stride, weight, eps, (__nv_bfloat16*)out, out_stride, inner, width);
     return launch_status();
   }
   if (dtype == 0)

@@ -175,10 +175,13 @@ def check_errors(device) -> None:
 
 
 def set_programmatic_launch(on) -> None:
-    """Programmatic dependent launch (off by default): a kernel may be scheduled, set up
-    its barriers and prefetch weights while the kernel before it finishes, and waits
-    for that kernel only before touching its results.  True or 1: every kernel; 2: the
-    weight-streaming products only."""
+    """Programmatic dependent launch: a kernel may be scheduled, set up its barriers and
+    prefetch weights while the kernel before it finishes, and waits for that kernel only
+    before touching its results.  True or 1: every kernel; 2: the weight-streaming
+    products; 0 (the default): only the small decode products that read their weights
+    straight from memory (up to 8 rows), which are launched so whatever is set here: a
+    0.6B layer's four take 12.7 us instead of 15.4, where larger kernels find no room
+    beside one another and lose."""
     lib = library()
     lib.arle_set_programmatic_launch.argtypes = [c_int]
     lib.arle_set_programmatic_launch.restype = None
@@ -1519,9 +1522,10 @@ def decay_memories(q, k, v, a, b, state, batch, out, heads: int, kq_heads: int, 
     n = decay_rows_chunks(batch, dim, ones_column)
     if n:
         scratch = batch.ws.get("decay_tiles", (n * heads * 4096,), torch.float32)
+        long_rows = sum(t > DECAY_TC_LONGEST for t in batch.q_lens)
         _check(library().arle_decay_rows_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(a), _ptr(b), _ptr(state),
-                                            state.stride(0), _ptr(batch.q_indptr), _ptr(batch.state_slots), _ptr(out), _ptr(scratch), n,
-                                            sum(t > DECAY_TC_LONGEST for t in batch.q_lens), batch.num_rows, heads, kq_heads, vdim, float(q_scale), DECAY_TC_LONGEST, _stream()), "decay_rows_tc")
+                                            state.stride(0), _ptr(batch.q_indptr), _ptr(batch.state_slots), _ptr(out), _ptr(scratch), n, long_rows,
+                                            batch.num_rows, heads, kq_heads, vdim, float(q_scale), DECAY_TC_LONGEST, _stream()), "decay_rows_tc")
         return
     _check(library().arle_decay_tc(_ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(a), _ptr(b), _ptr(state), state.stride(0),
                                    _ptr(batch.q_indptr), _ptr(batch.state_slots), _ptr(out), batch.num_rows, heads, kq_heads, dim, vdim, vcols,
@@ -2055,8 +2059,9 @@ def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: i
     heads * vdim * dim numbers are the memories, a head's transposed ([heads][vdim][dim]); out float32 [T, heads, vdim].
 
     With ``scratch`` (float32, ``delta_scan_scratch`` numbers; where ``delta_scan_takes_chunks`` says so) rows of 80 tokens and more run in chunks
-    on the tensor cores, for beta and decays in [0, 1] as ``delta_gates`` makes them.  Every row runs whatever the other two say: ``q_lens``, the rows' lengths on the host,
-    spares the launch for short rows where there are none; a ``max_q_len`` of 1 to 79 sends all rows to the scan."""
+    on the tensor cores, for beta and decays in [0, 1] as ``delta_gates`` makes them (with beta near 2, one key over and over and no decay they
+    are off from float64 by 3e-6, the scan by 5e-7).  Every row runs whatever the other two say: by ``q_lens``, the rows' lengths on the host, the
+    launches go by the rows that they run; a ``max_q_len`` of 1 to 79 sends all rows to the scan."""
     T = v.shape[0]
     R = state_slots.numel()
     if (q.shape != (T, kq_heads * dim) or k.shape != q.shape or v.shape != (T, heads * vdim) or q.dtype != k.dtype
