@@ -1519,7 +1519,7 @@ def decay_memories(q, k, v, a, b, state, batch, out, heads: int, kq_heads: int, 
         raise KernelError(f"decay_memories: state {tuple(state.shape)} must be float32 [slots, >= {heads * vcols * dim}]")
     if out.dtype != torch.float32 or tuple(out.shape) != (T, heads, vcols) or not out.is_contiguous():
         raise KernelError("decay_memories: out must be contiguous float32 [T, heads, vcols]")
-    n = decay_rows_chunks(batch, dim, ones_column)
+    n = decay_rows_chunks(batch, dim, ones_column, heads * -(-vdim // 16))
     if n:
         scratch = batch.ws.get("decay_tiles", (n * heads * 4096,), torch.float32)
         long_rows = sum(t > DECAY_TC_LONGEST for t in batch.q_lens)
@@ -1532,13 +1532,19 @@ def decay_memories(q, k, v, a, b, state, batch, out, heads: int, kq_heads: int, 
                                    float(q_scale), DECAY_TC_LONGEST, _stream()), "decay_tc")
 
 
-def decay_rows_chunks(batch, dim: int, ones_column: bool) -> int:
+def decay_rows_chunks(batch, dim: int, ones_column: bool, groups: int = 0) -> int:
     """The chunks of 64 tokens of a step's long rows, where ``decay_memories`` forms their scores side by side (4,096 float32 numbers of scratch a
-    chunk and head; 32 tokens a chunk at the least, which the mixers count); 0: one launch does it all.  The same bits either way, so the longest
-    row may decide: from three full chunks on the shorter chain gains more than the second launch costs."""
+    chunk and head; 32 tokens a chunk at the least, which the mixers count); 0: one launch does it all.  ``groups``: of 16 columns, of all heads
+    together.  The same bits either way, so the step may decide: from four full chunks on the shorter chain gains more than the second launch costs
+    (one row of 256 tokens, 32 heads of 64 columns 25 us and 30, 64 29 and 30, 128 38 and 38; four of them, 32 heads 38 and 38).  With three it does
+    while every group finds an SM (one row of 192, 32 heads 22.7 and 23.1), and once the one launch's blocks of four groups don't (256 heads 51 and
+    57; 12 rows of 200, 32 heads 81 and 100), but not in between (64 heads 26.2 and 23.4, 128 32.2 and 29.4; three rows, 32 heads 32.5 and 29.2)."""
     if dim != 128 or ones_column or batch.max_q_len < 3 * DECAY_CHUNK:
         return 0
-    n = sum(-(-t // DECAY_CHUNK) for t in batch.q_lens if t > DECAY_TC_LONGEST)
+    long = [t for t in batch.q_lens if t > DECAY_TC_LONGEST]
+    if batch.max_q_len < 4 * DECAY_CHUNK and 1 < groups * len(long) / sm_count(batch.device) <= 4:
+        return 0
+    n = sum(-(-t // DECAY_CHUNK) for t in long)
     return n if 32 * n <= batch.num_tokens else 0
 
 

@@ -55,6 +55,18 @@ def test_the_chain_goes_by_the_rows_that_it_runs(H, n):
 
 
 @pytest.mark.parametrize("H,G,vdim", [(128, 8, 40), (24, 6, 200)])      # four groups of columns a block: one block part full, and a last one with one group
-@pytest.mark.parametrize("lens", [[192], [300, 1, 33, 128, 20]], ids=["192", "300-1-33-128-20"])
+@pytest.mark.parametrize("lens", [[256], [300, 1, 33, 128, 20]], ids=["256", "300-1-33-128-20"])
 def test_four_groups_with_columns_left_over(monkeypatch, H, G, vdim, lens):
     test_the_bits_of_the_one_launch(monkeypatch, H, G, vdim, lens, "wild")
+
+
+@pytest.mark.parametrize("H,lens,split", [(32, [192], True), (64, [192], False), (64, [256], True), (32, [192] * 3, False), (32, [200] * 12, True),
+                                          (8, [192] + [1] * 60, True), (128, [191, 257], True)])
+def test_which_steps_are_split(H, lens, split):
+    """Four chunks and more always; three while every group of columns of the rows that run finds an SM, and once blocks of four groups don't."""
+    dim, vdim, T = 128, 64, sum(lens)
+    q, k, v = (torch.zeros(T, w, device=DEV, dtype=torch.bfloat16) for w in (dim, dim, H * vdim))
+    a, b = (torch.ones(T, H, device=DEV) for _ in range(2))
+    ctx, state, out = _ctx(lens, H * vdim * dim), torch.zeros(len(lens) + 1, H * vdim * dim, device=DEV), torch.empty(T, H, vdim, device=DEV)
+    ran = launched(lambda: ops.decay_memories(q, k, v, a, b, state, ctx, out, H, 1, dim, vdim, False, 1.0), r"decay\w*_tc_kernel")
+    assert ran == {"decay_rows_tc_kernel" if split else "decay_tc_kernel"}
