@@ -7,8 +7,9 @@
 // decay_rows_tc: a block has a head and 16 G columns of v for a whole row, four warps 16 columns; the groups share the chunk's q and k and
 // nothing else.  A warp forms the rows of a tile of 16 tokens and holds 32 rows of S.  A chunk has one barrier for the block and one for the group.
 // What bounds it: a block's chain of chunks, some 5 us each with four groups (the one launch: 9) and 2.2 with one; decay_tiles takes some 15 us of
-// 2,048 tokens.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 199 us (decay_tc 295), 32 heads 84 (216); three rows of 600 to 748 210
-// (301) and 80 (105); 300 tokens, 32 heads 29 (37); 100 tokens 23 (17), with 128 heads 29 (21).
+// 2,048 tokens, 35 with 128 heads.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 197 us (decay_tc 294), 32 heads 81 (215); three rows of
+// 600 to 748 207 (300) and 78 (104); 300 tokens, 32 heads 26.5 (35.6).  For heads of 128 alone, the size of the Mamba-2 layers that run prompts; other
+// sizes and a column of ones stay with the one launch.
 #include "common.cuh"
 #include "chunk_parts.cuh"
 using namespace arle;
@@ -388,8 +389,8 @@ ARLE_API int arle_decay_rows_tc(const void* q, const void* k, const void* v, int
   const int heads = H / kq_heads % kMostHeads == 0 ? kMostHeads : 1;
   launch_kernel(decay_tiles_kernel, dim3(num_chunks, H / heads), dim3(128), sizeof(TilesSmem), s, 1, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
                 (long)q_stride, (long)k_stride, a, b, q_indptr, R, longest, H, kq_heads, heads, q_scale, chunks);
-  // one group a block while two of them an SM hold all columns of the rows that run here (32 heads of 64 columns, 2,048 tokens: 84 us, with four
-  // groups 179), four beyond (128 heads: 226 with one or two groups, 199)
+  // one group a block while two of them an SM hold all columns of the rows that run here (32 heads of 64 columns, 2,048 tokens: 81 us, with four
+  // groups 179), four beyond (128 heads: 226 with one or two groups, 197)
   if ((long)((vdim + 15) / 16) * H * long_rows <= 296)
     return launch<1>(q, k, v, q_stride, k_stride, v_stride, chunks, state, slot_stride, q_indptr, state_slots, out, R, H, kq_heads, vdim, longest, s);
   return launch<4>(q, k, v, q_stride, k_stride, v_stride, chunks, state, slot_stride, q_indptr, state_slots, out, R, H, kq_heads, vdim, longest, s);

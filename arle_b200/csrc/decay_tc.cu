@@ -15,7 +15,7 @@
 //
 // Per chunk, eight warps: scores 16 rows x 64 (two warps each, half the columns of v), read-out of S_0 from its three parts in
 // shared memory, weighted scores times v, and the update, where a warp holds 16 (or 32) rows of S.
-// With 128 keys and no column of ones, steps with rows of three chunks and more take decay_rows_tc.cu, which has the same bits.
+// With 128 keys and no column of ones, most steps with rows of three chunks and all with four take decay_rows_tc.cu, which has the same bits.
 // Rows of up to `longest` tokens are left alone (the scan runs them).  A token's sums have one order for its place in its row, whatever
 // else is in the step; where a prompt is cut shows in the last bits.
 //
@@ -24,8 +24,8 @@
 //
 // What bounds it: the chain of chunks of a block (some 9 us each: the tensor cores' legacy path, a third of the time, then the matrix
 // loads and the barriers between the phases), with one block an SM.  A scheduler has two warps; one takes an early tile of rows and the other a
-// late one, which sees more keys.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 284 us (306 with two early or two late ones, the
-// scan 1,162), 8 heads of 256 x 513 305 us (326; 1,740 to 1,937 as the scan's mean of both).
+// late one, which sees more keys.  One row of 2,048 tokens: 128 heads of 128 x 64 in 8 groups 294 us (315 with two early or two late ones, the
+// scan 1,162), 8 heads of 256 x 513 304 us (325; 1,740 to 1,937 as the scan's mean of both).
 #include "common.cuh"
 #include "chunk_parts.cuh"
 using namespace arle;

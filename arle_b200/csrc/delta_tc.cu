@@ -23,7 +23,8 @@
 //
 // What bounds it: a block's chain of chunks, some 4 us each with one group and 6 with two (four phases with a barrier between them, the tensor
 // cores' legacy path about half of the time); delta_chunks takes some 20 us of a step of 2,000 tokens.  Rows of 819, 701 and 479 tokens, 32 heads
-// of 128 x 128: 219 us (the scan 530); one row of 2,048 218 (651), with 8 heads 138 (515); 300 tokens, 8 heads 37 (81).
+// of 128 x 128: 216 us (the scan 530); one row of 2,048 216 (650), with 8 heads 135 (510); 300 tokens, 8 heads 34 (79).  For keys of 128 alone, the size
+// of the layers that run prompts; others are scanned.
 #include "common.cuh"
 #include "chunk_parts.cuh"
 using namespace arle;

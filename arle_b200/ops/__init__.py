@@ -2101,7 +2101,8 @@ def delta_scan(q, k, v, beta, decay, state, q_indptr, state_slots, out, heads: i
 
 
 # Rows of the delta rule up to this length are scanned, also where longer rows run in chunks: a row's own length decides.  One row, 8 heads of 128:
-# 64 tokens 21 us scanned and 24 in chunks, 128 tokens 37 and 27; 32 heads 25 and 24, four rows of 80 83 and 63.
+# 80 tokens 24.4 us scanned and 23.7 in chunks, 96 27.2 and 24.2, 128 35.9 and 24.3; 32 heads 30 and 26, 35 and 27, 45 and 27; four rows of 80 83 and 61.
+# A step with rows on both sides pays for both launches: 8 heads, one row of 80 beside eight of one token 28.4 (24.6 all scanned), beside 25 of 79 147 (124).
 DELTA_SCAN_LONGEST = 79
 
 
