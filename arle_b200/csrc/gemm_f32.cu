@@ -9,7 +9,7 @@
 // kernel set runs it for every projection, so that a bfloat16 discrepancy can be put
 // down to the fast kernels or to the arithmetic.
 //
-// float32 A runs on one of four kernels, all with that order of sums, so all with the same bits:
+// float32 A runs on one of four kernels (but for bfloat16 W with K from 512 on in whole blocks of 64: gemm_f32_tc.cu), all with that order of sums, so all with the same bits:
 //  * gemm_f32_rows (up to 16 rows): a thread per column of C, W staged by cp.async.  Bound by W's bytes for one row, by the loads from
 //    shared memory for more.
 //  * gemm_f32_stages: tiles of 32 x 32 and 64 x 64, stages of 32 numbers of k as they lie in memory on their way by cp.async, three ahead.  For

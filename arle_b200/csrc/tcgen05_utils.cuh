@@ -155,6 +155,35 @@ inline int tensor_map_2d_bf16(const void* ptr, long long rows, int cols, int ld,
   return 0;
 }
 
+// Tensor map of a row-major [rows, cols] float32 matrix (row stride ld elements): boxes of box_rows x 64 elements, rows of 256 bytes one
+// after the other, zero fill out of bounds.  Cached per matrix.
+inline int tensor_map_2d_f32(const void* ptr, long long rows, int cols, int ld, int box_rows, CUtensorMap* out) {
+  static std::unordered_map<TensorMapKey, CUtensorMap, TensorMapKeyHash> cache;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  const TensorMapKey key{ptr, rows, cols, ld, box_rows};
+  auto it = cache.find(key);
+  if (it != cache.end()) {
+    *out = it->second;
+    return 0;
+  }
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return ARLE_E_UNSUPPORTED;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUtensorMap m;
+  CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return ARLE_E_BADARG;
+  if (cache.size() > 8192) cache.clear();
+  cache.emplace(key, m);
+  *out = m;
+  return 0;
+}
+
 // Tensor map of a cache [rows, hd] bfloat16 (hd a multiple of 64) seen as [hd / 64, rows, 64]:
 // a box is 16 rows of the whole head and lands as hd / 64 blocks of [16 rows x 128 bytes],
 // each 128-byte swizzled, one after the other.  Cached per cache.

@@ -6,8 +6,9 @@ tensors the caller provides; nothing here allocates device memory.  There is no
 CPU path: the first call loads the library (building it when needed) and raises
 if that fails or if a tensor is not on a CUDA device.
 
-Matrix products: the float32 path uses the package's own FFMA kernel
-(``gemm_f32.cu``: true 32-bit, fixed summation order).  The bfloat16 path has two
+Matrix products: the float32 path uses the package's own kernels (true 32-bit, fixed
+summation order): ``gemm_f32_tc.cu`` for bfloat16 weights with long rows, on the tensor cores
+in three exact pieces, FFMA (``gemm_f32.cu``) otherwise.  The bfloat16 path has two
 kernels of its own: weight streaming for up to 8 rows (``gemm_skinny.cu``, every
 decode step of up to 8 requests) and tcgen05 / TMA / TMEM for many rows
 (``gemm_tcgen05.cu``, switched on with ``set_tcgen05_min_rows``).  Otherwise it calls
@@ -79,6 +80,7 @@ _SIGNATURES = {
     "arle_paged_attention_prefill_tc": [_P, _I, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _P, _P, _I, _I,
                                         _I, _I, _I, _P, _I, _F, _I, _P, _P],
     "arle_gemm_f32": [_P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P],
+    "arle_gemm_f32_tc": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _P, _P],
     "arle_gemm_plain_bf16": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
     "arle_gemm_skinny": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _P],
     "arle_gemm_skinny_gated": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _P],
@@ -425,6 +427,10 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, sink: "ResidualSink" = None) -> 
     if x.dtype == torch.float32:
         if out.dtype != torch.float32 or x.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
             raise KernelError("gemm: the float32 path takes float32 activations with unit inner stride")
+        if f32_pieces_supported(x, w):
+            _check(library().arle_gemm_f32_tc(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K,
+                                              _ptr(error_flag(x.device)), _stream()), "gemm_f32_tc")
+            return False
         _check(library().arle_gemm_f32(_ptr(x), _ptr(w), _dt(w), _ptr(out), M, N, K, x.stride(0), w.stride(0),
                                        out.stride(0), _stream()), "gemm_f32")
         return False
@@ -451,6 +457,16 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, sink: "ResidualSink" = None) -> 
     else:
         raise KernelError(f"gemm: output type {out.dtype}")
     return False
+
+
+def f32_pieces_supported(x, w) -> bool:
+    """Whether a product of float32 rows runs on the tensor cores in three exact bfloat16 pieces (``gemm_f32_tc.cu``): a bfloat16 w, K a multiple
+    of 64 and at least 512, N at least 256, rows on 16-byte boundaries.  Sizes of w alone decide, never the number of rows, so that a
+    token's bits do not depend on how its prompt was cut.  Shorter sums are done sooner by the FFMA kernels (one row of 4,096 x 256 8.4 us, 9.4 in
+    pieces), and a few columns fill too few of the tiles of 128."""
+    N, K = w.shape
+    return (_KERNEL_SET == "fast" and w.dtype == torch.bfloat16 and K >= 512 and K % 64 == 0 and N >= 256 and x.stride(0) % 4 == 0
+            and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 _TCGEN05_MIN_ROWS = 1 << 30
