@@ -276,7 +276,6 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(
     int bt_width, int page_size, int ps_shift, float scale_log2, HeadTail<__nv_bfloat16> tail, int window, int stages, Prep prep, const int* __restrict__ plan,
     int* __restrict__ err) {
   pdl_launch_dependents();
-  pdl_wait();
   constexpr uint32_t OPERAND = kTile * HD * 2;            // bytes of the keys (or the values) of one stage
   constexpr uint32_t STAGE = 2 * OPERAND;
   constexpr uint32_t BOX = 16 * HD * 2;                   // bytes of one box: 16 keys, as HD / 64 blocks of [16 x 128 bytes]
@@ -314,6 +313,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(
     const CUtensorMap* m = warp > kConsumerWarps ? &map_v : &map_k;
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(m) : "memory");
   }
+  pdl_wait();
   __shared__ int plan_units, plan_per;
   int first_pages = 0;                                    // a producer lane's page id of the CTA's first piece (with a plan)
   if (plan) {
@@ -650,22 +650,23 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(
         consumer_sync();
         if (is_last) {
           __threadfence();
+          constexpr int kAtOnce = 16;                          // pieces whose loads are in flight together
           const size_t base = (size_t)first_cta * G;
           for (int i = tid; i < G * HD / 2; i += kConsumers) {
             const int row = i / (HD / 2), d = (i % (HD / 2)) * 2;
             const float2* po = reinterpret_cast<const float2*>(part_o + (base + row) * HD + d);
             const float2* pml = reinterpret_cast<const float2*>(part_ml) + base + row;
             float M = -INFINITY, L = 0.f, O0 = 0.f, O1 = 0.f;
-            for (int sp0 = 0; sp0 < pieces; sp0 += 8) {        // eight pieces' loads in flight together
-              float2 ml[8], ov[8];
+            for (int sp0 = 0; sp0 < pieces; sp0 += kAtOnce) {
+              float2 ml[kAtOnce], ov[kAtOnce];
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
+              for (int k = 0; k < kAtOnce; ++k) {
                 const int sp = min(sp0 + k, pieces - 1);
                 ml[k] = __ldcg(pml + (size_t)sp * G);
                 ov[k] = __ldcg(po + (size_t)sp * G * HD / 2);
               }
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
+              for (int k = 0; k < kAtOnce; ++k) {
                 if (sp0 + k < pieces && ml[k].y > 0.f) {
                   const float Mn = fmaxf(M, ml[k].x);
                   const float c = exp2f(M - Mn), f = exp2f(ml[k].x - Mn);
@@ -720,10 +721,20 @@ int launch_stream(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, i
   int stages = (int)(((size_t)max_smem - fixed) / stage);
   if (stages > kMaxStages) stages = kMaxStages;
   stages &= ~1;
+  // No more stages than a CTA can have tiles, and no more than four in front of a small product (up to 8 rows, whose heads are 2,048 numbers at
+  // most: gemm_skinny.cu reads such weights without a ring) while there are few tiles: the product's blocks start in the shared memory that
+  // is left, before this kernel has ended.  Steps of 8 layers of Qwen3-0.6B sizes, us, six stages, four and two: one request of 100 tokens
+  // 269, 250 and 249, four of 1,000 300, 274 and 284, eight of 300 311, 274 and 284, eight of 2,048 (14 tiles a CTA) 380, 349 and 400.  Nothing
+  // starts beside it at 8B sizes: eight requests of 2,048 tokens 828, 836 and 886.
+  const long long row_tiles = ((long long)bt_width * page_size + kTile - 1) / kTile, per = (row_tiles * rows * nkv + ctas - 1) / ctas;
+  if (rows <= 8 && nq * HD <= 2048 && per <= 32 && stages > 4) stages = 4;
+  if (per < stages) stages = per <= 2 ? 2 : (int)((per + 1) & ~1ll);
   const size_t smem = fixed - kStaticSmem + (size_t)stages * stage;
   e = cudaFuncSetAttribute(decode_stream_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - kStaticSmem);
   if (e != cudaSuccess) return (int)e;
-  e = launch_kernel(decode_stream_kernel<HD>, dim3(ctas), dim3(kThreads), smem, s, 1, mk, mv, (const __nv_bfloat16*)q,
+  // A step that decodes only (it prepares its heads here) is a chain of short kernels: this one starts as soon as the one in front has started
+  // its last block.  Behind a prompt portion's attention it would only hold SMs while it waits (a mixed layer 185 us instead of 181).
+  e = launch_kernel_as(prep.on != 0 || (pdl_enabled() & 1) != 0, decode_stream_kernel<HD>, dim3(ctas), dim3(kThreads), smem, s, 1, mk, mv, (const __nv_bfloat16*)q,
                     q_row_stride, (__nv_bfloat16*)out, q_indptr, kv_lens, block_table, bt_stride, part_o, part_ml, counters,
                     rows, nq, nkv, bt_width, page_size, ps_shift, scale * 1.4426950408889634f, tail, window, stages, prep, plan, err);
   if (e != cudaSuccess) return (int)e;
