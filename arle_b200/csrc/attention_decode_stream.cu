@@ -133,7 +133,7 @@ constexpr int kPlanHeader = 4;               // units, units per CTA, shared out
 
 // The rows' table and the CTAs' shares, by all threads of a block (kThreads of them).  prefix [R + 1], kvl [R], tok [R]
 // and the scalars are in shared memory; the scalars own_* are those of CTA `cta`.  Ends with a barrier.
-__device__ __forceinline__ void stream_shares(const int* __restrict__ q_indptr, const int* __restrict__ kv_lens, int R, int nkv,
+__device__ __forceinline__ void stream_shares(const int* q_indptr, const int* kv_lens, int R, int nkv,
                                               int window, int C, int cta, int* prefix, int* kvl, int* tok, int* units_out,
                                               int* per_out, int* by_pair_out, int* own_row_out, int* own_first_out,
                                               int* own_k_out) {
@@ -267,14 +267,14 @@ __global__ void __launch_bounds__(kThreads) decode_stream_plan_kernel(const int*
   }
 }
 
+// Plain loads, and no promise that an array is read alone: the kernel lives beside the one in front of it, which writes what it reads, and the
+// non-coherent path is for memory that nobody writes while a kernel lives.
 template <int HD>
 __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-    const __nv_bfloat16* __restrict__ q, int q_row_stride, __nv_bfloat16* __restrict__ out,
-    const int* __restrict__ q_indptr, const int* __restrict__ kv_lens, const int* __restrict__ block_table, int bt_stride,
-    float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ counters, int R, int nq, int nkv,
-    int bt_width, int page_size, int ps_shift, float scale_log2, HeadTail<__nv_bfloat16> tail, int window, int stages, Prep prep, const int* __restrict__ plan,
-    int* __restrict__ err) {
+    const __nv_bfloat16* q, int q_row_stride, __nv_bfloat16* out, const int* q_indptr, const int* kv_lens, const int* block_table, int bt_stride,
+    float* part_o, float* part_ml, int* counters, int R, int nq, int nkv,
+    int bt_width, int page_size, int ps_shift, float scale_log2, HeadTail<__nv_bfloat16> tail, int window, int stages, Prep prep, const int* plan, int* err) {
   pdl_launch_dependents();
   constexpr uint32_t OPERAND = kTile * HD * 2;            // bytes of the keys (or the values) of one stage
   constexpr uint32_t STAGE = 2 * OPERAND;
@@ -365,14 +365,14 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stream_kernel(
       // Page ids come 32 at a time, one per lane, and a second 32 ahead of them, so that no
       // tile waits for a read of the block table; a lane picks its page with a shuffle.
       int p0 = page_index(tile0 * kTile);
-      int cur = (plan && u == u0) ? first_pages : __ldg(bt + min(p0 + lane, bt_width - 1));
-      int nxt = __ldg(bt + min(p0 + 32 + lane, bt_width - 1));
+      int cur = (plan && u == u0) ? first_pages : bt[min(p0 + lane, bt_width - 1)];
+      int nxt = bt[min(p0 + 32 + lane, bt_width - 1)];
       int key0 = tile0 * kTile + c * 16;
       for (int i = 0; i < ntile; ++i) {
         while (page_index(key0 - c * 16) - p0 >= 32) {
           cur = nxt;
           p0 += 32;
-          nxt = __ldg(bt + min(p0 + 32 + lane, bt_width - 1));
+          nxt = bt[min(p0 + 32 + lane, bt_width - 1)];
         }
         const bool active = wanted(key0);
         const int pi = page_index(key0);

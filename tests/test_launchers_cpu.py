@@ -33,3 +33,14 @@ def test_kernels_that_always_start_early_read_plainly():
     body = re.sub(r"//[^\n]*", "", text[first:last])
     assert "direct_gemm_kernel(" in body and "pdl_wait();" in body
     assert not re.search(r"\.nc\b|__ldg\(", body)
+
+
+def test_the_streamed_decode_attention_starts_early_and_reads_plainly():
+    text = (CSRC / "attention_decode_stream.cu").read_text()
+    assert "launch_kernel_as(prep.on != 0" in text
+    kernel = text[text.index("decode_stream_kernel("): text.index("size_t fixed_smem(")]
+    for part in (kernel, text[text.index("void prep_head("): text.index("constexpr int kPlanHeader")], text[text.index("void stream_shares("): text.index("void own_units(")]):
+        body = re.sub(r"//[^\n]*", "", part)
+        assert not re.search(r"\.nc\b|__ldg\(|__restrict__", body)
+    body = re.sub(r"//[^\n]*", "", kernel)
+    assert body.index("pdl_wait();") < min(body.index(x) for x in ("q_indptr[", "plan[", "rows_plan[i]", "stream_shares(q_indptr", "block_table +") if x in body)
