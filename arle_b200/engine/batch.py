@@ -32,6 +32,7 @@ class Workspace:
         self.device = torch.device(device)
         self._bufs: Dict[Tuple[str, torch.dtype], torch.Tensor] = {}
         self._views: Dict[Tuple[str, torch.dtype], Tuple[Tuple[int, ...], torch.Tensor]] = {}     # the shape asked for last, and its view
+        self._cuts: Dict[Tuple[str, torch.dtype], Dict[Tuple[int, int], torch.Tensor]] = {}                # columns of those views
         self.frozen = False
         self.generation = 0            # counts (re)allocations: addresses handed out earlier may be stale after one
 
@@ -52,6 +53,7 @@ class Workspace:
             self.generation += 1
         view = buf[:n].view(shape)
         self._views[key] = (tuple(shape), view)
+        self._cuts.pop(key, None)
         return view
 
     def get_zeroed(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
@@ -73,7 +75,21 @@ class Workspace:
             self.generation += 1
         view = buf[:n].view(shape)
         self._views[key] = (tuple(shape), view)
+        self._cuts.pop(key, None)
         return view
+
+    def cut(self, name: str, view: torch.Tensor, first: int, last: int) -> torch.Tensor:
+        """``view[:, first: last]`` of a view that ``get`` handed out under this name.  Kept as long as the view is: making one costs the host as
+        much as a launch."""
+        key = (name, view.dtype)
+        last_view = self._views.get(key)
+        if last_view is None or last_view[1] is not view:
+            return view[:, first: last]
+        cuts = self._cuts.setdefault(key, {})
+        piece = cuts.get((first, last))
+        if piece is None:
+            piece = cuts[(first, last)] = view[:, first: last]
+        return piece
 
     def nbytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._bufs.values())

@@ -23,6 +23,7 @@ from ctypes import c_float, c_int, c_void_p
 import torch
 
 from . import build as _build
+from . import launchers as _launchers
 
 _LIB = None
 _LAUNCHES = 0
@@ -112,6 +113,8 @@ _SIGNATURES = {
     "arle_conv_silu": [_P, _I, _I, _P, _P, _P, ctypes.c_long, ctypes.c_long, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "arle_gated_group_norm": [_P, _P, _I, _I, _P, _I, _P, _I, _P, _F, _P, _I, _I, _I, _I, _P],
     "arle_moe_select": [_P, _I, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P, _I, _P],
+    "arle_moe_plan_ints": [_I, _I],
+    "arle_set_programmatic_launch": [_I],
     "arle_moe_plan": [_P, _I, _I, _I, _P, _P, _P, _P, _P, _P],
     "arle_moe_gemm": [_P, _I, _P, _P, _I, ctypes.c_long, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _P, _I, _P],
     "arle_moe_rows": [_P, _I, _P, _P, _I, _I, _P],
@@ -130,17 +133,11 @@ class KernelError(RuntimeError):
     pass
 
 
-def library() -> ctypes.CDLL:
-    """The loaded CUDA library; built on first use.  Raises if it cannot be had."""
+def library():
+    """The loaded CUDA library, a callable for each of its launchers; built on first use.  Raises if it cannot be had."""
     global _LIB
     if _LIB is None:
-        path = _build.library_path()
-        lib = ctypes.CDLL(path)
-        for name, args in _SIGNATURES.items():
-            fn = getattr(lib, name)
-            fn.argtypes = args
-            fn.restype = c_int
-        _LIB = lib
+        _LIB = _launchers.load(_build.library_path(), _SIGNATURES)
     return _LIB
 
 
@@ -184,10 +181,7 @@ def set_programmatic_launch(on) -> None:
     straight from memory (up to 8 rows), which are launched so whatever is set here: a
     0.6B layer's four take 12.7 us instead of 15.4, where larger kernels find no room
     beside one another and lose."""
-    lib = library()
-    lib.arle_set_programmatic_launch.argtypes = [c_int]
-    lib.arle_set_programmatic_launch.restype = None
-    lib.arle_set_programmatic_launch(int(on))
+    library().arle_set_programmatic_launch(int(on))
 
 
 _KERNEL_SET = "fast"
@@ -239,9 +233,9 @@ def _ptr(t, name="tensor"):
 
 
 def _stream():
-    # torch's raw-stream query: a plain C call (torch.cuda.current_stream() builds a Python object and costs
-    # some 15 us, once per launch)
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    # torch's raw-stream query: plain C calls (torch.cuda.current_stream() builds a Python object and costs some 15 us, once per
+    # launch, and torch.cuda.current_device() asks first whether CUDA is up, which a tensor among the arguments says)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _check(code: int, what: str):
@@ -1752,10 +1746,7 @@ def moe_select(z, correction, scratch, experts: int, top: int, groups: int, keep
 
 def moe_plan_size(experts: int, pairs: int) -> int:
     """int32 entries of the plan that ``moe_plan`` writes."""
-    lib = library()
-    lib.arle_moe_plan_ints.argtypes = [c_int, c_int]
-    lib.arle_moe_plan_ints.restype = c_int
-    return int(lib.arle_moe_plan_ints(int(experts), int(pairs)))
+    return library().arle_moe_plan_ints(int(experts), int(pairs))
 
 
 def moe_plan(ids, experts: int, plan, place_of_pair, row_of_place, weights=None, weight_of_place=None) -> None:
@@ -1956,7 +1947,8 @@ def normed_sum(xs, biases, weights, scales, eps: float, out) -> None:
     wptrs = (ctypes.c_void_p * n)(*[_ptr(w_) for w_ in weights])
     strides = (ctypes.c_int * n)(*[x_.stride(0) for x_ in xs])
     sc = (ctypes.c_float * n)(*[float(v) for v in scales])
-    _check(library().arle_normed_sum(ptrs, strides, bptrs, wptrs, sc, n, _ptr(out), _dt(out), out.stride(0), T, H, float(eps), _stream()),
+    p, st, bp, wp, sp = (ctypes.addressof(a) for a in (ptrs, strides, bptrs, wptrs, sc))      # read by the launcher during the call
+    _check(library().arle_normed_sum(p, st, bp, wp, sp, n, _ptr(out), _dt(out), out.stride(0), T, H, float(eps), _stream()),
            "normed_sum")
 
 

@@ -426,7 +426,8 @@ class Attention(Mixer):
             ops.gemm(x, self.w_qkv[: nq * hd], qkv)
             ops.attention_prep(qkv, ctx.positions, None, self.q_norm, None, eps, inv_freq, rdim, None, None, nq, 0, hd,
                                cache.page_size, angles=self._angles(qkv, ctx, inv_freq, rdim))
-        ops.paged_attention(qkv[:, : nq * hd], attn, cache.k, cache.v, ctx.positions, ctx.row_of_token,
+        q = ctx.ws.cut("qkv" if cache.writable else "q_only", qkv, 0, nq * hd)
+        ops.paged_attention(q, attn, cache.k, cache.v, ctx.positions, ctx.row_of_token,
                             cache.block_table, nq, nkv, hd, cache.page_size, s.scale, s.window, batch=ctx)
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)
         if ops.gemm(attn, self.w_o, out, sink=sink):

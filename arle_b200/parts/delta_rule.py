@@ -112,12 +112,12 @@ class GatedDeltaRule(Mixer):
         pre = ctx.ws.get("delta_pre", (T, 2 * H), torch.float32)
         ops.gemm(x, self.w_gates, pre)
         qkv = ctx.ws.get("delta_conv", (T, C), x.dtype)
-        ops.causal_conv(proj[:, :C], None, self.conv, None, "silu", state, self.conv_offset, ctx.q_indptr, ctx.row_of_token,
+        ops.causal_conv(ctx.ws.cut("delta_in", proj, 0, C), None, self.conv, None, "silu", state, self.conv_offset, ctx.q_indptr, ctx.row_of_token,
                         ctx.state_slots, qkv)
         beta, decay = (ctx.ws.get(n, (T, H), torch.float32) for n in ("delta_beta", "delta_decay"))
         ops.delta_gates(pre, self.a_log, self.dt_bias, beta, decay)
         o = ctx.ws.get("delta_o", (T, H, s.value_dim), torch.float32)
-        q, k, v = qkv[:, :dqk], qkv[:, dqk: 2 * dqk], qkv[:, 2 * dqk:]
+        q, k, v = (ctx.ws.cut("delta_conv", qkv, i, j) for i, j in ((0, dqk), (dqk, 2 * dqk), (2 * dqk, C)))
         chunks = {}
         if ops.delta_scan_takes_chunks(q, s.value_dim, s.key_dim, ctx.max_q_len):
             n = ops.delta_scan_scratch(T, ctx.state_slots.numel(), H)
@@ -125,7 +125,7 @@ class GatedDeltaRule(Mixer):
         ops.delta_scan(q, k, v, beta, decay, state, ctx.q_indptr, ctx.state_slots, o, H, s.num_kq_heads, s.key_dim, s.value_dim,
                        float(s.key_dim) ** -0.5, s.unit_eps, **chunks)
         gated = ctx.ws.get("delta_gated", (T, inner), x.dtype)
-        ops.gla_out(o.view(T, inner), proj[:, C:], self.norm, s.norm_eps, 1.0, gated, H, s.value_dim)
+        ops.gla_out(o.view(T, inner), ctx.ws.cut("delta_in", proj, C, C + inner), self.norm, s.norm_eps, 1.0, gated, H, s.value_dim)
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)
         ops.gemm(gated, self.w_o, out)
         return out

@@ -165,11 +165,11 @@ class LatentAttention(Mixer):
         ops.gemm(x, self.w_in, proj)
         if s.q_rank is not None:
             cq = ctx.ws.get("latent_cq", (T, s.q_rank), x.dtype)
-            ops.rms_rows(proj[:, : s.q_rank], self.q_latent_norm, s.norm_eps, cq)
+            ops.rms_rows(ctx.ws.cut("latent_in", proj, 0, s.q_rank), self.q_latent_norm, s.norm_eps, cq)
             q = ctx.ws.get("latent_q_up", (T, self.q_width), x.dtype)
             ops.gemm(cq, self.w_uq, q)
         else:
-            q = proj[:, : self.q_width]
+            q = ctx.ws.cut("latent_in", proj, 0, self.q_width)
         records = cache.streams[0]
         stores = cache.writable and s.own_latent
         places = ops.latent_built_places(ctx, q, dn, dr, s.value_dim, rank, cache.page_size, s.window) if self.w_ukv is not None else 0
@@ -182,7 +182,7 @@ class LatentAttention(Mixer):
                             pairing=getattr(self.position, "pairing", "half"), amplitude=getattr(self.position, "amplitude", 1.0))
 
         if stores or dr:
-            prepare(q_abs, proj[:, self.first: self.first + self.record] if s.own_latent else None, stores)
+            prepare(q_abs, ctx.ws.cut("latent_in", proj, self.first, self.first + self.record) if s.own_latent else None, stores)
         heads_out = ctx.ws.get("attn_out", (T, H, s.value_dim), x.dtype)
         gate = proj[:, self.gate_at: self.gate_at + H * s.value_dim] if s.out_gate else None
         if not all_built:

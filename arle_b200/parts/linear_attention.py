@@ -121,13 +121,14 @@ class GatedLinearAttention(Mixer):
         H, dk, dv = s.num_heads, s.key_dim, s.value_dim
         proj = ctx.ws.get("gla_in", (T, self.rows), x.dtype)
         ops.gemm(x, self.w_in, proj)
-        at = self.at
+        def part(role, width):
+            return ctx.ws.cut("gla_in", proj, self.at[role], self.at[role] + width)
+
         alpha = ctx.ws.get("gla_alpha", (T, H * dk), torch.float32)
-        ops.gla_decay(proj[:, at["low"]: at["low"] + s.decay_rank], self.w_decay, self.decay_bias, s.tau, alpha)
+        ops.gla_decay(part("low", s.decay_rank), self.w_decay, self.decay_bias, s.tau, alpha)
         o = ctx.ws.get("gla_o", (T, H * dv), torch.float32)
-        ops.gla_scan(proj[:, at["q"]: at["q"] + H * dk], proj[:, at["k"]: at["k"] + H * dk], proj[:, at["v"]: at["v"] + H * dv],
-                     alpha, state, ctx.q_indptr, ctx.state_slots, o, H, dk, dv, self.q_scale, ctx.max_q_len)
-        ops.gla_out(o, proj[:, at["gate"]: at["gate"] + H * dv], self.norm, s.norm_eps, scale, into, H, dv)
+        ops.gla_scan(part("q", H * dk), part("k", H * dk), part("v", H * dv), alpha, state, ctx.q_indptr, ctx.state_slots, o, H, dk, dv, self.q_scale, ctx.max_q_len)
+        ops.gla_out(o, part("gate", H * dv), self.norm, s.norm_eps, scale, into, H, dv)
 
     def forward(self, x, ctx, cache, state, sink=None):
         s = self.spec

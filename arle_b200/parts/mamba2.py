@@ -60,7 +60,7 @@ class Mamba2(Mixer):
         self.channels = self.inner + 2 * self.bc             # what the convolution runs over
         self.main_rows = self.inner + self.channels          # z, x, B, C
         self.conv_offset = spec.num_heads * spec.head_dim * spec.state_dim
-        self.w_in = self.w_o = self.conv = self.conv_bias = self.dt_bias = self.a_log = self.skip = self.norm = None
+        self.w_in = self.w_main = self.w_dt = self.w_o = self.conv = self.conv_bias = self.dt_bias = self.a_log = self.skip = self.norm = None
         self.in_chunks = False                               # whether long prompts' chunks keep something in step buffers
 
     def _name(self, role: str) -> str:
@@ -83,6 +83,7 @@ class Mamba2(Mixer):
         self.in_chunks = dtype == torch.bfloat16 and self.spec.state_dim == 128 and self.spec.head_dim % 8 == 0
         w, o = tensors[self._name("in")], tensors[self._name("o")]
         self.w_in = w.to(device=device, dtype=kept(w)).contiguous()
+        self.w_main, self.w_dt = self.w_in[: self.main_rows], self.w_in[self.main_rows:]
         self.w_o = o.to(device=device, dtype=kept(o)).contiguous()
         self.conv, self.conv_bias, self.dt_bias, self.a_log, self.skip, self.norm = (
             tensors[self._name(n)].to(device=device, dtype=torch.float32).contiguous()
@@ -108,18 +109,19 @@ class Mamba2(Mixer):
         T = x.shape[0]
         H, P, N, inner, bc = s.num_heads, s.head_dim, s.state_dim, self.inner, self.bc
         zxbc = ctx.ws.get("ssm_in", (T, self.main_rows), x.dtype)
-        ops.gemm(x, self.w_in[: self.main_rows], zxbc)
+        ops.gemm(x, self.w_main, zxbc)
         dt_raw = ctx.ws.get("ssm_dt", (T, H), torch.float32)
-        ops.gemm(x, self.w_in[self.main_rows:], dt_raw)
+        ops.gemm(x, self.w_dt, dt_raw)
         xbc = ctx.ws.get("ssm_conv", (T, self.channels), x.dtype)
-        ops.conv_silu(zxbc[:, inner:], self.conv, self.conv_bias, state, self.conv_offset, ctx.q_indptr, ctx.row_of_token,
+        ops.conv_silu(ctx.ws.cut("ssm_in", zxbc, inner, inner + self.channels), self.conv, self.conv_bias, state, self.conv_offset, ctx.q_indptr, ctx.row_of_token,
                       ctx.state_slots, xbc)
         a, b = (ctx.ws.get(n, (T, H), torch.float32) for n in ("scan_a", "scan_b"))
         ops.ssm_gates(dt_raw, self.dt_bias, self.a_log, a, b)
         y = ctx.ws.get("scan_out", (T, H, P), torch.float32)
-        ops.decay_memories(xbc[:, inner + bc:], xbc[:, inner: inner + bc], xbc[:, :inner], a, b, state, ctx, y, H, s.groups, N, P, False, 1.0)
+        u, B, C = (ctx.ws.cut("ssm_conv", xbc, i, j) for i, j in ((0, inner), (inner, inner + bc), (inner + bc, self.channels)))
+        ops.decay_memories(C, B, u, a, b, state, ctx, y, H, s.groups, N, P, False, 1.0)
         gated = ctx.ws.get("ssm_gated", (T, inner), x.dtype)
-        ops.gated_group_norm(y.view(T, inner), xbc[:, :inner], self.skip, P, zxbc[:, :inner], self.norm, s.norm_eps, gated, s.norm_groups)
+        ops.gated_group_norm(y.view(T, inner), u, self.skip, P, ctx.ws.cut("ssm_in", zxbc, 0, inner), self.norm, s.norm_eps, gated, s.norm_groups)
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)
         return None if ops.gemm(gated, self.w_o, out, sink=sink) else out
 

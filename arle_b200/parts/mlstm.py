@@ -112,12 +112,14 @@ class MatrixLstm(Mixer):
         ops.gemm(x, self.w_gates, pre)
         a, b, floor = (ctx.ws.get(n, (T, H), torch.float32) for n in ("scan_a", "scan_b", "mlstm_floor"))
         ops.mlstm_gates(pre, self.bias_i, self.bias_f, s.gate_cap, ctx.q_indptr, ctx.state_slots, state, self.m_offset, a, b, floor)
-        at = self.at
+
+        def part(role, width):
+            return ctx.ws.cut("mlstm_in", proj, self.at[role], self.at[role] + width)
+
         num = ctx.ws.get("scan_out", (T, H, dv + 1), torch.float32)
-        ops.decay_memories(proj[:, at["q"]: at["q"] + H * dk], proj[:, at["k"]: at["k"] + H * dk], proj[:, at["v"]: at["v"] + H * dv],
-                           a, b, state, ctx, num, H, H, dk, dv, True, dk ** -0.5)
+        ops.decay_memories(part("q", H * dk), part("k", H * dk), part("v", H * dv), a, b, state, ctx, num, H, H, dk, dv, True, dk ** -0.5)
         gated = ctx.ws.get("mlstm_gated", (T, H * dv), x.dtype)
-        ops.mlstm_out(num, floor, proj[:, at["gate"]: at["gate"] + H * dv], self.norm, s.norm_eps, gated, H, dv)
+        ops.mlstm_out(num, floor, part("gate", H * dv), self.norm, s.norm_eps, gated, H, dv)
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)
         return None if ops.gemm(gated, self.w_o, out, sink=sink) else out
 
