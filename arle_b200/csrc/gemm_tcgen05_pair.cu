@@ -13,19 +13,20 @@
 // first CTA's TMEM, rows 128-255 in the second's.
 //
 // Per CTA, by warp:
-//   warp 4, one lane : producer.  Waits for a free stage (its own `empty` barrier) and issues two TMA loads
+//   warp 8, one lane : producer.  Waits for a free stage (its own `empty` barrier) and issues two TMA loads
 //                      into its own shared memory whose bytes are counted on the FIRST CTA's `full` barrier
 //                      of the stage (cp.async.bulk.tensor with cta_group::2 and that barrier's cluster
 //                      address); the first CTA's producer arms that barrier with the bytes of both CTAs.
-//   warp 5, one lane : in the first CTA only, the MMA issuer: waits for a full stage, issues four
+//   warp 9, one lane : in the first CTA only, the MMA issuer: waits for a full stage, issues four
 //                      tcgen05.mma (256 x 256 x 16 over the pair), and hands the stage back to both
 //                      producers with one tcgen05.commit that arrives on the `empty` barrier of both CTAs
 //                      (multicast over the cluster); after a tile's last block a commit on both CTAs'
-//                      `acc_full`.  Warp 5 of both CTAs allocates and frees the TMEM columns (cta_group::2).
-//   warps 0-3        : epilogue of the CTA's own 128 rows: tcgen05.ld 32 columns at a time, convert (or apply
+//                      `acc_full`.  Warp 9 of both CTAs allocates and frees the TMEM columns (cta_group::2).
+//   warps 0-7        : epilogue of the CTA's own 128 rows, two warps to 32 rows with every second 32 columns each: tcgen05.ld, convert (or apply
 //                      the gate to neighbouring columns), store; then arrive on the first CTA's `acc_empty`.
 // The accumulators are double-buffered (2 x 256 of the 512 TMEM columns): the tensor cores fill one while the
-// epilogue drains the other.  Edges: TMA zero-fills rows beyond M or N and columns beyond K; stores are
+// epilogue drains the other (with four warps and an exact division in the gate it took longer than the products of a short K: gated, 1,685 rows
+// of 6,144 x 1,024 46.5 us, now 30.8; 2,048 of 24,576 x 4,096 294 and 290.  The last round's tiles in halves of 128 columns: no change).  Edges: TMA zero-fills rows beyond M or N and columns beyond K; stores are
 // guarded.  Every wait is bounded; a CTA whose wait runs out raises the error flag, stops issuing and runs to
 // its end (its partner's waits then run out in turn), and both meet at the cluster barrier before they free
 // their tensor memory.  No TMA load here is a multicast; the only cluster-wide operation besides the MMA is
@@ -42,8 +43,8 @@ constexpr int BM = 128;                      // rows of x per CTA (256 per pair)
 constexpr int BNH = 128;                     // weight rows per CTA (256 per pair)
 constexpr int BN = 256;
 constexpr int BK = 64;                       // 64 bfloat16 = 128 bytes = one swizzle span
-constexpr int kEpilogueWarps = 4;
-constexpr int kThreads = 192;
+constexpr int kEpilogueWarps = 8, kProducer = kEpilogueWarps, kIssuer = kProducer + 1;
+constexpr int kThreads = (kIssuer + 1) * 32;
 constexpr uint32_t kTmemCols = 512;
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_pair_kernel(const __
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
-  if (warp == 5) {
+  if (warp == kIssuer) {
     tmem_alloc_pair(smem_addr(&tmem_base_slot), kTmemCols);
     tmem_relinquish_pair();
   }
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_pair_kernel(const __
   const uint32_t tmem_base = tmem_base_slot;
   const volatile int* aborted = &abort_flag;
 
-  if (warp == 4) {
+  if (warp == kProducer) {
     if (lane == 0) {
       int issued = 0;
       for (int t = pair; t < num_tiles && !*aborted; t += npairs) {
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_pair_kernel(const __
         }
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == kIssuer) {
     if (lane == 0 && leader) {
       constexpr uint32_t idesc = idesc_bf16(2 * BM, BN);
       int consumed = 0, iter = 0;
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_pair_kernel(const __
       }
     }
   } else {
-    // epilogue of this CTA's 128 rows: warp i reads TMEM lanes 32 i .. 32 i + 31
+    // epilogue of this CTA's 128 rows: warps i and i + 4 read TMEM lanes 32 i .. 32 i + 31
     int iter = 0;
     const uint32_t acc_empty_leader[2] = {map_to_rank(smem_addr(&acc_empty[0]), 0), map_to_rank(smem_addr(&acc_empty[1]), 0)};
     for (int t = pair; t < num_tiles; t += npairs, ++iter) {
@@ -213,11 +214,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_pair_kernel(const __
       if (!ready) abort_flag = 1;
       if (__any_sync(0xffffffffu, !ready || *aborted)) break;
       tc_fence_after();
-      const int row = m0 + warp * 32 + lane;
+      const int row = m0 + (warp & 3) * 32 + lane;
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = warp >> 2; c < BN / 32; c += kEpilogueWarps / 4) {
         uint32_t r[32];
-        tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * BN + c * 32), r);
+        tmem_ld32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(buf * BN + c * 32), r);
         tmem_ld_wait();
         const int col = n0 + c * 32;
         if (row >= M || col >= N) continue;
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_pair_kernel(const __
           for (int i = 0; i < 16; ++i) {
             const float g = __uint_as_float(r[2 * i]), u = __uint_as_float(r[2 * i + 1]);
             v[i] = (act == 2 ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)))
-                             : g / (1.0f + __expf(-g))) * u;
+                             : times_sigmoid<__nv_bfloat16>(g, g)) * u;
           }
           if (col + 32 <= N && (((uintptr_t)dst) & 15) == 0) {
             uint32_t p[8];
@@ -290,12 +291,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_pair_kernel(const __
   }
   // A producer whose wait ran out may still have copies under way into its shared memory: wait for them
   // (bounded) before the CTA ends.  They are counted on the first CTA's barriers, so only it can look.
-  if (warp == 4 && lane == 0 && leader && *aborted)
+  if (warp == kProducer && lane == 0 && leader && *aborted)
     for (int s = 0; s < STAGES; ++s) mbar_wait_plain(smem_addr(&full_bar[s]), 0), mbar_wait_plain(smem_addr(&full_bar[s]), 1);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                                      // neither CTA frees tensor memory the other's MMAs may still write
-  if (warp == 5) {
+  if (warp == kIssuer) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, kTmemCols);
   }

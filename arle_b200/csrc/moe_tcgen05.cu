@@ -7,24 +7,28 @@
 // expert's c tokens are cut into ceil(c / 256) equal parts, rounded up to a multiple of 32.  Decoded tokens then cost what reading
 // the weights costs, and a prompt's tiles are 84 to 95 % tokens.
 //
-// Operands: the weights (K-major rows) come as 128 x 64 boxes by TMA, the tokens' rows, side by side in place order, as boxes of 16 rows.
+// Operands: the weights (K-major rows) come as 128 x 64 boxes by TMA, the tokens' rows, side by side in place order, as boxes of 128, 64, 32 and
+// 16 rows, one of each at most (in boxes of 16 alone, eight of them a stage, a block of K took 820 cycles instead of 660, of which the MMAs 512).
 // The caller copies them there first (moe_rows: 14 us for 8,192 places of 4,096 numbers); fetched from where they stand by
 // tile::gather4, four rows an instruction, the product of a prompt of 2,048 tokens with 32 matrices of 6,144 rows took 1,101 us instead of
 // 491, and 32 places gained nothing either.  Each CTA of the pair loads half of a tile's tokens.  Places past an expert's last one are computed from whatever row is there and not
 // stored.
 //
-// Per CTA, by warp (the roles and barriers of gemm_tcgen05_pair.cu): warp 4 producer; warp 5 allocates TMEM and, in the first CTA,
-// issues the MMAs; warps 0-3 epilogue.  The accumulators (256 columns) are double-buffered.  In the epilogue a lane holds one
+// Per CTA, by warp (the roles and barriers of gemm_tcgen05_pair.cu): warp 8 producer; warp 9 allocates TMEM and, in the first CTA,
+// issues the MMAs; warps 0-7 epilogue, two to a quarter of the
+// lanes with every second 32 tokens each (four warps took longer than the products where K is 1,024).  The accumulators (256 columns) are double-buffered.  In the epilogue a lane holds one
 // weight row and a register one token; neighbouring lanes exchange halves, so that a lane holds both numbers of a pair of rows
 // (gate_i and up_i, or two neighbouring outputs) for every second token: the gate is applied to the float32 sums and a lane stores
 // a whole pair.
 // Persistent grid: the tiles of an expert with the token part running fastest, then the weight rows, so the pairs that run together
 // read an expert's matrix once and share its tokens in L2.
 //
-// What bounds it: the weights' bytes for decoded tokens, the tensor cores (under the power cap) and the part of a tile that is padding
-// for prompts.  32 experts of 3 x 3,072 x 4,096, 4 of them a token, first and second product: 274 and 133 us for 64 tokens (1.61 and
-// 0.81 GB: 5.9 and 6.1 TB/s), 491 and 249 us for 2,048 tokens (0.84 and 0.83 PFLOP/s of tokens).  The mma.sync tiles of 64 x 128 that
-// ran these before took 563 us for both (64 tokens) and 2,538 us (2,048), with a gate kernel of 21 us behind the first.
+// What bounds it: the weights' bytes for decoded tokens, the tensor cores (under the power cap), the part of a tile that is padding and the last
+// round of tiles for prompts.  32 experts of 3 x 3,072 x 4,096, 4 of them a token, first and second product: 274 and 136 us for 64 tokens (1.61
+// and 0.81 GB: 5.9 TB/s), 462 and 232 us for 2,048 tokens (0.89 PFLOP/s of tokens; 509 and 256 with four warps in the epilogue and boxes of
+// 16); 16 experts of 3 x 768 x 1,024, 2,048 tokens 38.8 and 30.8 (57.0 and 43.4).  Tried and left: tiles of 512 weight rows, a block in each
+// accumulator (half the reads of the tokens, no second buffer: 454 and 239); runs of tiles of equal cost for the pairs, each at experts of its own
+// (598 and 306: the experts' tokens then fall out of L2).
 //
 // Every wait is bounded; a CTA whose wait runs out raises the error flag and runs to its end.
 #include "common.cuh"
@@ -36,8 +40,8 @@ namespace {
 constexpr int BM = 128;                      // weight rows per CTA (256 per pair)
 constexpr int BNMAX = 256;                   // tokens of a tile
 constexpr int BK = 64;
-constexpr int kEpilogueWarps = 4;
-constexpr int kThreads = 192;
+constexpr int kEpilogueWarps = 8, kProducer = kEpilogueWarps, kIssuer = kProducer + 1;
+constexpr int kThreads = (kIssuer + 1) * 32;
 constexpr uint32_t kTmemCols = 512;
 constexpr int kStages = 6;
 constexpr int kMaxExperts = 1024;
@@ -85,6 +89,12 @@ __device__ __forceinline__ float finish_pair(float g, float u, float limit, floa
   return g / (1.0f + expf(-alpha * g)) * (u + 1.0f);        // as clamped_glu: the full exponential and division
 }
 
+// The tokens' rows in boxes of 16, 32, 64 and 128: half a tile's tokens are one of each at most.
+constexpr int kBoxes = 4;
+struct RowMaps {
+  CUtensorMap of[kBoxes];
+};
+
 // The tiles of a product: expert e has cuts[e + 1] - cuts[e] equal token parts.
 struct Walk {
   const int* plan;
@@ -105,7 +115,7 @@ struct Walk {
 };
 
 template <int FINISH>
-__global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+__global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_constant__ RowMaps map_x, const __grid_constant__ CUtensorMap map_w,
                                                                   const int* __restrict__ plan, int E,
                                                                   __nv_bfloat16* __restrict__ out, int ldo, int N, int K,
                                                                   const float* __restrict__ place_scale, float limit, float alpha,
@@ -141,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
-  if (warp == 5) {
+  if (warp == kIssuer) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&tmem_base_slot)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
   }
@@ -177,12 +187,14 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
   Walk walk{plan, cuts, (N + 2 * BM - 1) / (2 * BM), 0};
   int n_tile, p0, count, part;
 
-  if (warp == 4) {
+  if (warp == kProducer) {
     int issued = 0;
     bool dead = false;
     for (int t = pair; !dead && walk.at(t, E, n_tile, p0, count, part); t += npairs) {
       const int half = part >> 1;                          // this CTA's tokens: 16 .. 128
       const int mine = p0 + (int)rank * half;
+      const bool boxed = lane < kBoxes && (half >> (4 + lane) & 1);      // lane l brings 16 << l rows, behind those of the larger boxes
+      const int box_row = half & ~((32 << (lane & 3)) - 1);
       const int wrow = walk.expert * N + n_tile * 2 * BM + (int)rank * BM;
       for (int kb = 0; kb < kblocks; ++kb, ++issued) {
         const int s = issued % kStages;
@@ -200,10 +212,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
           tma_load_2d_pair(a_dst, &map_w, kb * BK, wrow, bar);
         }
         __syncwarp();
-        if (lane * 16 < half) tma_load_2d_pair(a_dst + A_BYTES + (uint32_t)lane * (16 * BK * 2), &map_x, kb * BK, mine + lane * 16, bar);
+        if (boxed) tma_load_2d_pair(a_dst + A_BYTES + (uint32_t)box_row * (BK * 2), &map_x.of[lane & 3], kb * BK, mine + box_row, bar);
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == kIssuer) {
     if (lane == 0 && leader) {
       int consumed = 0, iter = 0;
       for (int t = pair; !*aborted && walk.at(t, E, n_tile, p0, count, part); t += npairs, ++iter) {
@@ -243,12 +255,12 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
       if (!ready) abort_flag = 1;
       if (__any_sync(0xffffffffu, !ready || *aborted)) break;
       tc_fence_after();
-      const int n0 = n_tile * 2 * BM + (int)rank * BM + warp * 32 + (lane & ~1);       // this lane's pair of weight rows
+      const int n0 = n_tile * 2 * BM + (int)rank * BM + (warp & 3) * 32 + (lane & ~1);       // this lane's pair of weight rows
       const int odd = lane & 1;
 #pragma unroll 1
-      for (int c = 0; c < part; c += 32) {
+      for (int c = (warp >> 2) * 32; c < part; c += kEpilogueWarps * 8) {
         uint32_t r[32];
-        tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * BNMAX + c), r);
+        tmem_ld32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(buf * BNMAX + c), r);
         tmem_ld_wait();
         if (c >= count) continue;
         const float scale = place_scale && c + lane < count ? place_scale[p0 + c + lane] : 1.f;
@@ -289,12 +301,12 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
   }
   // A producer whose wait ran out may still have copies under way into its shared memory: wait for them
   // (bounded) before the CTA ends.  They are counted on the first CTA's barriers, so only it can look.
-  if (warp == 4 && lane == 0 && leader && *aborted)
+  if (warp == kProducer && lane == 0 && leader && *aborted)
     for (int s = 0; s < kStages; ++s) mbar_wait_plain(smem_addr(&full_bar[s]), 0), mbar_wait_plain(smem_addr(&full_bar[s]), 1);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                                      // neither CTA frees tensor memory the other's MMAs may still write
-  if (warp == 5) {
+  if (warp == kIssuer) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
@@ -304,8 +316,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
 template <int FINISH>
 int launch(const void* x, int ldx, int x_rows, const void* W, void* out, int ldo, const int* plan, int E, int pairs, int N, int K,
            const float* place_scale, float limit, float alpha, int* err, cudaStream_t s) {
-  CUtensorMap mx, mw;
-  int rc = tensor_map_2d_bf16(x, x_rows, K, ldx, 16, &mx);
+  RowMaps mx;
+  CUtensorMap mw;
+  int rc = 0;
+  for (int i = 0; i < kBoxes && rc == 0; ++i) rc = tensor_map_2d_bf16(x, x_rows, K, ldx, 16 << i, &mx.of[i]);
   if (rc) return rc;
   rc = tensor_map_2d_bf16(W, (long long)E * N, K, K, BM, &mw);
   if (rc) return rc;

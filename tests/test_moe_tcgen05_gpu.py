@@ -62,6 +62,16 @@ def test_products_at_tile_edges(counts, N, K, gathered):
     ops.check_errors(DEV)
 
 
+def test_every_set_of_boxes():
+    """Half a tile's tokens are 16 to 128: boxes of 128, 64, 32 and 16 rows, one of each at most; the last expert's end where x does."""
+    x, rows, w, plan, z, mag = _setup([32 * i - i % 2 for i in range(1, 9)] + [480, 31 + 256], 300, 136, False, seed=5)
+    out = torch.full((z.shape[0] + 1, 300), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.moe_gemm(x, None, w, out[:-1], plan, w.shape[0])
+    assert ((out[:-1].double() - z).abs() <= 136 * 2.0 ** -23 * mag + 2.0 ** -8 * z.abs() + 1e-30).all()
+    assert (out[-1] == 7.0).all()
+    ops.check_errors(DEV)
+
+
 @pytest.mark.parametrize("counts", [COUNTS[1], COUNTS[2], [300]], ids=["small", "mid", "one"])
 @pytest.mark.parametrize("act", ["silu", "gelu_tanh", "clamped_glu"])
 def test_gated_products(counts, act):
