@@ -23,10 +23,10 @@ __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, i
   }
 }
 
-// Eight elements per thread and step for bfloat16 rows whose width is a multiple of 8.
+// Eight elements per thread and step for bfloat16 rows whose width is a multiple of 8.  Few rows are launched programmatically: plain loads, as
+// the kernel then lives beside the product that writes what it reads.
 template <int ACT>
-__global__ void silu_mul_bf16_vec_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int inter,
-                                         size_t total8, int out_stride) {
+__global__ void silu_mul_bf16_vec_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out, int inter, size_t total8, int out_stride) {
   pdl_launch_dependents();
   pdl_wait();
   const int i8 = inter >> 3;
@@ -65,7 +65,8 @@ static int act_mul_launch(const void* gu, void* out, int dtype, int num_tokens, 
     const size_t total8 = total / 8;
     size_t b8 = (total8 + threads - 1) / threads;
     if (b8 > 148 * 32) b8 = 148 * 32;
-    launch_kernel(silu_mul_bf16_vec_kernel<ACT>, dim3((int)b8), dim3(threads), 0, s, 1, (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, inter, total8, out_stride);
+    launch_kernel_as(num_tokens <= kEarlyRows || (pdl_enabled() & 1) != 0, silu_mul_bf16_vec_kernel<ACT>, dim3((int)b8), dim3(threads), 0, s, 1,
+                     (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, inter, total8, out_stride);
     return launch_status();
   }
   if (dtype == 0)

@@ -138,11 +138,15 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 
 // Bit 0: every kernel is launched with programmatic stream serialisation allowed; bit 1:
 // the weight-streaming products only (they fill their weight ring while the kernel before
-// them finishes).  Off by default.  (The small products of gemm_skinny.cu are always launched so.)
+// them finishes).  Off by default.  (Always launched so: the small products of gemm_skinny.cu, the streamed attention of steps that decode
+// only, norms and gates of up to kEarlyRows rows.)
 inline int& pdl_enabled() {
   static int on = 0;
   return on;
 }
+
+// Rows up to which the norms and gates between a step's products are launched programmatically.
+constexpr int kEarlyRows = 256;
 
 // kernel<<<grid, block, smem, stream>>>(args...) with the programmatic-launch attribute
 // (and a cluster dimension when cluster > 1).

@@ -177,10 +177,11 @@ def set_programmatic_launch(on) -> None:
     """Programmatic dependent launch: a kernel may be scheduled, set up its barriers and
     prefetch weights while the kernel before it finishes, and waits for that kernel only
     before touching its results.  True or 1: every kernel; 2: the weight-streaming
-    products; 0 (the default): only the small decode products that read their weights
-    straight from memory (up to 8 rows), which are launched so whatever is set here: a
-    0.6B layer's four take 12.7 us instead of 15.4, where larger kernels find no room
-    beside one another and lose."""
+    products; 0 (the default): only the kernels that are launched so whatever is set here,
+    the small decode products that read their weights straight from memory (up to 8 rows; a
+    0.6B layer's four take 12.7 us instead of 15.4), the streamed attention of steps that
+    decode only, and norms and gates of up to 256 rows.  Larger kernels find no room beside
+    one another and lose."""
     library().arle_set_programmatic_launch(int(on))
 
 
