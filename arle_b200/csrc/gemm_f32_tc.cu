@@ -15,7 +15,7 @@
 // piece).  Roles by warp:
 //   sums    : four warps.  Warp i owns TMEM lanes 32 i .. 32 i + 31, a column of C a thread; adds up the blocks' sums of BN rows in
 //             registers, stores them (lanes: neighbouring columns).
-//   cutters : eight warps (four).  Groups of BN / 16 warps take turns at the blocks: cut 64 numbers of k of the BN rows and lay the
+//   cutters : eight warps (four, ten).  Groups of BN / 16 warps take turns at the blocks: cut 64 numbers of k of the BN rows and lay the
 //             three tiles down as the MMA reads them (128-byte swizzle).
 //   loader  : one lane, W's tile and the rows of A by TMA.
 //   issuer  : one lane, four MMAs a block; its warp owns the TMEM.
@@ -27,7 +27,7 @@
 // for each who waits, took 900), many rows shared memory (A's rows come in, are read, go back in three pieces and are read by the MMAs).
 // Rows of A fetched by the cutters' own loads: each proxy fence waited for them, 950 cycles a block.  All cutters at one block at a time:
 // 1,400 cycles a block of 64 rows instead of 1,000.
-// Measured (us, the FFMA kernels and this one): 301 rows, 6,144 x 1,024 117 and 27; 4,096 x 1,024 87 and 27; 1,024 x 2,048 62 and 19; 1,024 x
+// Measured (us, the FFMA kernels and this one): 301 rows, 6,144 x 1,024 117 and 27; 4,096 x 1,024 87 and 20; 1,024 x 2,048 62 and 19; 1,024 x
 // 3,072 91 and 25; 1,024 rows of 24,576 x 4,096 4,420 and 795 (259 TFLOP/s); 16 rows of 1,024 x 3,072 84 and 21; one row of 151,936 x
 // 1,024 58 and 60, of 4,096 x 12,288 93 and 70, of 1,024 x 2,048 17 and 17.
 #include "common.cuh"
@@ -43,12 +43,12 @@ template <int BN, int CTAS>                                // CTAS: a SM
 struct Layout {
   // What TMA brings (W's tile, then the rows of A as they are) and, in a ring of their own, the pieces.
   static constexpr uint32_t W = kRowsW * kBK * 2, RAW = BN * kBK * 4, STAGE = W + RAW, PIECE = BN * kBK * 2;
-  static constexpr int PIECE_WARPS = CTAS == 2 ? 4 : 8, LOAD_WARP = kSumWarps + PIECE_WARPS, MMA_WARP = LOAD_WARP + 1, THREADS = (MMA_WARP + 1) * 32;
+  static constexpr int PIECE_WARPS = CTAS == 2 ? 4 : BN == 80 ? 10 : 8, LOAD_WARP = kSumWarps + PIECE_WARPS, MMA_WARP = LOAD_WARP + 1, THREADS = (MMA_WARP + 1) * 32;
   static constexpr int GROUP = BN / 16, GROUPS = PIECE_WARPS / GROUP;      // warps that cut a block together, blocks cut side by side
-  static constexpr int STAGES = BN == 64 || CTAS == 2 ? 4 : BN == 32 ? 6 : 8, RING = BN == 64 ? 3 : BN == 32 ? 5 : STAGES;
+  static constexpr int STAGES = BN >= 64 || CTAS == 2 ? 4 : BN == 32 ? 6 : 8, RING = BN == 80 ? 2 : BN == 64 ? 3 : BN == 32 ? 5 : STAGES;
   static_assert(RING >= GROUPS, "a group's next block has a place of its own");
   static constexpr size_t SMEM = (size_t)STAGES * STAGE + (size_t)RING * 3 * PIECE + 1024;
-  static constexpr int COLS = 3 * BN, BUFFERS = BN == 64 ? 2 : 4;      // accumulators in TMEM: a column for each piece of each row
+  static constexpr int COLS = 3 * BN, BUFFERS = BN >= 64 ? 2 : 4;      // accumulators in TMEM: a column for each piece of each row
   static constexpr uint32_t TMEM = BN == 16 ? 256 : 512;
   static_assert(COLS * BUFFERS <= (int)TMEM && CTAS * (SMEM + 2048) <= 228 * 1024, "TMEM, shared memory");
 };
@@ -331,12 +331,14 @@ ARLE_API int arle_gemm_f32_tc(const float* A, int lda, const void* W, int ldw, f
   if ((long long)((N + kRowsW - 1) / kRowsW) * ((M + 15) / 16) * (K / kBK) > 0x7fffffffll) return ARLE_E_UNSUPPORTED;
   const __nv_bfloat16* w = (const __nv_bfloat16*)W;
   // Rounds of tiles times what a block of 64 numbers of k takes (us): 301 rows of 6,144 x 1,024 43.5, 33.3 and 27.1 us in tiles of 16, 32 and 64
-  // rows, of 1,024 x 3,072 37.4, 25.1 and 33.3, 100 rows of 4,096 x 1,024 16.8, 12.7 and 16.9.  Two CTAs an SM with half the stages each
+  // rows, of 1,024 x 3,072 37.4, 25.1 and 33.3, 100 rows of 4,096 x 1,024 16.8, 12.7 and 16.9; of 4,096 x 1,024 with 301 rows 27.6 in tiles of 64 (a
+  // second round for 12 of 160), 20.0 in tiles of 80 (128), which take longer where both have as many rounds (6,144 x 1,024 33.7).  Two CTAs an SM with half the stages each
   // take more tiles at a time (one row of 24,576 x 4,096 45.5 us, with one CTA 52.5) and longer for one (1,024 x 3,072 25.0, 21.0).
   auto tiles = [&](int bn) { return (long long)((N + kRowsW - 1) / kRowsW) * ((M + bn - 1) / bn); };
   auto rounds = [](long long t, int at_once) { return (float)((t + at_once - 1) / at_once); };
   const bool few = tiles(16) <= 148;
-  const float c16 = few ? 0.316f : 0.47f * rounds(tiles(16), 296), c32 = 0.39f * rounds(tiles(32), 148), c64 = 0.53f * rounds(tiles(64), 148);
+  const float c16 = few ? 0.316f : 0.47f * rounds(tiles(16), 296), c32 = 0.39f * rounds(tiles(32), 148), c64 = 0.53f * rounds(tiles(64), 148), c80 = 0.77f * rounds(tiles(80), 148);
+  if (c80 < fminf(c16, fminf(c32, c64))) return launch<80, 1>(A, lda, w, ldw, C, ldc, M, N, K, err, s);
   if (c16 <= fminf(c32, c64))
     return few ? launch<16, 1>(A, lda, w, ldw, C, ldc, M, N, K, err, s) : launch<16, 2>(A, lda, w, ldw, C, ldc, M, N, K, err, s);
   if (c32 <= c64) return launch<32, 1>(A, lda, w, ldw, C, ldc, M, N, K, err, s);

@@ -65,7 +65,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = u;
 }
 
-// Up to kEarlyRows rows are launched programmatically (they stand between two products of some 10 us each; with the gates 4 layers of 0.6B sizes,
+// Up to kEarlyRows rows are launched programmatically (they stand between two products of some 10 us each; with the gates 8 layers of 0.6B sizes,
 // 20 requests, 483 -> 463 us a step, 8 layers of 8B sizes, 15 requests, 988 -> 984): plain loads, since the kernel lives beside the
 // one that writes what it reads, and all of them ahead of the first store, which without restrict they could not pass.
 template <typename TA>

@@ -1,4 +1,4 @@
-"""float32 rows times a bfloat16 W in three exact pieces on the tensor cores: against float64 at the edges of the tiles (16, 32 and 64 rows by
+"""float32 rows times a bfloat16 W in three exact pieces on the tensor cores: against float64 at the edges of the tiles (16, 32, 64 and 80 rows by
 128 columns), rows of other tensors untouched; no further off than the FFMA kernels; a row's bits whatever stands beside it; infinities,
 NaNs and the ends of float32's range."""
 import pytest
@@ -26,7 +26,7 @@ def ffma(x, w):
 
 @pytest.mark.parametrize("M,N,K,kernel", [
     (1, 256, 512, "<16, 1>"), (16, 300, 576, "<16, 1>"), (17, 4097, 1024, "<16, 1>"), (1, 20000, 512, "<16, 2>"), (16, 37900, 1024, "<16, 2>"),
-    (200, 2050, 640, "<32, 1>"), (129, 3000, 1024, "<32, 1>"), (301, 1024, 3072, "<32, 1>"), (301, 6145, 512, "<64, 1>"), (640, 2304, 4096, "<64, 1>"),
+    (200, 2050, 640, "<32, 1>"), (129, 3000, 1024, "<32, 1>"), (301, 1024, 3072, "<32, 1>"), (301, 6145, 512, "<64, 1>"), (640, 2304, 4096, "<80, 1>"), (80, 15000, 640, "<80, 1>"), (301, 4096, 512, "<80, 1>"),
     (64, 20000, 512, "<64, 1>")])
 def test_against_float64(M, N, K, kernel):
     x, w = inputs(M, N, K)
@@ -44,14 +44,14 @@ def test_against_float64(M, N, K, kernel):
 
 
 def test_a_row_has_the_same_bits_whatever_stands_beside_it():
-    x, w = inputs(301, 1536, 1024)
-    want = torch.empty(301, 1536, device=DEV)
+    x, w = inputs(301, 4096, 1024)
+    want = torch.empty(301, 4096, device=DEV)
     ops.gemm(x, w, want)
-    for rows in (slice(0, 1), slice(300, 301), slice(7, 23), slice(7, 24), slice(40, 140), slice(0, 257)):
-        got = torch.empty(x[rows].shape[0], 1536, device=DEV)
+    for rows in (slice(0, 1), slice(300, 301), slice(7, 23), slice(7, 24), slice(40, 140), slice(40, 200), slice(0, 257)):
+        got = torch.empty(x[rows].shape[0], 4096, device=DEV)
         ops.gemm(x[rows], w, got)
         assert torch.equal(got, want[rows])
-    wide = torch.empty(301, 1536 + 12, device=DEV)[:, 8:-4]
+    wide = torch.empty(301, 4096 + 12, device=DEV)[:, 8:-4]
     ops.gemm(torch.empty(301, 1028, device=DEV)[:, :1024].copy_(x), w, wide)
     assert torch.equal(wide, want)
 
