@@ -349,8 +349,8 @@ __global__ void __launch_bounds__(kPrepVecWarps * 32, 4) attention_prep_bf16_tok
 }
 
 // out[t][i] = (cos, sin)(positions[t] * inv_freq[i]): what every layer of a step would evaluate again.
-__global__ void rotary_angles_kernel(const int* __restrict__ positions, const float* __restrict__ inv_freq,
-                                     float2* __restrict__ out, int half, long long total) {
+__global__ void rotary_angles_kernel(const int* positions, const float* inv_freq,
+                                     float2* out, int half, long long total) {
   pdl_launch_dependents();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -367,7 +367,7 @@ ARLE_API int arle_rotary_angles(const int* positions, const float* inv_freq, flo
                                 cudaStream_t s) {
   if (num_tokens <= 0 || half <= 0) return 0;
   const long long total = (long long)num_tokens * half;
-  launch_kernel(rotary_angles_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, s, 1, positions, inv_freq,
+  launch_early(rotary_angles_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, s, 1, positions, inv_freq,
                 reinterpret_cast<float2*>(angles), half, total);
   return launch_status();
 }

@@ -139,7 +139,7 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // Bit 0: every kernel is launched with programmatic stream serialisation allowed; bit 1:
 // the weight-streaming products only (they fill their weight ring while the kernel before
 // them finishes).  Off by default.  (Always launched so: the small products of gemm_skinny.cu, the streamed attention of steps that decode
-// only, norms and gates of up to kEarlyRows rows.)
+// only, norms and gates of up to kEarlyRows rows, what goes through launch_early.)
 inline int& pdl_enabled() {
   static int on = 0;
   return on;
@@ -181,6 +181,14 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                  int cluster, Args&&... args) {
   return launch_kernel_as((pdl_enabled() & 1) != 0, kernel, grid, block, smem, stream, cluster, std::forward<Args>(args)...);
+}
+
+// A short kernel between others: launched as soon as the one in front has started its last block, whatever is set.  It waits for that one before
+// it reads anything and reads by plain loads (no restrict, no __ldg).  Not for kernels of few long blocks: those that start early gather on the
+// SMs that have room just then (a gated linear attention's scan of 128 blocks beside the decays in front of it took twice its time).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_early(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, Args&&... args) {
+  return launch_kernel_as(true, kernel, grid, block, smem, stream, cluster, std::forward<Args>(args)...);
 }
 
 // A kernel's limit of dynamic shared memory is a setting of the device it runs on, and a process may run models on several: a launcher

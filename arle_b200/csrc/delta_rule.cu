@@ -28,8 +28,8 @@
 #include "scan_utils.cuh"
 using namespace arle;
 
-__global__ void delta_gates_kernel(const float* __restrict__ pre, int pre_stride, const float* __restrict__ a_log,
-                                   const float* __restrict__ dt_bias, float* __restrict__ beta, float* __restrict__ decay, int H,
+__global__ void delta_gates_kernel(const float* pre, int pre_stride, const float* a_log,
+                                   const float* dt_bias, float* beta, float* decay, int H,
                                    size_t total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -51,7 +51,7 @@ ARLE_API int arle_delta_gates(const float* pre, int pre_stride, const float* a_l
   const size_t total = (size_t)num_tokens * H;
   size_t blocks = (total + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  launch_kernel(delta_gates_kernel, dim3((int)blocks), dim3(256), 0, s, 1, pre, pre_stride, a_log, dt_bias, beta, decay, H, total);
+  launch_early(delta_gates_kernel, dim3((int)blocks), dim3(256), 0, s, 1, pre, pre_stride, a_log, dt_bias, beta, decay, H, total);
   return launch_status();
 }
 

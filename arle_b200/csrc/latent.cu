@@ -28,10 +28,10 @@
 using namespace arle;
 
 template <typename T>
-__global__ void latent_prep_kernel(const T* q, int q_stride, const T* __restrict__ dkv, int dkv_stride,
-                                   const int* __restrict__ positions, const int* __restrict__ slot_mapping,
-                                   const float* __restrict__ c_weight, float eps, const float* __restrict__ inv_freq,
-                                   int rot_dims, int pairing, float amplitude, T* __restrict__ cache, T* q_out, long out_stride, int out_head,
+__global__ void latent_prep_kernel(const T* q, int q_stride, const T* dkv, int dkv_stride,
+                                   const int* positions, const int* slot_mapping,
+                                   const float* c_weight, float eps, const float* inv_freq,
+                                   int rot_dims, int pairing, float amplitude, T* cache, T* q_out, long out_stride, int out_head,
                                    int out_at, int H, int dn, int dr, int rank) {
   pdl_launch_dependents();
   pdl_wait();
@@ -49,34 +49,68 @@ __global__ void latent_prep_kernel(const T* q, int q_stride, const T* __restrict
   // unit i of a rotated vector p into o: the pair i (pairing 0: numbers i and i + half; 1: neighbours 2i and 2i + 1), or past the
   // pairs one of the numbers that pass
   const int units = half + dr - rot_dims;
-  auto turned = [&](const T* p, T* o, int i) {
+  auto read = [&](const T* p, int i, T& u, T& v) {
     if (i >= half) {
-      o[i - half + rot_dims] = p[i - half + rot_dims];
+      u = p[i - half + rot_dims];
       return;
     }
-    const int e0 = pairing ? 2 * i : i, e1 = pairing ? 2 * i + 1 : i + half;
-    const float cs = turn[i].x, sn = turn[i].y;
-    const float u = to_f32(p[e0]), v = to_f32(p[e1]);
-    o[e0] = from_f32<T>(u * cs - v * sn);
-    o[e1] = from_f32<T>(v * cs + u * sn);
+    u = p[pairing ? 2 * i : i], v = p[pairing ? 2 * i + 1 : i + half];
   };
+  auto write = [&](T* o, int i, T u, T v) {
+    if (i >= half) {
+      o[i - half + rot_dims] = u;
+      return;
+    }
+    const float cs = turn[i].x, sn = turn[i].y, x = to_f32(u), y = to_f32(v);
+    o[pairing ? 2 * i : i] = from_f32<T>(x * cs - y * sn);
+    o[pairing ? 2 * i + 1 : i + half] = from_f32<T>(y * cs + x * sn);
+  };
+  // Loads go ahead of stores a few at a time: q_out may be q, so that the compiler keeps their order.
+  constexpr int AHEAD = 4;
   const T* kv = dkv + (size_t)t * dkv_stride;
   if (cache != nullptr) {
-    float ss = 0.f;
-    for (int c = threadIdx.x; c < rank; c += blockDim.x) {
-      const float x = to_f32(kv[c]);
-      ss += x * x;
+    float x[AHEAD], ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) {
+      const int c = threadIdx.x + k * blockDim.x;
+      x[k] = c < rank ? to_f32(kv[c]) : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) ss += x[k] * x[k];
+    for (int c = threadIdx.x + AHEAD * blockDim.x; c < rank; c += blockDim.x) {
+      const float y = to_f32(kv[c]);
+      ss += y * y;
     }
     const float total = block_sum(ss, red);
     const float inv = 1.0f / sqrtf(total / (float)rank + eps);
     T* dst = cache + (size_t)slot_mapping[t] * kd;
-    for (int c = threadIdx.x; c < rank; c += blockDim.x) dst[c] = from_f32<T>(to_f32(kv[c]) * inv * c_weight[c]);
-    for (int i = threadIdx.x; i < units; i += blockDim.x) turned(kv + rank, dst + rank, i);
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) {
+      const int c = threadIdx.x + k * blockDim.x;
+      if (c < rank) dst[c] = from_f32<T>(x[k] * inv * c_weight[c]);
+    }
+    for (int c = threadIdx.x + AHEAD * blockDim.x; c < rank; c += blockDim.x) dst[c] = from_f32<T>(to_f32(kv[c]) * inv * c_weight[c]);
+    for (int i = threadIdx.x; i < units; i += blockDim.x) {
+      T u, v;
+      read(kv + rank, i, u, v);
+      write(dst + rank, i, u, v);
+    }
   }
-#pragma unroll 4
-  for (int idx = threadIdx.x; idx < H * units; idx += blockDim.x) {
-    const int h = idx / units, i = idx - h * units;
-    turned(q + (size_t)t * q_stride + (size_t)h * (dn + dr) + dn, q_out + (size_t)t * out_stride + (size_t)h * out_head + out_at, i);
+  const T* qt = q + (size_t)t * q_stride + dn;
+  T* ot = q_out + (size_t)t * out_stride + out_at;
+  for (int i0 = threadIdx.x; i0 < H * units; i0 += AHEAD * blockDim.x) {
+    T u[AHEAD], v[AHEAD];
+    int head[AHEAD], at[AHEAD];
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) {
+      const int idx = i0 + k * blockDim.x;
+      head[k] = idx / units;
+      at[k] = idx - head[k] * units;
+      if (idx < H * units) read(qt + (size_t)head[k] * (dn + dr), at[k], u[k], v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k)
+      if (i0 + k * blockDim.x < H * units) write(ot + (size_t)head[k] * out_head, at[k], u[k], v[k]);
   }
 }
 
@@ -92,11 +126,11 @@ ARLE_API int arle_latent_prep(const void* q, int q_stride, const void* dkv, int 
   const size_t smem = (size_t)rot_dims / 2 * sizeof(float2);
   if (smem > 40 * 1024) return ARLE_E_UNSUPPORTED;
   if (dtype == 0)
-    launch_kernel(latent_prep_kernel<float>, dim3(num_tokens), dim3(threads), smem, s, 1, (const float*)q, q_stride, (const float*)dkv,
+    launch_early(latent_prep_kernel<float>, dim3(num_tokens), dim3(threads), smem, s, 1, (const float*)q, q_stride, (const float*)dkv,
                   dkv_stride, positions, slot_mapping, c_weight, eps, inv_freq, rot_dims, pairing, amplitude, (float*)cache, (float*)q_out,
                   out_stride, out_head, out_at, H, dn, dr, rank);
   else if (dtype == 1)
-    launch_kernel(latent_prep_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), smem, s, 1, (const __nv_bfloat16*)q, q_stride,
+    launch_early(latent_prep_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), smem, s, 1, (const __nv_bfloat16*)q, q_stride,
                   (const __nv_bfloat16*)dkv, dkv_stride, positions, slot_mapping, c_weight, eps, inv_freq, rot_dims, pairing, amplitude,
                   (__nv_bfloat16*)cache, (__nv_bfloat16*)q_out, out_stride, out_head, out_at, H, dn, dr, rank);
   else

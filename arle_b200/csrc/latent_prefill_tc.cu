@@ -102,8 +102,8 @@ __device__ __forceinline__ unsigned int draw_ticket(int nblocks, int slot) {
 
 // plan: [R] (first key, place of that key in the built arrays of its group or -1).  A row is built from at most max(most * its queries,
 // floor) records, a group holds at most `room`.
-__global__ void __launch_bounds__(32) latent_plan_kernel(const int* __restrict__ q_indptr, const int* __restrict__ kv_lens, int R, int least,
-                                                         int most, int floor, int room, int window, int2* __restrict__ plan) {
+__global__ void __launch_bounds__(32) latent_plan_kernel(const int* q_indptr, const int* kv_lens, int R, int least,
+                                                         int most, int floor, int room, int window, int2* plan) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x;
@@ -135,10 +135,10 @@ constexpr int kGatherThreads = 256, kGatherSteps = 16 * (512 + 64) / 8 / kGather
 
 // A block copies 16 neighbouring records (pages hold a multiple of 16), 16 bytes a thread and step.  kd: numbers of a stored record, ko
 // of a gathered one.
-__global__ void __launch_bounds__(kGatherThreads) latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table,
-                                                                       int bt_stride, const int* __restrict__ kv_lens,
-                                                                       const int2* __restrict__ plan, int R, int page_size, int rank, int kd, int ko,
-                                                                       __nv_bfloat16* __restrict__ out) {
+__global__ void __launch_bounds__(kGatherThreads) latent_gather_kernel(const __nv_bfloat16* cache, const int* block_table,
+                                                                       int bt_stride, const int* kv_lens,
+                                                                       const int2* plan, int R, int page_size, int rank, int kd, int ko,
+                                                                       __nv_bfloat16* out) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ int bad[16];                                  // records whose latent holds an infinity or a NaN
@@ -667,7 +667,7 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mr, 
 ARLE_API int arle_latent_plan(const int* q_indptr, const int* kv_lens, int R, int least, int most, int floor, int room, int window, int* plan,
                               cudaStream_t s) {
   if (R <= 0) return 0;
-  launch_kernel(latent_plan_kernel, dim3(1), dim3(32), 0, s, 1, q_indptr, kv_lens, R, least, most, floor, room, window, (int2*)plan);
+  launch_early(latent_plan_kernel, dim3(1), dim3(32), 0, s, 1, q_indptr, kv_lens, R, least, most, floor, room, window, (int2*)plan);
   return launch_status();
 }
 
@@ -679,7 +679,7 @@ ARLE_API int arle_latent_gather(const void* cache, const int* block_table, int b
   if (page_size % 16 || rank <= 0 || rank > 512 || rank % 8 || dr < 0 || dr > 64 || dr % 8 || places % 16 || ((uintptr_t)cache & 15) ||
       ((uintptr_t)out & 15))
     return ARLE_E_UNSUPPORTED;
-  launch_kernel(latent_gather_kernel, dim3(places / 16), dim3(kGatherThreads), 0, s, 1, (const __nv_bfloat16*)cache, block_table, bt_stride, kv_lens,
+  launch_early(latent_gather_kernel, dim3(places / 16), dim3(kGatherThreads), 0, s, 1, (const __nv_bfloat16*)cache, block_table, bt_stride, kv_lens,
                 (const int2*)plan, R, page_size, rank, rank + dr, rank + gathered_tail(dr), (__nv_bfloat16*)out);
   return launch_status();
 }

@@ -103,8 +103,8 @@ __global__ void moe_select_kernel(const float* __restrict__ z, int z_stride, con
 // in 4 groups, 64 tokens 4.1 us (12.6 there), 2,048 tokens 4.8 (14.1).
 constexpr int kSelectWarps = 4;
 template <int PER, bool GROUPS>
-__global__ void moe_select_warp_kernel(const float* __restrict__ z, int z_stride, const float* __restrict__ correction, int E, int top, int groups,
-                                       int keep, float scale, int mode, int* __restrict__ ids, float* __restrict__ wts, int num_tokens) {
+__global__ void moe_select_warp_kernel(const float* z, int z_stride, const float* correction, int E, int top, int groups,
+                                       int keep, float scale, int mode, int* ids, float* wts, int num_tokens) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -206,7 +206,7 @@ ARLE_API int arle_moe_select(const float* z, int z_stride, const float* correcti
     auto kernel = keep < groups ? (E <= 32 ? moe_select_warp_kernel<1, true> : E <= 64 ? moe_select_warp_kernel<2, true> : moe_select_warp_kernel<8, true>)
                                 : (E <= 32 ? moe_select_warp_kernel<1, false> : E <= 64 ? moe_select_warp_kernel<2, false> : moe_select_warp_kernel<8, false>);
     const int warps = num_tokens <= 592 ? 1 : kSelectWarps;
-    launch_kernel(kernel, dim3((num_tokens + warps - 1) / warps), dim3(32 * warps), 0, s, 1, z, z_stride, correction, E, top, groups, keep, scale, mode, ids, wts,
+    launch_early(kernel, dim3((num_tokens + warps - 1) / warps), dim3(32 * warps), 0, s, 1, z, z_stride, correction, E, top, groups, keep, scale, mode, ids, wts,
                   num_tokens);
     return launch_status();
   }
@@ -218,38 +218,63 @@ ARLE_API int arle_moe_select(const float* z, int z_stride, const float* correcti
 constexpr int kMoeTile = 64;
 constexpr int kMoeMaxExperts = 1024;
 
-// plan (int32): [0, E] offsets of the experts' runs; [E + 1] tiles in use; then per tile (expert, first place, places).
-__global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ ids, int pairs, int top, int E, int* __restrict__ plan,
-                                                        int* __restrict__ place_of_pair, int* __restrict__ row_of_place, int max_tiles,
-                                                        const float* __restrict__ wts, float* __restrict__ weight_of_place) {
+// plan (int32): [0, E] offsets of the experts' runs; [E + 1] tiles in use; then per tile (expert, first place, places).  One block; a warp's pairs
+// of one expert are counted and placed together (the 32 experts of a prompt are 32 words of shared memory), a warp writes the runs and their tiles.
+__global__ void __launch_bounds__(1024) moe_plan_kernel(const int* ids, int pairs, int top, int E, int* plan,
+                                                        int* place_of_pair, int* row_of_place, int max_tiles,
+                                                        const float* wts, float* weight_of_place) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ int count[kMoeMaxExperts], offset[kMoeMaxExperts + 1], cursor[kMoeMaxExperts];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = cursor[e] = 0;
+  __shared__ int count[kMoeMaxExperts], cursor[kMoeMaxExperts];          // cursor: the next place of an expert's run
+  const int lane = threadIdx.x & 31, stride = blockDim.x;
+  for (int e = threadIdx.x; e < E; e += stride) count[e] = 0;
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&count[ids[p]], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0, tiles = 0;
-    int* tt = plan + E + 2;
-    for (int e = 0; e < E; ++e) {
-      offset[e] = at;
-      plan[e] = at;
-      for (int r0 = 0; r0 < count[e] && tiles < max_tiles; r0 += kMoeTile, ++tiles) {
-        tt[3 * tiles] = e;
-        tt[3 * tiles + 1] = at + r0;
-        tt[3 * tiles + 2] = min(kMoeTile, count[e] - r0);
-      }
-      at += count[e];
-    }
-    offset[E] = at;
-    plan[E] = at;
-    plan[E + 1] = tiles;
+  // The lanes of a warp that have the same expert count as one; first: the first of them.
+  auto together = [&](int p, int& e, uint32_t& same) {
+    e = p < pairs ? ids[p] : -1;
+    same = __match_any_sync(0xffffffffu, e);
+    return e >= 0 && __ffs(same) - 1 == lane;
+  };
+  for (int p0 = 0; p0 < pairs; p0 += stride) {
+    int e;
+    uint32_t same;
+    if (together(p0 + threadIdx.x, e, same)) atomicAdd(&count[e], __popc(same));
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const int e = ids[p];
-    const int place = offset[e] + atomicAdd(&cursor[e], 1);
+  if (threadIdx.x < 32) {                                  // the runs' first places and the first of their tiles
+    int* tt = plan + E + 2;
+    int at = 0, tiles = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, c = e < E ? count[e] : 0, k = (c + kMoeTile - 1) / kMoeTile;
+      int places = c, used = k;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, places, o), v = __shfl_up_sync(0xffffffffu, used, o);
+        if (lane >= o) places += u, used += v;
+      }
+      const int first = at + places - c, tile = tiles + used - k;
+      if (e < E) {
+        plan[e] = cursor[e] = first;
+        for (int j = 0; j < k && tile + j < max_tiles; ++j) {
+          tt[3 * (tile + j)] = e;
+          tt[3 * (tile + j) + 1] = first + j * kMoeTile;
+          tt[3 * (tile + j) + 2] = min(kMoeTile, c - j * kMoeTile);
+        }
+      }
+      at += __shfl_sync(0xffffffffu, places, 31);
+      tiles += __shfl_sync(0xffffffffu, used, 31);
+    }
+    if (lane == 0) plan[E] = at, plan[E + 1] = min(tiles, max_tiles);
+  }
+  __syncthreads();
+  for (int p0 = 0; p0 < pairs; p0 += stride) {
+    const int p = p0 + threadIdx.x;
+    int e, base = 0;
+    uint32_t same;
+    if (together(p, e, same)) base = atomicAdd(&cursor[e], __popc(same));
+    base = __shfl_sync(0xffffffffu, base, __ffs(same) - 1);
+    if (e < 0) continue;
+    const int place = base + __popc(same & ((1u << lane) - 1));
     place_of_pair[p] = place;
     row_of_place[place] = p / top;
     if (wts) weight_of_place[place] = wts[p];
@@ -263,7 +288,7 @@ ARLE_API int arle_moe_plan(const int* ids, int pairs, int top, int E, int* plan,
   if (pairs <= 0) return 0;
   if (E <= 0 || E > kMoeMaxExperts || top <= 0) return ARLE_E_UNSUPPORTED;
   if ((wts == nullptr) != (weight_of_place == nullptr)) return ARLE_E_BADARG;
-  launch_kernel(moe_plan_kernel, dim3(1), dim3(1024), 0, s, 1, ids, pairs, top, E, plan, place_of_pair, row_of_place,
+  launch_early(moe_plan_kernel, dim3(1), dim3(1024), 0, s, 1, ids, pairs, top, E, plan, place_of_pair, row_of_place,
                 pairs / kMoeTile + E + 1, wts, weight_of_place);
   return launch_status();
 }
@@ -530,9 +555,9 @@ ARLE_API int arle_moe_gemm(const void* A, int lda, const int* rows, const void* 
 
 // VEC columns a thread, one column tile of a token a block: every load of a thread is asked for before the sum is formed.
 template <typename T, int VEC>
-__global__ void moe_combine_kernel(const T* __restrict__ y, int y_stride, const int* __restrict__ place_of_pair,
-                                   const float* __restrict__ wts, int top, const T* __restrict__ shared, int shared_stride,
-                                   const float* __restrict__ gate, int gate_stride, T* __restrict__ out, int out_stride, int width) {
+__global__ void moe_combine_kernel(const T* y, int y_stride, const int* place_of_pair,
+                                   const float* wts, int top, const T* shared, int shared_stride,
+                                   const float* gate, int gate_stride, T* out, int out_stride, int width) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
@@ -569,10 +594,10 @@ ARLE_API int arle_moe_combine(const void* y, int y_stride, const int* place_of_p
   const int per = threads * (vec ? n : 1);
   const dim3 grid(num_tokens, (width + per - 1) / per);
   if (dtype == 0)
-    launch_kernel(vec ? moe_combine_kernel<float, 4> : moe_combine_kernel<float, 1>, grid, dim3(threads), 0, s, 1, (const float*)y, y_stride, place_of_pair, wts, top,
+    launch_early(vec ? moe_combine_kernel<float, 4> : moe_combine_kernel<float, 1>, grid, dim3(threads), 0, s, 1, (const float*)y, y_stride, place_of_pair, wts, top,
                   (const float*)shared, shared_stride, gate, gate_stride, (float*)out, out_stride, width);
   else if (dtype == 1)
-    launch_kernel(vec ? moe_combine_kernel<__nv_bfloat16, 8> : moe_combine_kernel<__nv_bfloat16, 1>, grid, dim3(threads), 0, s, 1, (const __nv_bfloat16*)y, y_stride,
+    launch_early(vec ? moe_combine_kernel<__nv_bfloat16, 8> : moe_combine_kernel<__nv_bfloat16, 1>, grid, dim3(threads), 0, s, 1, (const __nv_bfloat16*)y, y_stride,
                   place_of_pair, wts, top, (const __nv_bfloat16*)shared, shared_stride, gate, gate_stride, (__nv_bfloat16*)out,
                   out_stride, width);
   else

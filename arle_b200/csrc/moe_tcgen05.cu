@@ -342,13 +342,22 @@ int launch(const void* x, int ldx, int x_rows, const void* W, void* out, int ldo
 }
 
 // dst[place] = x[rows[place]], 16 bytes a thread and step.
-__global__ void __launch_bounds__(256) moe_rows_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int* __restrict__ rows,
-                                                       __nv_bfloat16* __restrict__ dst, int K) {
+__global__ void __launch_bounds__(256) moe_rows_kernel(const __nv_bfloat16* x, int ldx, const int* rows,
+                                                       __nv_bfloat16* dst, int K) {
   pdl_launch_dependents();
   pdl_wait();
   const uint4* from = reinterpret_cast<const uint4*>(x + (size_t)rows[blockIdx.x] * ldx);
   uint4* to = reinterpret_cast<uint4*>(dst + (size_t)blockIdx.x * K);
-  for (int i = threadIdx.x; i < K / 8; i += 256) to[i] = from[i];
+  constexpr int AHEAD = 4;                                 // loads in front of the stores, which they could not pass
+  for (int i0 = threadIdx.x; i0 < K / 8; i0 += 256 * AHEAD) {
+    uint4 v[AHEAD];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+      if (i0 + j * 256 < K / 8) v[j] = from[i0 + j * 256];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+      if (i0 + j * 256 < K / 8) to[i0 + j * 256] = v[j];
+  }
 }
 
 }  // namespace
@@ -357,7 +366,7 @@ __global__ void __launch_bounds__(256) moe_rows_kernel(const __nv_bfloat16* __re
 ARLE_API int arle_moe_rows(const void* x, int ldx, const int* rows, void* dst, int pairs, int K, cudaStream_t s) {
   if (pairs <= 0) return 0;
   if (K <= 0 || K % 8 || ldx % 8 || (((uintptr_t)x | (uintptr_t)dst) & 15)) return ARLE_E_UNSUPPORTED;
-  launch_kernel(moe_rows_kernel, dim3(pairs), dim3(256), 0, s, 1, (const __nv_bfloat16*)x, ldx, rows, (__nv_bfloat16*)dst, K);
+  launch_early(moe_rows_kernel, dim3(pairs), dim3(256), 0, s, 1, (const __nv_bfloat16*)x, ldx, rows, (__nv_bfloat16*)dst, K);
   return launch_status();
 }
 

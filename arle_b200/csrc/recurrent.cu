@@ -430,8 +430,8 @@ ARLE_API int arle_mlstm_out(const float* num, const float* floor_, const void* g
 }
 
 // ------------------------------------------------------------------------------------------------ state space
-__global__ void ssm_gates_kernel(const float* __restrict__ dt_raw, int dt_stride, const float* __restrict__ dt_bias,
-                                 const float* __restrict__ a_log, float* __restrict__ a, float* __restrict__ b, int H, size_t total) {
+__global__ void ssm_gates_kernel(const float* dt_raw, int dt_stride, const float* dt_bias,
+                                 const float* a_log, float* a, float* b, int H, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
@@ -451,7 +451,7 @@ ARLE_API int arle_ssm_gates(const float* dt_raw, int dt_stride, const float* dt_
   const size_t total = (size_t)num_tokens * H;
   size_t blocks = (total + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  launch_kernel(ssm_gates_kernel, dim3((int)blocks), dim3(256), 0, s, 1, dt_raw, dt_stride, dt_bias, a_log, a, b, H, total);
+  launch_early(ssm_gates_kernel, dim3((int)blocks), dim3(256), 0, s, 1, dt_raw, dt_stride, dt_bias, a_log, a, b, H, total);
   return launch_status();
 }
 

@@ -36,22 +36,38 @@ __global__ void rms_rows_warp_kernel(const TI* __restrict__ x, int x_stride, con
   for (int c = lane; c < n; c += 32) orow[c] = from_f32<TO>(to_f32(xr[c]) * inv * (weight ? weight[c] : 1.0f));
 }
 
+// The first 2,048 numbers of a row are kept in registers: read once, all loads under way together (2,048 rows of 1,536, bfloat16, 9.5 us when they
+// were read twice).  Launched early: plain loads.
 template <typename TI, typename TO>
-__global__ void rms_rows_block_kernel(const TI* __restrict__ x, int x_stride, const float* __restrict__ weight, TO* __restrict__ out,
-                                      int out_stride, int n, float eps) {
+__global__ void rms_rows_block_kernel(const TI* x, int x_stride, const float* weight, TO* out, int out_stride, int n, float eps) {
   pdl_launch_dependents();
   pdl_wait();
+  constexpr int KEPT = 8;
   __shared__ float red[33];
   const int t = blockIdx.x;
   const TI* xr = x + (size_t)t * x_stride;
-  float ss = 0.f;
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    const float v = to_f32(xr[c]);
-    ss += v * v;
+  float v[KEPT], w[KEPT], ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < KEPT; ++k) {
+    const int c = threadIdx.x + k * blockDim.x;
+    v[k] = c < n ? to_f32(xr[c]) : 0.f;
+    w[k] = weight && c < n ? weight[c] : 1.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < KEPT; ++k) ss += v[k] * v[k];
+  for (int c = threadIdx.x + KEPT * blockDim.x; c < n; c += blockDim.x) {
+    const float u = to_f32(xr[c]);
+    ss += u * u;
   }
   const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)n + eps);
   TO* orow = out + (size_t)t * out_stride;
-  for (int c = threadIdx.x; c < n; c += blockDim.x) orow[c] = from_f32<TO>(to_f32(xr[c]) * inv * (weight ? weight[c] : 1.0f));
+#pragma unroll
+  for (int k = 0; k < KEPT; ++k) {
+    const int c = threadIdx.x + k * blockDim.x;
+    if (c < n) orow[c] = from_f32<TO>(v[k] * inv * w[k]);
+  }
+  for (int c = threadIdx.x + KEPT * blockDim.x; c < n; c += blockDim.x)
+    orow[c] = from_f32<TO>(to_f32(xr[c]) * inv * (weight ? weight[c] : 1.0f));
 }
 
 template <typename TI, typename TO>
@@ -62,7 +78,7 @@ static int launch_rms_rows(const void* x, int x_stride, const float* weight, voi
     launch_kernel(rms_rows_warp_kernel<TI, TO>, dim3((num_rows + warps - 1) / warps), dim3(warps * 32), 0, s, 1, (const TI*)x, x_stride,
                   weight, (TO*)out, out_stride, n, eps, num_rows);
   } else {
-    launch_kernel(rms_rows_block_kernel<TI, TO>, dim3(num_rows), dim3(256), 0, s, 1, (const TI*)x, x_stride, weight, (TO*)out, out_stride,
+    launch_early(rms_rows_block_kernel<TI, TO>, dim3(num_rows), dim3(256), 0, s, 1, (const TI*)x, x_stride, weight, (TO*)out, out_stride,
                   n, eps);
   }
   return launch_status();

@@ -44,3 +44,30 @@ def test_the_streamed_decode_attention_starts_early_and_reads_plainly():
         assert not re.search(r"\.nc\b|__ldg\(|__restrict__", body)
     body = re.sub(r"//[^\n]*", "", kernel)
     assert body.index("pdl_wait();") < min(body.index(x) for x in ("q_indptr[", "plan[", "rows_plan[i]", "stream_shares(q_indptr", "block_table +") if x in body)
+
+
+def test_kernels_that_are_launched_early_read_plainly():
+    """Every kernel that goes through launch_early, or through launch_kernel_as with a condition of its own: no restrict on what it reads, no
+    __ldg, and a wait before anything else."""
+    found = set()
+    for f in sorted(CSRC.glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", f.read_text())
+        names = set()
+        for m in re.finditer(r"launch_(?:early\(|kernel_as\()([^;]*);", text):
+            names |= set(re.findall(r"\b\w+_kernel\b", m.group(1)))
+            if re.match(r"\s*kernel\b", m.group(1)):
+                names |= set(re.findall(r"\b\w+_kernel\b", text[text.rindex("auto kernel", 0, m.start()): m.start()]))
+        for name in names:
+            at = re.search(r"__global__[^;{]*?\b" + name + r"\s*\(", text)
+            if at is None:
+                continue
+            end = text.index("\n}\n", at.end())
+            body = text[at.end(): end]
+            assert not re.search(r"\.nc\b|__ldg\(", body), name
+            if name in ("skinny_gemm_kernel", "direct_gemm_kernel"):      # their weights and rows go through loads of their own
+                continue
+            assert "__restrict__" not in body and "pdl_wait();" in body, name
+            found.add(name)
+    assert {"moe_plan_kernel", "moe_rows_kernel", "moe_combine_kernel", "moe_select_warp_kernel", "latent_prep_kernel", "latent_gather_kernel",
+            "latent_plan_kernel", "rms_rows_block_kernel", "rmsnorm_vec_kernel", "silu_mul_bf16_vec_kernel", "decode_stream_kernel",
+            "delta_gates_kernel", "ssm_gates_kernel", "rotary_angles_kernel"} <= found
