@@ -19,7 +19,8 @@
 //    over the column's lanes.  What bounds it is a warp's instructions: a scheduler of the SM has one warp of a single prompt.  So
 //    two channels are one packed instruction (fma.rn.f32x2), and the sums of eight tokens and four columns are added over the 32 lanes
 //    together, 31 exchanges instead of 48.  The next chunk's loads are pinned in front
-//    of the work that hides them (plain ones were moved behind it).  16 heads of 128 x 128, 2,048 tokens: 213 us (444 with single
+//    of the work that hides them (plain ones were moved behind it), and where there are few blocks four warps more bring them.  16 heads of
+//    128 x 128, 2,048 tokens: 190 us (213 where the same warps bring them, 444 with single
 //    numbers and a token's sums by themselves, 269 before the loads were pinned).  The order of every sum depends on (dim, vdim) only: a token's result
 //    does not depend on how the prompt was cut or on what else is in the batch.
 //    With a bonus u (one number per head and key channel) the read-out comes before the update and sees the current
@@ -123,8 +124,20 @@ constexpr int few_blocks() {
   if (LPC == 1) return 3;
   return VEC && !BONUS && LPC >= 4 ? 5 : 4;
 }
-template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool LONG>
-__global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LPC, VEC, BONUS>()) gla_scan_kernel(
+// SPLIT (32 lanes of four channels a column): four warps more, which bring the chunks, so that the four that hold the memory do nothing else.  Chunks
+// of eight tokens go through a ring of kRing places, two more are under way in the loaders' registers.
+constexpr int kRing = 3;
+__device__ __forceinline__ void named_sync(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(2 * kScanThreads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "n"(2 * kScanThreads) : "memory");
+}
+
+template <typename T, int DPT, int LPC, bool VEC, bool BONUS, bool LONG, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 2 * kScanThreads : kScanThreads, SPLIT ? 2 : LONG ? 1 : few_blocks<T, DPT, LPC, VEC, BONUS>()) gla_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, int in_stride,
     const float* __restrict__ alpha, const float* __restrict__ bonus, float* __restrict__ state, long slot_stride, const int* __restrict__ q_indptr,
     const int* __restrict__ state_slots, float* __restrict__ out, int heads, int dim, int vdim, float q_scale) {
@@ -136,15 +149,17 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
   constexpr int PAD = DPT == 4 ? 4 : DPT + 4;    // floats a thread's channels take in shared memory: 16-byte rows, spread over the banks
   constexpr int DPAD = PAD * LPC;
   // float32 rows with a bonus, decoded: at 16 tokens a chunk the numbers under way spill at four blocks an SM
-  constexpr int CHUNK = DSPAN >= 512 ? 4 : (DSPAN >= 256 || (!LONG && BONUS && sizeof(T) == 4) ? 8 : 16);
+  constexpr int CHUNK = SPLIT ? 8 : DSPAN >= 512 ? 4 : (DSPAN >= 256 || (!LONG && BONUS && sizeof(T) == 4) ? 8 : 16);
   constexpr int QUADS = CHUNK * DSPAN / 4;       // groups of four channels in a chunk
   constexpr int QPT = (QUADS + kScanThreads - 1) / kScanThreads;
   constexpr int VPT = (CHUNK * COLS + kScanThreads - 1) / kScanThreads;
-  __shared__ __align__(16) float qs[CHUNK * DPAD], ks[CHUNK * DPAD], as[CHUNK * DPAD];
+  constexpr int PLACES = SPLIT ? kRing : 1;
+  __shared__ __align__(16) float qs[PLACES * CHUNK * DPAD], ks[PLACES * CHUNK * DPAD], as[PLACES * CHUNK * DPAD];
   constexpr int VD = LONG && LPC >= 4 ? 2 : 1;           // v's numbers stand twice side by side (a factor of both halves of a pair), where there is room
-  __shared__ __align__(16) float vs[CHUNK * COLS * VD];
+  __shared__ __align__(16) float vs[PLACES * CHUNK * COLS * VD];
   const int r = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * COLS;
-  const int l = threadIdx.x & (LPC - 1), jl = threadIdx.x / LPC;
+  const int tid = threadIdx.x & (kScanThreads - 1);    // among the loaders, or among those that hold the memory
+  const int l = tid & (LPC - 1), jl = tid / LPC;
   const int jb = j0 + jl * CPT;                  // this thread's first column
   const int t_begin = q_indptr[r], t_end = q_indptr[r + 1];
   // the state of a head is kept as [vdim][dim]: a thread's channels of a column are contiguous
@@ -161,7 +176,7 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
   f32x2 S[CPT][DPT / 2];                         // channels 2i and 2i + 1 of a column
 #pragma unroll
   for (int cc = 0; cc < CPT; ++cc) {
-    const bool col_ok = jb + cc < vdim;
+    const bool col_ok = jb + cc < vdim && !(SPLIT && threadIdx.x >= kScanThreads);
     const float* sp = S_g + (size_t)(col_ok ? jb + cc : 0) * dim;
 #pragma unroll
     for (int i = 0; i < DPT; i += 4) {
@@ -180,16 +195,21 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
   const size_t hq = (size_t)h * dim, hv = (size_t)h * vdim;
   const size_t a_stride = (size_t)heads * dim;
   using RawT = typename Raw4<T, VEC>::type;
-  RawT rq[QPT], rk[QPT];
-  float4 ra[QPT];
-  T rv[VPT];
+  struct Raw {
+    RawT q[QPT], k[QPT];
+    float4 a[QPT];
+    T v[VPT];
+  };
 
   // The chunk's numbers into registers; nothing waits on them yet.  Loads are unconditional (a place outside the
   // chunk reads the row's first token instead and is zeroed when staged), so that they are all under way at once.
-  auto fetch = [&](int t0, int n) {
+  auto fetch = [&](Raw& raw, int t0, int n) {
+    RawT (&rq)[QPT] = raw.q, (&rk)[QPT] = raw.k;
+    float4 (&ra)[QPT] = raw.a;
+    T (&rv)[VPT] = raw.v;
 #pragma unroll
     for (int u = 0; u < QPT; ++u) {
-      const int idx = threadIdx.x + u * kScanThreads;
+      const int idx = tid + u * kScanThreads;
       const int tt = idx / (DSPAN / 4), c = (idx - tt * (DSPAN / 4)) * 4;
       const bool ok = idx < QUADS && tt < n && c < dim;
       const size_t row = ok ? (size_t)(t0 + tt) : (size_t)t_begin;
@@ -221,7 +241,7 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
     }
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
-      const int idx = threadIdx.x + u * kScanThreads;
+      const int idx = tid + u * kScanThreads;
       const int tt = idx / COLS, c = idx - tt * COLS;
       const bool ok = idx < CHUNK * COLS && tt < n && j0 + c < vdim;
       const T* vp = v + (ok ? (size_t)(t0 + tt) : (size_t)t_begin) * in_stride + hv + (ok ? j0 + c : 0);
@@ -229,12 +249,15 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
       else rv[u] = *vp;
     }
   };
-  auto stage = [&](int n) {                      // registers to shared memory, widened, q scaled on the way
+  auto stage = [&](const Raw& raw, int n, int place) {   // registers to shared memory, widened, q scaled on the way
+    const RawT (&rq)[QPT] = raw.q, (&rk)[QPT] = raw.k;
+    const float4 (&ra)[QPT] = raw.a;
+    const T (&rv)[VPT] = raw.v;
 #pragma unroll
     for (int u = 0; u < QPT; ++u) {
-      const int idx = threadIdx.x + u * kScanThreads;
+      const int idx = tid + u * kScanThreads;
       const int tt = idx / (DSPAN / 4), c = (idx - tt * (DSPAN / 4)) * 4;
-      const int at = tt * DPAD + (c / DPT) * PAD + (c % DPT);
+      const int at = (place * CHUNK + tt) * DPAD + (c / DPT) * PAD + (c % DPT);
       if (idx >= QUADS) continue;
       const bool ok = tt < n && c < dim;
       const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -245,31 +268,65 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
     }
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
-      const int idx = threadIdx.x + u * kScanThreads;
+      const int idx = tid + u * kScanThreads;
       const int tt = idx / COLS, c = idx - tt * COLS;
       if (idx < CHUNK * COLS) {
         const float x = (tt < n && j0 + c < vdim) ? to_f32(rv[u]) : 0.f;
-        if (VD == 2) *reinterpret_cast<float2*>(vs + VD * idx) = make_float2(x, x);
-        else vs[idx] = x;
+        if (VD == 2) *reinterpret_cast<float2*>(vs + VD * (place * CHUNK * COLS + idx)) = make_float2(x, x);
+        else vs[place * CHUNK * COLS + idx] = x;
       }
     }
   };
 
-  if (t_begin < t_end) fetch(t_begin, min(CHUNK, t_end - t_begin));
+  Raw raw;
+  if constexpr (SPLIT) {
+    // Barriers 1 .. kRing: a place is full; kRing + 1 .. 2 kRing: it has been read (waited for, and arrived at, where a later chunk needs it).
+    const int chunks = (t_end - t_begin + CHUNK - 1) / CHUNK;
+    if (threadIdx.x >= kScanThreads) {
+      Raw other;
+      auto get = [&](Raw& to, int c) {
+        if (c < chunks) fetch(to, t_begin + c * CHUNK, min(CHUNK, t_end - t_begin - c * CHUNK));
+      };
+      auto put = [&](Raw& from, int c) {
+        if (c >= chunks) return;
+        const int place = c % kRing;
+        if (c >= kRing) named_sync(kRing + 1 + place);
+        stage(from, min(CHUNK, t_end - t_begin - c * CHUNK), place);
+        named_arrive(1 + place);
+        get(from, c + 2);
+      };
+      get(raw, 0);
+      get(other, 1);
+      for (int c = 0; c < chunks; c += 2) {
+        put(raw, c);
+        put(other, c + 1);
+      }
+      return;
+    }
+  } else if (t_begin < t_end) {
+    fetch(raw, t_begin, min(CHUNK, t_end - t_begin));
+  }
+  int place = 0;
   for (int t0 = t_begin; t0 < t_end; t0 += CHUNK) {
     const int n = min(CHUNK, t_end - t0);
-    __syncthreads();                             // the chunk before has been read by everyone
-    stage(n);
-    __syncthreads();
-    if (t0 + CHUNK < t_end) fetch(t0 + CHUNK, min(CHUNK, t_end - t0 - CHUNK));
+    if constexpr (SPLIT) {
+      named_sync(1 + place);
+    } else {
+      __syncthreads();                           // the chunk before has been read by everyone
+      stage(raw, n, 0);
+      __syncthreads();
+      if (t0 + CHUNK < t_end) fetch(raw, t0 + CHUNK, min(CHUNK, t_end - t0 - CHUNK));
+    }
+    const float *qp = qs + place * CHUNK * DPAD, *kp = ks + place * CHUNK * DPAD, *ap = as + place * CHUNK * DPAD;
+    const float* vp = vs + place * CHUNK * COLS * VD;
     // one token: the memory's step and the thread's part of its columns' sums
     auto token = [&](int tt, float (&o)[CPT]) {
       if constexpr (!LONG) {                     // single numbers: the same roundings in fewer registers
-        const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT);
+        const float4 v4 = *reinterpret_cast<const float4*>(vp + tt * COLS + jl * CPT);
         const float vj[CPT] = {v4.x, v4.y, v4.z, v4.w};
-        const float4* qt = reinterpret_cast<const float4*>(qs + tt * DPAD + l * PAD);
-        const float4* kt = reinterpret_cast<const float4*>(ks + tt * DPAD + l * PAD);
-        const float4* at = reinterpret_cast<const float4*>(as + tt * DPAD + l * PAD);
+        const float4* qt = reinterpret_cast<const float4*>(qp + tt * DPAD + l * PAD);
+        const float4* kt = reinterpret_cast<const float4*>(kp + tt * DPAD + l * PAD);
+        const float4* at = reinterpret_cast<const float4*>(ap + tt * DPAD + l * PAD);
         float lo[CPT], hi[CPT];
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) lo[cc] = hi[cc] = 0.f;
@@ -297,16 +354,16 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
       }
       f32x2 vj[CPT];
       if constexpr (VD == 2) {
-        const ulonglong2 va = *reinterpret_cast<const ulonglong2*>(vs + (tt * COLS + jl * CPT) * 2);
-        const ulonglong2 vb = *reinterpret_cast<const ulonglong2*>(vs + (tt * COLS + jl * CPT) * 2 + 4);
+        const ulonglong2 va = *reinterpret_cast<const ulonglong2*>(vp + (tt * COLS + jl * CPT) * 2);
+        const ulonglong2 vb = *reinterpret_cast<const ulonglong2*>(vp + (tt * COLS + jl * CPT) * 2 + 4);
         vj[0] = va.x, vj[1] = va.y, vj[2] = vb.x, vj[3] = vb.y;
       } else {
-        const float4 v4 = *reinterpret_cast<const float4*>(vs + tt * COLS + jl * CPT);
+        const float4 v4 = *reinterpret_cast<const float4*>(vp + tt * COLS + jl * CPT);
         vj[0] = pair2(v4.x, v4.x), vj[1] = pair2(v4.y, v4.y), vj[2] = pair2(v4.z, v4.z), vj[3] = pair2(v4.w, v4.w);
       }
-      const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(qs + tt * DPAD + l * PAD);
-      const ulonglong2* kt = reinterpret_cast<const ulonglong2*>(ks + tt * DPAD + l * PAD);
-      const ulonglong2* at = reinterpret_cast<const ulonglong2*>(as + tt * DPAD + l * PAD);
+      const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(qp + tt * DPAD + l * PAD);
+      const ulonglong2* kt = reinterpret_cast<const ulonglong2*>(kp + tt * DPAD + l * PAD);
+      const ulonglong2* at = reinterpret_cast<const ulonglong2*>(ap + tt * DPAD + l * PAD);
       f32x2 o2[CPT];
 #pragma unroll
       for (int cc = 0; cc < CPT; ++cc) o2[cc] = 0;
@@ -384,6 +441,10 @@ __global__ void __launch_bounds__(kScanThreads, LONG ? 1 : few_blocks<T, DPT, LP
           if (l == 0 && jb + cc < vdim) out[(size_t)(t0 + tt) * heads * vdim + hv + jb + cc] = x;
         }
       }
+    }
+    if constexpr (SPLIT) {
+      if (t0 + kRing * CHUNK < t_end) named_arrive(kRing + 1 + place);
+      place = place + 1 == kRing ? 0 : place + 1;
     }
   }
 #pragma unroll
@@ -524,6 +585,12 @@ ARLE_API int arle_gla_decay(const void* low, int dtype, int low_stride, const fl
 
 namespace {
 
+// Loaders beside the memory's warps, while no SM has more than two such blocks.  Without them bringing the chunks and the barriers around that are
+// 60 of 213 us.  16 heads of 128 x 128, us, without and with: one row of 2,048 tokens (128 blocks) 213.5 and 189.8, of 512 57.9 and 51.8, 32 heads,
+// 1,024 tokens (256 blocks) 153.7 and 149.8; but three rows of 600 to 748 (384 blocks, three an SM without) 156.1 and 169.4, 16 rows of 13 25.1
+// and 29.1.
+inline bool takes_loaders(dim3 grid) { return (long long)grid.x * grid.y * grid.z <= 296; }
+
 template <typename T, int DPT, int LPC>
 int scan_launch(const void* q, const void* k, const void* v, int in_stride, const float* alpha, const float* bonus, float* state, long slot_stride, const int* q_indptr,
                 const int* state_slots, float* out, int rows, int heads, int dim, int vdim, float q_scale, int max_q_len, cudaStream_t s) {
@@ -532,13 +599,22 @@ int scan_launch(const void* q, const void* k, const void* v, int in_stride, cons
   const size_t eb = sizeof(T) * 4;               // bytes of four elements of q or k
   const bool vec = dim % 4 == 0 && in_stride % 4 == 0 && ((uintptr_t)q % eb) == 0 && ((uintptr_t)k % eb) == 0 &&
                    ((uintptr_t)alpha % 16) == 0;
-  auto kernel = max_q_len >= 8 ? (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, true> : gla_scan_kernel<T, DPT, LPC, false, true, true>)
-                                        : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, true> : gla_scan_kernel<T, DPT, LPC, false, false, true>))
-                       : (bonus ? (vec ? gla_scan_kernel<T, DPT, LPC, true, true, false> : gla_scan_kernel<T, DPT, LPC, false, true, false>)
-                                : (vec ? gla_scan_kernel<T, DPT, LPC, true, false, false> : gla_scan_kernel<T, DPT, LPC, false, false, false>));
-  launch_kernel(kernel, grid, dim3(kScanThreads), 0, s, 1, (const T*)q, (const T*)k, (const T*)v, in_stride, alpha, bonus, state, slot_stride,
-                q_indptr, state_slots, out, heads, dim, vdim, q_scale);
-  return launch_status();
+  auto run = [&](auto kernel, int threads) {
+    launch_kernel(kernel, grid, dim3(threads), 0, s, 1, (const T*)q, (const T*)k, (const T*)v, in_stride, alpha, bonus, state, slot_stride, q_indptr,
+                  state_slots, out, heads, dim, vdim, q_scale);
+    return launch_status();
+  };
+#define ARLE_FORM(LONG, SPLIT)                                                                                                    \
+  return bonus ? (vec ? run(gla_scan_kernel<T, DPT, LPC, true, true, LONG, SPLIT>, SPLIT ? 2 * kScanThreads : kScanThreads)       \
+                      : run(gla_scan_kernel<T, DPT, LPC, false, true, LONG, SPLIT>, SPLIT ? 2 * kScanThreads : kScanThreads))     \
+               : (vec ? run(gla_scan_kernel<T, DPT, LPC, true, false, LONG, SPLIT>, SPLIT ? 2 * kScanThreads : kScanThreads)      \
+                      : run(gla_scan_kernel<T, DPT, LPC, false, false, LONG, SPLIT>, SPLIT ? 2 * kScanThreads : kScanThreads))
+  if (max_q_len < 8) ARLE_FORM(false, false);
+  if constexpr (LPC == 32 && DPT == 4) {
+    if (takes_loaders(grid)) ARLE_FORM(true, true);
+  }
+  ARLE_FORM(true, false);
+#undef ARLE_FORM
 }
 
 // The split of the key channels among threads depends on dim alone, so the order of a token's sums does too: four
