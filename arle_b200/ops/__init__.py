@@ -18,6 +18,7 @@ cuBLAS through ``torch.mm``, as cklxx/arle calls cuBLASLt for all its projection
 from __future__ import annotations
 
 import ctypes
+import threading
 from ctypes import c_float, c_int, c_void_p
 
 import torch
@@ -26,6 +27,7 @@ from . import build as _build
 from . import launchers as _launchers
 
 _LIB = None
+_LIB_LOCK = threading.Lock()          # two threads' first calls: one builds
 _LAUNCHES = 0
 
 
@@ -137,7 +139,9 @@ def library():
     """The loaded CUDA library, a callable for each of its launchers; built on first use.  Raises if it cannot be had."""
     global _LIB
     if _LIB is None:
-        _LIB = _launchers.load(_build.library_path(), _SIGNATURES)
+        with _LIB_LOCK:
+            if _LIB is None:
+                _LIB = _launchers.load(_build.library_path(), _SIGNATURES)
     return _LIB
 
 
