@@ -31,11 +31,6 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
   return __float2bfloat16_rn(v);
 }
 
-// x * sigmoid(g), for a result that is rounded into T: in front of a bfloat16 rounding the fast exponential and division (a few units in the last
-// place of float32, a few instructions instead of some 30 and no branch), else the exact ones.
-template <typename T> __device__ __forceinline__ float times_sigmoid(float x, float g) { return x / (1.0f + expf(-g)); }
-template <> __device__ __forceinline__ float times_sigmoid<__nv_bfloat16>(float x, float g) { return __fdividef(x, 1.0f + __expf(-g)); }
-
 // Whether one of two bfloat16 numbers is an infinity or a NaN.
 __device__ __forceinline__ bool bf16x2_odd(uint32_t w) { return (w & 0x7f80u) == 0x7f80u || (w & 0x7f800000u) == 0x7f800000u; }
 

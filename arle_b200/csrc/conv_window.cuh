@@ -1,10 +1,12 @@
 // A causal convolution of four taps per channel over the tokens of every row, several tokens a thread: the four inputs of a token
 // slide through registers, so a row of x is read once (and the three before a thread's first token once more) instead of four times,
 // VEC channels an access.  Sums in the order of the kernels that take a token a thread (causal_conv, conv_silu): the same bits.
-// What bounds it: instructions (silu's exponential and division; memory is at half of its rate), and with exact ones in front of a bfloat16
-// rounding twice as much: 2,048 tokens of 10,240 channels, bfloat16, 84 MB 27.4 us in a graph (38 with the exact ones), 1,999 tokens of
-// 8,192 21.8 (33), 300 of 2,304 7.2.  Four channels a thread leave room for six blocks an SM; eight channels and three blocks 32.3, 27.7 and 8.9,
-// seven blocks 27.9, eight spill, two channels 30.6, 8 or 32 tokens a thread 29.8 and 29.1, eight tokens ahead 29.2.
+// What bounds it: instructions, the exponentials and divisions of silu above all (37 an element, and a division has a branch of its own, so that
+// the next one waits); memory is at a third of its rate.  Four channels a thread leave room for six blocks an SM: 2,048 tokens of 10,240
+// channels, bfloat16, 84 MB 37.2 us in a graph, 1,999 tokens of 8,192 30.0, 300 of 2,304 10.0 (eight channels a thread and three blocks an SM, five
+// blocks, two channels, 32 tokens a thread: all slower; eight blocks spill).  The fast exponential and division, 26.5 us, are
+// not taken: they round to another bfloat16 in one of 1,000 places; in front of a look at whether they could, with the full ones behind it, 34 us, but 55
+// where numbers are large.
 #pragma once
 #include "common.cuh"
 
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(kConvThreads, sizeof(TI) + sizeof(TO) == 4 ? 6
         win[0][i] = win[1][i];
         win[1][i] = win[2][i];
         win[2][i] = in;
-        y[i] = act == 1 ? times_sigmoid<TO>(acc, acc) : acc;
+        y[i] = act == 1 ? acc / (1.0f + expf(-acc)) : acc;
       }
       store_vec<TO, VEC>(out + (size_t)t * out_stride + c, y);
     }

@@ -25,8 +25,8 @@
 //   warps 0-7        : epilogue of the CTA's own 128 rows, two warps to 32 rows with every second 32 columns each: tcgen05.ld, convert (or apply
 //                      the gate to neighbouring columns), store; then arrive on the first CTA's `acc_empty`.
 // The accumulators are double-buffered (2 x 256 of the 512 TMEM columns): the tensor cores fill one while the
-// epilogue drains the other (with four warps and an exact division in the gate it took longer than the products of a short K: gated, 1,685 rows
-// of 6,144 x 1,024 46.5 us, now 30.8; 2,048 of 24,576 x 4,096 294 and 290.  The last round's tiles in halves of 128 columns: no change).  Edges: TMA zero-fills rows beyond M or N and columns beyond K; stores are
+// epilogue drains the other (with four warps it took longer than the products of a short K: gated, 1,685 rows of 6,144 x 1,024 47.0 us,
+// now 33.8; 2,048 of 24,576 x 4,096 294 and 294.  The last round's tiles in halves of 128 columns: no change).  Edges: TMA zero-fills rows beyond M or N and columns beyond K; stores are
 // guarded.  Every wait is bounded; a CTA whose wait runs out raises the error flag, stops issuing and runs to
 // its end (its partner's waits then run out in turn), and both meet at the cluster barrier before they free
 // their tensor memory.  No TMA load here is a multicast; the only cluster-wide operation besides the MMA is
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_pair_kernel(const __
           for (int i = 0; i < 16; ++i) {
             const float g = __uint_as_float(r[2 * i]), u = __uint_as_float(r[2 * i + 1]);
             v[i] = (act == 2 ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)))
-                             : times_sigmoid<__nv_bfloat16>(g, g)) * u;
+                             : g / (1.0f + __expf(-g))) * u;
           }
           if (col + 32 <= N && (((uintptr_t)dst) & 15) == 0) {
             uint32_t p[8];

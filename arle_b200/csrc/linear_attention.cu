@@ -476,7 +476,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float a, float b, float
 
 // VEC4: four numbers a lane and access.  ONE: a head fits in one round of them (vdim up to 128): its gate and weights are asked for beside it and
 // nothing is read twice.  Bound by instructions (exponentials, divisions, the warp's sum): 1,999 tokens of
-// 32 heads of 128 19.6 us (23.7 with the exact exponential and division, 24.9 in two rounds with a division of 64-bit numbers), 2,048 of 16 11.9 (13.6, 14.7).
+// 32 heads of 128 22.8 us (24.9 in two rounds with a division of 64-bit numbers), 2,048 of 16 12.6 (14.7).
 template <typename T, bool VEC4, bool ONE>
 __global__ void gla_out_kernel(const float* __restrict__ o, const T* __restrict__ gate, int gate_stride,
                                const float* __restrict__ weight, float eps, float scale, T* __restrict__ out,
@@ -510,7 +510,7 @@ __global__ void gla_out_kernel(const float* __restrict__ o, const T* __restrict_
     if (gate) {
       const float gs[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) y[i] *= times_sigmoid<T>(sigmoid_gate ? 1.0f : gs[i], gs[i]);
+      for (int i = 0; i < 4; ++i) y[i] *= (sigmoid_gate ? 1.0f : gs[i]) / (1.0f + expf(-gs[i]));
     }
     store4(out + (size_t)t * out_stride + (size_t)h * vdim + e, y[0] * scale, y[1] * scale, y[2] * scale, y[3] * scale);
   } else if constexpr (VEC4) {                   // vdim a multiple of 4, rows on 16-byte (8-byte for bfloat16) boundaries
@@ -532,11 +532,11 @@ __global__ void gla_out_kernel(const float* __restrict__ o, const T* __restrict_
       if (gp) {
         const float4 g = widen4(load_raw4(gp + e));
         if (sigmoid_gate) {
-          y[0] *= times_sigmoid<T>(1.0f, g.x), y[1] *= times_sigmoid<T>(1.0f, g.y);
-          y[2] *= times_sigmoid<T>(1.0f, g.z), y[3] *= times_sigmoid<T>(1.0f, g.w);
+          y[0] *= 1.0f / (1.0f + expf(-g.x)), y[1] *= 1.0f / (1.0f + expf(-g.y));
+          y[2] *= 1.0f / (1.0f + expf(-g.z)), y[3] *= 1.0f / (1.0f + expf(-g.w));
         } else {
-          y[0] *= times_sigmoid<T>(g.x, g.x), y[1] *= times_sigmoid<T>(g.y, g.y);
-          y[2] *= times_sigmoid<T>(g.z, g.z), y[3] *= times_sigmoid<T>(g.w, g.w);
+          y[0] *= g.x / (1.0f + expf(-g.x)), y[1] *= g.y / (1.0f + expf(-g.y));
+          y[2] *= g.z / (1.0f + expf(-g.z)), y[3] *= g.w / (1.0f + expf(-g.w));
         }
       }
       store4(op + e, y[0] * scale, y[1] * scale, y[2] * scale, y[3] * scale);
@@ -550,7 +550,7 @@ __global__ void gla_out_kernel(const float* __restrict__ o, const T* __restrict_
       if (weight) y *= weight[e];
       if (gate) {
         const float g = to_f32(gate[(size_t)t * gate_stride + (size_t)h * vdim + e]);
-        y *= times_sigmoid<T>(sigmoid_gate ? 1.0f : g, g);
+        y *= (sigmoid_gate ? 1.0f : g) / (1.0f + expf(-g));
       }
       out[(size_t)t * out_stride + (size_t)h * vdim + e] = from_f32<T>(y * scale);
     }

@@ -409,7 +409,7 @@ __global__ void mlstm_out_kernel(const float* __restrict__ num, const float* __r
   for (int c = threadIdx.x; c < vdim; c += blockDim.x) {
     const float o = np[c] * inv_den * inv * weight[h * vdim + c];
     const float gz = to_f32(gate[(size_t)t * gate_stride + h * vdim + c]);
-    out[(size_t)t * out_stride + h * vdim + c] = from_f32<T>(times_sigmoid<T>(o, gz));
+    out[(size_t)t * out_stride + h * vdim + c] = from_f32<T>(o / (1.0f + expf(-gz)));
   }
 }
 
@@ -477,7 +477,7 @@ __global__ void conv_silu_kernel(const T* __restrict__ x, int x_stride, const fl
     const float xv = src >= 0 ? to_f32(x[(size_t)(beg + src) * x_stride + c]) : st[src + taps - 1];
     acc = fmaf(w[(size_t)c * taps + j], xv, acc);
   }
-  out[(size_t)t * out_stride + c] = from_f32<T>(times_sigmoid<T>(acc, acc));
+  out[(size_t)t * out_stride + c] = from_f32<T>(acc / (1.0f + expf(-acc)));
 }
 
 template <typename T>
@@ -549,7 +549,7 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const T* __
     float val = yr[c];
     if (skip) val = fmaf(skip[c / vdim], to_f32(x[(size_t)t * x_stride + c]), val);
     const float g = to_f32(z[(size_t)t * z_stride + c]);
-    val *= times_sigmoid<T>(g, g);
+    val *= g / (1.0f + expf(-g));
     ss += val * val;
   }
   const float total = block_sum(ss, red);
@@ -559,7 +559,7 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const T* __
     float val = yr[c];
     if (skip) val = fmaf(skip[c / vdim], to_f32(x[(size_t)t * x_stride + c]), val);
     const float g = to_f32(z[(size_t)t * z_stride + c]);
-    val *= times_sigmoid<T>(g, g);
+    val *= g / (1.0f + expf(-g));
     out[(size_t)t * out_stride + c] = from_f32<T>(val * inv * weight[c]);
   }
 }
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) gated_group_norm_vec_kernel(c
     }
 #pragma unroll
     for (int g = 0; g < 8; ++g) {
-      val[it][g] *= times_sigmoid<T>(zv[g], zv[g]);
+      val[it][g] *= zv[g] / (1.0f + expf(-zv[g]));
       ss += val[it][g] * val[it][g];
     }
   }

@@ -38,7 +38,7 @@ __global__ void causal_conv_kernel(const TI* __restrict__ x, int x_stride, const
     const float xv = src >= 0 ? to_f32(x[(size_t)(beg + src) * x_stride + c]) + ib : st[src + taps - 1];
     acc = fmaf(w[(size_t)c * taps + j], xv, acc);
   }
-  if (act == 1) acc = times_sigmoid<TO>(acc, acc);
+  if (act == 1) acc = acc / (1.0f + expf(-acc));
   out[(size_t)t * out_stride + c] = from_f32<TO>(acc);
 }
 
