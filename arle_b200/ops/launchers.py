@@ -4,7 +4,7 @@ A step of short rows is a chain of launches whose host side costs as much as the
 3 us before the launcher runs.  So the calls are compiled: for every argument list among the launchers a C function that converts its
 arguments and calls through the launcher's address (0.3 us), written out, compiled with the host's C compiler and kept beside the library
 under a name that holds the source's hash.  As with ctypes, the interpreter's lock is released during the call and a wrong argument raises.
-Where there is no compiler or no Python headers, the launchers are called through ctypes.
+Where the calls cannot be had (no compiler, no Python headers, nowhere to write), the launchers are called through ctypes.
 """
 from __future__ import annotations
 
@@ -18,6 +18,8 @@ import subprocess
 import sys
 import sysconfig
 import types
+
+from . import build as _build
 
 # ctypes' type of an argument -> (letter, C type, conversion)
 _KINDS = {ctypes.c_void_p: ("P", "void*", "as_pointer"), ctypes.c_int: ("I", "int", "as_int"), ctypes.c_float: ("F", "float", "as_float"),
@@ -103,20 +105,61 @@ def source(signatures) -> str:
     return "".join(out) + _TAIL % dict(rows="".join(rows))
 
 
+def _note(why) -> None:
+    print(f"[arle_b200] the launchers' compiled calls cannot be had, ctypes is used: {why}", file=sys.stderr, flush=True)
+
+
 def _compile(text: str, path: str) -> bool:
+    """Whether ``path`` now holds the compiled calls.  False where there is no compiler or no headers, or the compiler fails; OSError where
+    the folder cannot be written or the compiler cannot be started."""
     include, cc = sysconfig.get_paths()["include"], os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc")
     if cc is None or not os.path.isfile(os.path.join(include, "Python.h")):
         return False
     tmp = f"{path}.tmp{os.getpid()}"
-    with open(tmp + ".c", "w") as f:
-        f.write(text)
-    r = subprocess.run([*cc.split(), "-O2", "-shared", "-fPIC", "-I", include, "-o", tmp, tmp + ".c"], capture_output=True, text=True)
-    os.remove(tmp + ".c")
-    if r.returncode != 0:
-        print(f"[arle_b200] the launchers' calls were not compiled, ctypes is used:\n{r.stderr}", file=sys.stderr, flush=True)
-        return False
-    os.replace(tmp, path)
-    return True
+    try:
+        with open(tmp + ".c", "w") as f:
+            f.write(text)
+        r = subprocess.run([*cc.split(), "-O2", "-shared", "-fPIC", "-I", include, "-o", tmp, tmp + ".c"], capture_output=True, text=True)
+        if r.returncode != 0:
+            _note(r.stderr)
+            return False
+        os.replace(tmp, path)
+        return True
+    finally:
+        for left in (tmp + ".c", tmp):
+            if os.path.exists(left):
+                os.remove(left)
+
+
+def _module(path: str):
+    spec = importlib.util.spec_from_file_location("_arle_launch", path, loader=importlib.machinery.ExtensionFileLoader("_arle_launch", path))
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+def _calls(lib_path: str, text: str):
+    """The module of the compiled calls, from beside the library or, where that folder cannot be written, the folder that a build would go to;
+    compiled when it is missing or cannot be loaded.  None where it cannot be had."""
+    name = f"_arle_launch_{hashlib.sha256(text.encode()).hexdigest()[:16]}{sysconfig.get_config_var('EXT_SUFFIX')}"
+    paths, why = [os.path.join(os.path.dirname(lib_path), name)], None
+    try:
+        paths.append(os.path.join(_build.build_dir(), name))
+    except OSError as e:
+        why = e
+    for path in paths:
+        if os.path.isfile(path):
+            try:
+                return _module(path)
+            except (OSError, ImportError):
+                pass                                       # of another system, or cut short: compiled anew
+    for path in dict.fromkeys(paths):
+        try:
+            return _module(path) if _compile(text, path) else None
+        except (OSError, ImportError) as e:
+            why = e
+    _note(why)
+    return None
 
 
 def load(lib_path: str, signatures):
@@ -126,13 +169,8 @@ def load(lib_path: str, signatures):
         fn = getattr(lib, name)
         fn.argtypes = list(types_)
         fn.restype = ctypes.c_int
-    text = source(signatures)
-    tag = hashlib.sha256(text.encode()).hexdigest()[:16]
-    path = os.path.join(os.path.dirname(lib_path), f"_arle_launch_{tag}{sysconfig.get_config_var('EXT_SUFFIX')}")
-    if not os.path.isfile(path) and not _compile(text, path):
+    module = _calls(lib_path, source(signatures))
+    if module is None:
         return lib
-    spec = importlib.util.spec_from_file_location("_arle_launch", path, loader=importlib.machinery.ExtensionFileLoader("_arle_launch", path))
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
     return types.SimpleNamespace(**{name: module.bind(letters(types_), ctypes.cast(getattr(lib, name), ctypes.c_void_p).value)
                                     for name, types_ in signatures.items()})

@@ -1,10 +1,11 @@
 """The compiled calls of the launchers: arguments arrive as ctypes delivers them, wrong ones raise, and without a compiler ctypes is used."""
 import ctypes
+import os
 import subprocess
 
 import pytest
 
-from arle_b200.ops import launchers
+from arle_b200.ops import build, launchers
 
 P, I, F, L = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_long
 SIGNATURES = {"echo_all": [P, I, F, L, P, F, F, F, F, I, I, I, F, F, F, F, P], "echo_none": [P, P]}
@@ -50,3 +51,71 @@ def test_wrong_arguments_raise(lib, at, value):
         lib.echo_all(*args)
     with pytest.raises(TypeError):
         lib.echo_none(None)
+
+
+def _library(folder):
+    (folder / "e.c").write_text(C_SOURCE)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(folder / "e.so"), str(folder / "e.c")], check=True)
+    return str(folder / "e.so")
+
+
+def _answers(lib):
+    assert lib.echo_none(None, None) == 1 and lib.echo_none(None, 8) == 0
+
+
+@pytest.mark.parametrize("compiler", ["/no/such/compiler", "false"])
+def test_a_compiler_that_does_not_run_leaves_ctypes(compiler, tmp_path, monkeypatch):
+    monkeypatch.setenv("CC", compiler)
+    path = _library(tmp_path)
+    before = sorted(os.listdir(tmp_path))
+    loaded = launchers.load(path, SIGNATURES)
+    assert isinstance(loaded, ctypes.CDLL) and sorted(os.listdir(tmp_path)) == before
+    _answers(loaded)
+
+
+def _no_writing_below(folder, monkeypatch):
+    """open(..., "w") below ``folder`` fails, as for a user who may not write there (chmod does not stop root)."""
+    real = open
+
+    def guarded(file, mode="r", *args, **kwargs):
+        if str(file).startswith(str(folder)) and mode != "r":
+            raise PermissionError(13, "Permission denied", str(file))
+        return real(file, mode, *args, **kwargs)
+
+    monkeypatch.setattr(launchers, "open", guarded, raising=False)
+
+
+def test_a_folder_that_cannot_be_written(tmp_path, monkeypatch):
+    (tmp_path / "shared").mkdir(), (tmp_path / "own").mkdir()
+    path = _library(tmp_path / "shared")
+    monkeypatch.setattr(build, "build_dir", lambda: str(tmp_path / "own"))
+    _no_writing_below(tmp_path / "shared", monkeypatch)
+    loaded = launchers.load(path, SIGNATURES)              # the calls go to the user's folder
+    assert not isinstance(loaded, ctypes.CDLL) and len(os.listdir(tmp_path / "own")) == 1
+    _answers(loaded)
+    monkeypatch.setattr(launchers, "_compile", None)       # and are found there again
+    again = launchers.load(path, SIGNATURES)
+    assert not isinstance(again, ctypes.CDLL)
+    _answers(again)
+
+
+def test_no_folder_that_can_be_written(tmp_path, monkeypatch):
+    path = _library(tmp_path)
+    monkeypatch.setattr(build, "build_dir", lambda: str(tmp_path))
+    _no_writing_below(tmp_path, monkeypatch)
+    loaded = launchers.load(path, SIGNATURES)
+    assert isinstance(loaded, ctypes.CDLL)
+    _answers(loaded)
+
+
+def test_calls_that_cannot_be_loaded_are_compiled_anew(tmp_path):
+    (tmp_path / "first").mkdir(), (tmp_path / "other").mkdir()
+    path = _library(tmp_path / "first")
+    before = set(os.listdir(tmp_path / "first"))
+    launchers.load(path, SIGNATURES)
+    name, = set(os.listdir(tmp_path / "first")) - before
+    path = _library(tmp_path / "other")                    # a path that this process has not loaded yet
+    (tmp_path / "other" / name).write_text("not a library")
+    loaded = launchers.load(path, SIGNATURES)
+    assert not isinstance(loaded, ctypes.CDLL)
+    _answers(loaded)
