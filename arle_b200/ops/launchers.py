@@ -1,9 +1,10 @@
 """Python's way into the launchers of the CUDA library.
 
 A step of short rows is a chain of launches whose host side costs as much as the kernels: a call through ctypes with twenty arguments takes
-3 us before the launcher runs.  So the calls are compiled: for every argument list among the launchers a C function that converts its
-arguments and calls through the launcher's address (0.3 us), written out, compiled with the host's C compiler and kept beside the library
-under a name that holds the source's hash.  As with ctypes, the interpreter's lock is released during the call and a wrong argument raises.
+2.6 us before the launcher runs.  So the calls are compiled: for every argument list among the launchers a C function that converts its
+arguments and calls through the launcher's address (0.4 us), written out, compiled with the host's C compiler and kept beside the library
+under a name that holds the source's hash.  As with ctypes, the interpreter's lock is released during the call, numbers of other types (numpy's)
+are taken where they are what is wanted and a wrong argument raises; stricter than ctypes, a pointer is a plain int or None, never text or an array.
 Where the calls cannot be had (no compiler, no Python headers, nowhere to write), the launchers are called through ctypes.
 """
 from __future__ import annotations
@@ -36,15 +37,18 @@ static void* as_pointer(PyObject* o, int* bad) {
   return (void*)(uintptr_t)PyLong_AsUnsignedLongLongMask(o);
 }
 static long as_long(PyObject* o, int* bad) {
-  if (!PyLong_Check(o)) { *bad = 1; return 0; }
-  return (long)PyLong_AsUnsignedLongLongMask(o);
+  if (PyLong_Check(o)) return (long)PyLong_AsUnsignedLongLongMask(o);
+  o = PyNumber_Index(o);                       /* numpy's whole numbers; no floats */
+  if (!o) { PyErr_Clear(); *bad = 1; return 0; }
+  long v = (long)PyLong_AsUnsignedLongLongMask(o);
+  Py_DECREF(o);
+  return v;
 }
 static int as_int(PyObject* o, int* bad) { return (int)as_long(o, bad); }
 static float as_float(PyObject* o, int* bad) {
   if (PyFloat_CheckExact(o)) return (float)PyFloat_AS_DOUBLE(o);
-  if (!PyFloat_Check(o) && !PyLong_Check(o)) { *bad = 1; return 0.0f; }
-  double v = PyFloat_AsDouble(o);
-  if (PyErr_Occurred()) { PyErr_Clear(); *bad = 1; }
+  double v = PyFloat_AsDouble(o);              /* whole numbers and whatever says what it is as a float */
+  if (v == -1.0 && PyErr_Occurred()) { PyErr_Clear(); *bad = 1; }
   return (float)v;
 }
 static PyObject* refuse(Py_ssize_t got, int want) {

@@ -1,8 +1,10 @@
 """The compiled calls of the launchers: arguments arrive as ctypes delivers them, wrong ones raise, and without a compiler ctypes is used."""
 import ctypes
+import fractions
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 from arle_b200.ops import build, launchers
@@ -20,13 +22,17 @@ int echo_none(void* a, void* b) { return !a && !b; }
 """
 
 
+def _library(folder):
+    (folder / "e.c").write_text(C_SOURCE)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(folder / "e.so"), str(folder / "e.c")], check=True)
+    return str(folder / "e.so")
+
+
 @pytest.fixture(params=[True, False])
 def lib(request, tmp_path, monkeypatch):
-    (tmp_path / "e.c").write_text(C_SOURCE)
-    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "e.so"), str(tmp_path / "e.c")], check=True)
     if not request.param:
         monkeypatch.setattr(launchers, "_compile", lambda text, path: False)
-    loaded = launchers.load(str(tmp_path / "e.so"), SIGNATURES)
+    loaded = launchers.load(_library(tmp_path), SIGNATURES)
     assert isinstance(loaded, ctypes.CDLL) != request.param
     return loaded
 
@@ -40,23 +46,33 @@ def test_arguments_and_results(lib):
     assert lib.echo_none(None, None) == 1 and lib.echo_none(None, 8) == 0
 
 
-@pytest.mark.parametrize("at,value", [(0, 1.5), (0, "x"), (1, 2.0), (1, None), (2, "x"), (3, 1.0)])
+def _arguments(out):
+    return [ctypes.addressof(out), 5, 0.25, 1, 0, 1.0, 2, 3.0, 4.0, 1, 2, 3, 4.0, 3.0, 2.0, 1, None]
+
+
+@pytest.mark.parametrize("at,value", [(0, 1.5), (0, np.int64(8)), (1, 2.0), (1, None), (1, np.float32(2)), (2, "x"), (3, 1.0), (3, "x")])
 def test_wrong_arguments_raise(lib, at, value):
-    out = (ctypes.c_long * 8)()
-    args = [ctypes.addressof(out), 5, 0.25, 1, 0, 1.0, 2, 3.0, 4.0, 1, 2, 3, 4.0, 3.0, 2.0, 1, None]
+    args = _arguments((ctypes.c_long * 8)())
     args[at] = value
     with pytest.raises((TypeError, ctypes.ArgumentError)):
-        if at == 0 and value == "x" and isinstance(lib, ctypes.CDLL):
-            raise TypeError("ctypes takes text for a pointer")
         lib.echo_all(*args)
     with pytest.raises(TypeError):
         lib.echo_none(None)
 
 
-def _library(folder):
-    (folder / "e.c").write_text(C_SOURCE)
-    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(folder / "e.so"), str(folder / "e.c")], check=True)
-    return str(folder / "e.so")
+@pytest.mark.parametrize("value", ["x", b"x", (ctypes.c_long * 2)()])
+def test_compiled_calls_take_no_text_or_arrays_for_pointers(tmp_path, value):
+    loaded = launchers.load(_library(tmp_path), SIGNATURES)
+    with pytest.raises(TypeError):
+        loaded.echo_none(value, None)
+
+
+def test_numbers_of_other_types(lib):
+    out = (ctypes.c_long * 8)()
+    args = _arguments(out)
+    args[1:4] = np.int32(-5), np.float32(0.5), np.int64(-(1 << 40))
+    args[5:8] = fractions.Fraction(1), np.int64(2), np.float64(3)
+    assert lib.echo_all(*args) == -3 and list(out)[:5] == [-5, 500, -(1 << 40), 0, 4321]
 
 
 def _answers(lib):
