@@ -164,8 +164,9 @@ __global__ void __launch_bounds__(Layout<BN, CTAS>::THREADS, CTAS) gemm_f32_tc_k
           tma_load_2d(dst, &map_w, kb * kBK, n0, bar);
         }
       }
-      if (*aborted)                                        // the copies still under way land before the CTA gives its shared memory back
-        for (int i = max(0, issued - STAGES); i < issued; ++i) mbar_wait_plain(smem_addr(&full_bar[i % STAGES]), (i / STAGES) & 1);
+      // The copies still under way land before the CTA gives its shared memory back, whatever the flag says now: a cutter's wait may run out after
+      // this look.  The cutters have waited for them where none did.
+      for (int k = max(0, issued - STAGES); k < issued; ++k) mbar_wait_plain(smem_addr(&full_bar[k % STAGES]), (k / STAGES) & 1);
     }
   } else if (warp == L::MMA_WARP) {
     if (lane == 0) {
@@ -194,6 +195,8 @@ __global__ void __launch_bounds__(Layout<BN, CTAS>::THREADS, CTAS) gemm_f32_tc_k
           umma_commit(smem_addr(&done_bar[s]));
           ready = sums && cuts;
         }
+      // And the MMAs end before the TMEM is freed.
+      if (i > 0) mbar_wait_plain(smem_addr(&done_bar[(i - 1) % STAGES]), ((i - 1) / STAGES) & 1);
     }
   } else if (warp >= kSumWarps) {
     // Eight numbers of k a thread and unit: 16 bytes of each piece.

@@ -103,11 +103,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
           tma_load_2d(smem_addr(tiles + (size_t)s * (A_BYTES + B_BYTES) + A_BYTES), &map_w, kb * BK, n0, bar);
         }
       }
-      if (*aborted) {
-        // wait (bounded) for the copies still under way before the CTA gives its shared memory back
-        for (int i = max(0, issued - STAGES); i < issued; ++i)
-          mbar_wait_plain(smem_addr(&full_bar[i % STAGES]), (i / STAGES) & 1);
-      }
+      // wait (bounded) for the copies still under way before the CTA gives its shared memory back, whatever the flag says now: the issuer's
+      // wait may run out after this look
+      for (int i = max(0, issued - STAGES); i < issued; ++i)
+        mbar_wait_plain(smem_addr(&full_bar[i % STAGES]), (i / STAGES) & 1);
     }
   } else if (warp == 5) {
     if (lane == 0) {

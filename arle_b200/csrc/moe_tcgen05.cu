@@ -299,8 +299,10 @@ __global__ void __launch_bounds__(kThreads, 1) moe_tcgen05_kernel(const __grid_c
       if (lane == 0) mbar_arrive_cluster(acc_empty_leader[buf]);
     }
   }
-  // A producer whose wait ran out may still have copies under way into its shared memory: wait for them
-  // (bounded) before the CTA ends.  They are counted on the first CTA's barriers, so only it can look.
+  // Where a wait ran out, copies may still be under way into the pair's shared memory: wait for them (bounded) before the
+  // CTA ends.  They are counted on the first CTA's barriers, so only it can look, and it does when all its warps are here: any of them may
+  // be the one whose wait ran out.
+  __syncthreads();
   if (warp == kProducer && lane == 0 && leader && *aborted)
     for (int s = 0; s < kStages; ++s) mbar_wait_plain(smem_addr(&full_bar[s]), 0), mbar_wait_plain(smem_addr(&full_bar[s]), 1);
   tc_fence_before();
