@@ -460,13 +460,14 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, sink: "ResidualSink" = None) -> 
 
 def f32_pieces_supported(x, w) -> bool:
     """Whether a product of float32 rows runs on the tensor cores in three bfloat16 pieces (``gemm_f32_tc.cu``): a bfloat16 w, K a multiple
-    of 64 and at least 512, N at least 256, rows on 16-byte boundaries, not more than the 2^31 blocks that its counters take (16 rows by 128 columns
+    of 64 and at least 512, N at least 256, rows on 16-byte boundaries that do not overlap (what a tensor map is promised to take; x may be
+    one row repeated), not more than the 2^31 blocks that its counters take (16 rows by 128 columns
     by 64 numbers of k; some 150 GB).  Short of that the sizes of w and how the arrays lie in memory decide, never the number of rows, so that a token's
     bits do not depend on how its prompt was cut.  Shorter sums are done sooner by the FFMA kernels (one row of 4,096 x 256 8.4 us, 9.4 in
     pieces), and a few columns fill too few of the tiles of 128."""
     N, K = w.shape
-    return (_KERNEL_SET == "fast" and w.dtype == torch.bfloat16 and K >= 512 and K % 64 == 0 and N >= 256 and x.stride(0) % 4 == 0
-            and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+    return (_KERNEL_SET == "fast" and w.dtype == torch.bfloat16 and K >= 512 and K % 64 == 0 and N >= 256 and x.stride(0) >= K and x.stride(0) % 4 == 0
+            and w.stride(0) >= K and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and -(-N // 128) * -(-x.shape[0] // 16) * (K // 64) < 1 << 31)
 
 
