@@ -700,7 +700,7 @@ template <int HD>
 int launch_stream(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, int q_row_stride, void* out,
                   const int* q_indptr, const int* kv_lens, const int* block_table, int bt_stride, float* part_o,
                   float* part_ml, int* counters, int rows, int nq, int nkv, int bt_width, int page_size, float scale, HeadTail<__nv_bfloat16> tail, int window,
-                  int ctas, const Prep& prep, const int* plan, int* err, cudaStream_t s) {
+                  int ctas, const Prep& prep, const int* plan, int small_behind, int* err, cudaStream_t s) {
   int ps_shift = -1;
   if ((page_size & (page_size - 1)) == 0)
     for (ps_shift = 0; (1 << ps_shift) < page_size; ++ps_shift) {}
@@ -721,13 +721,14 @@ int launch_stream(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, i
   int stages = (int)(((size_t)max_smem - fixed) / stage);
   if (stages > kMaxStages) stages = kMaxStages;
   stages &= ~1;
-  // No more stages than a CTA can have tiles, and no more than four in front of a small product (up to 8 rows, whose heads are 2,048 numbers at
-  // most: gemm_skinny.cu reads such weights without a ring) while there are few tiles: the product's blocks start in the shared memory that
-  // is left, before this kernel has ended.  Steps of 8 layers of Qwen3-0.6B sizes, us, six stages, four and two: one request of 100 tokens
-  // 269, 250 and 249, four of 1,000 300, 274 and 284, eight of 300 311, 274 and 284, eight of 2,048 (14 tiles a CTA) 380, 349 and 400.  Nothing
-  // starts beside it at 8B sizes: eight requests of 2,048 tokens 828, 836 and 886.
+  // No more stages than a CTA can have tiles, and no more than four in front of a small product that reads its weights straight from memory
+  // (gemm_skinny.cu: plan_direct says which do) while there are few tiles: the product's blocks start in the shared memory that
+  // is left, before this kernel has ended.  Steps of 8 layers, 8 requests of 2,048 tokens (14 tiles a CTA), us, six stages, four and two:
+  // 2,048 numbers of heads into a hidden size of 1,024 330, 301 and 352, into 2,048 440, 437 and 489, 4,096 into 2,560 691, 658 and 709.  Into 4,096, where the
+  // product with its sums added into the residual goes to the ring, nothing starts beside it: 2,048 numbers 626, 632 and 682, 4,096 828, 836 and 886.
+  // With 56 tiles a CTA (8,192 tokens) four gain less and do not always: 564 and 545, 673 and 677, 917 and 891; 76 tiles 650 and 640, 762 and 767.
   const long long row_tiles = ((long long)bt_width * page_size + kTile - 1) / kTile, per = (row_tiles * rows * nkv + ctas - 1) / ctas;
-  if (rows <= 8 && nq * HD <= 2048 && per <= 32 && stages > 4) stages = 4;
+  if (small_behind && per <= 32 && stages > 4) stages = 4;
   if (per < stages) stages = per <= 2 ? 2 : (int)((per + 1) & ~1ll);
   const size_t smem = fixed - kStaticSmem + (size_t)stages * stage;
   e = cudaFuncSetAttribute(decode_stream_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - kStaticSmem);
@@ -750,7 +751,7 @@ ARLE_API int arle_paged_attention_decode_stream_prep(const void* q, int q_row_st
                                                      int page_size, float scale, const float* sinks, const void* gate, int gate_stride,
                                                      int window, int rows, int ctas, int fused,
                                                      const int* slot_mapping, const float* q_weight, const float* k_weight,
-                                                     float eps, const float* inv_freq, int rotary_dim, const float* bias, const int* plan, int* err,
+                                                     float eps, const float* inv_freq, int rotary_dim, const float* bias, const int* plan, int small_behind, int* err,
                                                      cudaStream_t s);
 
 // k_cache / v_cache: [cache_pages, nkv, page_size, hd].  Scratch: part_o float32
@@ -763,12 +764,12 @@ ARLE_API int arle_paged_attention_decode_stream(const void* q, int q_row_stride,
                                                 const int* kv_lens, const int* block_table, int bt_stride, int bt_width,
                                                 float* part_o, float* part_ml, int* counters, int nq, int nkv, int hd,
                                                 int page_size, float scale, const float* sinks, const void* gate, int gate_stride,
-                                                int window, int rows, int ctas, int* err,
+                                                int window, int rows, int ctas, int small_behind, int* err,
                                                 cudaStream_t s) {
   return arle_paged_attention_decode_stream_prep(q, q_row_stride, out, k_cache, v_cache, cache_pages, q_indptr, kv_lens,
                                                  block_table, bt_stride, bt_width, part_o, part_ml, counters, nq, nkv, hd,
                                                  page_size, scale, sinks, gate, gate_stride, window, rows, ctas, 0, nullptr, nullptr, nullptr, 0.f,
-                                                 nullptr, 0, nullptr, nullptr, err, s);
+                                                 nullptr, 0, nullptr, nullptr, small_behind, err, s);
 }
 
 // Ints of a step's plan for this many rows and CTAs.
@@ -799,7 +800,7 @@ ARLE_API int arle_paged_attention_decode_stream_prep(const void* q, int q_row_st
                                                      int page_size, float scale, const float* sinks, const void* gate, int gate_stride,
                                                      int window, int rows, int ctas, int fused,
                                                      const int* slot_mapping, const float* q_weight, const float* k_weight,
-                                                     float eps, const float* inv_freq, int rotary_dim, const float* bias, const int* plan, int* err,
+                                                     float eps, const float* inv_freq, int rotary_dim, const float* bias, const int* plan, int small_behind, int* err,
                                                      cudaStream_t s) {
   if (rows <= 0) return 0;
   if (fused && (!slot_mapping || ((uintptr_t)q & 15) || (q_row_stride % 8) != 0)) return ARLE_E_BADARG;
@@ -822,7 +823,7 @@ ARLE_API int arle_paged_attention_decode_stream_prep(const void* q, int q_row_st
   if (rc) return rc;
   if (hd == 128)
     return launch_stream<128>(mk, mv, q, q_row_stride, out, q_indptr, kv_lens, block_table, bt_stride, part_o, part_ml, counters,
-                              rows, nq, nkv, bt_width, page_size, scale, tail, window, ctas, prep, plan, err, s);
+                              rows, nq, nkv, bt_width, page_size, scale, tail, window, ctas, prep, plan, small_behind, err, s);
   return launch_stream<64>(mk, mv, q, q_row_stride, out, q_indptr, kv_lens, block_table, bt_stride, part_o, part_ml, counters,
-                           rows, nq, nkv, bt_width, page_size, scale, tail, window, ctas, prep, plan, err, s);
+                           rows, nq, nkv, bt_width, page_size, scale, tail, window, ctas, prep, plan, small_behind, err, s);
 }

@@ -735,6 +735,13 @@ int skinny_entry(const void* x, int ldx, const void* W, int ldw, void* out, int 
 
 }  // namespace
 
+// Whether a product of these sizes reads its weights straight from memory (1) or through the ring (0); sink: its sums go into the residual.
+ARLE_API int arle_gemm_skinny_direct(int M, int N, int K, int sink) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const DirectPlan p = plan_direct(M, N, K, sink != 0);
+  return p.rows && !p.last;
+}
+
 // out_dtype: 0 float32, 1 bfloat16.  Needs M <= 16, K a multiple of 32, ldx and ldw multiples of 8,
 // 16-byte aligned x and W.  err (may be null): set to 1 if a bounded wait ran out.
 ARLE_API int arle_gemm_skinny(const void* x, int ldx, const void* W, int ldw, void* out, int out_dtype, int ldo, int M, int N,

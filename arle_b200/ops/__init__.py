@@ -74,9 +74,9 @@ _SIGNATURES = {
     "arle_clamped_glu": [_P, _P, _I, _I, _I, _I, _F, _F, _P],
     "arle_paged_attention_decode": [_P, _I, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P],
     "arle_paged_attention_decode_stream": [_P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I,
-                                           _F, _P, _P, _I, _I, _I, _I, _P, _P],
+                                           _F, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     "arle_paged_attention_decode_stream_prep": [_P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I,
-                                                _F, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _P, _P],
+                                                _F, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _I, _P, _P],
     "arle_decode_stream_plan_ints": [_I, _I],
     "arle_decode_stream_plan": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "arle_paged_attention_prefill": [_P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P],
@@ -85,6 +85,7 @@ _SIGNATURES = {
     "arle_gemm_f32": [_P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P],
     "arle_gemm_f32_tc": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _P, _P],
     "arle_gemm_plain_bf16": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+    "arle_gemm_skinny_direct": [_I, _I, _I, _I],
     "arle_gemm_skinny": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _P],
     "arle_gemm_skinny_gated": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _P],
     "arle_gemm_skinny_fused": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _F, _F, _P, _I, _P, _P, _I, _P, _F, _P, _P, _P],
@@ -585,7 +586,7 @@ def attention_prep(qkv, positions, slot_mapping, q_weight, k_weight, eps, inv_fr
 
 def paged_attention(q, out, k_cache, v_cache, positions, row_of_token, block_table, nq: int, nkv: int, hd: int,
                     page_size: int, scale: float, window, batch=None, vd: int = None, sink=None, keep_first: int = 0,
-                    softcap: float = None, chunk: int = None, score_bias=None, gate=None) -> None:
+                    softcap: float = None, chunk: int = None, score_bias=None, gate=None, product=None) -> None:
     """Causal attention of this step's queries over the paged cache.
 
     ``chunk``: a query sees only the keys of its own chunk of that many positions, counted from position 0 (in a window's
@@ -604,7 +605,8 @@ def paged_attention(q, out, k_cache, v_cache, positions, row_of_token, block_tab
     q: [T, nq*hd] view (row stride free, unit inner stride); out: contiguous
     [T, nq*hd]; caches [pages, nkv, page_size, hd]; positions / row_of_token int32
     [T]; block_table int32 [rows, max_pages].  ``window`` None or <= 0 means all
-    keys.  ``batch`` (a StepContext) lets faster kernels pick their launch shape;
+    keys.  ``product`` (w, sink): the product of out that the caller launches next, ``gemm(out, w, ..., sink)``, for which the streamed
+    attention leaves room beside it where that starts early; it changes no result.  ``batch`` (a StepContext) lets faster kernels pick their launch shape;
     the general kernel does not need it."""
     T = q.shape[0]
     vd = hd if vd is None else int(vd)
@@ -644,7 +646,7 @@ def paged_attention(q, out, k_cache, v_cache, positions, row_of_token, block_tab
                 q, out, k_cache, v_cache, batch.q_indptr, batch.kv_lens, block_table, nq, nkv, hd, page_size, scale, window,
                 batch.ws.get("attn_piece_o", (slots * hd,), torch.float32),
                 batch.ws.get("attn_piece_ml", (slots * 2,), torch.float32),
-                batch.ws.get_zeroed("attn_piece_counters", (batch.num_rows * nkv,), torch.int32), ctas, sink=sink, gate=gate)
+                batch.ws.get_zeroed("attn_piece_counters", (batch.num_rows * nkv,), torch.int32), ctas, sink=sink, gate=gate, product=product)
         elif batch.num_single > 0:
             bound = block_table.shape[1] * page_size
             if window:
@@ -763,10 +765,18 @@ def stream_decode_supported(rows: int, page_size: int, group: int = 1) -> bool:
     return page_size % 16 == 0 and rows <= 2048 and group <= 16
 
 
+def _small_behind(rows: int, product) -> int:
+    """Whether the product that follows an attention reads its weights straight from memory (``gemm_skinny.cu``)."""
+    if product is None or not fused_gemm_shape_ok(rows, product[0]):
+        return 0
+    w, sink = product
+    return library().arle_gemm_skinny_direct(rows, w.shape[0], w.shape[1], int(sink is not None))
+
+
 def paged_attention_decode_stream(q, out, k_cache, v_cache, q_indptr, kv_lens, block_table, nq, nkv, hd, page_size, scale,
-                                  window, piece_o, piece_ml, counters, ctas: int, sink=None, gate=None) -> None:
+                                  window, piece_o, piece_ml, counters, ctas: int, sink=None, gate=None, product=None) -> None:
     """Attention of the rows that have exactly one query (others are skipped), as a
-    resident grid of ``ctas`` CTAs that share the batch's 64-key tiles evenly.
+    resident grid of ``ctas`` CTAs that share the batch's 64-key tiles evenly.  ``product`` as in ``paged_attention``.
     Scratch: piece_o float32 [(ctas + R*nkv) * (nq/nkv) * hd], piece_ml float32
     [(ctas + R*nkv) * (nq/nkv) * 2], counters int32 [R*nkv], zero before the first
     launch (the kernel leaves it zero)."""
@@ -785,7 +795,7 @@ def paged_attention_decode_stream(q, out, k_cache, v_cache, q_indptr, kv_lens, b
         _ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), k_cache.shape[0], _ptr(q_indptr), _ptr(kv_lens),
         _ptr(block_table), block_table.stride(0), block_table.shape[1], _ptr(piece_o), _ptr(piece_ml), _ptr(counters),
         nq, nkv, hd, page_size, float(scale), _ptr(_sinks(sink, nq, q.device)), *_gate_arg(gate, q, nq), int(window) if window else 0, R,
-        int(ctas), _ptr(error_flag(q.device)), _stream()), "paged_attention_decode_stream")
+        int(ctas), _small_behind(q.shape[0], product), _ptr(error_flag(q.device)), _stream()), "paged_attention_decode_stream")
 
 
 def fused_decode_supported(qkv, batch, cache_dtype, nq: int, nkv: int, hd: int, page_size: int, rotary_dim: int) -> bool:
@@ -800,13 +810,13 @@ def fused_decode_supported(qkv, batch, cache_dtype, nq: int, nkv: int, hd: int, 
 
 def decode_attention_with_prep(qkv, out, k_cache, v_cache, slot_mapping, q_weight, k_weight, eps: float, inv_freq,
                                block_table, nq: int, nkv: int, hd: int, page_size: int, scale: float, window, batch, rotary_dim: int = None,
-                               bias=None, sink=None, gate=None) -> None:
+                               bias=None, sink=None, gate=None, product=None) -> None:
     """Attention of a step in which every row is one decoded token, from the raw projection output
     qkv [T, (nq + 2 nkv) hd]: per-head norm and rotation of the queries and of the new keys, the store of
     the new keys and values into the cache, and the attention over the cache, in one launch of the
     streaming kernel.  ``q_weight`` / ``k_weight`` None: no norm; ``inv_freq`` None: no rotation; ``rotary_dim``: the first numbers
-    of a head that turn (None: all); ``bias`` (float32 [(nq + 2 nkv) hd]): added to q, k and v first; ``sink`` and ``gate`` as in
-    ``paged_attention``."""
+    of a head that turn (None: all); ``bias`` (float32 [(nq + 2 nkv) hd]): added to q, k and v first; ``sink``, ``gate`` and
+    ``product`` as in ``paged_attention``."""
     T = qkv.shape[0]
     rotary_dim = 0 if inv_freq is None else hd if rotary_dim is None else int(rotary_dim)
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != (nq + 2 * nkv) * hd or not bias.is_contiguous()):
@@ -851,7 +861,7 @@ def decode_attention_with_prep(qkv, out, k_cache, v_cache, slot_mapping, q_weigh
         _ptr(batch.kv_lens), _ptr(block_table), block_table.stride(0), block_table.shape[1], _ptr(piece_o), _ptr(piece_ml),
         _ptr(counters), nq, nkv, hd, page_size, float(scale), _ptr(_sinks(sink, nq, qkv.device)), *_gate_arg(gate, qkv, nq), int(window) if window else 0, R,
         int(ctas), 1, _ptr(slot_mapping), _ptr(q_weight), _ptr(k_weight), float(eps), _ptr(inv_freq), rotary_dim, _ptr(bias), _ptr(plan),
-        _ptr(error_flag(qkv.device)), _stream()), "decode_attention_with_prep")
+        _small_behind(T, product), _ptr(error_flag(qkv.device)), _stream()), "decode_attention_with_prep")
 
 
 def decode_splits(rows: int, nkv: int, kv_bound: int, device=None) -> int:

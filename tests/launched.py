@@ -12,8 +12,8 @@ def _shown(mangled: bytes) -> str:
     return ctypes.string_at(at).decode() if at else mangled.decode()
 
 
-def launched(run, pattern):
-    """The parts of the kernels' names (template arguments included) that ``pattern`` matches, after a first call by itself."""
+def kernels(run):
+    """The kernels' names (template arguments included) and launch parameters, in the graph's order, after a first call by itself."""
     from cuda.bindings import driver
 
     def ok(res):
@@ -28,13 +28,13 @@ def launched(run, pattern):
     raw = driver.CUgraph(graph.raw_cuda_graph())
     err, _, count = driver.cuGraphGetNodes(raw)
     assert err == driver.CUresult.CUDA_SUCCESS
-    found = set()
     for node in ok(driver.cuGraphGetNodes(raw, count))[:count]:
         if ok(driver.cuGraphNodeGetType(node)) != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
             continue
         p = ok(driver.cuGraphKernelNodeGetParams(node))
-        name = ok(driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern))
-        m = re.search(pattern, _shown(name))
-        if m:
-            found.add(m.group(0))
-    return found
+        yield _shown(ok(driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern))), p
+
+
+def launched(run, pattern):
+    """The parts of the kernels' names that ``pattern`` matches."""
+    return {m.group(0) for name, _ in kernels(run) for m in [re.search(pattern, name)] if m}

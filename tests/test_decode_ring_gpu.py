@@ -1,28 +1,40 @@
-"""Streamed decode attention with rings of two to eight stages (what the step's table bounds, and four in front of a small product), pairs in
-as many pieces as the last arriver reads at once and more, and a chain in which the kernels in front and behind start early."""
+"""Streamed decode attention with rings of two to eight stages (what the step's table bounds, and four in front of a product that reads its weights
+straight from memory), pairs in as many pieces as the last arriver reads at once and more, and a chain in which the products around it start early."""
 import math
 
 import pytest
 import torch
 
 from arle_b200 import ops
-from test_kernels_gpu import _fast_setup, _ref_attn, _stream_decode
+from launched import kernels
+from test_kernels_gpu import _fast_setup, _ref_attn
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
+def _stream_decode(q, out, kc, vc, qi, kv, bt, nq, nkv, hd, ps, window, ctas, scratch=None, product=None):
+    R = kv.numel()
+    slots = (ctas + R * nkv) * (nq // nkv)
+    if scratch is None:
+        scratch = (torch.zeros(slots * hd, device=DEV), torch.zeros(slots * 2, device=DEV), torch.zeros(R * nkv, dtype=torch.int32, device=DEV))
+    ops.paged_attention_decode_stream(q, out, kc, vc, qi, kv, bt, nq, nkv, hd, ps, 1 / math.sqrt(hd), window, *scratch, ctas, product=product)
+    return scratch
+
+
 @pytest.mark.parametrize("nq,nkv,lens", [
     (16, 8, [64]), (16, 8, [1153]), (16, 8, [1400] * 2), (16, 8, [2100] * 2), (16, 8, [300] * 8), (16, 8, [2100] * 8), (16, 8, [700, 1, 2300, 65] * 3),
     (32, 8, [700]), (32, 8, [2100] * 3), (16, 8, [16500] * 3), (2, 1, [64 * 16]), (2, 1, [64 * 16 + 1]), (2, 1, [64 * 33]), (4, 2, [64 * 50 + 7])])
-def test_rings_and_pieces(nq, nkv, lens):
+@pytest.mark.parametrize("behind", [None, 1024])           # columns of the product that follows
+def test_rings_and_pieces(nq, nkv, lens, behind):
+    product = None if behind is None else (torch.empty(behind, nq * 128, dtype=torch.bfloat16, device=DEV), None)
     q, kc, vc, pos, rows, bt, qi, kv = _fast_setup(nq, nkv, 128, 16, lens, [1] * len(lens), seed=4)
     out = torch.zeros(len(lens), nq * 128, dtype=torch.bfloat16, device=DEV)
     want = _ref_attn(q, kc, vc, pos, rows, bt, nq, nkv, 128, 16, None)
     scratch = None
     for _ in range(2):
         out.zero_()
-        scratch = _stream_decode(q, out, kc, vc, qi, kv, bt, nq, nkv, 128, 16, None, 148, scratch)
+        scratch = _stream_decode(q, out, kc, vc, qi, kv, bt, nq, nkv, 128, 16, None, 148, scratch, product)
         torch.testing.assert_close(out.float().cpu(), want, rtol=2e-2, atol=1e-2)      # P is rounded to bfloat16
         assert scratch[2].abs().sum().item() == 0
 
@@ -64,3 +76,18 @@ def test_a_chain_with_products_in_front_and_behind():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(torch.stack(xs[1:]), want)
+
+
+@pytest.mark.parametrize("nq,hidden,sums,room", [
+    (16, 1024, True, True), (16, 2048, True, True), (32, 2560, True, True), (32, 4096, False, True),
+    (16, 4096, True, False), (32, 4096, True, False), (64, 5120, True, False), (16, None, False, False)])
+def test_room_is_left_in_front_of_products_without_a_ring_alone(nq, hidden, sums, room):
+    """``sums``: the product adds into the residual.  A step of 8 requests of 2,048 tokens: rings of six stages, four where room is left."""
+    nkv, lens = 8, [2048] * 8
+    q, kc, vc, pos, rows, bt, qi, kv = _fast_setup(nq, nkv, 128, 16, lens, [1] * 8, seed=4)
+    out = torch.zeros(8, nq * 128, dtype=torch.bfloat16, device=DEV)
+    product = None if hidden is None else (torch.empty(hidden, nq * 128, dtype=torch.bfloat16, device=DEV), object() if sums else None)
+    scratch = _stream_decode(q, out, kc, vc, qi, kv, bt, nq, nkv, 128, 16, None, 148)
+    shared, = [p.sharedMemBytes for name, p in kernels(lambda: _stream_decode(q, out, kc, vc, qi, kv, bt, nq, nkv, 128, 16, None, 148, scratch, product))
+               if "decode_stream_kernel" in name]
+    assert shared // 32768 in ((4,) if room else (5, 6)), shared         # 32 KB a stage, and less than one for the rest
