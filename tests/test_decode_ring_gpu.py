@@ -1,11 +1,14 @@
 """Streamed decode attention with rings of two to eight stages (what the step's table bounds, and four in front of a product that reads its weights
-straight from memory), pairs in as many pieces as the last arriver reads at once and more, and a chain in which the products around it start early."""
+straight from memory), pairs in as many pieces as the last arriver reads at once and more, and chains: one in which the products around it start
+early, and one in which the attention does too (with its preparation in the same launch), each against the same calls one by one."""
 import math
+from types import SimpleNamespace
 
 import pytest
 import torch
 
 from arle_b200 import ops
+from arle_b200.engine import Workspace
 from launched import kernels
 from test_kernels_gpu import _fast_setup, _ref_attn
 
@@ -91,3 +94,61 @@ def test_room_is_left_in_front_of_products_without_a_ring_alone(nq, hidden, sums
     shared, = [p.sharedMemBytes for name, p in kernels(lambda: _stream_decode(q, out, kc, vc, qi, kv, bt, nq, nkv, 128, 16, None, 148, scratch, product))
                if "decode_stream_kernel" in name]
     assert shared // 32768 in ((4,) if room else (5, 6)), shared         # 32 KB a stage, and less than one for the rest
+
+
+@pytest.mark.parametrize("memo", [False, True])            # with a plan of the step, which the first layer's call makes
+@pytest.mark.parametrize("nq,nkv,hidden,lens", [(16, 8, 1024, [900, 130]), (16, 8, 1024, [4000, 1, 64]), (4, 1, 256, [33 * 64])])
+def test_a_chain_in_which_the_attention_starts_early(nq, nkv, hidden, lens, memo):
+    R, layers, hd, ps = len(lens), 6, 128, 16
+    _, kc0, vc0, pos, rows, bt, qi, kv = _fast_setup(nq, nkv, hd, ps, lens, [1] * R, seed=6)
+    last = kv.long() - 1
+    slots = (bt[torch.arange(R, device=DEV), last // ps].long() * ps + last % ps).to(torch.int32)
+    g = torch.Generator(device=DEV).manual_seed(1)
+    w_qkv = [(torch.randn((nq + 2 * nkv) * hd, hidden, generator=g, device=DEV) * 0.03).bfloat16() for _ in range(layers)]
+    w_o = [(torch.randn(hidden, nq * hd, generator=g, device=DEV) * 0.05).bfloat16() for _ in range(layers)]
+    norm = torch.rand(hd, generator=g, device=DEV) + 0.5
+    inv_freq = torch.pow(torch.tensor(1e4), -torch.arange(hd // 2, dtype=torch.float32) * 2 / hd).to(DEV)
+    xs = [torch.randn(R, hidden, generator=g, device=DEV).bfloat16()] + [torch.empty(R, hidden, dtype=torch.bfloat16, device=DEV) for _ in range(layers)]
+    caches = [(kc0.clone(), vc0.clone()) for _ in range(layers)]
+    qkv = torch.empty(R, (nq + 2 * nkv) * hd, dtype=torch.bfloat16, device=DEV)
+    attn = torch.empty(R, nq * hd, dtype=torch.bfloat16, device=DEV)
+    batch = SimpleNamespace(max_q_len=1, num_rows=R, ws=Workspace(DEV), q_indptr=qi, kv_lens=kv)       # scratch and counters of all layers
+
+    def chain(wait):
+        if memo:
+            batch.memo = {}
+        for i in range(layers):
+            k, v = caches[i]
+            for step in (lambda: ops.gemm(xs[i], w_qkv[i], qkv),
+                         lambda: ops.decode_attention_with_prep(qkv, attn, k, v, slots, norm, norm, 1e-6, inv_freq, bt, nq, nkv, hd, ps, 1 / math.sqrt(hd),
+                                                                None, batch, product=(w_o[i], None)),
+                         lambda: ops.gemm(attn, w_o[i], xs[i + 1])):
+                step()
+                if wait:
+                    torch.cuda.synchronize()
+
+    def clear():
+        for t in (*xs[1:], qkv, attn):
+            t.fill_(float("nan"))
+        for k, v in caches:
+            k.copy_(kc0), v.copy_(vc0)
+        torch.cuda.synchronize()
+
+    def result():
+        torch.cuda.synchronize()
+        ops.check_errors(DEV)
+        return [t.clone() for t in (*xs[1:], *(t for pair in caches for t in pair))]
+
+    clear()
+    chain(True)
+    want = result()
+    assert all(t.isfinite().all() for t in want[:layers]) and want[layers - 1].abs().max() > 0
+    assert not torch.equal(want[layers], kc0)              # the new keys are in the cache
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain(False)
+    for _ in range(4):
+        for run in (lambda: chain(False), graph.replay):
+            clear()
+            run()
+            assert all(torch.equal(a, b) for a, b in zip(result(), want))
