@@ -115,7 +115,8 @@ __global__ void __launch_bounds__(Layout<BN, CTAS>::THREADS, CTAS) gemm_f32_tc_k
   unsigned char* pieces = tiles + (size_t)STAGES * L::STAGE;
   __shared__ __align__(8) uint64_t full_bar[STAGES], done_bar[STAGES], cut_full[RING], acc_empty[kBuffers];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, loaded;                        // loaded: blocks whose copies have been issued
+  __shared__ __align__(8) uint64_t last_bar;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m = (M + BN - 1) / BN, num_tiles = tiles_m * ((N + kRowsW - 1) / kRowsW);      // rows of A fastest: W's tile stays in L2
@@ -127,7 +128,8 @@ __global__ void __launch_bounds__(Layout<BN, CTAS>::THREADS, CTAS) gemm_f32_tc_k
     }
     for (int p = 0; p < RING; ++p) mbar_init(smem_addr(&cut_full[p]), L::GROUP);
     for (int b = 0; b < kBuffers; ++b) mbar_init(smem_addr(&acc_empty[b]), kSumWarps);
-    abort_flag = 0;
+    mbar_init(smem_addr(&last_bar), 1);
+    abort_flag = loaded = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
@@ -164,9 +166,7 @@ __global__ void __launch_bounds__(Layout<BN, CTAS>::THREADS, CTAS) gemm_f32_tc_k
           tma_load_2d(dst, &map_w, kb * kBK, n0, bar);
         }
       }
-      // The copies still under way land before the CTA gives its shared memory back, whatever the flag says now: a cutter's wait may run out after
-      // this look.  The cutters have waited for them where none did.
-      for (int k = max(0, issued - STAGES); k < issued; ++k) mbar_wait_plain(smem_addr(&full_bar[k % STAGES]), (k / STAGES) & 1);
+      loaded = issued;
     }
   } else if (warp == L::MMA_WARP) {
     if (lane == 0) {
@@ -195,8 +195,6 @@ __global__ void __launch_bounds__(Layout<BN, CTAS>::THREADS, CTAS) gemm_f32_tc_k
           umma_commit(smem_addr(&done_bar[s]));
           ready = sums && cuts;
         }
-      // And the MMAs end before the TMEM is freed.
-      if (i > 0) mbar_wait_plain(smem_addr(&done_bar[(i - 1) % STAGES]), ((i - 1) / STAGES) & 1);
     }
   } else if (warp >= kSumWarps) {
     // Eight numbers of k a thread and unit: 16 bytes of each piece.
@@ -301,6 +299,15 @@ __global__ void __launch_bounds__(Layout<BN, CTAS>::THREADS, CTAS) gemm_f32_tc_k
   __syncwarp();                                            // the loader's and the issuer's other lanes have been here all along
   tc_fence_before();
   __syncthreads();
+  if (*aborted) {                                          // as all warps have left it: copies and MMAs under way end (bounded) before their memory is given back
+    if (warp == L::LOAD_WARP && lane == 0)
+      for (int i = max(0, loaded - STAGES); i < loaded; ++i) mbar_wait_plain(smem_addr(&full_bar[i % STAGES]), (i / STAGES) & 1);
+    if (warp == L::MMA_WARP && lane == 0) {
+      umma_commit(smem_addr(&last_bar));
+      mbar_wait_plain(smem_addr(&last_bar), 0);
+    }
+    __syncthreads();
+  }
   if (warp == L::MMA_WARP) {
     __syncwarp();
     tc_fence_after();
