@@ -81,23 +81,16 @@ __global__ void __launch_bounds__(1024) rmsnorm_vec_kernel(float* resid, const T
   const float* er = extra ? extra + (size_t)r * hidden : nullptr;
   const int n4 = hidden >> 2;
   float4 x[kVecMax], wv[kVecMax];
-  decltype(raw4(delta)) d[kVecMax];                          // as they lie in memory: 1,024 threads leave 64 registers each
+  decltype(raw4(delta)) d[kVecMax];                   // as they lie in memory: 1,024 threads leave 64 registers each
   float ss = 0.f;
-#pragma unroll
-  for (int k = 0; k < kVecMax; ++k) {
+  auto load = [&](int k) {
     const int c = threadIdx.x + k * blockDim.x;
     if (c < n4) {
       x[k] = load4(xr + 4 * c);
       if (dr) d[k] = raw4(dr + 4 * c);
     }
-  }
-#pragma unroll
-  for (int k = 0; k < kVecMax; ++k) {
-    const int c = threadIdx.x + k * blockDim.x;
-    if (c < n4) wv[k] = load4(weight + 4 * c);
-  }
-#pragma unroll
-  for (int k = 0; k < kVecMax; ++k) {
+  };
+  auto add = [&](int k) {
     const int c = threadIdx.x + k * blockDim.x;
     if (c < n4) {
       float4 v = x[k];
@@ -107,14 +100,23 @@ __global__ void __launch_bounds__(1024) rmsnorm_vec_kernel(float* resid, const T
         v.z = fmaf(delta_scale, dk.z, v.z), v.w = fmaf(delta_scale, dk.w, v.w);
       }
       if (er) {
-        const float4 ek = load4(er + 4 * c);
+        const float4 ek = raw4(er + 4 * c);
         v.x += ek.x; v.y += ek.y; v.z += ek.z; v.w += ek.w;
       }
       if (write_resid && (dr || er)) store4(xr + 4 * c, v);
       x[k] = v;
       ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
     }
+  };
+#pragma unroll
+  for (int k = 0; k < kVecMax; ++k) load(k);
+#pragma unroll
+  for (int k = 0; k < kVecMax; ++k) {                        // the gains too: not waited for after the reduction
+    const int c = threadIdx.x + k * blockDim.x;
+    if (c < n4) wv[k] = load4(weight + 4 * c);
   }
+#pragma unroll
+  for (int k = 0; k < kVecMax; ++k) add(k);
   const float total = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(total / (float)hidden + eps);
   TA* o = out + (size_t)i * hidden;
