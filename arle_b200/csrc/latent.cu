@@ -27,7 +27,7 @@
 #include "mma_utils.cuh"
 using namespace arle;
 
-template <typename T>
+template <typename T, int AHEAD>
 __global__ void latent_prep_kernel(const T* q, int q_stride, const T* dkv, int dkv_stride,
                                    const int* positions, const int* slot_mapping,
                                    const float* c_weight, float eps, const float* inv_freq,
@@ -65,8 +65,7 @@ __global__ void latent_prep_kernel(const T* q, int q_stride, const T* dkv, int d
     o[pairing ? 2 * i : i] = from_f32<T>(x * cs - y * sn);
     o[pairing ? 2 * i + 1 : i + half] = from_f32<T>(y * cs + x * sn);
   };
-  // Loads go ahead of stores a few at a time: q_out may be q, so that the compiler keeps their order.
-  constexpr int AHEAD = 4;
+  // Loads go ahead of stores AHEAD at a time: q_out may be q, so that the compiler keeps their order.
   const T* kv = dkv + (size_t)t * dkv_stride;
   if (cache != nullptr) {
     float x[AHEAD], ss = 0.f;
@@ -104,9 +103,10 @@ __global__ void latent_prep_kernel(const T* q, int q_stride, const T* dkv, int d
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k) {
       const int idx = i0 + k * blockDim.x;
+      if (idx >= H * units) break;
       head[k] = idx / units;
       at[k] = idx - head[k] * units;
-      if (idx < H * units) read(qt + (size_t)head[k] * (dn + dr), at[k], u[k], v[k]);
+      read(qt + (size_t)head[k] * (dn + dr), at[k], u[k], v[k]);
     }
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k)
@@ -125,12 +125,16 @@ ARLE_API int arle_latent_prep(const void* q, int q_stride, const void* dkv, int 
   const int threads = H * dr >= 1024 ? 256 : 128;
   const size_t smem = (size_t)rot_dims / 2 * sizeof(float2);
   if (smem > 40 * 1024) return ARLE_E_UNSUPPORTED;
+  // Few tokens start early: 64 of 32 heads 3.7 us behind one another, 4.5 in stream order, but 256 of 128 heads 11.2 and 8.9.  They wait for memory, so a thread
+  // with work for it has four loads under way (32 heads 3.5 us, 3.8 with two); many want the registers for more blocks (1,024 tokens 8.1 and 7.4,
+  // 2,048 of 16 heads 6.8 and 5.6).
+  const bool few = num_tokens <= kEarlyRows / 2, early = few || (pdl_enabled() & 1) != 0, four = few && threads == 256;
   if (dtype == 0)
-    launch_early(latent_prep_kernel<float>, dim3(num_tokens), dim3(threads), smem, s, 1, (const float*)q, q_stride, (const float*)dkv,
+    launch_kernel_as(early, four ? latent_prep_kernel<float, 4> : latent_prep_kernel<float, 2>, dim3(num_tokens), dim3(threads), smem, s, 1, (const float*)q, q_stride, (const float*)dkv,
                   dkv_stride, positions, slot_mapping, c_weight, eps, inv_freq, rot_dims, pairing, amplitude, (float*)cache, (float*)q_out,
                   out_stride, out_head, out_at, H, dn, dr, rank);
   else if (dtype == 1)
-    launch_early(latent_prep_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), smem, s, 1, (const __nv_bfloat16*)q, q_stride,
+    launch_kernel_as(early, four ? latent_prep_kernel<__nv_bfloat16, 4> : latent_prep_kernel<__nv_bfloat16, 2>, dim3(num_tokens), dim3(threads), smem, s, 1, (const __nv_bfloat16*)q, q_stride,
                   (const __nv_bfloat16*)dkv, dkv_stride, positions, slot_mapping, c_weight, eps, inv_freq, rot_dims, pairing, amplitude,
                   (__nv_bfloat16*)cache, (__nv_bfloat16*)q_out, out_stride, out_head, out_at, H, dn, dr, rank);
   else
