@@ -46,28 +46,49 @@ def test_the_streamed_decode_attention_starts_early_and_reads_plainly():
     assert body.index("pdl_wait();") < min(body.index(x) for x in ("q_indptr[", "plan[", "rows_plan[i]", "stream_shares(q_indptr", "block_table +") if x in body)
 
 
+def _functions(text):
+    """Name -> arguments and body of the functions that are defined in ``text`` (of all, where several have a name)."""
+    found = {}
+    for m in re.finditer(r"\b(\w+)\s*\(", text):
+        depth, i = 1, m.end()
+        while depth and i < len(text):
+            depth += (text[i] == "(") - (text[i] == ")")
+            i += 1
+        rest = re.match(r"\s*\{", text[i:])
+        if rest is None or m.group(1) in ("if", "for", "while", "switch"):
+            continue
+        depth, j = 1, i + rest.end()
+        while depth and j < len(text):
+            depth += (text[j] == "{") - (text[j] == "}")
+            j += 1
+        found[m.group(1)] = found.get(m.group(1), "") + text[m.end(): j]
+    return found
+
+
 def test_kernels_that_are_launched_early_read_plainly():
     """Every kernel that goes through launch_early, or through launch_kernel_as with a condition of its own: no restrict on what it reads, no
-    __ldg, and a wait before anything else."""
+    __ldg in it nor in a function that it calls, and a wait before anything else."""
+    headers = {f: re.sub(r"//[^\n]*", "", f.read_text()) for f in CSRC.glob("*.cuh")}
+    shared = _functions("\n".join(headers.values()))
     found = set()
     for f in sorted(CSRC.glob("*.cu")):
         text = re.sub(r"//[^\n]*", "", f.read_text())
-        names = set()
+        here = _functions(text)
+        kernels = set(re.findall(r"__global__[^;{]*?\b(\w+)\s*\((?!\s*(?:THREADS|\d))", re.sub(r"__launch_bounds__\s*\((?:[^()]|\([^()]*\))*\)", "", text)))
         for m in re.finditer(r"launch_(?:early\(|kernel_as\()([^;]*);", text):
-            names |= set(re.findall(r"\b\w+_kernel\b", m.group(1)))
-            if re.match(r"\s*kernel\b", m.group(1)):
-                names |= set(re.findall(r"\b\w+_kernel\b", text[text.rindex("auto kernel", 0, m.start()): m.start()]))
-        for name in names:
-            at = re.search(r"__global__[^;{]*?\b" + name + r"\s*\(", text)
-            if at is None:
-                continue
-            end = text.index("\n}\n", at.end())
-            body = text[at.end(): end]
-            assert not re.search(r"\.nc\b|__ldg\(", body), name
-            if name in ("skinny_gemm_kernel", "direct_gemm_kernel"):      # their weights and rows go through loads of their own
-                continue
-            assert "__restrict__" not in body and "pdl_wait();" in body, name
-            found.add(name)
+            names = kernels & set(re.findall(r"\b\w+\b", m.group(1)))
+            for var in set(re.findall(r"\bauto (\w+) =", text[: m.start()])) & set(re.findall(r"\b\w+\b", m.group(1))):
+                names |= kernels & set(re.findall(r"\b\w+\b", text[text.rindex(f"auto {var} =", 0, m.start()): m.start()]))
+            assert names, f"{f.name}: {m.group(0)[:80]}"
+            for name in names - {"skinny_gemm_kernel"}:                 # early where a switch asks for it alone
+                body = here[name]
+                called = {name} | (set(re.findall(r"\b(\w+)\s*(?:<[^<>;]*>)?\s*\(", body)) & (set(here) | set(shared)))
+                for c in called - {"launch_early"}:
+                    assert not re.search(r"\.nc\b|__ldg\(", here.get(c) or shared[c]), (name, c)
+                if name == "direct_gemm_kernel":                         # its weights and rows go through loads of their own
+                    continue
+                assert "__restrict__" not in body and "pdl_wait();" in body, name
+                found.add(name)
     assert {"moe_plan_kernel", "moe_rows_kernel", "moe_combine_kernel", "moe_select_warp_kernel", "latent_prep_kernel", "latent_gather_kernel",
             "latent_plan_kernel", "rms_rows_block_kernel", "rmsnorm_vec_kernel", "silu_mul_bf16_vec_kernel", "decode_stream_kernel",
             "delta_gates_kernel", "ssm_gates_kernel", "rotary_angles_kernel"} <= found
