@@ -1,8 +1,9 @@
 // float32 rows times a bfloat16 W on the tensor cores, without giving up 32 bits:
 //     C[M, N] = A[M, K] (float32) . W[N, K]^T (bfloat16)
 //
-// A number of A is cut into three bfloat16 pieces of eight bits each (cut off, not rounded: the three add up to it exactly, and none
-// overflows), so A . W is three products of bfloat16 numbers, each exact in float32.  What is left to chance is the sums.  The
+// A number of A is cut into three bfloat16 pieces of eight bits each (cut off, not rounded: none overflows, and the three add up to it
+// exactly from 2^-110 on; below that the last piece ends at bfloat16's smallest number, 2^-133, so that a number keeps fewer than 24 bits: off by
+// less than 2^-133), so A . W is three products of bfloat16 numbers, each exact in float32.  What is left to chance is the sums.  The
 // tensor cores add into their accumulator without rounding to nearest, so a long sum there drifts towards zero; here an accumulator in
 // TMEM holds 64 numbers of k of one piece only, and float32 registers add up the three pieces' sums, the smallest first, and those of the
 // blocks, k ascending, rounded to nearest.  Off from float64 by 1.2e-7 to 2.8e-7 of the result's norm at K of 1,024 to 12,288, where
@@ -21,16 +22,18 @@
 //   issuer  : one lane, four MMAs a block; its warp owns the TMEM.
 // NaN: a piece that is zero times an infinite W is NaN where the number itself times it is infinite.  A sum that comes out as NaN is
 // formed once more from the numbers themselves, k ascending, until it is NaN there too.
-// Every wait is bounded; when one runs out the error flag is raised and the CTA leaves with its copies landed and its TMEM freed.
+// Every wait is bounded; when one runs out the error flag is raised and the CTA leaves with its copies landed, its MMAs done and its TMEM freed.
 //
 // What bounds it: few rows, the issuer (some 600 cycles a block of its looks at barriers, MMAs and commit; three commits a block, a barrier
 // for each who waits, took 900); many rows, the chain of a block through cutters, MMAs and sums, with two accumulators (301 rows of 6,144 x 1,024:
 // 1,000 cycles a block of 64 rows, issue slots 45 % used, tensor pipe and shared memory 18 % each).
 // Rows of A fetched by the cutters' own loads: each proxy fence waited for them, 950 cycles a block.  All cutters at one block at a time:
 // 1,400 cycles a block of 64 rows instead of 1,000.
-// Measured (us, the FFMA kernels and this one): 301 rows, 6,144 x 1,024 117 and 27; 4,096 x 1,024 87 and 20; 1,024 x 2,048 62 and 19; 1,024 x
-// 3,072 91 and 25; 1,024 rows of 24,576 x 4,096 4,420 and 795 (259 TFLOP/s); 16 rows of 1,024 x 3,072 84 and 21; one row of 151,936 x
-// 1,024 58 and 60, of 4,096 x 12,288 93 and 70, of 1,024 x 2,048 17 and 17.
+// Measured (us, the FFMA kernels and this one): 301 rows, 6,144 x 1,024 117 and 26; 4,096 x 1,024 87 and 18; 1,024 x 2,048 62 and 17; 1,024 x
+// 3,072 91 and 24; 1,024 rows of 24,576 x 4,096 4,420 and 805 (256 TFLOP/s); 16 rows of 1,024 x 3,072 84 and 19; four rows of 256 to 4,096 x 1,024 13.0 and
+// 8.9, of 512 7.3 and 6.2.  One row is done sooner by FFMAs where K is short (256 to 4,096 x 512 4.7 and 6.2, x 1,024 8.0 and 8.9, x 2,048 14.6 and 14.0,
+// x 4,096 27.9 and 24.3, x 12,288 80 and 66; 151,936 x 1,024 57.6 and 58.1), but a row's order of sums may not depend on how many there are; steps of one
+// row are no slower as a whole (28 layers of 0.6B sizes 2,811 and 2,687, 8 layers of a hidden size of 512 583 and 584).
 #include "common.cuh"
 #include "tcgen05_utils.cuh"
 using namespace arle;

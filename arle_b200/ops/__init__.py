@@ -8,7 +8,7 @@ if that fails or if a tensor is not on a CUDA device.
 
 Matrix products: the float32 path uses the package's own kernels (true 32-bit, fixed
 summation order): ``gemm_f32_tc.cu`` for bfloat16 weights with long rows, on the tensor cores
-in three exact pieces, FFMA (``gemm_f32.cu``) otherwise.  The bfloat16 path has two
+in three pieces, FFMA (``gemm_f32.cu``) otherwise.  The bfloat16 path has two
 kernels of its own: weight streaming for up to 8 rows (``gemm_skinny.cu``, every
 decode step of up to 8 requests) and tcgen05 / TMA / TMEM for many rows
 (``gemm_tcgen05.cu``, switched on with ``set_tcgen05_min_rows``).  Otherwise it calls
@@ -185,8 +185,8 @@ def set_programmatic_launch(on) -> None:
     products; 0 (the default): only the kernels that are launched so whatever is set here,
     the small decode products that read their weights straight from memory (up to 8 rows; a
     0.6B layer's four take 12.7 us instead of 15.4), the streamed attention of steps that
-    decode only, and norms and gates of up to 256 rows.  Larger kernels find no room beside
-    one another and lose."""
+    decode only, norms and gates of up to 256 rows, and the short kernels around experts,
+    latents and recurrences.  Larger kernels find no room beside one another and lose."""
     library().arle_set_programmatic_launch(int(on))
 
 

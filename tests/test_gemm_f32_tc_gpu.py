@@ -1,4 +1,4 @@
-"""float32 rows times a bfloat16 W in three exact pieces on the tensor cores: against float64 at the edges of the tiles (16, 32, 64 and 80 rows by
+"""float32 rows times a bfloat16 W in three pieces on the tensor cores: against float64 at the edges of the tiles (16, 32, 64 and 80 rows by
 128 columns), rows of other tensors untouched; no further off than the FFMA kernels; a row's bits whatever stands beside it; infinities,
 NaNs and the ends of float32's range."""
 import pytest
