@@ -206,9 +206,12 @@ ARLE_API int arle_moe_select(const float* z, int z_stride, const float* correcti
     auto kernel = keep < groups ? (E <= 32 ? moe_select_warp_kernel<1, true> : E <= 64 ? moe_select_warp_kernel<2, true> : moe_select_warp_kernel<8, true>)
                                 : (E <= 32 ? moe_select_warp_kernel<1, false> : E <= 64 ? moe_select_warp_kernel<2, false> : moe_select_warp_kernel<8, false>);
     const int warps = num_tokens <= 592 ? 1 : kSelectWarps;
+    const dim3 grid((num_tokens + warps - 1) / warps), block(32 * warps);
     // Early while there are few blocks: 300 tokens 3.6 us behind one another (4.1 in stream order), 1,024 4.0 (4.2), 2,048 6.4 (4.8).
-    launch_kernel_as(num_tokens <= 1024 || (pdl_enabled() & 1) != 0, kernel, dim3((num_tokens + warps - 1) / warps), dim3(32 * warps), 0, s, 1, z, z_stride, correction, E, top, groups, keep, scale, mode, ids, wts,
-                  num_tokens);
+    if (num_tokens <= 1024)
+      launch_early(kernel, grid, block, 0, s, 1, z, z_stride, correction, E, top, groups, keep, scale, mode, ids, wts, num_tokens);
+    else
+      launch_kernel(kernel, grid, block, 0, s, 1, z, z_stride, correction, E, top, groups, keep, scale, mode, ids, wts, num_tokens);
     return launch_status();
   }
   launch_kernel(moe_select_kernel, dim3((num_tokens + 63) / 64), dim3(64), 0, s, 1, z, z_stride, correction, scratch, E, top, groups,

@@ -296,10 +296,14 @@ class Attention(Mixer):
                                 cache.page_size)
         attn = ctx.ws.get("attn_out", (T, nq * vd), x.dtype)
         ops.paged_attention(proj[:, : nq * hd], attn, cache.k, cache.v, ctx.positions, ctx.row_of_token, cache.block_table,
-                            nq, nkv, hd, cache.page_size, s.scale, s.window, batch=ctx, vd=vd, sink=s.sink, product=(self.w_o, None))
+                            nq, nkv, hd, cache.page_size, s.scale, s.window, batch=ctx, vd=vd, sink=s.sink, **self._next_product(T, None))
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)
         ops.gemm(attn, self.w_o, out)
         return out
+
+    def _next_product(self, rows, sink):
+        """What the attention is told of the output projection behind it: where that may be one of the small products that start early."""
+        return {"product": (self.w_o, sink)} if ops.fused_gemm_shape_ok(rows, self.w_o) else {}
 
     # ------------------------------------------------- biases, convolution, kept first tokens, capped scores, sinks
     def _forward_general(self, x, ctx, cache, state, sink=None):
@@ -319,7 +323,7 @@ class Attention(Mixer):
                 and ops.fused_decode_supported(proj, ctx, cache.k.dtype, nq, nkv, hd, cache.page_size, rdim)):
             ops.decode_attention_with_prep(proj, attn, cache.k, cache.v, cache.slot_mapping, self.q_norm, self.k_norm, s.qk_norm_eps or 0.0,
                                            inv_freq if rdim else None, cache.block_table, nq, nkv, hd, cache.page_size, s.scale, s.window,
-                                           ctx, rotary_dim=rdim, bias=self.b_qkv, sink=self.sinks, gate=gate, product=(self.w_o, sink))
+                                           ctx, rotary_dim=rdim, bias=self.b_qkv, sink=self.sinks, gate=gate, **self._next_product(T, sink))
             return self._output_general(attn, out, sink)
         bias = self.b_qkv
         if s.conv_taps:
@@ -336,7 +340,7 @@ class Attention(Mixer):
                                     cache.k, cache.v, nq, nkv, hd, vd, cache.page_size, norm_first=True, bias=bias)
         ops.paged_attention(proj[:, : nq * hd], attn, cache.k, cache.v, ctx.positions, ctx.row_of_token, cache.block_table,
                             nq, nkv, hd, cache.page_size, s.scale, s.window, batch=ctx, vd=vd, keep_first=s.keep_first, softcap=s.softcap,
-                            sink=self.sinks, gate=gate, product=(self.w_o, sink))
+                            sink=self.sinks, gate=gate, **self._next_product(T, sink))
         return self._output_general(attn, out, sink)
 
     def _output_general(self, attn, out, sink):
@@ -416,7 +420,7 @@ class Attention(Mixer):
                 # a step of decoded tokens only: norm, rotation, cache store and attention in one launch
                 ops.decode_attention_with_prep(qkv, attn, cache.k, cache.v, cache.slot_mapping, self.q_norm, self.k_norm, eps,
                                                inv_freq if rdim else None, cache.block_table, nq, nkv, hd, cache.page_size,
-                                               s.scale, s.window, ctx, product=(self.w_o, sink))
+                                               s.scale, s.window, ctx, **self._next_product(T, sink))
                 out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)
                 return None if ops.gemm(attn, self.w_o, out, sink=sink) else out
             ops.attention_prep(qkv, ctx.positions, cache.slot_mapping, self.q_norm, self.k_norm, eps, inv_freq, rdim,
@@ -428,7 +432,7 @@ class Attention(Mixer):
                                cache.page_size, angles=self._angles(qkv, ctx, inv_freq, rdim))
         q = ctx.ws.cut("qkv" if cache.writable else "q_only", qkv, 0, nq * hd)
         ops.paged_attention(q, attn, cache.k, cache.v, ctx.positions, ctx.row_of_token,
-                            cache.block_table, nq, nkv, hd, cache.page_size, s.scale, s.window, batch=ctx, product=(self.w_o, sink))
+                            cache.block_table, nq, nkv, hd, cache.page_size, s.scale, s.window, batch=ctx, **self._next_product(T, sink))
         out = ctx.ws.get("mixer_out", (T, s.hidden_size), x.dtype)
         if ops.gemm(attn, self.w_o, out, sink=sink):
             return None                       # summed into the residual by the product itself
