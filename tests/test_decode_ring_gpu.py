@@ -27,7 +27,7 @@ def _stream_decode(q, out, kc, vc, qi, kv, bt, nq, nkv, hd, ps, window, ctas, sc
 
 @pytest.mark.parametrize("nq,nkv,lens", [
     (16, 8, [64]), (16, 8, [1153]), (16, 8, [1400] * 2), (16, 8, [2100] * 2), (16, 8, [300] * 8), (16, 8, [2100] * 8), (16, 8, [700, 1, 2300, 65] * 3),
-    (32, 8, [700]), (32, 8, [2100] * 3), (16, 8, [16500] * 3), (2, 1, [64 * 16]), (2, 1, [64 * 16 + 1]), (2, 1, [64 * 33]), (4, 2, [64 * 50 + 7])])
+    (32, 8, [700]), (32, 8, [2100] * 3), (16, 8, [16500] * 3), (2, 1, [64 * 16]), (2, 1, [64 * 16 + 1]), (2, 1, [64 * 10]), (2, 1, [64 * 11]), (2, 1, [64 * 20]), (2, 1, [64 * 21]), (2, 1, [64 * 33]), (4, 2, [64 * 50 + 7])])
 @pytest.mark.parametrize("behind", [None, 1024])           # columns of the product that follows
 def test_rings_and_pieces(nq, nkv, lens, behind):
     product = None if behind is None else (torch.empty(behind, nq * 128, dtype=torch.bfloat16, device=DEV), None)
