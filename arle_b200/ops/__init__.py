@@ -370,7 +370,7 @@ def fused_gemm_supported(x, w) -> bool:
 def fused_gemm_shape_ok(rows: int, w: torch.Tensor, gated: bool = False) -> bool:
     """Whether a product of ``rows`` bfloat16 rows with ``w`` can take the fused kernel (asked by the
     parts before they hand out a sink or rows without their norm factor)."""
-    return (_KERNEL_SET == "fast" and w is not None and w.is_cuda and w.dtype == torch.bfloat16 and 0 < rows <= 8
+    return (0 < rows <= 8 and _KERNEL_SET == "fast" and w is not None and w.is_cuda and w.dtype == torch.bfloat16
             and w.shape[1] % 32 == 0 and w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0
             and (not gated or gated_gemm_fits(w.shape[1])))
 
